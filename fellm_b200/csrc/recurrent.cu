@@ -317,6 +317,7 @@ struct ScanArgs {
   // [item][block][H][dk].  scan_blocks_kernel then walks an item's blocks in order and turns blk_state into the states
   // IN FRONT of the blocks (and moves the slot's state on).  phase 3: every block again from that state, with outputs.
   int phase, blk; float* blk_state; float* blk_decay;
+  int skip_from;                                       // > 0: items of that many rows or more are another kernel's
 };
 
 template <int VE> __device__ __forceinline__ void load_vec(const float* p, float* out) {
@@ -574,6 +575,7 @@ __global__ void __launch_bounds__(SC_THREADS) scan_kernel(ScanArgs a) {
   const int h = blockIdx.x / col_tiles, col0 = (blockIdx.x - h * col_tiles) * COLS;
   const int item = blockIdx.y;
   int row_begin = a.item_start[item], n = a.item_start[item + 1] - row_begin;
+  if (a.skip_from > 0 && n >= a.skip_from) return;
   const int per_buf = a.tc * (4 * DKP + COLS + 4);          // (a multiple of four floats: the second buffer stays 16-byte aligned)
   const bool consumer = warp < SC_CONSUMERS;
   const int ks = lane % KS, cw = warp * CPW + lane / KS;          // (consumers) this thread's lane of rows and column
@@ -838,10 +840,12 @@ static int scan_launch(ScanArgs& a, int n_items, int max_item_rows, cudaStream_t
 // Gated delta rule.  qkv [T, ldq]: q heads at column 0 (G x dk), k at k_off, v at v_off (H x dv), after their
 // convolutions and SiLU.  small [T, lds]: beta's logit at column b_off + h; per-head decay: logit at a_off + h,
 // g = exp(-exp(A_log[h]) softplus(logit + dt_bias[h])); per-channel decay: gch [T, H*dk] holds g itself.
+// skip_from > 0 (here and below): items of that many rows or more are left alone (recurrent_chunk.cu takes them).
 FELLM_API int fellm_delta_scan(const void* qkv, int is_bf16, int ldq, int k_off, int v_off, const float* small, int lds,
                                int b_off, int a_off, const float* A_log, const float* dt_bias, const float* gch,
                                float* state, long long slot_stride, const int* item_start, const int* item_slot,
-                               float* out, int n_items, int H, int G, int dk, int dv, int max_item_rows, cudaStream_t stream) {
+                               float* out, int n_items, int H, int G, int dk, int dv, int max_item_rows, int skip_from,
+                               cudaStream_t stream) {
   if (n_items <= 0) return 0;
   if (dk < 1 || dk > 1024 || dv < 1 || G < 1 || H % G) return FELLM_ERR_SIZE;
   if (!qkv || !small || !state || !item_start || !item_slot || !out || (!gch && (!A_log || !dt_bias))) return FELLM_ERR_ARG;
@@ -849,6 +853,7 @@ FELLM_API int fellm_delta_scan(const void* qkv, int is_bf16, int ldq, int k_off,
   a.q = qkv; a.ld = ldq; a.k_off = k_off; a.v_off = v_off; a.small = small; a.lds = lds; a.b_off = b_off; a.a_off = a_off;
   a.A_log = A_log; a.dt_bias = dt_bias; a.gch = gch; a.state = state; a.slot_stride = slot_stride;
   a.item_start = item_start; a.item_slot = item_slot; a.out = out; a.H = H; a.G = G; a.dk = dk; a.dv = dv;
+  a.skip_from = skip_from;
   if (gch) return is_bf16 ? scan_launch<1, bf16>(a, n_items, max_item_rows, stream) : scan_launch<1, float>(a, n_items, max_item_rows, stream);
   return is_bf16 ? scan_launch<0, bf16>(a, n_items, max_item_rows, stream) : scan_launch<0, float>(a, n_items, max_item_rows, stream);
 }
@@ -857,13 +862,14 @@ FELLM_API int fellm_delta_scan(const void* qkv, int is_bf16, int ldq, int k_off,
 FELLM_API int fellm_decay_bonus_scan(const void* r, const void* k, const void* v, int is_bf16, int ld, const float* w,
                                      const float* u, float* state, long long slot_stride, const int* item_start,
                                      const int* item_slot, float* out, int n_items, int H, int dk, int max_item_rows,
-                                     cudaStream_t stream) {
+                                     int skip_from, cudaStream_t stream) {
   if (n_items <= 0) return 0;
   if (dk < 1 || dk > 1024 || H < 1) return FELLM_ERR_SIZE;
   if (!r || !k || !v || !w || !u || !state || !item_start || !item_slot || !out) return FELLM_ERR_ARG;
   ScanArgs a = {};
   a.q = r; a.k = k; a.v = v; a.ld = ld; a.gch = w; a.bonus = u; a.state = state; a.slot_stride = slot_stride;
   a.item_start = item_start; a.item_slot = item_slot; a.out = out; a.H = H; a.G = H; a.dk = dk; a.dv = dk;
+  a.skip_from = skip_from;
   return is_bf16 ? scan_launch<2, bf16>(a, n_items, max_item_rows, stream) : scan_launch<2, float>(a, n_items, max_item_rows, stream);
 }
 
@@ -920,14 +926,14 @@ gated_write_prep_kernel(float* __restrict__ z, int ld, int f_off, const float* _
 FELLM_API int fellm_gated_write_scan(float* z, int ld, int f_off, int v_off, const float* lower, const float* bias,
                                      float* state, long long slot_stride, const int* item_start, const int* item_slot,
                                      float* out, int n_items, int H, int dk, int dv, int max_item_rows, int blk,
-                                     float* scratch, float* prep, int T, cudaStream_t stream) {
+                                     float* scratch, float* prep, int T, int skip_from, cudaStream_t stream) {
   if (n_items <= 0) return 0;
   if (dk < 1 || dk > 1024 || dv < 1 || H < 1) return FELLM_ERR_SIZE;
   if (!z || !lower || !bias || !state || !item_start || !item_slot || !out) return FELLM_ERR_ARG;
   ScanArgs a = {};
   a.q = z; a.ld = ld; a.k_off = f_off; a.v_off = v_off; a.state = state; a.slot_stride = slot_stride;
   a.item_start = item_start; a.item_slot = item_slot; a.out = out; a.H = H; a.G = H; a.dk = dk; a.dv = dv;
-  a.lower = lower; a.fbias = bias;
+  a.lower = lower; a.fbias = bias; a.skip_from = skip_from;
   if (blk > 0 && scratch && max_item_rows > blk) {
     const size_t n_blocks = (size_t)(max_item_rows + blk - 1) / blk;
     a.phase = 1; a.blk = blk; a.blk_state = scratch; a.blk_decay = scratch + (size_t)n_items * n_blocks * H * dk * dv;

@@ -635,8 +635,44 @@ GATED_WRITE_BLOCK_MIN_ROWS = int(os.environ.get("FELLM_B200_GATED_WRITE_BLOCK_MI
 GATED_WRITE_PREP_MIN_ROWS = int(os.environ.get("FELLM_B200_GATED_WRITE_PREP_MIN_ROWS", 16))       # a step's longest portion from which the gates are prepared in front
 
 
+# Portions of prompts in chunks of 32 tokens (csrc/recurrent_chunk.cu) in the place of the token-by-token scan: from this many
+# rows of a request's portion on.
+RECURRENT_CHUNK_MIN_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_CHUNK_MIN_ROWS", 32))
+
+
+def recurrent_chunk_rows(dtype) -> int:
+    """What a mixer passes as chunk_rows: the bfloat16 engine's portions run in chunks; the 32-bit engine keeps the scan, and with
+    it the same bits for a prompt under every cut (0: no chunks)."""
+    return RECURRENT_CHUNK_MIN_ROWS if dtype == torch.bfloat16 else 0
+
+
+def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_items, max_item_rows, min_rows, H, G, dk, dv, out, *,
+                     small=None, b_off=0, a_off=0, A_log=None, dt_bias=None, gch=None, bonus=None, lower=None, fbias=None) -> bool:
+    """Runs the items of min_rows rows or more in chunks; False (nothing launched) for sizes and alignments the kernels do not
+    take: a lane reads dk / 32 neighbouring elements at once, a block keeps 16 value columns."""
+    es = q.element_size()
+    lane = dk // 32
+    if dk not in (64, 128) or dv % 16 or n_items > 65535 or H > 65535 or (mode == 3 and es == 2):
+        return False
+    if any(t.data_ptr() % (lane * es) for t in (q, k)) or ld % lane or any(t is not None and t.data_ptr() % (lane * 4) for t in (gch, bonus, lower, fbias)):
+        return False
+    if out.data_ptr() % 16 or not out.is_contiguous():
+        return False
+    T = out.shape[0]
+    need = _fn("recurrent_chunk", "fellm_recurrent_chunk_scratch", [_c_int] * 5)
+    need.restype = _c_ll
+    scratch = torch.empty(need(T, n_items, H, dk, dv), dtype=torch.float32, device=out.device)
+    sp, ss = _state_args(state)
+    f = _fn("recurrent_chunk", "fellm_recurrent_chunk",
+            [_c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int] + [_c_p] * 7 + [_c_ll] + [_c_p] * 4 + [_c_int] * 8 + [_c_p])
+    _check(f(mode, _p(q), _p(k), _p(v), _is_bf16(q), ld, int(v_off), _p(small), small.stride(0) if small is not None else 0, int(b_off),
+             int(a_off), _p(A_log), _p(dt_bias), _p(gch), _p(bonus), _p(lower), _p(fbias), sp, ss, _p(item_start), _p(item_slot), _p(out),
+             _p(scratch), T, n_items, int(max_item_rows), int(min_rows), H, G, dk, dv, _stream()), "recurrent_chunk")
+    return True
+
+
 def gated_write_scan(z, f_off, v_off, lower, bias, state, item_start, item_slot, n_items, H, dk, dv, out=None,
-                     max_item_rows=0, block=None, prepared=None):
+                     max_item_rows=0, block=None, prepared=None, chunk_rows=0):
     """Per head S = diag(f) S + (1 - f) v^T, o = S^T q, with q = SiLU(q raw) and f = lower + (1 - lower) sigmoid(f raw +
     bias).  z float32 [T, >= v_off + H*dv]: q raw at column 0 (H x dk), f raw at f_off, v at v_off (H x dv); lower, bias
     float32 [H*dk]; state float32 [slots, H, dk, dv] (the scan kernel's own layout).  Returns float32 [T, H*dv].
@@ -645,7 +681,9 @@ def gated_write_scan(z, f_off, v_off, lower, bias, state, item_start, item_slot,
     front of it), a walk over the blocks' states between the two; equal to the plain scan up to float32 rounding.
     prepared (default: where the longest portion has GATED_WRITE_PREP_MIN_ROWS rows or more): a kernel in front computes the
     gates once a token and head IN PLACE (z's q and f columns then hold f q and f) and the scan's producers only copy;
-    the same numbers as the one-launch form, which single tokens keep."""
+    the same numbers as the one-launch form, which single tokens keep.
+    chunk_rows > 0: items of that many rows or more run in chunks of 32 tokens where those kernels take the sizes (another
+    order of the sums)."""
     _dev(z, lower, bias, state, item_start, item_slot)
     T = z.shape[0]
     if dk > MAX_SCAN_KEY_DIM:
@@ -657,6 +695,12 @@ def gated_write_scan(z, f_off, v_off, lower, bias, state, item_start, item_slot,
     _i32(item_start, "item_start"), _i32(item_slot, "item_slot")
     if out is None:
         out = torch.empty((T, H * dv), dtype=torch.float32, device=z.device)
+    skip = 0
+    if 0 < chunk_rows <= max_item_rows and _recurrent_chunk(3, z, z[:, f_off:], z, z.stride(0), v_off, state, item_start, item_slot, n_items,
+                                                            max_item_rows, chunk_rows, H, H, dk, dv, out, lower=lower, fbias=bias):
+        if n_items == 1:
+            return out
+        skip, max_item_rows, block, prepared = chunk_rows, chunk_rows - 1, 0, False
     sp, ss = _state_args(state)
     if block is None:
         block = GATED_WRITE_BLOCK if max_item_rows >= max(GATED_WRITE_BLOCK_MIN_ROWS, 2) else 0
@@ -668,9 +712,9 @@ def gated_write_scan(z, f_off, v_off, lower, bias, state, item_start, item_slot,
     prep = torch.empty((T, H), dtype=torch.float32, device=z.device) if prepared else None
     f = _fn("recurrent", "fellm_gated_write_scan",
             [_c_p, _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int,
-             _c_int, _c_p, _c_p, _c_int, _c_p])
+             _c_int, _c_p, _c_p, _c_int, _c_int, _c_p])
     _check(f(_p(z), z.stride(0), int(f_off), int(v_off), _p(lower), _p(bias), sp, ss, _p(item_start), _p(item_slot), _p(out),
-             n_items, H, dk, dv, int(max_item_rows), int(block or 0), _p(scratch), _p(prep), T, _stream()), "gated_write_scan")
+             n_items, H, dk, dv, int(max_item_rows), int(block or 0), _p(scratch), _p(prep), T, skip, _stream()), "gated_write_scan")
     return out
 
 
@@ -700,13 +744,15 @@ def lowrank_expand(z, w2, bias=None, *, f_in="none", f_out="none", rate=None, pe
 
 
 def delta_scan(qkv, k_off, v_off, small, b_off, a_off, A_log, dt_bias, gch, state, item_start, item_slot, n_items,
-               H, G, dk, dv, out=None, max_item_rows=0):
+               H, G, dk, dv, out=None, max_item_rows=0, chunk_rows=0):
     """The gated delta rule over the step's portions.  qkv [T, *]: q (G x dk) at column 0, k at k_off, v (H x dv) at
     v_off, after convolution and SiLU; small float32 [T, *]: beta's logit at b_off + h and, for a decay per head,
     its logit at a_off + h (A_log, dt_bias [H]); gch float32 [T, H*dk]: the decay per head and key channel itself
     (then A_log and dt_bias are not read).  state float32 [slots, H, dk, dv] (the kernel's own: it keeps each
     head's matrix column by column there).  Returns o float32 [T, H*dv].
-    max_item_rows: the longest portion of the step, if known (sizes the staging buffers; no result depends on it)."""
+    max_item_rows: the longest portion of the step, if known (sizes the staging buffers; no result depends on it).
+    chunk_rows > 0: items of that many rows or more (max_item_rows known) run in chunks of 32 tokens where those kernels
+    take the sizes (another order of the sums)."""
     _dev(qkv, small, A_log, dt_bias, gch, state, item_start, item_slot)
     T = qkv.shape[0]
     if dk > MAX_SCAN_KEY_DIM:
@@ -717,20 +763,29 @@ def delta_scan(qkv, k_off, v_off, small, b_off, a_off, A_log, dt_bias, gch, stat
         assert gch.dtype == torch.float32 and gch.is_contiguous() and gch.shape == (T, H * dk)
     if out is None:
         out = torch.empty((T, H * dv), dtype=torch.float32, device=qkv.device)
+    skip = 0
+    if 0 < chunk_rows <= max_item_rows and _recurrent_chunk(
+            0 if gch is None else 1, qkv, qkv[:, k_off:], qkv, qkv.stride(0), v_off, state, item_start, item_slot, n_items, max_item_rows,
+            chunk_rows, H, G, dk, dv, out, small=small, b_off=b_off, a_off=a_off, A_log=A_log, dt_bias=dt_bias, gch=gch):
+        if n_items == 1:
+            return out
+        skip, max_item_rows = chunk_rows, chunk_rows - 1
     sp, ss = _state_args(state)
     f = _fn("recurrent", "fellm_delta_scan",
             [_c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p,
-             _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p])
+             _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p])
     _check(f(_p(qkv), _is_bf16(qkv), qkv.stride(0), k_off, v_off, _p(small), small.stride(0), b_off, a_off, _p(A_log),
              _p(dt_bias), _p(gch), sp, ss, _p(item_start), _p(item_slot), _p(out), n_items, H, G, dk, dv,
-             int(max_item_rows), _stream()),
+             int(max_item_rows), skip, _stream()),
            "delta_scan")
     return out
 
 
-def decay_bonus_scan(r, k, v, w, u, state, item_start, item_slot, n_items, H, dk, out=None, max_item_rows=0):
+def decay_bonus_scan(r, k, v, w, u, state, item_start, item_slot, n_items, H, dk, out=None, max_item_rows=0, chunk_rows=0):
     """o_t = (S + diag(u) k_t v_t^T)^T r_t; S = diag(w_t) S + k_t v_t^T per head.  r, k, v [T, H*dk] (one row stride),
-    w float32 [T, H*dk], u float32 [H, dk], state float32 [slots, H, dk, dk].  Returns o float32 [T, H*dk]."""
+    w float32 [T, H*dk], u float32 [H, dk], state float32 [slots, H, dk, dk].  Returns o float32 [T, H*dk].
+    chunk_rows > 0: items of that many rows or more (max_item_rows known) run in chunks of 32 tokens where those kernels
+    take the sizes (another order of the sums)."""
     _dev(r, k, v, w, u, state, item_start, item_slot)
     T = r.shape[0]
     if dk > MAX_SCAN_KEY_DIM:
@@ -740,11 +795,17 @@ def decay_bonus_scan(r, k, v, w, u, state, item_start, item_slot, n_items, H, dk
     assert state.shape[1:] == (H, dk, dk)
     if out is None:
         out = torch.empty((T, H * dk), dtype=torch.float32, device=r.device)
+    skip = 0
+    if 0 < chunk_rows <= max_item_rows and _recurrent_chunk(2, r, k, v, r.stride(0), 0, state, item_start, item_slot, n_items, max_item_rows,
+                                                            chunk_rows, H, H, dk, dk, out, gch=w, bonus=u):
+        if n_items == 1:
+            return out
+        skip, max_item_rows = chunk_rows, chunk_rows - 1
     sp, ss = _state_args(state)
     f = _fn("recurrent", "fellm_decay_bonus_scan",
-            [_c_p, _c_p, _c_p, _c_int, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p])
+            [_c_p, _c_p, _c_p, _c_int, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p])
     _check(f(_p(r), _p(k), _p(v), _is_bf16(r), r.stride(0), _p(w), _p(u), sp, ss, _p(item_start), _p(item_slot), _p(out),
-             n_items, H, dk, int(max_item_rows), _stream()), "decay_bonus_scan")
+             n_items, H, dk, int(max_item_rows), skip, _stream()), "decay_bonus_scan")
     return out
 
 

@@ -56,7 +56,8 @@ class Hgrn2(Mixer):
         w, n = self.w, self.H * self.dk
         z = linear(h, w["qfv.weight"], out_dtype=torch.float32)
         o = ops.gated_write_scan(z, n, 2 * n, w["lower"], w["f.bias"], cache.states, ctx.item_start, cache.item_slot,
-                                 ctx.n_items, self.H, self.dk, self.dv, max_item_rows=ctx.max_item_rows)
+                                 ctx.n_items, self.H, self.dk, self.dv, max_item_rows=ctx.max_item_rows,
+                                 chunk_rows=ops.recurrent_chunk_rows(h.dtype))
         y = ops.head_norm_gate(o, w["norm.weight"], False, None, None, self.eps, self.H, self.dv, h.dtype)
         linear(y, w["o.weight"], out=out, accumulate=not store)
         return out
@@ -65,4 +66,4 @@ class Hgrn2(Mixer):
         return [self.w["qfv.weight"], self.w["o.weight"]]
 
     def kernel_modules(self, dtype):
-        return linear_modules(dtype) + [("recurrent", None)]
+        return linear_modules(dtype) + [("recurrent", None)] + ([("recurrent_chunk", None)] if dtype == "bfloat16" else [])

@@ -70,7 +70,8 @@ class TimeMix(Mixer):
         z = linear(mixes[4], w["w1.weight"], out_dtype=torch.float32)
         decay = ops.lowrank_expand(z[:, :self.rank], w["w2.weight"], w["w0"], f_in="tanh", f_out="exp_neg_exp")
         o = ops.decay_bonus_scan(r, k, v, decay, w["u"], mat_state.states, ctx.item_start, mat_state.item_slot,
-                                 ctx.n_items, self.H, self.dk, max_item_rows=ctx.max_item_rows)
+                                 ctx.n_items, self.H, self.dk, max_item_rows=ctx.max_item_rows,
+                                 chunk_rows=ops.recurrent_chunk_rows(xn.dtype))
         y = ops.head_norm_gate(o, w["norm.weight"], True, g, "silu", self.eps, self.H, self.dk, xn.dtype)
         linear(y, w["o.weight"], out=out, accumulate=True)
         return out
@@ -80,4 +81,4 @@ class TimeMix(Mixer):
         return [w["r.weight"], w["k.weight"], w["v.weight"], w["g.weight"], w["w1.weight"], w["o.weight"]]
 
     def kernel_modules(self, dtype):
-        return linear_modules(dtype) + [("recurrent", None)]
+        return linear_modules(dtype) + [("recurrent", None)] + ([("recurrent_chunk", None)] if dtype == "bfloat16" else [])
