@@ -16,9 +16,11 @@
 // Two kernels.  `prep` (a block a chunk and head, all side by side): the token vectors, L and M with one running product a
 // column, the substitution for (P A) and V, the scaled B and K.  `walk` (a block a head and 16 value columns): chunk
 // after chunk, the state in registers, three small products a chunk; the next chunk's operands arrive by cp.async meanwhile.
-// Bound by: walk, its float32 multiply-adds (a chunk of 32 tokens at dk = 128: 0.16 M a block, 1,250 cycles at 128 a
-// cycle) and the shared-memory reads and five barriers around them; the scan walks one token after another, a reduction
-// over dk and ~500 cycles each.  16 columns a block: a prompt of 16 heads of 128 is 128 blocks for 148 SMs.
+// Bound by: the reads of shared memory.  A lane's tile of 4 x 4 (or 2 x 4) results takes a register from shared memory for
+// every two multiply-adds, and a block's chunk of 32 tokens at dk = 128 is 0.2 M of those: ~5,000 of the 5,800 cycles a
+// chunk takes.  The scan walks one token after another, a reduction over dk and ~750 cycles each.  16 columns a block: a
+// prompt of 16 heads of 128 is 128 blocks for 148 SMs.  2,048 tokens of 16 heads of 128 x 128, delta rule: scan 791 us, here
+// prep 75 + walk 188; three prompts of 1,537 tokens, 8 heads, gated write: 274 us, here 28 + 77.
 // 32 tokens a chunk: L and M cost 32 / 2 multiply-adds a token, channel and matrix, an eighth of the walk's.
 //
 // A later token's infinity or NaN stays out of an earlier token's sums, as in the walk token by token: masked pairs are
@@ -46,7 +48,7 @@ struct RkArgs {
   const int* item_start; const int* item_slot;
   float* state; long long slot_stride;
   float* out;                                                      // [T, H dv]
-  float* W; float* Q; float* K; float* U; float* M; float* P;      // per (chunk, head): [32][dk] x 3, [32][dv], [32][36], [dk]
+  float* image; float* U;                                          // per (chunk, head): an RkImage; [dv / 16][32][16]
   int H, G, dv, min_rows;
 };
 
@@ -69,9 +71,17 @@ template <int E> __device__ __forceinline__ void rk_store(float* p, const float*
 __device__ __forceinline__ float rk_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float rk_sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
 
+// What prep leaves for walk of a chunk and head, as it lies in walk's shared memory (its copies are then linear).
+template <bool DELTA, int DK>
+struct RkImage {
+  static constexpr int NR = DELTA ? 2 * RK_C : RK_C;          // rows of the product with the state: W above Q, or Q alone
+  static constexpr int AP = DK + 4;                           // their stride: eight rows' 16 bytes in different banks
+  static constexpr int A = 0, K = A + NR * AP, M = K + RK_C * DK, P = M + RK_C * RK_LP, FLOATS = P + DK;
+};
+
 // ---------------------------------------------------------------- prep
 template <int MODE, int DK, typename TA>
-__global__ void __launch_bounds__(RK_THREADS)
+__global__ void __launch_bounds__(RK_THREADS, 2)
 rk_prep_kernel(const RkArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* A = sm;                                   // [32][DK]
@@ -91,7 +101,7 @@ rk_prep_kernel(const RkArgs a) {
   const size_t cell = (size_t)(rk_first_chunk(r0, item) + c) * a.H + h;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = h / (a.H / a.G);
-  for (int x = tid; x < RK_C * RK_LP; x += RK_THREADS) Mm[x] = 0.f;
+  for (int x = tid; x < 2 * RK_C * RK_LP; x += RK_THREADS) Lt[x] = 0.f;          // (and Mm behind it)
 
   // ---- the token vectors: a warp takes tokens warp, warp + 8, ..; a lane E consecutive elements
   {
@@ -163,16 +173,21 @@ rk_prep_kernel(const RkArgs a) {
   }
   __syncthreads();
 
-  // ---- L and M: eight lanes a column s (four columns a warp), channels 4 ig + 32 m + e a lane; X = D_(t-1,s) K_s
+  // ---- L and M: eight lanes a column s (four columns a warp), channels 4 ig + 32 m + e a lane; X = D_(t-1,s) K_s.
+  // Four tokens a round: their (up to) eight sums go through the eight lanes together, seven shuffles for all of them.
   {
     constexpr int MB = DK / 32;
     const int ig = lane & 7, s = 4 * warp + (lane >> 3);
     unsigned long long X[2 * MB];
 #pragma unroll
     for (int m = 0; m < 2 * MB; ++m) X[m] = 0ull;
-    for (int t = 4 * warp; t < len; ++t) {
-      const int o = t * DK + 4 * ig;
-      if (t > 4 * warp) {
+#pragma unroll 1
+    for (int t0 = 4 * warp; t0 < len; t0 += 4) {
+      const bool first = t0 == 4 * warp;                       // the columns' own tokens
+      float sum[8];                                            // M of four tokens, L of four tokens
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = t0 + j, o = t * DK + 4 * ig;
         unsigned long long l2 = 0ull, m2 = 0ull;
 #pragma unroll
         for (int m = 0; m < MB; ++m) {
@@ -185,32 +200,60 @@ rk_prep_kernel(const RkArgs a) {
         }
         float lo, hi;
         unpack_f2(m2, lo, hi);
-        float ms = lo + hi, ls = 0.f;
-        if (DELTA) { unpack_f2(l2, lo, hi); ls = lo + hi; }
+        sum[j] = lo + hi;
+        unpack_f2(l2, lo, hi);
+        sum[4 + j] = lo + hi;
+        if (first) {
+          const bool own = t == s;
 #pragma unroll
-        for (int x = 1; x < 8; x <<= 1) {
-          ms += __shfl_xor_sync(0xffffffffu, ms, x);
-          if (DELTA) ls += __shfl_xor_sync(0xffffffffu, ls, x);
-        }
-        if (ig == 0 && t > s) {
-          Mm[t * RK_LP + s] = ms;
-          if (DELTA) Lt[s * RK_LP + t] = beta[t] * ls;
+          for (int m = 0; m < MB; ++m) {
+            const ulonglong2 gd = *(const ulonglong2*)(Gd + o + 32 * m);
+            const ulonglong2 kk = *(const ulonglong2*)(KK + o + 32 * m);
+            // (before its own token a column is not zero times a decay but zero)
+            X[2 * m] = own ? kk.x : t < s ? 0ull : mul_f2(X[2 * m], gd.x);
+            X[2 * m + 1] = own ? kk.y : t < s ? 0ull : mul_f2(X[2 * m + 1], gd.y);
+          }
+        } else {
+#pragma unroll
+          for (int m = 0; m < MB; ++m) {
+            const ulonglong2 gd = *(const ulonglong2*)(Gd + o + 32 * m);
+            X[2 * m] = mul_f2(X[2 * m], gd.x); X[2 * m + 1] = mul_f2(X[2 * m + 1], gd.y);
+          }
         }
       }
-      const bool own = t == s;
-      if (own && ig == 0) Mm[t * RK_LP + t] = cc[t];
+      // lane ig ends with the whole of sum[4 (ig & 1) + 2 ((ig >> 1) & 1) + (ig >> 2)]
+      const bool b0 = ig & 1, b1 = ig & 2, b2 = ig & 4;
+      float q4[4], q2[2], v;
+      if (DELTA) {
 #pragma unroll
-      for (int m = 0; m < MB; ++m) {
-        const ulonglong2 gd = *(const ulonglong2*)(Gd + o + 32 * m);
-        const ulonglong2 kk = *(const ulonglong2*)(KK + o + 32 * m);
-        // (before its own token a column is not zero times a decay but zero)
-        X[2 * m] = own ? kk.x : t < s ? 0ull : mul_f2(X[2 * m], gd.x);
-        X[2 * m + 1] = own ? kk.y : t < s ? 0ull : mul_f2(X[2 * m + 1], gd.y);
+        for (int j = 0; j < 4; ++j) {
+          const float give = b0 ? sum[j] : sum[4 + j], keep = b0 ? sum[4 + j] : sum[j];
+          q4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q4[j] = sum[j] + __shfl_xor_sync(0xffffffffu, sum[j], 1);
       }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float give = b1 ? q4[j] : q4[2 + j], keep = b1 ? q4[2 + j] : q4[j];
+        q2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+      }
+      {
+        const float give = b2 ? q2[0] : q2[1], keep = b2 ? q2[1] : q2[0];
+        v = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+      }
+      const int t = t0 + (b1 ? 2 : 0) + (b2 ? 1 : 0);
+      if (t > s) {
+        if (DELTA && b0) Lt[s * RK_LP + t] = beta[t] * v;
+        else if (!b0) Mm[t * RK_LP + s] = v;
+      } else if (t == s && !b0) Mm[t * RK_LP + t] = cc[t];
     }
   }
   __syncthreads();
 
+  using I = RkImage<DELTA, DK>;
+  float* img = a.image + cell * I::FLOATS;
   // ---- running products of the decays: forward into A and B (up to the token before), backward into K (behind the token)
   if (tid < DK) {
     float p = 1.f;
@@ -222,7 +265,7 @@ rk_prep_kernel(const RkArgs a) {
       B[o] *= p;
       p *= gd;
     }
-    a.P[cell * DK + tid] = p;
+    img[I::P + tid] = p;
   } else if (tid < 2 * DK) {
     float p = 1.f;
 #pragma unroll 8
@@ -233,15 +276,15 @@ rk_prep_kernel(const RkArgs a) {
     }
   }
   __syncthreads();
-  float* Qg = a.Q + cell * (RK_C * DK); float* Kg = a.K + cell * (RK_C * DK); float* Mg = a.M + cell * (RK_C * RK_LP);
   for (int x = tid * 4; x < RK_C * DK; x += RK_THREADS * 4) {
-    *(float4*)(Qg + x) = *(const float4*)(B + x);
-    *(float4*)(Kg + x) = *(const float4*)(KK + x);
+    const int t = x / DK, i = x - t * DK;
+    *(float4*)(img + I::A + (t + I::NR - RK_C) * I::AP + i) = *(const float4*)(B + x);
+    *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
   }
-  for (int x = tid * 4; x < RK_C * RK_LP; x += RK_THREADS * 4) *(float4*)(Mg + x) = *(const float4*)(Mm + x);
+  for (int x = tid * 4; x < RK_C * RK_LP; x += RK_THREADS * 4) *(float4*)(img + I::M + x) = *(const float4*)(Mm + x);
 
   // ---- (I + beta L) [W | U0] = beta [P A | V], a column a thread; without the delta rule U0 = V
-  float* Ug = a.U + cell * ((size_t)RK_C * a.dv); float* Wg = a.W + cell * (RK_C * DK);
+  float* Ug = a.U + cell * ((size_t)RK_C * a.dv);
   const TA* vp = (const TA*)a.v + a.v_off + (size_t)h * a.dv;
   for (int col = tid; col < (DELTA ? DK : 0) + a.dv; col += RK_THREADS) {
     const bool is_w = DELTA && col < DK;
@@ -261,16 +304,16 @@ rk_prep_kernel(const RkArgs a) {
 #pragma unroll
         for (int t0 = (s + 1) & ~3; t0 < RK_C; t0 += 4) {
           const float4 l = *(const float4*)(Lt + s * RK_LP + t0);
-          if (t0 > s) x[t0] = t0 < len ? fmaf(-l.x, x[s], x[t0]) : 0.f;
-          if (t0 + 1 > s) x[t0 + 1] = t0 + 1 < len ? fmaf(-l.y, x[s], x[t0 + 1]) : 0.f;
-          if (t0 + 2 > s) x[t0 + 2] = t0 + 2 < len ? fmaf(-l.z, x[s], x[t0 + 2]) : 0.f;
-          x[t0 + 3] = t0 + 3 < len ? fmaf(-l.w, x[s], x[t0 + 3]) : 0.f;
+          if (t0 > s) x[t0] = fmaf(-l.x, x[s], x[t0]);
+          if (t0 + 1 > s) x[t0 + 1] = fmaf(-l.y, x[s], x[t0 + 1]);
+          if (t0 + 2 > s) x[t0 + 2] = fmaf(-l.z, x[s], x[t0 + 2]);
+          x[t0 + 3] = fmaf(-l.w, x[s], x[t0 + 3]);
         }
     }
 #pragma unroll
     for (int t = 0; t < RK_C; ++t) {
-      if (is_w) Wg[t * DK + col] = x[t];
-      else Ug[(size_t)t * a.dv + j] = x[t];
+      if (is_w) img[I::A + t * I::AP + col] = x[t];
+      else Ug[((size_t)(j / RK_NV) * RK_C + t) * RK_NV + j % RK_NV] = x[t];
     }
   }
 }
@@ -280,66 +323,99 @@ __device__ __forceinline__ void rk_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-template <bool DELTA, int DK>
-struct RkStage {
-  static constexpr int NR = DELTA ? 2 * RK_C : RK_C;          // rows of the product with the state: W under Q, or Q alone
-  static constexpr int AP = DK + 4;                           // their stride: eight rows' 16 bytes in different banks
-  static constexpr int A = 0, K = A + NR * AP, M = K + RK_C * DK, U = M + RK_C * RK_LP, P = U + RK_C * RK_NV, FLOATS = P + DK;
-};
+// Two groups of eight warps.  The first walks the state: W S, U = U0 - W S, S = P S + K^T U; the second makes the
+// outputs, Q S + M U, from the state in front of the chunk as it lies in shared memory and the first group's U: what the
+// outputs cost runs beside the chain and not in it, and sixteen warps hide each other's waits.
+#define RK_WALK_THREADS 512
+#define RK_PP (RK_NV + 4)  // row stride of the partial sums
+
+__device__ __forceinline__ void rk_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void rk_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 template <bool DELTA, int DK>
-__device__ __forceinline__ void rk_fetch(const RkArgs& a, float* buf, size_t cell, int j0, int tid) {
-  using S = RkStage<DELTA, DK>;
-  constexpr int V = DK / 4;
-  const float* Qg = a.Q + cell * (RK_C * DK); const float* Kg = a.K + cell * (RK_C * DK); const float* Wg = a.W + cell * (RK_C * DK);
-  for (int x = tid; x < RK_C * V; x += RK_THREADS) {
-    const int t = x / V, i = (x - t * V) * 4;
-    if (DELTA) rk_copy16(buf + S::A + t * S::AP + i, Wg + t * DK + i);
-    rk_copy16(buf + S::A + (t + (DELTA ? RK_C : 0)) * S::AP + i, Qg + t * DK + i);
-    rk_copy16(buf + S::K + t * DK + i, Kg + t * DK + i);
-  }
-  const float* Mg = a.M + cell * (RK_C * RK_LP);
-  for (int x = tid; x < RK_C * RK_LP / 4; x += RK_THREADS) rk_copy16(buf + S::M + 4 * x, Mg + 4 * x);
-  const float* Ug = a.U + cell * ((size_t)RK_C * a.dv) + j0;
-  for (int x = tid; x < RK_C * RK_NV / 4; x += RK_THREADS) {
-    const int t = x / (RK_NV / 4), j = (x - t * (RK_NV / 4)) * 4;
-    rk_copy16(buf + S::U + t * RK_NV + j, Ug + (size_t)t * a.dv + j);
-  }
-  if (tid < DK / 4) rk_copy16(buf + S::P + 4 * tid, a.P + cell * DK + 4 * tid);
+__device__ __forceinline__ void rk_fetch(const RkArgs& a, float* buf, size_t cell, int tile, int tid) {
+  using I = RkImage<DELTA, DK>;
+  const float* img = a.image + cell * I::FLOATS;
+#pragma unroll
+  for (int x = 4 * tid; x < I::FLOATS; x += 4 * RK_WALK_THREADS) rk_copy16(buf + x, img + x);
+  const float* Ug = a.U + cell * ((size_t)RK_C * a.dv) + (size_t)tile * (RK_C * RK_NV);
+  if (tid < RK_C * RK_NV / 4) rk_copy16(buf + I::FLOATS + 4 * tid, Ug + 4 * tid);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
+// 32 rows (at A, stride AP) times the state, over a warp's KW key rows: a lane rows rg + 8 m, columns 4 cg + x; pairs of
+// key rows an operation.  The sums go to part [32][RK_PP].
+template <int KW, int AP>
+__device__ __forceinline__ void rk_rows_by_state(const float* A, const float* Sw, float* part, int rg, int cg) {
+  constexpr int GM = KW / 4 - 1;
+  unsigned long long acc[4][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) acc[m][x] = 0ull;
+  A += rg * AP;
+#pragma unroll
+  for (int kk = 0; kk < KW / 4; ++kk) {
+    ulonglong2 sv[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) sv[x] = *(const ulonglong2*)(Sw + (4 * cg + x) * KW + 4 * (kk ^ (cg & GM)));
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const ulonglong2 av = *(const ulonglong2*)(A + 8 * m * AP + 4 * kk);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) { acc[m][x] = fma_f2(av.x, sv[x].x, acc[m][x]); acc[m][x] = fma_f2(av.y, sv[x].y, acc[m][x]); }
+    }
+  }
+  part += rg * RK_PP + 4 * cg;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    float o[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) { float lo, hi; unpack_f2(acc[m][x], lo, hi); o[x] = lo + hi; }
+    *(float4*)(part + 8 * m * RK_PP) = make_float4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+// the eight warps' sums of a row and two columns, in warp order
+__device__ __forceinline__ float2 rk_gather(const float* part, int row, int col) {
+  float2 r = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const float2 p = *(const float2*)(part + (w * RK_C + row) * RK_PP + col);
+    r.x += p.x; r.y += p.y;
+  }
+  return r;
+}
+
 template <bool DELTA, int DK>
-__global__ void __launch_bounds__(RK_THREADS)
+__global__ void __launch_bounds__(RK_WALK_THREADS)
 rk_walk_kernel(const RkArgs a) {
   extern __shared__ __align__(16) float sm[];
-  using S = RkStage<DELTA, DK>;
+  using I = RkImage<DELTA, DK>;
+  constexpr int STAGE = I::FLOATS + RK_C * RK_NV;
   constexpr int KW = DK / 8;                       // key rows of the state a warp keeps
   constexpr int RPL = KW / 8;                      // of them a lane
-  constexpr int PP = RK_NV + 4;                    // row stride of the partial sums
-  float* part = sm + 2 * S::FLOATS;                // [8 warps][NR][PP]
-  float* Us = part + 8 * S::NR * PP;               // [32][16]
-  float* St = Us + RK_C * RK_NV;                   // [8 warps][16 columns][KW], 16-byte groups swizzled by column / 4
+  constexpr int GM = KW / 4 - 1;                   // 16-byte groups of a column, less one
+  float* partQ = sm + 2 * STAGE;                   // [8 warps][32][RK_PP]
+  float* St = partQ + 8 * RK_C * RK_PP;            // two of [8 warps][16 columns][KW], 16-byte groups swizzled by column / 4
+  float* partW = St + 2 * RK_NV * DK;              // (delta) as partQ
+  float* Us = partW + 8 * RK_C * RK_PP;            // (delta) [32][16]
   const int item = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * RK_NV;
   const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0;
   if (n < a.min_rows || n <= 0) return;
   const int chunks = (n + RK_C - 1) / RK_C;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, gtid = tid & 255, warp = (tid >> 5) & 7, lane = tid & 31;
+  const bool walker = tid < 256;
   const int rg = lane >> 2, cg = lane & 3;
   const size_t cell0 = (size_t)rk_first_chunk(r0, item) * a.H + h;
-  rk_fetch<DELTA, DK>(a, sm, cell0, j0, tid);
+  rk_fetch<DELTA, DK>(a, sm, cell0, blockIdx.x, tid);
 
-  // this lane's part of the state: rows warp * KW + RPL * rg + r, columns j0 + 4 cg + x
+  // a walker's part of the state: rows warp * KW + RPL * rg + r, columns j0 + 4 cg + x
   float* slot = a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv;
   const int i0 = warp * KW + RPL * rg;
   float s[RPL][4];
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) s[r][x] = slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r];
-  float* Sw = St + warp * (RK_NV * KW);
-  constexpr int GM = KW / 4 - 1;                   // 16-byte groups of a column, less one
-  auto put_state = [&]() {
+  auto put_state = [&](int c) {
+    float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
@@ -348,89 +424,33 @@ rk_walk_kernel(const RkArgs a) {
         Sw[col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3)] = s[r][x];
       }
   };
-  put_state();
+  if (walker) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) s[r][x] = slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r];
+    put_state(0);
+  }
+  const int row = gtid >> 3, jc = 2 * (gtid & 7);                // gathering: a thread a row and two columns
 
   for (int c = 0; c < chunks; ++c) {
-    const float* buf = sm + (c & 1) * S::FLOATS;
+    const float* buf = sm + (c & 1) * STAGE;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();                               // this chunk's operands are here; the other buffer, the sums and U are free
-    if (c + 1 < chunks) rk_fetch<DELTA, DK>(a, sm + ((c + 1) & 1) * S::FLOATS, cell0 + (size_t)(c + 1) * a.H, j0, tid);
-
-    // ---- [W; Q] S over this warp's key rows: a lane rows rg + 8 m, columns 4 cg + x; pairs of key rows an operation
-    {
-      constexpr int NM = S::NR / 8;
-      unsigned long long acc[NM][4];
-#pragma unroll
-      for (int m = 0; m < NM; ++m)
-#pragma unroll
-        for (int x = 0; x < 4; ++x) acc[m][x] = 0ull;
-      const float* Ab = buf + S::A + rg * S::AP + warp * KW;
-#pragma unroll
-      for (int kk = 0; kk < KW / 4; ++kk) {
-        ulonglong2 sv[4];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) sv[x] = *(const ulonglong2*)(Sw + (4 * cg + x) * KW + 4 * (kk ^ (cg & GM)));
-#pragma unroll
-        for (int m = 0; m < NM; ++m) {
-          const ulonglong2 av = *(const ulonglong2*)(Ab + 8 * m * S::AP + 4 * kk);
-#pragma unroll
-          for (int x = 0; x < 4; ++x) { acc[m][x] = fma_f2(av.x, sv[x].x, acc[m][x]); acc[m][x] = fma_f2(av.y, sv[x].y, acc[m][x]); }
-        }
+    __syncthreads();          // this chunk's operands and state are here; the other buffers, the sums and U are free
+    if (c + 1 < chunks) rk_fetch<DELTA, DK>(a, sm + ((c + 1) & 1) * STAGE, cell0 + (size_t)(c + 1) * a.H, blockIdx.x, tid);
+    const float* U = DELTA ? Us : buf + I::FLOATS;
+    const float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
+    if (walker) {
+      if (DELTA) {
+        rk_rows_by_state<KW, I::AP>(buf + I::A + warp * KW, Sw, partW + warp * (RK_C * RK_PP), rg, cg);
+        rk_bar_sync(1, 256);
+        const float2 r = rk_gather(partW, row, jc), u0 = *(const float2*)(buf + I::FLOATS + row * RK_NV + jc);
+        *(float2*)(Us + row * RK_NV + jc) = make_float2(u0.x - r.x, u0.y - r.y);
+        rk_bar_sync(1, 256);
+        rk_bar_arrive(2, 512);                     // U is there for the other group
       }
-      float* pw = part + (warp * S::NR + rg) * PP + 4 * cg;
-#pragma unroll
-      for (int m = 0; m < NM; ++m) {
-        float o[4];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) { float lo, hi; unpack_f2(acc[m][x], lo, hi); o[x] = lo + hi; }
-        *(float4*)(pw + 8 * m * PP) = make_float4(o[0], o[1], o[2], o[3]);
-      }
-    }
-    __syncthreads();
-
-    // ---- the eight warps' sums in warp order; a thread a row and four columns
-    const int row = tid >> 2, jc = 4 * (tid & 3);
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < S::NR) {
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const float4 p = *(const float4*)(part + (w * S::NR + row) * PP + jc);
-        r.x += p.x; r.y += p.y; r.z += p.z; r.w += p.w;
-      }
-    }
-    const float* U = buf + S::U;
-    if (DELTA) {
-      if (row < RK_C) {
-        const float4 u0 = *(const float4*)(U + row * RK_NV + jc);
-        *(float4*)(Us + row * RK_NV + jc) = make_float4(u0.x - r.x, u0.y - r.y, u0.z - r.z, u0.w - r.w);
-      }
-      __syncthreads();
-      U = Us;
-    }
-
-    // ---- O = Q S + M U: the threads that hold Q's rows
-    const int t = DELTA ? row - RK_C : row;
-    if (t >= 0 && t < RK_C) {
-      const int rows_here = min(RK_C, n - c * RK_C);
-      const float* Mt = buf + S::M + t * RK_LP;
-#pragma unroll 2
-      for (int x = 0; x < RK_C; x += 4) {
-        if (x > (t | 7)) break;                    // (a warp's eight rows end together)
-        const float4 m = *(const float4*)(Mt + x);
-        const float mm[4] = {m.x, m.y, m.z, m.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float4 u = *(const float4*)(U + (x + e) * RK_NV + jc);
-          if (x + e <= t) { r.x = fmaf(mm[e], u.x, r.x); r.y = fmaf(mm[e], u.y, r.y); r.z = fmaf(mm[e], u.z, r.z); r.w = fmaf(mm[e], u.w, r.w); }
-        }
-      }
-      if (t < rows_here) *(float4*)(a.out + (size_t)(r0 + c * RK_C + t) * ((size_t)a.H * a.dv) + (size_t)h * a.dv + j0 + jc) = r;
-    }
-
-    // ---- S = P S + K^T U
-    {
-      const float* Kb = buf + S::K + i0;
-      const float* Pb = buf + S::P + i0;
+      const float* Kb = buf + I::K + i0;
+      const float* Pb = buf + I::P + i0;
       float k1[RPL];
 #pragma unroll
       for (int q = 0; q < RPL; ++q) {
@@ -438,7 +458,7 @@ rk_walk_kernel(const RkArgs a) {
 #pragma unroll
         for (int x = 0; x < 4; ++x) s[q][x] *= p;
       }
-#pragma unroll 8
+#pragma unroll 16
       for (int t2 = 0; t2 < RK_C; ++t2) {
         if (RPL == 2) { const float2 f = *(const float2*)(Kb + t2 * DK); k1[0] = f.x; k1[RPL - 1] = f.y; }
         else k1[0] = Kb[t2 * DK];
@@ -449,15 +469,32 @@ rk_walk_kernel(const RkArgs a) {
           s[q][2] = fmaf(k1[q], u.z, s[q][2]); s[q][3] = fmaf(k1[q], u.w, s[q][3]);
         }
       }
+      put_state(c + 1);
+    } else {
+      rk_rows_by_state<KW, I::AP>(buf + I::A + (I::NR - RK_C) * I::AP + warp * KW, Sw, partQ + warp * (RK_C * RK_PP), rg, cg);
+      rk_bar_sync(3, 256);
+      float2 r = rk_gather(partQ, row, jc);
+      if (DELTA) rk_bar_sync(2, 512);
+      const float* Mt = buf + I::M + row * RK_LP;
+#pragma unroll 2
+      for (int x = 0; x <= (row | 3); x += 4) {    // (a warp's four rows end together)
+        const float4 m = *(const float4*)(Mt + x);
+        const float mm[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 u = *(const float2*)(U + (x + e) * RK_NV + jc);
+          if (x + e <= row) { r.x = fmaf(mm[e], u.x, r.x); r.y = fmaf(mm[e], u.y, r.y); }
+        }
+      }
+      if (c * RK_C + row < n) *(float2*)(a.out + (size_t)(r0 + c * RK_C + row) * ((size_t)a.H * a.dv) + (size_t)h * a.dv + j0 + jc) = r;
     }
-    __syncwarp();
-    put_state();
-    __syncwarp();
   }
+  if (walker) {
 #pragma unroll
-  for (int x = 0; x < 4; ++x)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r] = s[r][x];
+      for (int r = 0; r < RPL; ++r) slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r] = s[r][x];
+  }
 }
 
 // ---------------------------------------------------------------- launches
@@ -465,20 +502,24 @@ template <int MODE, int DK, typename TA>
 static int rk_launch(const RkArgs& a, int n_items, int max_rows, cudaStream_t stream) {
   constexpr bool DELTA = MODE <= RK_DELTA_CHANNEL;
   const size_t sm_prep = (size_t)(4 * RK_C * DK + 2 * RK_C * RK_LP + 2 * RK_C) * sizeof(float);
-  using S = RkStage<DELTA, DK>;
-  const size_t sm_walk = (size_t)(2 * S::FLOATS + 8 * S::NR * (RK_NV + 4) + RK_C * RK_NV + RK_NV * DK) * sizeof(float);
+  const size_t sm_walk = (size_t)(2 * (RkImage<DELTA, DK>::FLOATS + RK_C * RK_NV) + 8 * RK_C * RK_PP + 2 * RK_NV * DK +
+                                  (DELTA ? 8 * RK_C * RK_PP + RK_C * RK_NV : 0)) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(rk_prep_kernel<MODE, DK, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_prep);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(rk_walk_kernel<DELTA, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
   if (e != cudaSuccess) return (int)e;
   rk_prep_kernel<MODE, DK, TA><<<dim3((max_rows + RK_C - 1) / RK_C, a.H, n_items), RK_THREADS, sm_prep, stream>>>(a);
-  rk_walk_kernel<DELTA, DK><<<dim3(a.dv / RK_NV, a.H, n_items), RK_THREADS, sm_walk, stream>>>(a);
+  rk_walk_kernel<DELTA, DK><<<dim3(a.dv / RK_NV, a.H, n_items), RK_WALK_THREADS, sm_walk, stream>>>(a);
   return launch_status();
 }
 
+static long long rk_image_floats(int mode, int dk) {
+  if (dk == 128) return mode <= RK_DELTA_CHANNEL ? RkImage<true, 128>::FLOATS : RkImage<false, 128>::FLOATS;
+  return mode <= RK_DELTA_CHANNEL ? RkImage<true, 64>::FLOATS : RkImage<false, 64>::FLOATS;
+}
+
 // Floats of scratch for a step of T rows.
-FELLM_API long long fellm_recurrent_chunk_scratch(int T, int n_items, int H, int dk, int dv) {
-  const long long chunks = T / RK_C + n_items;
-  return chunks * H * ((long long)RK_C * (3 * dk + dv + RK_LP) + dk);
+FELLM_API long long fellm_recurrent_chunk_scratch(int mode, int T, int n_items, int H, int dk, int dv) {
+  return (T / RK_C + (long long)n_items) * H * (rk_image_floats(mode, dk) + (long long)RK_C * dv);
 }
 
 // mode 0 / 1: the delta rule with a decay per head / channel (q, k [T, G dk] and v [T, H dv] in rows of ld elements, as
@@ -506,8 +547,7 @@ FELLM_API int fellm_recurrent_chunk(int mode, const void* q, const void* k, cons
   a.item_start = item_start; a.item_slot = item_slot; a.state = state; a.slot_stride = slot_stride; a.out = out;
   a.H = H; a.G = G; a.dv = dv; a.min_rows = min_rows;
   const size_t cells = (size_t)(T / RK_C + n_items) * H;
-  a.W = scratch; a.Q = a.W + cells * (RK_C * dk); a.K = a.Q + cells * (RK_C * dk); a.U = a.K + cells * (RK_C * dk);
-  a.M = a.U + cells * ((size_t)RK_C * dv); a.P = a.M + cells * (RK_C * RK_LP);
+  a.image = scratch; a.U = scratch + cells * (size_t)rk_image_floats(mode, dk);
 #define RK_GO(MODE_, TA_) (dk == 128 ? rk_launch<MODE_, 128, TA_>(a, n_items, max_rows, stream) : rk_launch<MODE_, 64, TA_>(a, n_items, max_rows, stream))
   if (mode == 0) return is_bf16 ? RK_GO(0, bf16) : RK_GO(0, float);
   if (mode == 1) return is_bf16 ? RK_GO(1, bf16) : RK_GO(1, float);

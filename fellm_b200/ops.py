@@ -636,7 +636,7 @@ GATED_WRITE_PREP_MIN_ROWS = int(os.environ.get("FELLM_B200_GATED_WRITE_PREP_MIN_
 
 
 # Portions of prompts in chunks of 32 tokens (csrc/recurrent_chunk.cu) in the place of the token-by-token scan: from this many
-# rows of a request's portion on.
+# rows of a request's portion on, a whole chunk (the scan costs ~0.3 us a token; a chunk 3 us behind two launches of ~10).
 RECURRENT_CHUNK_MIN_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_CHUNK_MIN_ROWS", 32))
 
 
@@ -659,9 +659,9 @@ def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_i
     if out.data_ptr() % 16 or not out.is_contiguous():
         return False
     T = out.shape[0]
-    need = _fn("recurrent_chunk", "fellm_recurrent_chunk_scratch", [_c_int] * 5)
+    need = _fn("recurrent_chunk", "fellm_recurrent_chunk_scratch", [_c_int] * 6)
     need.restype = _c_ll
-    scratch = torch.empty(need(T, n_items, H, dk, dv), dtype=torch.float32, device=out.device)
+    scratch = torch.empty(need(mode, T, n_items, H, dk, dv), dtype=torch.float32, device=out.device)
     sp, ss = _state_args(state)
     f = _fn("recurrent_chunk", "fellm_recurrent_chunk",
             [_c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int] + [_c_p] * 7 + [_c_ll] + [_c_p] * 4 + [_c_int] * 8 + [_c_p])
