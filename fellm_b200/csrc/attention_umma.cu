@@ -11,6 +11,9 @@
 // A sink per head (a.sinks): exp(sink) joins the softmax's denominator once, with no key and no value.
 // With -DAU_EXT the kernel also takes a sliding window (the pages in front of a CTA's first window are not
 // walked), a soft cap on the scores and a gate on the outputs (o times sigmoid(gate), element by element).
+// With -DAU_GEN (which has AU_EXT in it) also chunks (a query reads only its own block of `chunk` positions), a bias by
+// distance per head, a query temperature by position, a gate per head, and values that are the keys (the keys' tile is then
+// the second product's operand too: half the page traffic).
 // A page-layer record of the pool is the keys [G][64][AU_KD], then the values [G][64][AU_VD].
 // The accumulator is scaled by 2^-m with m a row's REFERENCE maximum, which moves only when a tile's
 // maximum exceeds it by 2^8: only then is the accumulator read, scaled and written back.
@@ -40,6 +43,12 @@
 #endif
 #ifndef AU_VD
 #define AU_VD 64
+#endif
+#ifdef AU_GEN
+#define AU_EXT 1
+constexpr bool AU_GENERAL = true;
+#else
+constexpr bool AU_GENERAL = false;
 #endif
 #ifdef AU_EXT
 constexpr bool AU_EXTENDED = true;
@@ -77,6 +86,10 @@ struct AuArgs {
   const bf16* og;                      // AU_EXT: a gate [T, ldog] (null: none), a window (0: none), a soft cap (cap_log2 0: none)
   int ldog, window;
   float cap_log2;
+  // AU_GEN: slopes [H] of a bias by distance (null: none), a query temperature 1 + qt_coef ln(floor((p + 1) / qt_every) + 1)
+  // (qt_every 0: none), blocks of `chunk` positions (0: none), a gate float32 [T, ldhg] of a number per head (null: none)
+  const float* slopes; const float* hg;
+  float qt_coef; int qt_every, chunk, ldhg, v_is_k;
 };
 
 __device__ __forceinline__ unsigned au_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -215,7 +228,8 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
   const int pos0 = a.positions[row_begin] + tok0;              // position of the block's first token
   const int k_last = pos0 + n_tok - 1;
   // tiles = pages first_page .. that of the last token; first_page: 0, or that of the first token's window
-  const int first_page = (AU_EXTENDED && a.window > 0) ? max(pos0 - a.window + 1, 0) / AU_PT : 0;
+  const int first_key = max((AU_EXTENDED && a.window > 0) ? pos0 - a.window + 1 : 0, (AU_GENERAL && a.chunk > 0) ? pos0 / a.chunk * a.chunk : 0);
+  const int first_page = first_key / AU_PT;
   const int n_tiles = k_last / AU_PT + 1 - first_page;
   const int* bt = a.block_table + (size_t)a.row_slot[row_begin] * a.max_pages + first_page;
 
@@ -255,11 +269,13 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
         const int page = max(bt[j], 0);                        // an unmapped entry (-1) must never become an address
         const int rec = page * a.layers_in_group + a.layer;
         const unsigned dst = stage0 + s * AU_STAGE_B;
-        au_mbar_expect_tx(full0 + 8 * s, AU_STAGE_B);
+        const bool values = !AU_GENERAL || !a.v_is_k;
+        au_mbar_expect_tx(full0 + 8 * s, values ? AU_STAGE_B : AU_KA * AU_ATOM_B);
 #pragma unroll
         for (int i = 0; i < AU_KA; ++i) au_tma_load_3d(dst + i * AU_ATOM_B, &k_map, 64 * i, g * AU_PT, rec, full0 + 8 * s);
+        if (values)
 #pragma unroll
-        for (int i = 0; i < AU_VA; ++i) au_tma_load_3d(dst + (AU_KA + i) * AU_ATOM_B, &v_map, 64 * i, g * AU_PT, rec, full0 + 8 * s);
+          for (int i = 0; i < AU_VA; ++i) au_tma_load_3d(dst + (AU_KA + i) * AU_ATOM_B, &v_map, 64 * i, g * AU_PT, rec, full0 + 8 * s);
       }
     }
   } else if (warp == 1) {
@@ -289,7 +305,7 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const unsigned long long dp = au_desc(p_s0 + (2 * grp + (i & 1)) * AU_ROWS * 128);
-        const unsigned long long dv = au_desc(stage0 + s * AU_STAGE_B + AU_KA * AU_ATOM_B, true);
+        const unsigned long long dv = au_desc(stage0 + s * AU_STAGE_B + ((AU_GENERAL && a.v_is_k) ? 0 : AU_KA * AU_ATOM_B), true);
 #pragma unroll
         for (int k = 0; k < AU_PT / 16; ++k)                   // 16 keys further: 32 bytes along P's rows, 16 rows (2048 bytes) down V
           au_mma(tmem_base + AU_COL_O + grp * AU_VC * 32, dp + (unsigned long long)(k * 2), dv + (unsigned long long)(k * 128), idesc_o,
@@ -319,9 +335,15 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
     const unsigned t_acc = t_row + AU_COL_O + grp * AU_VC * 32;
     const unsigned s_full = s_full0 + 16 * grp, p_full = p_full0 + 16 * grp, o_full = o_full0 + 16 * grp;
     const bool capped = AU_EXTENDED && a.cap_log2 > 0.f;
-    const float scale = capped ? a.cap_log2 : a.scale_log2;      // (capped: of tanh's values)
+    float scale = capped ? a.cap_log2 : a.scale_log2;            // (capped: of tanh's values)
+    if (AU_GENERAL && a.qt_every > 0) scale *= 1.0f + a.qt_coef * logf((float)((pos + 1) / a.qt_every + 1));
+    const bool sloped = AU_GENERAL && a.slopes != nullptr;
+    const float slope = sloped ? a.slopes[g * R + head] * 1.4426950408889634f : 0.f;
+    const float raw_scale = scale;
+    if (sloped) scale = 1.f;                                     // (the scores are then scaled where their bias is added)
     const float cap_in = capped ? a.scale_log2 / a.cap_log2 : 0.f;
-    const int lo = (AU_EXTENDED && a.window > 0) ? pos - a.window + 1 : 0;         // the first key the row sees
+    int lo = (AU_EXTENDED && a.window > 0) ? pos - a.window + 1 : 0;               // the first key the row sees
+    if (AU_GENERAL && a.chunk > 0) lo = max(lo, pos / a.chunk * a.chunk);
     // The accumulator of P V stays in tensor memory, scaled by 2^-m where m is the row's REFERENCE
     // maximum; m only moves when a tile's maximum exceeds it by AU_RESCALE_AT (P then stays below 2^8,
     // well inside bfloat16 and float32), and only then is the accumulator read, scaled and written back.
@@ -334,7 +356,10 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
         // rows past the last key hold whatever the page held before: zero the V rows, so that 0 * V is 0
         ok = au_wait(full0 + 8 * s, (j / AU_STAGES) & 1, fail, a.status, 315);
         if (!ok) break;
-        const unsigned v_s = stage0 + s * AU_STAGE_B + AU_KA * AU_ATOM_B;
+        // (keys that are the values too are written over once the scores have read them)
+        if (AU_GENERAL && a.v_is_k) ok = au_wait(s_full + 8 * (i & 1), (i >> 1) & 1, fail, a.status, 316);
+        if (!ok) break;
+        const unsigned v_s = stage0 + s * AU_STAGE_B + ((AU_GENERAL && a.v_is_k) ? 0 : AU_KA * AU_ATOM_B);
         for (int e = (k_last + 1 - key0) * 8 + row; e < AU_PT * 8; e += AU_ROWS) {
 #pragma unroll
           for (int i = 0; i < AU_VA; ++i) au_st_shared16(v_s + i * AU_ATOM_B + au_off(e >> 3, e & 7), make_uint4(0, 0, 0, 0));
@@ -365,6 +390,15 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
         } else {
 #pragma unroll
           for (int c = 0; c < AU_PT; ++c) sc[c] = tanh_any(sc[c]);
+        }
+      }
+      if (sloped) {
+        const float b0 = slope * (float)(key0 - pos);
+        const unsigned long long f2 = pack_f2(raw_scale, raw_scale), s2 = pack_f2(slope, slope);
+#pragma unroll
+        for (int c = 0; c < AU_PT; c += 2) {
+          const unsigned long long bias = fma_f2(s2, pack_f2((float)c, (float)(c + 1)), pack_f2(b0, b0));
+          unpack_f2(fma_f2(pack_f2(sc[c], sc[c + 1]), f2, bias), sc[c], sc[c + 1]);
         }
       }
       if (key0 + AU_PT - 1 > pos) {
@@ -491,6 +525,11 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
           }
         }
       }
+      if (AU_GENERAL && a.hg) {
+        const float z = 1.0f / (1.0f + expf(-a.hg[(size_t)(row_begin + tok0 + tok) * a.ldhg + g * R + head]));
+#pragma unroll
+        for (int d = 0; d < AU_VD; ++d) o[d] *= z;
+      }
       uint4* dst = (uint4*)(a.out + out_row);
 #pragma unroll
       for (int ch = 0; ch < AU_VD / 8; ++ch) {
@@ -510,17 +549,17 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
 }
 
 // A page-layer record's keys (or values) as a 3-D tensor [elements of a head, rows of all heads, records]: a box is
-// 64 elements of the 64 rows of one kv head.  Kept per (base, records, G).
+// 64 elements of the 64 rows of one kv head.  Kept per (base, records, G, sizes); per_key: elements of a record per key.
 typedef CUresult (*AuEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static int au_pool_map(const bf16* base, int size, long long records, int G, CUtensorMap* out) {
+static int au_pool_map(const bf16* base, int size, int per_key, long long records, int G, CUtensorMap* out) {
   static std::mutex mu;
-  static struct { const void* base; long long records; int G, size; CUtensorMap map; } cache[16];
+  static struct { const void* base; long long records; int G, size, per_key; CUtensorMap map; } cache[16];
   static int n_cached = 0, next = 0;
   std::lock_guard<std::mutex> lock(mu);
   for (int i = 0; i < n_cached; ++i)
-    if (cache[i].base == base && cache[i].records == records && cache[i].G == G && cache[i].size == size) { *out = cache[i].map; return 0; }
+    if (cache[i].base == base && cache[i].records == records && cache[i].G == G && cache[i].size == size && cache[i].per_key == per_key) { *out = cache[i].map; return 0; }
   static AuEncodeTiledFn fn = nullptr;
   if (!fn) {
     void* p = nullptr;
@@ -530,7 +569,7 @@ static int au_pool_map(const bf16* base, int size, long long records, int G, CUt
     fn = (AuEncodeTiledFn)p;
   }
   cuuint64_t dims[3] = {(cuuint64_t)size, (cuuint64_t)G * AU_PT, (cuuint64_t)records};
-  cuuint64_t strides[2] = {(cuuint64_t)size * 2, (cuuint64_t)G * AU_PT * (AU_KD + AU_VD) * 2};
+  cuuint64_t strides[2] = {(cuuint64_t)size * 2, (cuuint64_t)G * AU_PT * per_key * 2};
   cuuint32_t box[3] = {64, AU_PT, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUtensorMap m;
@@ -538,7 +577,7 @@ static int au_pool_map(const bf16* base, int size, long long records, int G, CUt
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return 1000 + (int)r;
-  cache[next].base = base; cache[next].records = records; cache[next].G = G; cache[next].size = size; cache[next].map = m;
+  cache[next].base = base; cache[next].records = records; cache[next].G = G; cache[next].size = size; cache[next].per_key = per_key; cache[next].map = m;
   next = (next + 1) % 16;
   if (n_cached < 16) ++n_cached;
   *out = m;
@@ -557,17 +596,23 @@ FELLM_API int fellm_attn_prefill_umma_takes(int H, int G, int hd, int vd, int pa
 // item_start[i]..item_start[i+1], its positions are consecutive from positions[item_start[i]]; max_item_rows: the longest
 // item of the step.  sinks: float32 [H] or null.  status: device int32 that a role sets (311..317) if a wait ran out.
 // With -DAU_EXT also window (0: none), softcap (0: none) and og [T, ldog] bfloat16 (null: none), the outputs times its sigmoid.
+// With -DAU_GEN also slopes (float32 [H], null: none), qt_coef and qt_every (0: none), chunk (0: none), hg float32 [T, ldhg] (a
+// number per head, null: none) and v_is_k (the records are the keys alone).
 // FELLM_ERR_SIZE for sizes it does not take.
 FELLM_API int fellm_attn_prefill_umma(const void* q, int ldq, const void* pool, long long n_pages, const int* block_table,
                                       int max_pages, const int* positions, const int* row_slot, const int* item_start,
                                       int n_items, int max_item_rows, void* out, int T, int H, int G, int hd, int vd,
                                       int page_tokens, int layer, int layers_in_group, float scale, int window,
-                                      const float* sinks, int* status, float softcap, const void* og, int ldog, cudaStream_t stream) {
+                                      const float* sinks, int* status, float softcap, const void* og, int ldog, const float* slopes,
+                                      float qt_coef, int qt_every, int chunk, const float* hg, int ldhg, int v_is_k, cudaStream_t stream) {
   if (T <= 0 || n_items <= 0) return 0;
   if (!q || !pool || !block_table || !positions || !row_slot || !item_start || !out) return FELLM_ERR_ARG;
   if (!fellm_attn_prefill_umma_takes(H, G, hd, vd, page_tokens, window)) return FELLM_ERR_SIZE;
   if (!(scale > 0.f)) return FELLM_ERR_ARG;                    // a row's maximum is taken of the unscaled scores
   if (!AU_EXTENDED && (softcap > 0.f || og)) return FELLM_ERR_SIZE;
+  if (!AU_GENERAL && (slopes || qt_every > 0 || chunk > 0 || hg || v_is_k)) return FELLM_ERR_SIZE;
+  // (a row's maximum is taken before a temperature is known to be positive)
+  if (qt_every < 0 || chunk < 0 || (qt_every > 0 && qt_coef < 0.f) || (v_is_k && AU_KD != AU_VD) || (hg && ldhg < H)) return FELLM_ERR_ARG;
   if (softcap < 0.f || (og && (ldog < H * vd || (ldog & 7) || ((uintptr_t)og & 15)))) return FELLM_ERR_ARG;
   const long long records = n_pages * layers_in_group;
   if (records >= (1ll << 31) || ldq < H * hd || (ldq % 8) || ((uintptr_t)pool & 15) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15))
@@ -577,9 +622,12 @@ FELLM_API int fellm_attn_prefill_umma(const void* q, int ldq, const void* pool, 
   a.out = (bf16*)out; a.status = status; a.sinks = sinks; a.max_pages = max_pages; a.H = H; a.G = G; a.layer = layer;
   a.layers_in_group = layers_in_group; a.scale_log2 = scale * 1.4426950408889634f;
   a.og = (const bf16*)og; a.ldog = ldog; a.window = window > 0 ? window : 0; a.cap_log2 = softcap * 1.4426950408889634f;
+  a.slopes = slopes; a.hg = hg; a.qt_coef = qt_coef; a.qt_every = qt_every; a.chunk = chunk; a.ldhg = ldhg; a.v_is_k = v_is_k ? 1 : 0;
   CUtensorMap k_map, v_map;
-  int e = au_pool_map((const bf16*)pool, AU_KD, records, G, &k_map);
-  if (!e) e = au_pool_map((const bf16*)pool + (size_t)G * AU_PT * AU_KD, AU_VD, records, G, &v_map);
+  const int per_key = AU_KD + (v_is_k ? 0 : AU_VD);
+  int e = au_pool_map((const bf16*)pool, AU_KD, per_key, records, G, &k_map);
+  if (!e && v_is_k) v_map = k_map;
+  else if (!e) e = au_pool_map((const bf16*)pool + (size_t)G * AU_PT * AU_KD, AU_VD, per_key, records, G, &v_map);
   if (e) return e;
   const int tokb = AU_ROWS / (H / G);
   size_t smem = (size_t)AU_FIXED_B + (size_t)AU_STAGES * AU_STAGE_B + 1024;     // Q, the P tiles, the stages

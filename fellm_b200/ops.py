@@ -1999,9 +1999,11 @@ def attention_prefill(q, pool, block_table, positions, row_slot, item_start, n_i
     return out
 
 
-def _umma_defines(hd: int, vd: int, ext: bool = False):
+def _umma_defines(hd: int, vd: int, ext: bool = False, general: bool = False):
     d = {} if hd == vd == 64 else {"AU_KD": hd, "AU_VD": vd}
-    if ext:
+    if general:
+        d["AU_GEN"] = 1                 # and chunks, biases by distance, a query temperature, a gate per head, values that are keys
+    elif ext:
         d["AU_EXT"] = 1                 # with a window, a soft cap and a gate on the outputs
     return d or None
 
@@ -2020,16 +2022,20 @@ def umma_prefill_takes(H: int, G: int, hd: int, vd: int, page_tokens: int, windo
 
 
 def _prefill_umma(q, ldq, H, G, hd, vd, pool, block_table, positions, row_slot, item_start, n_items, max_item_rows, layer,
-                  page_tokens, scale, sinks, out, *, window=None, softcap=None, gate=None, ext=False):
+                  page_tokens, scale, sinks, out, *, window=None, softcap=None, gate=None, ext=False, general=False, chunk=None,
+                  head_gate=None, slopes=None, q_temp=None, values_are_keys=False):
     T = q.shape[0]
+    qt_coef, qt_every = q_temp if q_temp else (0.0, 0)
     f = _fn("attention_umma", "fellm_attn_prefill_umma",
             [_c_p, _c_int, _c_p, ctypes.c_longlong, _c_p, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int,
-             _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_p, _c_p, _c_f, _c_p, _c_int, _c_p],
-            defines=_umma_defines(hd, vd, ext))
+             _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_p, _c_p, _c_f, _c_p, _c_int, _c_p, _c_f, _c_int, _c_int, _c_p,
+             _c_int, _c_int, _c_p],
+            defines=_umma_defines(hd, vd, ext, general))
     _check(f(_p(q), int(ldq), _p(pool), pool.shape[0], _p(block_table), block_table.shape[1], _p(positions), _p(row_slot),
              _p(item_start), n_items, max_item_rows, _p(out), T, H, G, hd, vd, page_tokens, layer, pool.shape[1],
              float(scale), int(window or 0), _p(sinks), _p(umma_status(q.device)), float(softcap or 0.0), _p(gate),
-             gate.stride(0) if gate is not None else 0, _stream()), "attention_prefill (tcgen05)")
+             gate.stride(0) if gate is not None else 0, _p(slopes), float(qt_coef), int(qt_every), int(chunk or 0), _p(head_gate),
+             head_gate.stride(0) if head_gate is not None else 0, int(bool(values_are_keys)), _stream()), "attention_prefill (tcgen05)")
     return out
 
 
@@ -2221,12 +2227,14 @@ def _prefill_biased(qkv, pool, block_table, positions, row_slot, item_start, n_i
 
 def attention_prefill_general(qkv, H, pool, block_table, positions, row_slot, item_start, n_items, max_item_rows, layer,
                               scale, *, window=None, chunk=None, softcap=None, gate=None, slopes=None, q_temp=None,
-                              values_are_keys=None, out=None):
+                              values_are_keys=None, out=None, out_gate=None):
     """Portions of prompts on tensor cores (bfloat16; keys and values of one size, the one the library is compiled
     for) with the part's soft cap, chunks and gate: q is read in place from rows [T, >= H*hd] (heads at column 0),
     gate float32 [T, >= H].  pool [pages, layers, 2, G, page_tokens, hd].  slopes float32 [H] and q_temp = (coef,
     every) as in paged_attention_general.  values_are_keys = (G, page_tokens, hd): the pool is [pages, layers,
-    G * page_tokens * hd], keys alone, read as the values too."""
+    G * page_tokens * hd], keys alone, read as the values too.  out_gate [T, H*hd] bfloat16: the result times its sigmoid,
+    element by element.  Heads of 64 and pages of 64 tokens: tcgen05 (which gates its float32 sums; elsewhere the gate is a
+    kernel behind the rounded result)."""
     _dev(qkv, pool, block_table, positions, row_slot, item_start, gate, slopes)
     T = qkv.shape[0]
     if values_are_keys:
@@ -2244,10 +2252,23 @@ def attention_prefill_general(qkv, H, pool, block_table, positions, row_slot, it
         assert gate.dtype == torch.float32 and gate.stride(1) == 1
     if out is None:
         out = torch.empty((T, H * hd), dtype=torch.bfloat16, device=qkv.device)
+    # measured beside the mma.sync kernel: 2,048 tokens, 16 heads, window 1,024, values that are the keys 89 -> 35 us
+    if general_umma_takes(H, G, hd, page_tokens, scale, q_temp) and qkv.stride(0) % 8 == 0 and not (
+            (qkv.data_ptr() | out.data_ptr() | pool.data_ptr()) % 16) and (
+            out_gate is None or (out_gate.stride(0) % 8 == 0 and out_gate.data_ptr() % 16 == 0)):
+        return _prefill_umma(qkv, qkv.stride(0), H, G, hd, hd, pool, block_table, positions, row_slot, item_start, n_items, max_item_rows,
+                             layer, page_tokens, scale, None, out, window=window, softcap=softcap, gate=out_gate, general=True, chunk=chunk,
+                             head_gate=gate, slopes=slopes, q_temp=q_temp, values_are_keys=bool(values_are_keys))
     _prefill_biased(qkv, pool, block_table, positions, row_slot, item_start, n_items, max_item_rows, out, T, H, G, hd, hd,
                     page_tokens, layer, scale, window, chunk=chunk, softcap=softcap, gate=gate, slopes=slopes, q_temp=q_temp,
                     values_are_keys=values_are_keys)
-    return out
+    return out if out_gate is None else gate_mul(out, out_gate)
+
+
+def general_umma_takes(H: int, G: int, hd: int, page_tokens: int, scale: float, q_temp=None) -> bool:
+    """Whether attention_prefill_general runs on tcgen05: heads of 64, pages of 64 tokens, and a query temperature that is
+    positive everywhere (a row's maximum is taken of the unscaled scores)."""
+    return hd == 64 and umma_prefill_takes(H, G, hd, hd, page_tokens, None, scale) and (not q_temp or q_temp[0] >= 0)
 
 
 def attention_modules(dtype: str, head_dim: int):

@@ -326,7 +326,10 @@ class Attention(Mixer):
             if self._on_tensor_cores(qkv):
                 a = ops.attention_prefill_general(qkv, H, cache.pool, cache.block_table, ctx.positions, ctx.row_slot,
                                                   ctx.item_start, ctx.n_items, ctx.max_item_rows, cache.layer, self.scale,
-                                                  window=self.window, chunk=self.chunk, softcap=self.softcap)
+                                                  window=self.window, chunk=self.chunk, softcap=self.softcap,
+                                                  out_gate=qkv[:, self.gate_off:self.gate_off + H * vd] if self.out_gate else None)
+                linear(a, self.w["out_proj.weight"], self.w.get("out_proj.bias"), out=out, accumulate=not store)
+                return out
             else:
                 a = ops.paged_attention_general(qkv, H, hd, vd, cache.pool, cache.block_table, ctx.positions,
                                                 ctx.row_slot, cache.layer, cache.page_tokens, self.G, self.scale, **kw)
@@ -349,5 +352,7 @@ class Attention(Mixer):
         if self.general:
             mma = dtype == "bfloat16" and self.vd == self.hd and self.hd % 16 == 0 and self.H // self.G <= 64
             extra = ([("qk_rope_write", None)] if self.in_place else []) + ([("sublayer", None)] if self.out_gate else [])
+            if mma and ops.general_umma_takes(self.H, self.G, self.hd, 64, self.scale, self.q_temp):
+                extra.append(("attention_umma", ops._umma_defines(64, 64, general=True)))
             return linear_modules(dtype) + [("attention_simt", None)] + ([("attention_mma", {"HD": self.hd})] if mma else []) + extra
         return linear_modules(dtype) + [("qk_rope_write", None)] + ops.attention_modules(dtype, self.hd)

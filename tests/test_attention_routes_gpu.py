@@ -1,0 +1,119 @@
+"""Attention kernels of portions and of single rows that a layer's sizes choose: tcgen05 with chunks, biases, temperatures,
+gates and values that are the keys.  Against float64 over whole contexts, at the edges of pages, windows, chunks and of a
+block's 128 rows."""
+from __future__ import annotations
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def attend(q, k, v, pos, scale, window=None, chunk=None, cap=None, slopes=None, temp=None, sinks=None):
+    """q [n, H, dk] at positions pos [n]; k, v [len, G, .] -> [n, H, dv], all float64."""
+    H, G = q.shape[1], k.shape[1]
+    j = torch.arange(k.shape[0])
+    see = j[None] <= pos[:, None]
+    if window:
+        see &= pos[:, None] - j[None] < window
+    if chunk:
+        see &= pos[:, None] // chunk == j[None] // chunk
+    if temp:
+        q = q * (1 + temp[0] * torch.log(torch.floor((pos.double() + 1) / temp[1]) + 1))[:, None, None]
+    out = torch.empty(q.shape[0], H, v.shape[2], dtype=torch.float64)
+    for h in range(H):
+        s = q[:, h] @ k[:, h // (H // G)].T * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        if slopes is not None:
+            s = s - slopes[h] * (pos[:, None] - j[None])
+        s = s.masked_fill(~see, -math.inf)
+        m = s.max(-1, keepdim=True).values
+        if sinks is not None:
+            m = m.clamp(min=float(sinks[h]))
+        p = torch.exp(s - m)
+        out[:, h] = (p / (p.sum(-1, keepdim=True) + (torch.exp(sinks[h] - m) if sinks is not None else 0))) @ v[:, h // (H // G)]
+    return out
+
+
+class Pages:
+    """Requests with the given numbers of tokens, their keys and values in pages handed out in a mixed order; what no request
+    wrote is NaN."""
+
+    def __init__(self, lens, G, hd, vd, page, seed):
+        g = torch.Generator().manual_seed(seed)
+        self.lens, self.page = lens, page
+        n_pages = [-(-n // page) for n in lens]
+        order = torch.randperm(sum(n_pages), generator=g).tolist()
+        self.k = [torch.randn(n, G, hd, generator=g).bfloat16() for n in lens]
+        self.v = [torch.randn(n, G, vd, generator=g).bfloat16() for n in lens] if vd else self.k
+        width = max(n_pages) + 1
+        self.table = torch.full((len(lens), width), -1, dtype=torch.int32)
+        pool = torch.full((len(order), 2, G * page * (hd + vd)), float("nan"), dtype=torch.bfloat16)
+        for r, n in enumerate(lens):
+            for i in range(n_pages[r]):
+                p = order.pop()
+                self.table[r, i] = p
+                part = slice(i * page, min(n, (i + 1) * page))
+                m = part.stop - part.start
+                rec = pool[p, 1]
+                rec[:G * page * hd].view(G, page, hd)[:, :m] = self.k[r][part].transpose(0, 1)
+                if vd:
+                    rec[G * page * hd:].view(G, page, vd)[:, :m] = self.v[r][part].transpose(0, 1)
+        self.pool = pool.cuda()
+
+    def five(self, G, hd):
+        return self.pool.view(self.pool.shape[0], 2, 2, G, self.page, hd)
+
+
+def close(got, want):
+    # bfloat16 probabilities and results: 2^-8 of the result's size each, with room for the sums
+    assert float((got.double().cpu() - want).norm() / want.norm()) < 6e-3
+    assert float((got.double().cpu() - want).abs().max() / want.pow(2).mean().sqrt()) < 0.06
+
+
+FORMS = [dict(window=70), dict(chunk=48), dict(window=100, slopes=True, temp=(0.25, 16)), dict(cap=4.0, chunk=100, gate=True), dict(slopes=True),
+         dict(window=1, temp=(0.5, 128)), dict(window=64, out_gate=True), dict()]
+
+
+def form(spec, T, H, g):
+    kw = dict(spec)
+    slopes = torch.rand(H, generator=g) * 0.2 if kw.pop("slopes", False) else None
+    gate = torch.randn(T, H + 3, generator=g) if kw.pop("gate", False) else None
+    out_gate = torch.randn(T, H * 64 + 8, generator=g).bfloat16() if kw.pop("out_gate", False) else None
+    return kw, slopes, gate, out_gate
+
+
+def gated(want, H, gate, out_gate):
+    if gate is not None:
+        want = want * torch.sigmoid(gate[:, :H].double())[:, :, None]
+    want = want.reshape(want.shape[0], -1)
+    return want if out_gate is None else want * torch.sigmoid(out_gate[:, :want.shape[1]].double())
+
+
+@pytest.mark.parametrize("spec", FORMS)
+@pytest.mark.parametrize("H,G,keys_alone", [(4, 1, True), (4, 2, False), (8, 8, False)])
+def test_portions_on_tcgen05(spec, H, G, keys_alone):
+    from fellm_b200 import ops
+    g = torch.Generator().manual_seed(H + G)
+    lens, rows = [200, 64, 300, 1], [37, 64, 130, 1]                   # tokens of every request, of which the last `rows` are the step's
+    pages = Pages(lens, G, 64, 0 if keys_alone else 64, 64, 3)
+    T = sum(rows)
+    q = torch.randn(T, H * 64 + 24, generator=g).bfloat16()
+    pos = torch.cat([torch.arange(n - m, n) for n, m in zip(lens, rows)])
+    kw, slopes, gate, out_gate = form(spec, T, H, g)
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()  # noqa: E731
+    starts = [sum(rows[:i]) for i in range(len(rows) + 1)]
+    got = ops.attention_prefill_general(
+        q.cuda(), H, pages.pool if keys_alone else pages.five(G, 64), pages.table.cuda(), i32(pos), i32([r for r, m in enumerate(rows) for _ in range(m)]),
+        i32(starts), len(rows), max(rows), 1, 0.125, window=kw.get("window"), chunk=kw.get("chunk"), softcap=kw.get("cap"), q_temp=kw.get("temp"),
+        slopes=None if slopes is None else slopes.cuda(), gate=None if gate is None else gate.cuda(),
+        out_gate=None if out_gate is None else out_gate.cuda()[:, :H * 64], values_are_keys=(G, 64, 64) if keys_alone else None)
+    ops.check_umma_status(torch.device("cuda"))
+    for r in range(len(rows)):
+        at = slice(starts[r], starts[r + 1])
+        want = attend(q[at, :H * 64].double().view(-1, H, 64), pages.k[r].double(), pages.v[r].double(), pos[at], 0.125,
+                      slopes=None if slopes is None else slopes.double(), **kw)
+        close(got[at], gated(want, H, None if gate is None else gate[at], None if out_gate is None else out_gate[at]))
