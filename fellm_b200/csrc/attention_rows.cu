@@ -1,0 +1,257 @@
+// Attention of single rows (decode steps) over the paged bfloat16 cache with float32 scores, probabilities and sums on CUDA
+// cores, for the forms the tensor-core decode kernels do not take (biases by distance, query temperatures, chunks, values
+// that are the keys) and wherever probabilities are to stay 32-bit: what paged_attention_simt_kernel (attention_simt.cu)
+// computes for such a row, for key sizes of 64 and 128 and 1, 2 or 4 heads a kv head.
+//
+// That kernel has a block a (row, head) and a lane a key: every head of a group reads the group's keys again, a lane's
+// loads are a key's 128 bytes one after another, and the values are read row by row behind them (48 us for 12 rows of 16
+// heads over 1,024 keys; 13 MB of cache).  Here a warp takes 32 keys for ALL heads of the group: LPK lanes a key, 16 bytes a
+// lane, the 32 keys' K and V all in flight at once; the partial dot products of 32 keys go through the lanes by a
+// transposing butterfly that leaves lane j with the whole scores of key j; the softmax runs on a key a lane; then every lane
+// adds its 8 elements of its keys' values, the probabilities by shuffles.  A row and kv head's keys are dealt out in tiles of
+// 32 over the warps of a cluster of up to eight blocks (as many as fill the device: ~1 tile a warp for a window of 1,024 at
+// 48 rows x kv heads), merged through shared memory and then through the cluster's.  Bound by: latency, one round trip to
+// memory for the page numbers, one for keys and values, the two merges.
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+#define AR_WARPS 4
+
+struct ArArgs {
+  const bf16* q; const bf16* pool; const int* block_table; const int* positions; const int* row_slot;
+  bf16* out; int* status;
+  const float* gate; const float* slopes; const bf16* og;
+  int ldq, max_pages, H, G, page_shift, layer, layers_in_group, window, chunk, ldg, ldog, qt_every, new_k_off, new_v_off;
+  float scale, softcap, qt_coef;
+};
+
+__device__ __forceinline__ void ar_unpack(const uint4& raw, float* f) {
+  const __nv_bfloat162* h = (const __nv_bfloat162*)&raw;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) { const float2 v = __bfloat1622float2(h[e]); f[2 * e] = v.x; f[2 * e + 1] = v.y; }
+}
+
+// What a part's sums are multiplied by on the way to the maximum M; a part without keys (m = -inf, l = 0) counts nothing,
+// one whose scores were no numbers keeps them.
+__device__ __forceinline__ float ar_factor(float m, float l, float M) { return (m == -INFINITY && l == 0.f) ? 0.f : expf(m - M); }
+
+template <int HD, int R, bool VK>
+__global__ void __launch_bounds__(AR_WARPS * 32)
+attention_rows_kernel(const ArArgs a) {
+  constexpr int LPK = HD / 8, KPI = 32 / LPK, NI = 32 / KPI;        // lanes a key, keys a load, loads a tile (= LPK)
+  __shared__ __align__(16) float part[AR_WARPS][R][HD + 4];          // a warp's sums, then m, l
+  __shared__ __align__(16) float rec[R][HD + 4];                     // the block's
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = gridDim.x, rank = blockIdx.x, g = blockIdx.y, row = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPK, sub = lane % LPK;
+  const int pos = a.positions[row];
+  const int* bt = a.block_table + (size_t)a.row_slot[row] * a.max_pages;
+  int k_begin = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
+  if (a.chunk > 0) k_begin = max(k_begin, pos / a.chunk * a.chunk);
+  const int pt = 1 << a.page_shift;
+  const size_t record = (size_t)a.G * pt * (VK ? HD : 2 * HD);
+  const bf16* qrow = a.q + (size_t)row * a.ldq;
+  const bool fused = a.new_k_off >= 0;
+
+  float q[R][8];
+  const float qt = a.qt_every > 0 ? 1.0f + a.qt_coef * logf((float)((pos + 1) / a.qt_every + 1)) : 1.0f;
+  float slope[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    ar_unpack(*(const uint4*)(qrow + (size_t)(g * R + r) * HD + 8 * sub), q[r]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q[r][e] *= qt;
+    slope[r] = a.slopes ? a.slopes[g * R + r] : 0.f;
+  }
+  float acc[R][8], m[R], l[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    m[r] = -INFINITY; l[r] = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
+  }
+
+  for (int k0 = k_begin + 32 * (rank * AR_WARPS + warp); k0 <= pos; k0 += 32 * AR_WARPS * cs) {
+    const int mine = min(k0 + lane, pos);
+    const int page = max(bt[mine >> a.page_shift], 0);               // an unmapped entry (-1) must never become an address
+    uint4 kr[NI], vr[VK ? 1 : NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int j = i * KPI + grp, kj = min(k0 + j, pos);            // (beyond the row: the row's own key once more, masked below)
+      const int pg = __shfl_sync(0xffffffffu, page, j);
+      const bf16* krow = a.pool + ((size_t)pg * a.layers_in_group + a.layer) * record + ((size_t)g * pt + (kj & (pt - 1))) * HD;
+      const bf16* vrow = krow + (size_t)a.G * pt * HD;
+      if (fused && kj == pos) {
+        krow = qrow + a.new_k_off + (size_t)g * HD;
+        vrow = qrow + a.new_v_off + (size_t)g * HD;
+      }
+      kr[i] = *(const uint4*)(krow + 8 * sub);
+      if (!VK) vr[i] = *(const uint4*)(vrow + 8 * sub);
+    }
+    float s[R][NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      float kf[8];
+      ar_unpack(kr[i], kf);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float d = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d = fmaf(q[r][e], kf[e], d);
+        s[r][i] = d;
+      }
+    }
+    // a key's LPK partial sums, for NI = LPK keys of this lane group: lane `sub` ends with the whole of key sub * KPI + grp
+    float p[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int w = LPK / 2; w > 0; w >>= 1) {
+        const bool up = sub & w;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+          const float give = up ? s[r][i] : s[r][i + w], keep = up ? s[r][i + w] : s[r][i];
+          s[r][i] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+        }
+      }
+    }
+    const int kj = k0 + sub * KPI + grp;
+    const bool seen = kj <= pos;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float x = s[r][0] * a.scale;
+      if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+      x -= slope[r] * (float)(pos - kj);
+      x = seen ? x : -INFINITY;
+      const float mn = fmaxf(m[r], warp_max(x));                     // (a tile holds a key that the row sees)
+      p[r] = seen ? expf(x - mn) : 0.f;
+      const float corr = expf(m[r] - mn);
+      m[r] = mn;
+      l[r] = fmaf(l[r], corr, p[r]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[r][e] *= corr;
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const bool live = k0 + i * KPI + grp <= pos;                   // (a masked key's value is not touched: 0 * NaN)
+      float vf[8];
+      ar_unpack(VK ? kr[i] : vr[VK ? 0 : i], vf);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float pr = __shfl_sync(0xffffffffu, p[r], i, LPK);
+        if (live) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(pr, vf[e], acc[r][e]);
+        }
+      }
+    }
+  }
+
+  // the step's own key and value into their page: nobody in this launch reads them from there
+  if (fused && rank == 0 && warp == 0) {
+    const int page = bt[pos >> a.page_shift];
+    if (page < 0) {
+      if (lane == 0 && a.status) atomicExch(a.status, 2);
+    } else if (lane < LPK) {
+      bf16* krow = const_cast<bf16*>(a.pool) + ((size_t)page * a.layers_in_group + a.layer) * record + ((size_t)g * pt + (pos & (pt - 1))) * HD;
+      *(uint4*)(krow + 8 * lane) = *(const uint4*)(qrow + a.new_k_off + (size_t)g * HD + 8 * lane);
+      if (!VK) *(uint4*)(krow + (size_t)a.G * pt * HD + 8 * lane) = *(const uint4*)(qrow + a.new_v_off + (size_t)g * HD + 8 * lane);
+    }
+  }
+
+  // lane groups, then warps, then blocks
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    l[r] = warp_sum(l[r]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int w = LPK; w < 32; w <<= 1) acc[r][e] += __shfl_xor_sync(0xffffffffu, acc[r][e], w);
+    if (grp == 0) {
+      *(float4*)&part[warp][r][8 * sub] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      *(float4*)&part[warp][r][8 * sub + 4] = make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]);
+    }
+    if (lane == 0) { part[warp][r][HD] = m[r]; part[warp][r][HD + 1] = l[r]; }
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < R * HD; x += AR_WARPS * 32) {
+    const int r = x / HD, e = x - r * HD;
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < AR_WARPS; ++w) M = fmaxf(M, part[w][r][HD]);
+    float o = 0.f, L = 0.f;
+#pragma unroll
+    for (int w = 0; w < AR_WARPS; ++w) {
+      const float f = ar_factor(part[w][r][HD], part[w][r][HD + 1], M);
+      o = fmaf(part[w][r][e], f, o); L = fmaf(part[w][r][HD + 1], f, L);
+    }
+    rec[r][e] = o;
+    if (e == 0) { rec[r][HD] = M; rec[r][HD + 1] = L; }
+  }
+  if (cs > 1) cluster.sync(); else __syncthreads();
+  // every block finishes its share of the elements
+  const int share = R * HD / cs;
+  for (int x = rank * share + threadIdx.x; x < (rank + 1) * share; x += AR_WARPS * 32) {
+    const int r = x / HD, e = x - r * HD, h = g * R + r;
+    float M = -INFINITY;
+    for (int c = 0; c < cs; ++c) M = fmaxf(M, cs > 1 ? cluster.map_shared_rank(&rec[0][0], c)[r * (HD + 4) + HD] : rec[r][HD]);
+    float o = 0.f, L = 0.f;
+    for (int c = 0; c < cs; ++c) {
+      const float* rc = (cs > 1 ? cluster.map_shared_rank(&rec[0][0], c) : &rec[0][0]) + r * (HD + 4);
+      const float f = ar_factor(rc[HD], rc[HD + 1], M);
+      o = fmaf(rc[e], f, o); L = fmaf(rc[HD + 1], f, L);
+    }
+    float inv = 1.0f / L;
+    if (a.gate) inv *= 1.0f / (1.0f + expf(-a.gate[(size_t)row * a.ldg + h]));
+    o *= inv;
+    if (a.og) o *= 1.0f / (1.0f + expf(-__bfloat162float(a.og[(size_t)row * a.ldog + (size_t)h * HD + e])));
+    a.out[((size_t)row * a.H + h) * HD + e] = __float2bfloat16_rn(o);
+  }
+  if (cs > 1) cluster.sync();                                        // nobody leaves while its sums are being read
+}
+
+template <int HD, int R, bool VK>
+static int ar_launch(const ArArgs& a, int T, int cs, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs, a.G, T); cfg.blockDim = dim3(AR_WARPS * 32); cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, attention_rows_kernel<HD, R, VK>, a);
+  if (e != cudaSuccess) return (int)e;
+  return launch_status();
+}
+
+// Rows of q [T, ldq] (heads at column 0, H x hd bfloat16), each at its own position of its own slot; the other arguments as
+// fellm_paged_attention_general's, vd 0 (values that are the keys) or hd; og [T, ldog] bfloat16 (null: none): the result times
+// its sigmoid, element by element; cluster: 1, 2, 4 or 8 blocks a (row, kv head).
+FELLM_API int fellm_attention_rows(const void* q, const void* pool, const int* block_table, int max_pages, const int* positions,
+                                   const int* row_slot, void* out, int T, int H, int G, int hd, int vd, int page_tokens, int layer,
+                                   int layers_in_group, float scale, int window, int ldq, float softcap, int chunk, const float* gate,
+                                   int ldg, const float* slopes, float qt_coef, int qt_every, int new_k_off, int new_v_off, int* status,
+                                   const void* og, int ldog, int cluster, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (!q || !pool || !block_table || !positions || !row_slot || !out) return FELLM_ERR_ARG;
+  if (G < 1 || H % G || (hd != 64 && hd != 128) || (vd && vd != hd) || T > 65535 || G > 65535) return FELLM_ERR_SIZE;
+  const int R = H / G;
+  if ((R != 1 && R != 2 && R != 4) || page_tokens < 1 || (page_tokens & (page_tokens - 1))) return FELLM_ERR_SIZE;
+  if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return FELLM_ERR_ARG;
+  if ((((uintptr_t)q | (uintptr_t)pool) & 15) || (ldq & 7) || (new_k_off >= 0 && ((new_k_off & 7) || (vd && (new_v_off & 7))))) return FELLM_ERR_SIZE;
+  ArArgs a;
+  a.q = (const bf16*)q; a.pool = (const bf16*)pool; a.block_table = block_table; a.positions = positions; a.row_slot = row_slot;
+  a.out = (bf16*)out; a.status = status; a.gate = gate; a.slopes = slopes; a.og = (const bf16*)og;
+  a.ldq = ldq; a.max_pages = max_pages; a.H = H; a.G = G; a.layer = layer; a.layers_in_group = layers_in_group;
+  a.window = window; a.chunk = chunk; a.ldg = ldg; a.ldog = ldog; a.qt_every = qt_every; a.new_k_off = new_k_off; a.new_v_off = new_v_off;
+  a.scale = scale; a.softcap = softcap; a.qt_coef = qt_coef;
+  a.page_shift = 0;
+  while ((1 << a.page_shift) < page_tokens) ++a.page_shift;
+#define AR_R(HD_, VK_) (R == 1 ? ar_launch<HD_, 1, VK_>(a, T, cluster, stream) : R == 2 ? ar_launch<HD_, 2, VK_>(a, T, cluster, stream) \
+                      : ar_launch<HD_, 4, VK_>(a, T, cluster, stream))
+  if (hd == 64) return vd ? AR_R(64, false) : AR_R(64, true);
+  return vd ? AR_R(128, false) : AR_R(128, true);
+#undef AR_R
+}

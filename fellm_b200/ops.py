@@ -1222,7 +1222,7 @@ ATTENTION_SIMT_MAX_HD = 1024       # the CUDA-core attention kernel's largest ke
 
 def paged_attention_general(q, H, hd, vd, pool, block_table, positions, row_slot, layer, page_tokens, G, scale, *,
                             window=None, chunk=None, softcap=None, gate=None, slopes=None, q_temp=None, warps=1, write_new=None,
-                            sinks=None, out_dim=None, out=None):
+                            sinks=None, out_dim=None, out=None, out_gate=None):
     """Attention on CUDA cores with float32 arithmetic for every form the part describes: q read in place from rows
     [T, >= H*hd] (heads at column 0), values of size vd, scores soft-capped (softcap * tanh(s / softcap)), keys limited
     to the last `window` positions and to the query's own block of `chunk` positions, and gate float32 [T, >= H]
@@ -1233,7 +1233,11 @@ def paged_attention_general(q, H, hd, vd, pool, block_table, positions, row_slot
     write_new = (k_off, v_off, status): a decode step (every row its request's only one): the rows' own keys and values,
     at those columns of q's rows, are read from there and written into their pages by this kernel (no kv_write in front).
     sinks float32 [H]: exp(sinks[h]) joins head h's softmax denominator (no key, no value, not scaled).  out_dim (with
-    vd == 0): only the first out_dim elements of a key are read out as its value.
+    vd == 0): only the first out_dim elements of a key are read out as its value.  out_gate [T, H*vd] in q's dtype: the result
+    times its sigmoid, element by element.
+    A bfloat16 decode step (write_new given, or out_gate) of the sizes `attention_rows_takes` names runs on a kernel that shares a
+    key's reading among its heads and a row's keys among blocks (csrc/attention_rows.cu; the same float32 arithmetic in another
+    order).
     Returns [T, H*vd] (H*hd, or H*out_dim, when the values are the keys) in q's dtype."""
     _dev(q, pool, block_table, positions, row_slot, gate, slopes, sinks)
     if sinks is not None:
@@ -1255,6 +1259,19 @@ def paged_attention_general(q, H, hd, vd, pool, block_table, positions, row_slot
     if out is None:
         out = torch.empty((T, H * (vd or od or hd)), dtype=q.dtype, device=q.device)
     qt_coef, qt_every = q_temp if q_temp else (0.0, 0)
+    if (write_new or out_gate is not None) and sinks is None and not od and attention_rows_takes(q, pool, H, G, hd, vd, page_tokens, write_new):
+        nk, nv, status = write_new if write_new else (-1, -1, None)
+        if out_gate is not None:
+            assert out_gate.dtype == q.dtype and out_gate.stride(1) == 1 and out_gate.shape == out.shape
+        f = _fn("attention_rows", "fellm_attention_rows",
+                [_c_p, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p] + [_c_int] * 8 + [_c_f, _c_int, _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_f,
+                 _c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_p])
+        _check(f(_p(q), _p(pool), _p(block_table), block_table.shape[1], _p(positions), _p(row_slot), _p(out), T, H, G, hd, vd, page_tokens,
+                 layer, pool.shape[1], float(scale), int(window or 0), q.stride(0), float(softcap or 0.0), int(chunk or 0), _p(gate),
+                 gate.stride(0) if gate is not None else 0, _p(slopes), float(qt_coef), int(qt_every), int(nk), int(nv), _p(status),
+                 _p(out_gate), out_gate.stride(0) if out_gate is not None else 0, attention_rows_cluster(T * G, window, chunk), _stream()),
+               "attention_rows")
+        return out
     f = _fn("attention_simt", "fellm_paged_attention_general",
             [_c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
              _c_int, _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_f, _c_int, _c_int, _c_int,
@@ -1265,7 +1282,25 @@ def paged_attention_general(q, H, hd, vd, pool, block_table, positions, row_slot
              float(scale), int(window or 0), vd, q.stride(0), float(softcap or 0.0), int(chunk or 0), _p(gate),
              gate.stride(0) if gate is not None else 0, _p(slopes), float(qt_coef), int(qt_every), int(warps), int(nk), int(nv),
              _p(status), _p(sinks), od, _stream()), "paged_attention_general")
-    return out
+    return out if out_gate is None else gate_mul(out, out_gate)
+
+
+def attention_rows_takes(q, pool, H: int, G: int, hd: int, vd: int, page_tokens: int, write_new=None) -> bool:
+    """bfloat16, keys of 64 or 128 with values of their size (or that are the keys), 1, 2 or 4 heads a kv head, pages of a power
+    of two, and rows and offsets that start on 16 bytes."""
+    return (q.dtype == pool.dtype == torch.bfloat16 and hd in (64, 128) and vd in (0, hd) and H % G == 0 and H // G in (1, 2, 4)
+            and page_tokens & (page_tokens - 1) == 0 and q.stride(0) % 8 == 0 and not (q.data_ptr() | pool.data_ptr()) % 16
+            and q.shape[0] <= 65535 and (not write_new or not (write_new[0] % 8 or (vd and write_new[1] % 8))))
+
+
+def attention_rows_cluster(items: int, window=None, chunk=None) -> int:
+    """Blocks (of four warps, a tile of 32 keys at a time) that share a row and kv head's keys: enough for two blocks an SM, no
+    more than have a tile each."""
+    tiles = -(-min(window or 4096, chunk or 4096, 4096) // 32)
+    n = 1
+    while n < 8 and items * n < 2 * sm_count() and 8 * n <= tiles:
+        n *= 2
+    return n
 
 
 def latent_prep(z, q_off, rq, c_off, rk, r_off, dr, wq, wc, eps, freq, n_rot, mag, positions, row_slot, cache, out_dtype,

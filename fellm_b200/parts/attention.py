@@ -314,27 +314,23 @@ class Attention(Mixer):
         if self.position.inv_freq is not None or self.unit_qk_norm:
             ops.qk_rotate_norm(qkv, H, G, H * hd, hd, self.rot_dim, self.position.inv_freq, self.position.pairing,
                                ctx.positions, self.eps, unit_norm=self.unit_qk_norm)
-        kw = dict(window=self.window, chunk=self.chunk, softcap=self.softcap, warps=self.simt_warps)
+        kw = dict(window=self.window, chunk=self.chunk, softcap=self.softcap,
+                  out_gate=qkv[:, self.gate_off:self.gate_off + H * vd] if self.out_gate else None)
         if ctx.all_single:
             write = None if self.shares_cache else (H * hd, (H + G) * hd, ctx.status)
             a = ops.paged_attention_general(qkv, H, hd, vd, cache.pool, cache.block_table, ctx.positions, ctx.row_slot,
-                                            cache.layer, cache.page_tokens, self.G, self.scale, write_new=write, **kw)
+                                            cache.layer, cache.page_tokens, self.G, self.scale, write_new=write,
+                                            warps=self.simt_warps, **kw)
         else:
             if not self.shares_cache:
                 ops.kv_write(qkv, H * hd, (H + G) * hd, cache.pool, cache.block_table, ctx.positions, ctx.row_slot,
                              cache.layer, cache.page_tokens, G, hd, vd, status=ctx.status)
             if self._on_tensor_cores(qkv):
                 a = ops.attention_prefill_general(qkv, H, cache.pool, cache.block_table, ctx.positions, ctx.row_slot,
-                                                  ctx.item_start, ctx.n_items, ctx.max_item_rows, cache.layer, self.scale,
-                                                  window=self.window, chunk=self.chunk, softcap=self.softcap,
-                                                  out_gate=qkv[:, self.gate_off:self.gate_off + H * vd] if self.out_gate else None)
-                linear(a, self.w["out_proj.weight"], self.w.get("out_proj.bias"), out=out, accumulate=not store)
-                return out
+                                                  ctx.item_start, ctx.n_items, ctx.max_item_rows, cache.layer, self.scale, **kw)
             else:
-                a = ops.paged_attention_general(qkv, H, hd, vd, cache.pool, cache.block_table, ctx.positions,
-                                                ctx.row_slot, cache.layer, cache.page_tokens, self.G, self.scale, **kw)
-        if self.out_gate:
-            ops.gate_mul(a, qkv[:, self.gate_off:self.gate_off + H * vd])
+                a = ops.paged_attention_general(qkv, H, hd, vd, cache.pool, cache.block_table, ctx.positions, ctx.row_slot,
+                                                cache.layer, cache.page_tokens, self.G, self.scale, warps=self.simt_warps, **kw)
         linear(a, self.w["out_proj.weight"], self.w.get("out_proj.bias"), out=out, accumulate=not store)
         return out
 
@@ -352,6 +348,8 @@ class Attention(Mixer):
         if self.general:
             mma = dtype == "bfloat16" and self.vd == self.hd and self.hd % 16 == 0 and self.H // self.G <= 64
             extra = ([("qk_rope_write", None)] if self.in_place else []) + ([("sublayer", None)] if self.out_gate else [])
+            if dtype == "bfloat16" and self.hd in (64, 128) and self.vd == self.hd and self.H // self.G in (1, 2, 4):
+                extra.append(("attention_rows", None))
             if mma and ops.general_umma_takes(self.H, self.G, self.hd, 64, self.scale, self.q_temp):
                 extra.append(("attention_umma", ops._umma_defines(64, 64, general=True)))
             return linear_modules(dtype) + [("attention_simt", None)] + ([("attention_mma", {"HD": self.hd})] if mma else []) + extra

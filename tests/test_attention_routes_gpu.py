@@ -117,3 +117,53 @@ def test_portions_on_tcgen05(spec, H, G, keys_alone):
         want = attend(q[at, :H * 64].double().view(-1, H, 64), pages.k[r].double(), pages.v[r].double(), pos[at], 0.125,
                       slopes=None if slopes is None else slopes.double(), **kw)
         close(got[at], gated(want, H, None if gate is None else gate[at], None if out_gate is None else out_gate[at]))
+
+
+@pytest.mark.parametrize("spec", FORMS)
+@pytest.mark.parametrize("H,G,hd,page,keys_alone,cluster", [(4, 1, 64, 64, True, 8), (4, 2, 64, 16, False, 2), (3, 3, 128, 64, False, 4),
+                                                           (8, 2, 64, 256, False, 1), (8, 2, 128, 32, True, 8)])
+def test_rows_over_a_cluster(spec, H, G, hd, page, keys_alone, cluster, monkeypatch):
+    from fellm_b200 import ops
+    if hd != 64 and "out_gate" in spec:
+        return
+    monkeypatch.setattr(ops, "attention_rows_cluster", lambda *a: cluster)
+    g = torch.Generator().manual_seed(H + G)
+    lens = [1, 31, 33, 130, 700]
+    vd = 0 if keys_alone else hd
+    pages = Pages(lens, G, hd, vd, page, 5)
+    T = len(lens)
+    q = torch.randn(T, (H + 2 * G) * hd + 8, generator=g).bfloat16()
+    for r in range(T):                                                 # the step's own keys and values lie in the rows
+        pages.k[r][-1] = q[r, H * hd:(H + G) * hd].view(G, hd)
+        if vd:
+            pages.v[r][-1] = q[r, (H + G) * hd:(H + 2 * G) * hd].view(G, hd)
+    pos = torch.tensor([n - 1 for n in lens])
+    kw, slopes, gate, out_gate = form(spec, T, H, g)
+    pool = pages.pool if keys_alone else pages.five(G, hd)
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()  # noqa: E731
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def call(write, with_gate=True):
+        return ops.paged_attention_general(
+            q.cuda(), H, hd, vd, pool, pages.table.cuda(), i32(pos), i32(range(T)), 1, page, G, hd ** -0.5, window=kw.get("window"),
+            chunk=kw.get("chunk"), softcap=kw.get("cap"), q_temp=kw.get("temp"), slopes=None if slopes is None else slopes.cuda(),
+            gate=None if gate is None else gate.cuda(), write_new=write,
+            out_gate=out_gate.cuda()[:, :H * hd] if out_gate is not None and with_gate else None)
+    write = (H * hd, (H + G) * hd, status)
+    assert ops.attention_rows_takes(q.cuda(), pool, H, G, hd, vd, page, write)
+    got = call(write)
+    assert int(status) == 0
+    again = call(None, with_gate=False)          # the CUDA-core kernel, which reads the rows' keys and values from their pages now
+    for r in range(T):
+        want = attend(q[r:r + 1, :H * hd].double().view(1, H, hd), pages.k[r].double(), pages.v[r].double(), pos[r:r + 1], hd ** -0.5,
+                      slopes=None if slopes is None else slopes.double(), **kw)
+        whole = gated(want, H, None if gate is None else gate[r:r + 1], None if out_gate is None else out_gate[r:r + 1])
+        # float32 throughout, one rounding to bfloat16 at the end: 2^-9 of an element at most
+        assert float((got[r:r + 1].double().cpu() - whole).norm() / whole.norm()) < 2.5e-3
+        plain = gated(want, H, None if gate is None else gate[r:r + 1], None)
+        assert float((again[r:r + 1].double().cpu() - plain).norm() / plain.norm()) < 2.5e-3
+    pages.table[2, (lens[2] - 1) // page] = -1                          # no page for the row's position: nothing written, a status
+    before = pool.clone()
+    call(write)
+    torch.cuda.synchronize()
+    assert int(status) == 2 and torch.equal(before.view(torch.int16), pool.view(torch.int16))
