@@ -14,6 +14,9 @@
 // With -DAU_GEN (which has AU_EXT in it) also chunks (a query reads only its own block of `chunk` positions), a bias by
 // distance per head, a query temperature by position, a gate per head, and values that are the keys (the keys' tile is then
 // the second product's operand too: half the page traffic).
+// With -DAU_LAT (which has AU_EXT in it) the keys and values are not pages but rows of matrices that a latent-attention layer
+// has made out of its cached latents for this step (fellm_attn_latent_umma below): per key the heads' unrotated parts and
+// values side by side, and one rotated part for all heads.
 // A page-layer record of the pool is the keys [G][64][AU_KD], then the values [G][64][AU_VD].
 // The accumulator is scaled by 2^-m with m a row's REFERENCE maximum, which moves only when a tile's
 // maximum exceeds it by 2^8: only then is the accumulator read, scaled and written back.
@@ -49,6 +52,12 @@
 constexpr bool AU_GENERAL = true;
 #else
 constexpr bool AU_GENERAL = false;
+#endif
+#ifdef AU_LAT
+#define AU_EXT 1
+constexpr bool AU_LATENT = true;
+#else
+constexpr bool AU_LATENT = false;
 #endif
 #ifdef AU_EXT
 constexpr bool AU_EXTENDED = true;
@@ -90,7 +99,9 @@ struct AuArgs {
   // (qt_every 0: none), blocks of `chunk` positions (0: none), a gate float32 [T, ldhg] of a number per head (null: none)
   const float* slopes; const float* hg;
   float qt_coef; int qt_every, chunk, ldhg, v_is_k;
+  int key_rows;                        // AU_LAT: rows of the matrices per item; an item's first is the page of its first row's first key
 };
+#define AU_LAT_ROPE 64                 // AU_LAT: elements of a key that all heads share (the last of AU_KD)
 
 __device__ __forceinline__ unsigned au_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void au_mbar_init(unsigned bar, unsigned count) {
@@ -266,6 +277,19 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % AU_STAGES;
         if (j >= AU_STAGES && !au_wait(empty0 + 8 * s, (j / AU_STAGES - 1) & 1, fail, a.status, 311)) break;
+        if constexpr (AU_LATENT) {
+          const int p0 = a.positions[row_begin];
+          const int key_row = item * a.key_rows + (first_page + j) * AU_PT - max(p0 - a.window + 1, 0) / AU_PT * AU_PT;
+          const unsigned to = stage0 + s * AU_STAGE_B;
+          au_mbar_expect_tx(full0 + 8 * s, AU_STAGE_B);
+#pragma unroll
+          for (int i = 0; i < AU_KA - 1; ++i) au_tma_load_3d(to + i * AU_ATOM_B, &k_map, g * (AU_KD - AU_LAT_ROPE + AU_VD) + 64 * i, key_row, 0, full0 + 8 * s);
+          au_tma_load_3d(to + (AU_KA - 1) * AU_ATOM_B, &v_map, 0, key_row, 0, full0 + 8 * s);
+#pragma unroll
+          for (int i = 0; i < AU_VA; ++i)
+            au_tma_load_3d(to + (AU_KA + i) * AU_ATOM_B, &k_map, g * (AU_KD - AU_LAT_ROPE + AU_VD) + AU_KD - AU_LAT_ROPE + 64 * i, key_row, 0, full0 + 8 * s);
+          continue;
+        }
         const int page = max(bt[j], 0);                        // an unmapped entry (-1) must never become an address
         const int rec = page * a.layers_in_group + a.layer;
         const unsigned dst = stage0 + s * AU_STAGE_B;
@@ -635,4 +659,59 @@ FELLM_API int fellm_attn_prefill_umma(const void* q, int ldq, const void* pool, 
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ce != cudaSuccess) return (int)ce;
   return launch_k_class(launch_class_for_rows(T, 0), kern, dim3(ceil_div(max_item_rows, tokb) * G, 1, n_items), dim3(AU_THREADS), smem, stream, 1, k_map, v_map, a);
+}
+
+// ---------------------------------------------------------------- latent attention of portions, keys and values per head
+// A latent-attention layer with a window: kv [n_items * key_rows, H * (AU_KD - 64 + AU_VD)] bfloat16, per key and head the
+// unrotated part and the value (a product of the cached latents with the layer's up projections); rope [n_items * key_rows, 64]:
+// the keys' rotated parts.  Item i's keys are rows i * key_rows + (key - first), first: the position of the page of the first
+// key that the item's first row sees; rows past its last key are zeros.  q [T, ldq]: head h at column h * AU_KD, rotated.
+// Against the form that keeps the queries in the latents' space (latent_attention_mma.cu) a pair of query and key costs 320
+// multiply-adds a head and not 1,088 (heads of 128 + 64, values of 128, a latent of 512).
+FELLM_API int fellm_attn_latent_umma(const void* q, int ldq, const void* kv, const void* rope, int key_rows, const int* positions,
+                                     const int* item_start, int n_items, int max_item_rows, void* out, int T, int H, float scale,
+                                     int window, const float* sinks, int* status, cudaStream_t stream) {
+#ifdef AU_LAT
+  if (T <= 0 || n_items <= 0) return 0;
+  if (!q || !kv || !rope || !positions || !item_start || !out) return FELLM_ERR_ARG;
+  static_assert(AU_KD % 64 == 0 && AU_VD % 64 == 0 && AU_KD > 64, "whole atoms");
+  const long long rows = (long long)n_items * key_rows;
+  if (!(scale > 0.f) || window < 1) return FELLM_ERR_ARG;
+  if (H < 1 || key_rows < 1 || (key_rows % AU_PT) || rows >= (1ll << 31) || key_rows < window - 1 + AU_PT - 1 + max_item_rows || ldq < H * AU_KD ||
+      (ldq % 8) || (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)rope | (uintptr_t)out) & 15)) return FELLM_ERR_SIZE;
+  AuArgs a = {};
+  a.q = (const bf16*)q; a.ldq = ldq; a.positions = positions; a.item_start = item_start; a.out = (bf16*)out; a.status = status;
+  a.block_table = positions; a.row_slot = positions;            // (there are no pages: addresses that are valid, times max_pages = 0)
+  a.max_pages = 0; a.sinks = sinks; a.H = H; a.G = H; a.layers_in_group = 1; a.scale_log2 = scale * 1.4426950408889634f;
+  a.window = window; a.key_rows = key_rows;
+  static AuEncodeTiledFn fn = nullptr;
+  if (!fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess)
+      return FELLM_ERR_ARG;
+    fn = (AuEncodeTiledFn)p;
+  }
+  CUtensorMap maps[2];
+  const cuuint64_t cols[2] = {(cuuint64_t)H * (AU_KD - AU_LAT_ROPE + AU_VD), AU_LAT_ROPE};
+  const void* base[2] = {kv, rope};
+  for (int i = 0; i < 2; ++i) {
+    cuuint64_t dims[3] = {cols[i], (cuuint64_t)rows, 1};
+    cuuint64_t strides[2] = {cols[i] * 2, cols[i] * 2 * (cuuint64_t)rows};
+    cuuint32_t box[3] = {64, AU_PT, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base[i]), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return 1000 + (int)r;
+  }
+  const size_t smem = (size_t)AU_FIXED_B + (size_t)AU_STAGES * AU_STAGE_B + 1024;
+  auto kern = attention_prefill_umma_kernel;
+  cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (ce != cudaSuccess) return (int)ce;
+  return launch_k_class(launch_class_for_rows(T, 0), kern, dim3(ceil_div(max_item_rows, AU_ROWS) * H, 1, n_items), dim3(AU_THREADS), smem,
+                        stream, 1, maps[0], maps[1], a);
+#else
+  return FELLM_ERR_SIZE;
+#endif
 }

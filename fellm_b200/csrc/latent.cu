@@ -205,3 +205,61 @@ FELLM_API int fellm_latent_rotate_q(const void* q, int bf16_, int ldq, int H, in
   return launch_k_class(cls, latent_rotate_q_kernel<float>, dim3(T), dim3(128), 0, stream, 1, (const float*)q, ldq, H, dn, dr,
                         (float*)q_abs, rk, freq, n_rot, mag, positions);
 }
+
+// ---------------------------------------------------------------- portions: the latents a step's rows see, side by side
+// Blocks [0, T): a row's queries' rotated parts (dr elements behind the dn unrotated ones of every head), rotated where they
+// lie.  The others: a warp a key row of item i: the cached row of position first_i + k, first_i the position of the page of
+// the first key that the item's first row sees through the window; its rk latent elements into `lat`, its rotated part into
+// `rope`; zeros behind the item's last key (and where no page is mapped).
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(bf16* q, int ldq, int H, int dn, int dr, const float* __restrict__ freq, int n_rot, float mag,
+                     const int* __restrict__ positions, const int* __restrict__ row_slot, const int* __restrict__ item_start,
+                     const int* __restrict__ block_table, int max_pages, const bf16* __restrict__ pool, int page_tokens, int layer,
+                     int layers_in_group, int rk, int window, int key_rows, int T, bf16* __restrict__ lat, bf16* __restrict__ rope) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if ((int)blockIdx.x < T) {
+    const int row = blockIdx.x, half = n_rot / 2;
+    const float pos = (float)positions[row];
+    bf16* qr = q + (size_t)row * ldq;
+    for (int i = threadIdx.x; i < H * half; i += blockDim.x) {
+      const int h = i / half, p = i - h * half;
+      __nv_bfloat162* at = (__nv_bfloat162*)(qr + (size_t)h * (dn + dr) + dn + 2 * p);
+      float2 v = __bfloat1622float2(*at);
+      float sn, cs;
+      sincosf(pos * freq[p], &sn, &cs);
+      sn *= mag; cs *= mag;
+      *at = __floats2bfloat162_rn(v.x * cs - v.y * sn, v.y * cs + v.x * sn);
+    }
+    return;
+  }
+  const int w = (blockIdx.x - T) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int item = w / key_rows, k = w - item * key_rows;
+  const int r0 = item_start[item], n = item_start[item + 1] - r0;
+  const int p0 = n > 0 ? positions[r0] : 0, key = max(p0 - window + 1, 0) / page_tokens * page_tokens + k;
+  const int D = rk + dr;
+  int page = -1;
+  if (n > 0 && key < p0 + n) page = block_table[(size_t)row_slot[r0] * max_pages + key / page_tokens];
+  const uint4* src = (const uint4*)(pool + (((size_t)max(page, 0) * layers_in_group + layer) * page_tokens + key % page_tokens) * D);
+  for (int i = lane; i < D / 8; i += 32) {
+    const uint4 v = page >= 0 ? src[i] : make_uint4(0, 0, 0, 0);
+    if (i < rk / 8) *(uint4*)(lat + (size_t)w * rk + 8 * i) = v;
+    else *(uint4*)(rope + (size_t)w * dr + 8 * i - rk) = v;
+  }
+}
+
+// key_rows: a multiple of 8 and of the page, at least window - 1 + page - 1 + the longest item's rows.
+FELLM_API int fellm_latent_gather(void* q, int ldq, int H, int dn, int dr, const float* freq, int n_rot, float mag, const int* positions,
+                                  const int* row_slot, const int* item_start, const int* block_table, int max_pages, const void* pool,
+                                  int page_tokens, int layer, int layers_in_group, int rk, int window, int key_rows, int T, int n_items,
+                                  void* lat, void* rope, cudaStream_t stream) {
+  if (T <= 0 || n_items <= 0) return 0;
+  if (!q || !positions || !row_slot || !item_start || !block_table || !pool || !lat || !rope || (n_rot && !freq)) return FELLM_ERR_ARG;
+  if (H < 1 || dn < 0 || dr < 0 || n_rot < 0 || n_rot > dr || (n_rot & 1) || window < 1 || key_rows < 8 || key_rows % 8 || page_tokens < 1 ||
+      rk % 8 || dr % 8 || (dn & 1) || (ldq & 1) || (((uintptr_t)pool | (uintptr_t)lat | (uintptr_t)rope) & 15) || ((uintptr_t)q & 3)) return FELLM_ERR_SIZE;
+  const long long blocks = T + (long long)n_items * key_rows / 8;
+  if (blocks >= (1ll << 28)) return FELLM_ERR_SIZE;
+  return launch_k_class(launch_class_for_rows(T, 0), latent_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, 1, (bf16*)q, ldq, H, dn, dr,
+                        freq, n_rot, mag, positions, row_slot, item_start, block_table, max_pages, (const bf16*)pool, page_tokens, layer,
+                        layers_in_group, rk, window, key_rows, T, (bf16*)lat, (bf16*)rope);
+}

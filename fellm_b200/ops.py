@@ -1347,6 +1347,62 @@ LATENT_SINGLE_ROWS = 32        # up to this many (token, head) rows an item: the
 LATENT_MAX_SPLITS = 16
 
 
+LATENT_EXPAND = os.environ.get("FELLM_B200_LATENT_EXPAND", "1") != "0"
+
+
+def latent_expand_key_rows(H: int, dn: int, dr: int, dv: int, rk: int, window, page_tokens: int, n_rows: int, n_items: int, max_item_rows: int) -> int:
+    """Rows of keys an item when a portion's keys and values are made per head out of the cached latents (latent_expanded_attention),
+    or 0 where the queries rather go into the latents' space (latent_attention).  Sizes: what the tcgen05 library is compiled for, a
+    window (the rows an item can see are then known without its positions), pages of 64.  Worth it: a key row costs a product of
+    rk x H (dn + dv) (~8 ns at 16 heads of 128, a latent of 512), a query row in the latents' space 0.2 us more over a window of
+    1,024 than per head, so up to 16 key rows a query row; below that a step is mostly single tokens or the last few of a prompt."""
+    if not LATENT_EXPAND or not window or page_tokens != 64 or (dn, dr, dv) != (128, 64, 128) or rk % 64 or window > 4096:
+        return 0
+    rows = -(-(int(window) - 1 + 63 + max_item_rows) // 64) * 64
+    return rows if n_items * rows <= 16 * n_rows and n_rows >= 64 else 0
+
+
+def latent_expand_defines():
+    return {"AU_KD": 192, "AU_VD": 128, "AU_GROUPS": 1, "AU_LAT": 1}
+
+
+def latent_gather(q, H: int, dn: int, dr: int, freq, n_rot: int, mag: float, rk: int, cache, ctx, window: int, key_rows: int):
+    """Rotates the queries' rotated parts where they lie (q bfloat16 [T, >= H (dn + dr)]) and brings the cached rows that the
+    step's rows see side by side: (latents [n_items * key_rows, rk], rotated parts [n_items * key_rows, dr]), zeros behind an
+    item's last key."""
+    _dev(q, freq, cache.pool, ctx.positions, ctx.row_slot, ctx.item_start)
+    assert q.dtype == cache.pool.dtype == torch.bfloat16 and q.stride(1) == 1 and cache.pool.is_contiguous()
+    assert cache.pool[0, 0].numel() == cache.page_tokens * (rk + dr)
+    _i32(ctx.positions, "positions"), _i32(ctx.row_slot, "row_slot"), _i32(ctx.item_start, "item_start"), _i32(cache.block_table, "block_table")
+    n = ctx.n_items * key_rows
+    lat = torch.empty((n, rk), dtype=q.dtype, device=q.device)
+    rope = torch.empty((n, dr), dtype=q.dtype, device=q.device)
+    f = _fn("latent", "fellm_latent_gather",
+            [_c_p, _c_int, _c_int, _c_int, _c_int, _c_p, _c_int, _c_f, _c_p, _c_p, _c_p, _c_p, _c_int, _c_p] + [_c_int] * 8 + [_c_p] * 3)
+    _check(f(_p(q), q.stride(0), H, dn, dr, _p(freq), int(n_rot), float(mag), _p(ctx.positions), _p(ctx.row_slot), _p(ctx.item_start),
+             _p(cache.block_table), cache.block_table.shape[1], _p(cache.pool), cache.page_tokens, cache.layer, cache.pool.shape[1], rk,
+             int(window), int(key_rows), q.shape[0], ctx.n_items, _p(lat), _p(rope), _stream()), "latent_gather")
+    return lat, rope
+
+
+def latent_expanded_attention(q, H: int, kv, rope, key_rows: int, ctx, scale: float, window: int, sinks=None):
+    """Attention of prompt portions with keys and values per head: q [T, H * 192] rotated, kv [n_items * key_rows, H * 256] (per head
+    128 unrotated key elements, 128 of the value), rope [n_items * key_rows, 64]; -> [T, H * 128]."""
+    _dev(q, kv, rope, ctx.positions, ctx.item_start, sinks)
+    assert q.dtype == kv.dtype == rope.dtype == torch.bfloat16 and kv.is_contiguous() and rope.is_contiguous() and q.stride(1) == 1
+    assert kv.shape == (ctx.n_items * key_rows, H * 256) and rope.shape == (ctx.n_items * key_rows, 64) and q.shape[1] >= H * 192
+    if sinks is not None:
+        assert sinks.dtype == torch.float32 and sinks.numel() == H and sinks.is_contiguous()
+    T = q.shape[0]
+    out = torch.empty((T, H * 128), dtype=q.dtype, device=q.device)
+    f = _fn("attention_umma", "fellm_attn_latent_umma",
+            [_c_p, _c_int, _c_p, _c_p, _c_int, _c_p, _c_p, _c_int, _c_int, _c_p, _c_int, _c_int, _c_f, _c_int, _c_p, _c_p, _c_p],
+            defines=latent_expand_defines())
+    _check(f(_p(q), q.stride(0), _p(kv), _p(rope), int(key_rows), _p(ctx.positions), _p(ctx.item_start), ctx.n_items, ctx.max_item_rows,
+             _p(out), T, H, float(scale), int(window), _p(sinks), _p(umma_status(q.device)), _stream()), "latent attention (tcgen05)")
+    return out
+
+
 def latent_attention_takes(q_abs, pool, rk: int, dr: int, page_tokens: int) -> bool:
     """Whether the tensor-core kernel takes a latent-attention layer of these sizes: bfloat16 queries and cache, a
     latent of a multiple of 32 up to 512, rows of a multiple of 16 elements, pages of a multiple of 64 tokens."""

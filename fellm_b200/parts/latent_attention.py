@@ -11,7 +11,10 @@ normed key-value latent (rk elements) and ONE rotated key part (dr elements) sha
 Nothing per head is ever stored: with qa_i,h = W_uk,h^T qn_i,h the unrotated part of the score is qa_i,h . c_j, and
 sum_j p_ij v_j,h = W_uv,h sum_j p_ij c_j.  So the attention kernel runs over the cached rows [c_j | rot_j(kr_j)] with
 queries [qa_i,h | rot_i(qr_i,h)], one key "head" for all query heads, the keys read as the values and only their
-first rk elements read out; a product per head before it (W_uk^T) and one behind it (W_uv) do the rest.  `scale` is
+first rk elements read out; a product per head before it (W_uk^T) and one behind it (W_uv) do the rest.  Prompt portions
+of a layer with a window go the other way round where the sizes allow (ops.latent_expand_key_rows): the latents that the
+step's rows see are gathered, kn and v of all heads are one product, and attention runs per head on tcgen05 with keys of
+dn + dr; a pair of query and key then costs dn + dr + dv multiply-adds a head and not 2 rk + dr.  `scale` is
 the layer's own and is used as given.  The rotation is the position part's (pairs (2i, 2i+1) or, r elements being
 rotated, (i, i + r/2); scaled frequencies and a magnitude where the part has them); norms, angles, scores and the softmax are float32 in both engines.
 """
@@ -92,10 +95,16 @@ class LatentAttention(Mixer):
         w["uq.weight"] = _pad_rows(w["uq.weight"])
         # per head: W_uk,h^T as [rk, dn] rows (qa = W_uk,h^T qn) and W_uv,h [dv, rk]
         uk = w.pop("uk.weight")
+        if self._expands(uk.dtype):
+            # portions of prompts: keys and values per head out of the latents, one product, rows [head: W_uk,h | W_uv,h]
+            w["kv.weight"] = torch.cat([uk.view(H, dn, rk), w["uv.weight"].view(H, dv, rk).to(uk.dtype)], 1).reshape(H * (dn + dv), rk).contiguous()
         w["ukT.weight"] = uk.view(H, dn, rk).transpose(1, 2).contiguous()
         w["uv.weight"] = w["uv.weight"].view(H, dv, rk).contiguous()
         w["o.weight"] = w["o.weight"].contiguous()
         self.position.to(uk.device)
+
+    def _expands(self, dtype) -> bool:
+        return dtype == torch.bfloat16 and bool(ops.latent_expand_key_rows(self.H, self.dn, self.dr, self.dv, self.rk, self.window, 64, 1 << 20, 1, 1))
 
     can_store = True       # forward(store=True) writes the float32 rows `out` instead of adding into them
     input_rows = "down.weight"      # forward(pre=z): the float32 product of the layer's input with these rows, made elsewhere
@@ -111,6 +120,12 @@ class LatentAttention(Mixer):
                              xn.dtype, status=ctx.status)
         q = linear(cq, w["uq.weight"])
         T = q.shape[0]
+        if "kv.weight" in w and q.dtype == torch.bfloat16 and q.data_ptr() % 16 == 0 and q.stride(0) % 8 == 0:
+            key_rows = ops.latent_expand_key_rows(H, dn, dr, dv, rk, self.window, cache.page_tokens, T, ctx.n_items, ctx.max_item_rows)
+            if key_rows:
+                lat, rope = ops.latent_gather(q, H, dn, dr, self.position.inv_freq, self.n_rot, self.magnitude, rk, cache, ctx, self.window, key_rows)
+                o = ops.latent_expanded_attention(q, H, linear(lat, w["kv.weight"]), rope, key_rows, ctx, self.scale, self.window, w.get("sink"))
+                return self._project(o, out, store)
         on_mma = ops.latent_attention_takes(q, cache.pool, rk, dr, cache.page_tokens)
         if on_mma and ctx.max_item_rows * H <= ops.LATENT_SINGLE_ROWS and ops.latent_rotate_fusable(q, dn + dr, dn):
             # single tokens: the attention kernel rotates the queries' rotated parts itself, on their way into shared
@@ -141,6 +156,10 @@ class LatentAttention(Mixer):
         w = self.w
         o = torch.empty((T, self.H * self.dv), dtype=a.dtype, device=a.device)
         ops.head_gemm(a, w["uv.weight"], o, a_head=self.rk, out_head=self.dv)
+        return self._project(o, out, store)
+
+    def _project(self, o, out, store):
+        w = self.w
         if store:
             linear(o, w["o.weight"], out=out, out_dtype=torch.float32)
         else:
@@ -154,4 +173,6 @@ class LatentAttention(Mixer):
         mods = linear_modules(dtype) + [("latent", None), ("attention_simt", None)]
         if dtype == "bfloat16" and self.rk % 32 == 0 and 32 <= self.rk <= 512 and (self.rk + self.dr) % 16 == 0:
             mods += ops.latent_attention_modules(self.rk, self.dr)
+            if self._expands(torch.bfloat16):
+                mods.append(("attention_umma", ops.latent_expand_defines()))
         return mods

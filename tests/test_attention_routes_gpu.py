@@ -1,9 +1,11 @@
 """Attention kernels of portions and of single rows that a layer's sizes choose: tcgen05 with chunks, biases, temperatures,
-gates and values that are the keys.  Against float64 over whole contexts, at the edges of pages, windows, chunks and of a
+gates and values that are the keys; keys and values per head out of cached latents; and rows whose keys are dealt out over
+a cluster.  Against float64 over whole contexts, at the edges of pages, windows, chunks and of a
 block's 128 rows."""
 from __future__ import annotations
 
 import math
+import types
 
 import pytest
 import torch
@@ -167,3 +169,43 @@ def test_rows_over_a_cluster(spec, H, G, hd, page, keys_alone, cluster, monkeypa
     call(write)
     torch.cuda.synchronize()
     assert int(status) == 2 and torch.equal(before.view(torch.int16), pool.view(torch.int16))
+
+
+@pytest.mark.parametrize("window,sink", [(64, True), (100, False), (1, True)])
+def test_latents_taken_out_per_head(window, sink):
+    from fellm_b200 import ops
+    H, rk, dr = 3, 128, 64
+    g = torch.Generator().manual_seed(window)
+    lens, rows = [200, 130, 64, 300], [65, 130, 1, 128]
+    pages = Pages(lens, 1, rk + dr, 0, 64, 4)
+    T = sum(rows)
+    q = torch.randn(T, H * 192, generator=g).bfloat16()
+    wk, wv = ((torch.randn(H, 128, rk, generator=g) * rk ** -0.5).bfloat16() for _ in range(2))
+    sinks = torch.randn(H, generator=g) if sink else None
+    pos = torch.cat([torch.arange(n - m, n) for n, m in zip(lens, rows)])
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()  # noqa: E731
+    starts = [sum(rows[:i]) for i in range(len(rows) + 1)]
+    freq = torch.tensor([10000.0 ** (-2 * i / 32) for i in range(16)])                  # half of the rotated part turns
+    ctx = types.SimpleNamespace(positions=i32(pos), row_slot=i32([r for r, m in enumerate(rows) for _ in range(m)]), item_start=i32(starts),
+                                n_items=len(rows), max_item_rows=max(rows))
+    cache = types.SimpleNamespace(pool=pages.pool, block_table=pages.table.cuda(), page_tokens=64, layer=1)
+    key_rows = -(-(window - 1 + 63 + max(rows)) // 64) * 64
+    qd = q.cuda()
+    lat, rope = ops.latent_gather(qd, H, 128, dr, freq.cuda(), 32, 1.5, rk, cache, ctx, window, key_rows)
+    kv = (lat.float() @ torch.cat([wk, wv], 1).reshape(H * 256, rk).cuda().float().T).bfloat16()
+    assert torch.isfinite(kv).all()
+    got = ops.latent_expanded_attention(qd, H, kv, rope, key_rows, ctx, 0.1, window, None if sinks is None else sinks.cuda())
+    ops.check_umma_status(torch.device("cuda"))
+    a = (pos.float()[:, None] * freq[None]).double()
+    q64 = q.double().view(T, H, 192).clone()
+    u, v = q64[..., 128:160:2].clone(), q64[..., 129:160:2].clone()
+    c, s = (torch.cos(a) * 1.5)[:, None], (torch.sin(a) * 1.5)[:, None]
+    q64[..., 128:160:2], q64[..., 129:160:2] = u * c - v * s, v * c + u * s
+    for r in range(len(rows)):
+        at = slice(starts[r], starts[r + 1])
+        row = pages.k[r][:, 0].double()
+        k = torch.cat([torch.einsum("nr,hdr->nhd", row[:, :rk], wk.double()), row[:, None, rk:].expand(-1, H, dr)], -1)
+        want = attend(q64[at], k, torch.einsum("nr,hdr->nhd", row[:, :rk], wv.double()), pos[at], 0.1, window=window,
+                      sinks=None if sinks is None else sinks.double())
+        # (keys, values and rotated queries are rounded once more than in `close`'s other callers)
+        assert float((got[at].double().cpu() - want.reshape(rows[r], -1)).norm() / want.norm()) < 1e-2
