@@ -1192,6 +1192,15 @@ def paged_attention_simt(q, pool, block_table, positions, row_slot, layer, scale
     _i32(block_table, "block_table"), _i32(positions, "positions"), _i32(row_slot, "row_slot")
     if out is None:
         out = torch.empty((T, H * hd), dtype=q.dtype, device=q.device)
+    if (hd == 64 and H // G in (1, 2, 4) and q.dtype == pool.dtype == torch.float32 and out.dtype == torch.float32
+            and not (q.data_ptr() | pool.data_ptr()) % 16):
+        # heads of 64: neighbouring rows share the reading of their keys (201 rows of 16 heads behind 250 tokens: 104 us in the
+        # kernel below)
+        f = _fn("attention_f32", "fellm_attention_f32",
+                [_c_p, _c_int, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p] + [_c_int] * 7 + [_c_f, _c_int, _c_p])
+        _check(f(_p(q), H * hd, _p(pool), _p(block_table), block_table.shape[1], _p(positions), _p(row_slot), _p(out), T, H, G, hd,
+                 page_tokens, layer, pool.shape[1], float(scale), int(window or 0), _stream()), "attention_f32")
+        return out
     f = _fn("attention_simt", "fellm_paged_attention_simt",
             [_c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
              _c_int, _c_int, _c_int, _c_f, _c_int, _c_p])
@@ -2388,6 +2397,8 @@ def general_umma_takes(H: int, G: int, hd: int, page_tokens: int, scale: float, 
 
 def attention_modules(dtype: str, head_dim: int):
     mods = [("attention_simt", None)]
+    if dtype == "float32" and head_dim == 64:
+        mods.append(("attention_f32", None))
     if dtype == "bfloat16":
         mods.append(("attention_mma", {"HD": head_dim}))
         if head_dim == 64 and USE_UMMA_PREFILL:

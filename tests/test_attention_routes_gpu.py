@@ -209,3 +209,27 @@ def test_latents_taken_out_per_head(window, sink):
                       sinks=None if sinks is None else sinks.double())
         # (keys, values and rotated queries are rounded once more than in `close`'s other callers)
         assert float((got[at].double().cpu() - want.reshape(rows[r], -1)).norm() / want.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("H,G,page,window", [(4, 4, 16, None), (4, 2, 64, None), (8, 2, 32, None), (4, 2, 64, 40), (3, 3, 64, 1)])
+def test_float32_rows_share_their_keys(H, G, page, window):
+    """The 32-bit attention: near float64, and a row's bits whatever else is in the launch."""
+    from fellm_b200 import ops
+    g = torch.Generator().manual_seed(H * G)
+    lens, rows = [131, 64, 300, 1, 33], [37, 64, 5, 1, 33]
+    pages = Pages(lens, G, 64, 64, page, 6)
+    pool = pages.five(G, 64).float()
+    T = sum(rows)
+    q = torch.randn(T, H, 64, generator=g)
+    pos = torch.cat([torch.arange(n - m, n) for n, m in zip(lens, rows)])
+    slot = torch.tensor([r for r, m in enumerate(rows) for _ in range(m)])
+    i32 = lambda x: x.to(torch.int32).cuda()  # noqa: E731
+    got = ops.paged_attention_simt(q.cuda(), pool, pages.table.cuda(), i32(pos), i32(slot), 1, 0.125, window)
+    for r in range(len(rows)):
+        at = slice(sum(rows[:r]), sum(rows[:r + 1]))
+        want = attend(q[at].double(), pages.k[r].double(), pages.v[r].double(), pos[at], 0.125, window=window).reshape(rows[r], -1)
+        # scores of 64 products, sums of up to 300 terms, each rounded to 2^-24, exponentials to 2^-22
+        assert float((got[at].double().cpu() - want).norm() / want.norm()) < 2e-6
+    for part in (slice(0, 40), slice(7, 8), slice(36, 75), slice(100, T)):
+        one = ops.paged_attention_simt(q[part].cuda(), pool, pages.table.cuda(), i32(pos[part]), i32(slot[part]), 1, 0.125, window)
+        assert torch.equal(one, got[part])
