@@ -1,7 +1,7 @@
 // Causal GQA attention over the paged float32 cache, heads of 64, 1, 2 or 4 of them a kv head: the 32-bit engine's attention
 // of the LFM2 shapes, float32 arithmetic on CUDA cores.  What paged_attention_simt_kernel (attention_simt.cu) computes; there a
 // block is a (row, head), so every row and head reads its keys and values again, a lane a key (104 us for 201 rows of 16
-// heads behind 250 tokens each).
+// heads behind 250 tokens each; 44 here).
 //
 // Here a block of four warps takes a kv head and RB neighbouring rows: a tile of 32 keys is read once for its RB x R queries,
 // 8 lanes a key and 32 bytes a lane.  The partial dot products of a lane's eight keys go through the eight lanes by a

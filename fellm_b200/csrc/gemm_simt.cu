@@ -76,11 +76,13 @@ gemm_tn_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const fl
 }
 
 // All three float32, rows that start on 16 bytes and K a multiple of 4: the same chains, fed by cp.async through a ring of
-// FP_STAGES stages of 32 k.  A thread keeps 4 x 4 outputs whose rows and columns are TBM / 4 and TBN / 4 apart, and reads four
-// k of a row at a time (row stride 36 floats: the 8 rows of a quarter warp in different banks).  Bound by those reads: 32
-// floats from shared memory for 64 multiply-adds a thread.  The tile is the largest of 64 x 64, 32 x 64 and 16 x 32 whose
-// tiles fill the SMs (or the smallest): a kernel of 8 warps an SM with no loads in flight under its sums took 95 us for
-// [201, 2048, 1024] and as much for [201, 1024, 1024].
+// FP_STAGES stages of 32 k.  A thread keeps TM x TN outputs whose rows and columns are TBM / TM and TBN / TN apart, and reads
+// four k of a row at a time (row stride 36 floats: the 8 rows of a quarter warp in different banks).  Bound by those reads
+// where rows are many (4 x 4 outputs: 32 floats from shared memory for 64 multiply-adds) and by the warps' latency: 8 x 4
+// outputs a thread halve the warps and take 49 and 63 us where 4 x 4 take 48 ([201, 2048, 1024]) and 44 ([201, 1024, 1024]); the
+// kernel above, without loads in flight under its sums, takes 95 for either.  Tiles of 64 x 64 where they fill three
+// quarters of the SMs, of 32 x 64 where those fill half, else 16 x 32 and 8 x 32 with few outputs a thread: a product of a
+// decode step is a few chains of K dependent multiply-adds, and more warps walk them side by side.
 #define FP_STAGES 4
 #define FP_BK 32
 #define FP_LD 36
@@ -89,13 +91,13 @@ __device__ __forceinline__ void fp_copy16(float* dst, const float* src, bool liv
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
 }
 
-template <int TBM, int TBN, int EPI>
-__global__ void __launch_bounds__(TBM * TBN / 16)
+template <int TBM, int TBN, int TM, int TN, int EPI>
+__global__ void __launch_bounds__(TBM * TBN / (TN * TM))
 gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
                    float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
   FELLM_TRACE_SCOPE(TRACE_GEMM_SIMT);
   extern __shared__ __align__(16) float fp_smem[];
-  constexpr int THREADS = TBM * TBN / 16, TX = TBN / 4, TY = TBM / 4, STAGE = (TBM + TBN) * FP_LD;
+  constexpr int THREADS = TBM * TBN / (TN * TM), TX = TBN / TN, TY = TBM / TM, STAGE = (TBM + TBN) * FP_LD;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
   auto fetch = [&](int step) {
@@ -115,11 +117,11 @@ gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, con
     if (s < steps) fetch(s);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
-  float acc[4][4];
+  float acc[TM][TN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
   for (int s = 0; s < steps; ++s) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(FP_STAGES - 2) : "memory");
     __syncthreads();                               // this stage is here; the one before it is free
@@ -129,15 +131,15 @@ gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, con
     const float* Ws = fp_smem + (s % FP_STAGES) * STAGE + (TBM + tx) * FP_LD;
 #pragma unroll
     for (int k = 0; k < FP_BK; k += 4) {
-      float4 a[4], w[4];
+      float4 a[TM], w[TN];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = *(const float4*)(As + TY * i * FP_LD + k);
+      for (int i = 0; i < TM; ++i) a[i] = *(const float4*)(As + TY * i * FP_LD + k);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = *(const float4*)(Ws + TX * j * FP_LD + k);
+      for (int j = 0; j < TN; ++j) w[j] = *(const float4*)(Ws + TX * j * FP_LD + k);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {              // (each output's chain in the order of k)
+        for (int j = 0; j < TN; ++j) {              // (each output's chain in the order of k)
           acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]); acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
           acc[i][j] = fmaf(a[i].z, w[j].z, acc[i][j]); acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
         }
@@ -145,11 +147,11 @@ gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, con
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < TM; ++i) {
     const int gm = m0 + ty + TY * i;
     if (gm >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < TN; ++j) {
       const int gn = n0 + tx + TX * j;
       if (gn >= N) continue;
       float v = acc[i][j];
@@ -161,14 +163,14 @@ gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, con
   }
 }
 
-template <int TBM, int TBN>
+template <int TBM, int TBN, int TM, int TN>
 static int launch_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc, int epi,
                       cudaStream_t s) {
-  auto kern = epi == 2 ? gemm_tn_f32_kernel<TBM, TBN, 2> : epi ? gemm_tn_f32_kernel<TBM, TBN, 1> : gemm_tn_f32_kernel<TBM, TBN, 0>;
+  auto kern = epi == 2 ? gemm_tn_f32_kernel<TBM, TBN, TM, TN, 2> : epi ? gemm_tn_f32_kernel<TBM, TBN, TM, TN, 1> : gemm_tn_f32_kernel<TBM, TBN, TM, TN, 0>;
   const int smem = FP_STAGES * (TBM + TBN) * FP_LD * (int)sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  kern<<<dim3(ceil_div(N, TBN), ceil_div(M, TBM)), TBM * TBN / 16, smem, s>>>(A, W, bias, C, M, N, K, lda, ldw, ldc);
+  kern<<<dim3(ceil_div(N, TBN), ceil_div(M, TBM)), TBM * TBN / (TN * TM), smem, s>>>(A, W, bias, C, M, N, K, lda, ldw, ldc);
   return launch_status();
 }
 
@@ -197,9 +199,10 @@ FELLM_API int fellm_gemm_simt(const void* A, int a_dt, const void* W, int w_dt, 
     const float *a = (const float*)A, *w = (const float*)W;
     int sms = 0, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    if (M > 32 && (long long)ceil_div(N, 64) * ceil_div(M, 64) >= sms * 3 / 4) return launch_f32<64, 64>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
-    if (M > 16 && (long long)ceil_div(N, 64) * ceil_div(M, 32) >= sms / 2) return launch_f32<32, 64>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
-    return launch_f32<16, 32>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
+    if (M > 32 && (long long)ceil_div(N, 64) * ceil_div(M, 64) >= sms * 3 / 4) return launch_f32<64, 64, 4, 4>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
+    if (M > 16 && (long long)ceil_div(N, 64) * ceil_div(M, 32) >= sms / 2) return launch_f32<32, 64, 4, 4>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
+    if (M > 8) return launch_f32<16, 32, 2, 2>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
+    return launch_f32<8, 32, 2, 1>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
   }
   switch (key) {
     case 0: return launch_epi<float, float, float>(A, W, bias, C, M, N, K, lda, ldw, ldc, epi, s);

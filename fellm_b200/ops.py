@@ -1195,7 +1195,7 @@ def paged_attention_simt(q, pool, block_table, positions, row_slot, layer, scale
     if (hd == 64 and H // G in (1, 2, 4) and q.dtype == pool.dtype == torch.float32 and out.dtype == torch.float32
             and not (q.data_ptr() | pool.data_ptr()) % 16):
         # heads of 64: neighbouring rows share the reading of their keys (201 rows of 16 heads behind 250 tokens: 104 us in the
-        # kernel below)
+        # kernel below, 44 there)
         f = _fn("attention_f32", "fellm_attention_f32",
                 [_c_p, _c_int, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p] + [_c_int] * 7 + [_c_f, _c_int, _c_p])
         _check(f(_p(q), H * hd, _p(pool), _p(block_table), block_table.shape[1], _p(positions), _p(row_slot), _p(out), T, H, G, hd,
