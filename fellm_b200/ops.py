@@ -492,7 +492,7 @@ def conv_product_takes(M: int, N: int, K: int, taps: int) -> bool:
     key = (M, N, K, taps)
     hit = _conv_takes_cache.get(key)
     if hit is None:
-        if M <= 16 and not _swap_rows(M, N, K):
+        if M <= 16:
             f = _fn("gemm_skinny", "fellm_gemm_skinny_conv_takes", [_c_int, _c_int, _c_int, _c_int])
             hit = bool(f(M, N, K, taps))
         else:
@@ -501,7 +501,7 @@ def conv_product_takes(M: int, N: int, K: int, taps: int) -> bool:
             # width 2048 (64 rows) 1.298 -> 1.318 ms: tiles of 96 rows cost the wider product more than the launch saves;
             # at 96 and 128 rows the two ways lie within 2% of each other (width 1024: 1.061 / 1.065 and 1.283 / 1.271
             # ms; width 1536: 1.289 / 1.264 and 1.580 / 1.543 ms), so the kernel of its own stays there
-            hit = bool(_swap_rows(M, N, K) and FUSE_SWAP_CONV and M <= SWAP_CONV_MAX_ROWS and K <= SWAP_CONV_MAX_K and f(M, N, K, taps))
+            hit = bool(_swap_rows(M, N) and FUSE_SWAP_CONV and M <= SWAP_CONV_MAX_ROWS and K <= SWAP_CONV_MAX_K and f(M, N, K, taps))
         _conv_takes_cache[key] = hit
     return hit
 
@@ -523,10 +523,10 @@ def gemm_bf16_conv(x, w_blocked, bias, conv_w, conv_bias, state, row_slot, *, no
     if out is None:
         out = torch.empty((M, d), dtype=torch.bfloat16, device=x.device)
     assert out.dtype == torch.bfloat16 and out.stride(1) == 1
-    if M > 16 or _swap_rows(M, N, K):
-        # the tcgen05 product of few rows (up to 64 of them), the convolution in its owners' epilogue
+    if M > 16:
+        # 17..64 requests: the tcgen05 product of few rows, the convolution in its owners' epilogue
         if norm is not None or x.dtype != torch.bfloat16:
-            raise KernelError("gemm_bf16_conv: the tcgen05 product takes bfloat16 rows (normed before, or a handed-on norm's)")
+            raise KernelError("gemm_bf16_conv: more than 16 rows take bfloat16 rows (normed before, or a handed-on norm's)")
         if not conv_product_takes(M, N, K, taps):
             raise KernelError(f"gemm_bf16_conv does not take a product of {M} x {N} x {K} with {taps} taps")
         if row_scale is not None:
@@ -1497,8 +1497,6 @@ FUSE_SWAP_CONV = os.environ.get("FELLM_B200_FUSE_SWAP_CONV", "1") != "0"     # t
 SWAP_CONV_MAX_K = int(os.environ.get("FELLM_B200_SWAP_CONV_MAX_K", 1536))
 SWAP_CONV_MAX_ROWS = int(os.environ.get("FELLM_B200_SWAP_CONV_MAX_ROWS", 64))
 SWAP_MIN_ROWS = int(os.environ.get("FELLM_B200_SWAP_MIN_ROWS", 17))     # fewer rows: the weight-streaming kernel (norm and convolution fused)
-SWAP_ODD_MIN_ROWS = int(os.environ.get("FELLM_B200_SWAP_ODD_MIN_ROWS", 2))      # the same for widths of no power of two of K slices (_swap_from)
-SWAP_WIDE_MIN_ROWS = int(os.environ.get("FELLM_B200_SWAP_WIDE_MIN_ROWS", 9))    # and for widths of 2048 and more
 SWAP_MAX_ROWS = int(os.environ.get("FELLM_B200_SWAP_MAX_ROWS", 128))     # more rows: the persistent tcgen05 product (width 1024, 128 rows: 1.68 ms a step there, 1.28 here)
 SWAP_MAX_N = 16384                                                       # wider (the vocabulary head): the persistent tcgen05 product
 
@@ -1610,7 +1608,7 @@ def _single_shot(M: int, N: int, K: int, norm: bool) -> bool:
 # into x is followed by an RMSNorm with weights g"; norm_handoff(x, g) gives the reader what was left, if
 # it is still good (same tensor, same weights, nothing written to x since).
 NORM_HANDOFF = os.environ.get("FELLM_B200_NORM_HANDOFF", "1") != "0"
-HANDOFF_MAX_ROWS = 128       # up to 16 rows: the weight-streaming kernel on both sides; up to 128, where _swap_rows says so: the tcgen05 product of few rows
+HANDOFF_MAX_ROWS = 128       # up to 16 rows: the weight-streaming kernel on both sides; 17..128: the tcgen05 product of few rows
 _handoff_bufs = {}          # device -> (xg bfloat16 [16 * width], ssq float32 [16 * width / 16], width)
 _handoff_retired = []
 _expected_norm = None       # (data_ptr of x, norm weights)
@@ -1673,41 +1671,19 @@ def norm_handoff(x, norm_w):
     return h
 
 
-def _swap_from(N: int, K: int) -> int:
-    """The fewest rows that a [N, K] product gives to the tcgen05 product of few rows; fewer stay with the weight-streaming
-    kernel.  By the model's width, the smaller extent of its matrices, so that the products of a step agree and a norm can be
-    handed on among them.  The weight-streaming kernel cuts K into slices of 8..10 chunks of 32 and puts a power of two of them
-    into a block: a width that is no power of two of such slices (1536: six) leaves it with clusters of three that are not
-    resident together, one of 2048 with twice the instructions from nine rows on (its MMA holds eight).  Decode steps of 16
-    layers on B200, there and here: width 1536 4 rows 0.699 and 0.623 ms, 8 rows 0.706 and 0.637, 16 rows 0.882 and 0.606 (1 row
-    0.624 and 0.613); width 2048 8 rows 0.818 and 0.855, 12 rows 0.867 and 0.829, 16 rows 0.878 and 0.828; width 1024 16 rows
-    0.415 there, 17 rows 0.442 here."""
-    width = min(N, K)
-    if width > 1024:
-        chunks = width // 32
-        if width % 32 or not any(8 <= chunks / (1 << i) <= 10 and chunks % (1 << i) == 0 for i in range(8)):
-            return min(SWAP_ODD_MIN_ROWS, SWAP_MIN_ROWS)
-        if width >= 2048:
-            return min(SWAP_WIDE_MIN_ROWS, SWAP_MIN_ROWS)
-    return SWAP_MIN_ROWS
+def _swap_rows(M: int, N: int) -> bool:
+    """Whether gemm_bf16 gives a product of M rows and N columns to the tcgen05 product of few rows."""
+    return USE_UMMA and USE_UMMA_SWAP and max(SWAP_MIN_ROWS, 17) <= M <= SWAP_MAX_ROWS and N <= SWAP_MAX_N
 
 
-def _swap_rows(M: int, N: int, K: int) -> bool:
-    """Whether gemm_bf16 gives a product of M rows with an [N, K] matrix to the tcgen05 product of few rows."""
-    return USE_UMMA and USE_UMMA_SWAP and _swap_from(N, K) <= M <= SWAP_MAX_ROWS and N <= SWAP_MAX_N
-
-
-few_rows_on_umma = _swap_rows
-
-
-def row_scale_takes(M: int, N: int, K: int, parts=None) -> bool:
-    """Whether a product of these sizes can take a handed-on norm's input (left in `parts` sums a row): the single-shot
-    weight-streaming kernel takes sums of 16 columns, the tcgen05 product of few rows sums of 128."""
+def row_scale_takes(M: int, N: int, K: int) -> bool:
+    """Whether a product of these sizes can take a handed-on norm's input: up to 16 rows the single-shot
+    weight-streaming kernel, 17..128 rows the tcgen05 product of few rows."""
     if K % 8:
         return False
-    if _swap_rows(M, N, K):
-        return parts is None or (K % 128 == 0 and parts == K // 128)
-    return M <= 16 and (parts is None or (K % 16 == 0 and parts == K // 16)) and _single_shot(M, N, K, False)
+    if M <= 16:
+        return _single_shot(M, N, K, False)
+    return _swap_rows(M, N)
 
 
 def _announce_handoff(exp, out, M: int, N: int, K: int, norm_fused: bool):
@@ -1716,14 +1692,14 @@ def _announce_handoff(exp, out, M: int, N: int, K: int, norm_fused: bool):
     global _handoff
     if exp is None or M > HANDOFF_MAX_ROWS or not out.is_contiguous() or norm_fused:
         return
-    if _swap_rows(M, N, K):
-        if N % 128:
-            return
-        module, per_part = "gemm_umma", 128
-    else:
-        if M > 16 or N % 16 or not _single_shot(M, N, K, False):
+    if M <= 16:
+        if N % 16 or not _single_shot(M, N, K, False):
             return
         module, per_part = "gemm_skinny", 16
+    else:
+        if N % 128 or not _swap_rows(M, N):
+            return
+        module, per_part = "gemm_umma", 128
     xg, ssq, width = _handoff_bufs[out.device]
     _handoff = None                      # the buffers are about to be rewritten
     f = _fn(module, f"fellm_{module}_next_norm", [_c_p, _c_p, _c_int, _c_p])
@@ -1739,7 +1715,7 @@ def _announce_row_scale(row_scale, M: int, N: int, K: int, own_plan: bool = Fals
     if not own_plan and not row_scale_takes(M, N, K):
         raise KernelError(f"a product of {M} x {N} x {K} does not take a handed-on norm")
     assert ssq.dtype == torch.float32 and ssq.numel() >= M * parts
-    module = "gemm_umma" if M > 16 or _swap_rows(M, N, K) else "gemm_skinny"
+    module = "gemm_skinny" if M <= 16 else "gemm_umma"
     _fn(module, f"fellm_{module}_row_scale", [_c_p, _c_int, _c_f])(_p(ssq), int(parts), float(eps))
 
 
@@ -1800,12 +1776,12 @@ def gemm_bf16(x, w, bias=None, *, out=None, out_dtype=None, accumulate=False, sw
     # (measured at 64 rows: 14 us against 26 us for [1024, 4608], 8 against 9-11 for K = 1024, but 13
     # against 11 for the 9216 rows of gate/up, which stays with tcgen05 beyond 32 rows)
     expected = residual_written(out) if accumulate else None
-    if umma_ok and _swap_rows(M, N, K):
-        # a decode step of few rows: tcgen05 with the weights as the MMA's 128 rows.  It asks for no next matrix: its own
-        # stream is short of bandwidth, not of latency (a step of 2..16 rows at width 1536 3-6% longer with it, at 2048 10%)
+    if umma_ok and USE_UMMA_SWAP and SWAP_MIN_ROWS <= M <= SWAP_MAX_ROWS and N <= SWAP_MAX_N and (row_scale is None or M > 16):
+        # a decode step of 17..128 rows: tcgen05 with the weights as the MMA's 128 rows
+        _announce_next("gemm_umma", w, M)
         if row_scale is not None:
             _announce_row_scale(row_scale, M, N, K)
-        left = _announce_handoff(expected, out, M, N, K, False)
+        left = _announce_handoff(expected, out, M, N, K, False) if M > 16 else None
         gemm_umma_swap(x, w, bias, out=out, epi=epi, written=True)
         if left is not None:
             _handoff = left
@@ -1819,7 +1795,7 @@ def gemm_bf16(x, w, bias=None, *, out=None, out_dtype=None, accumulate=False, sw
         _announce_next("gemm_skinny", w, M)
         if row_scale is not None:
             _announce_row_scale(row_scale, M, N, K)
-        left = _announce_handoff(expected, out, M, N, K, norm is not None) if M <= 16 and not _swap_rows(M, N, K) else None
+        left = _announce_handoff(expected, out, M, N, K, norm is not None) if M <= 16 else None
         f = _fn("gemm_skinny", "fellm_gemm_skinny", _SKINNY_ARGS)
         if norm is not None:
             code = f(None, _p(x), _p(norm[0]), float(norm[1]), _p(w), _p(bias), _p(out), epi, M, N, K, x.stride(0),

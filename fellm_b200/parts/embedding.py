@@ -55,7 +55,7 @@ class LinearHead(Head):
             return False                 # (a positive scale and the soft cap keep the order of a row's logits)
         rows = xf.shape[0]
         h = xf.handed_on() if isinstance(xf, LazyNorm) else None
-        if h is not None and ops.row_scale_takes(rows, w.shape[0], w.shape[1], h.parts):
+        if h is not None and ops.row_scale_takes(rows, w.shape[0], w.shape[1]):
             need = ops.head_argmax_scratch(rows, w.shape[0], w.shape[1], False)
             if need and need <= keys.numel():
                 ops.gemm_bf16_argmax(h.xg, w, None, keys, out_tokens, row_scale=(h.ssq, h.parts, xf.norm.eps))

@@ -52,7 +52,7 @@ def linear(x, w, bias=None, *, out=None, out_dtype=None, accumulate=False, swigl
     if isinstance(x, LazyNorm):
         h = x.handed_on()
         if (h is not None and ops.fast_gemm_takes(h.xg, w) and w.data_ptr() % 16 == 0
-                and ops.row_scale_takes(h.rows, w.shape[0], w.shape[1], h.parts)
+                and ops.row_scale_takes(h.rows, w.shape[0], w.shape[1])
                 and not (swiglu and out is not None and out.stride(0) % 8)):
             return ops.gemm_bf16(h.xg, w, bias, out=out, out_dtype=out_dtype, accumulate=accumulate, swiglu=swiglu, act=act,
                                  row_scale=(h.ssq, h.parts, x.norm.eps))

@@ -60,13 +60,10 @@ class ShortConv(Mixer):
         if self.blocked and FUSE_DECODE_CONV and ctx.all_single and ops.conv_product_takes(ctx.n_rows, 3 * self.size, self.size, self.taps):
             # a decode step: product and convolution in one launch
             h = xn.handed_on() if isinstance(xn, LazyNorm) else None
-            on_umma = ops.few_rows_on_umma(ctx.n_rows, 3 * self.size, self.size)
-            if h is not None and h.parts * (128 if on_umma else 16) != self.size:
-                h = None                 # left by the other kernel
             scale = None
             if h is not None:
                 x, norm, scale = h.xg, None, (h.ssq, h.parts, xn.norm.eps)
-            elif not on_umma and isinstance(xn, LazyNorm) and xn.fusable_with(w_in):
+            elif ctx.n_rows <= 16 and isinstance(xn, LazyNorm) and xn.fusable_with(w_in):
                 x, norm = xn.x, (xn.norm.w["weight"], xn.norm.eps)
             else:
                 x, norm = (xn.tensor() if isinstance(xn, LazyNorm) else xn), None
