@@ -25,7 +25,7 @@ from ..weights.random_init import random_tensors
 from ..sampling.params import GenParams, GenStats
 from ..sampling.sampler import Sampler
 from .scheduler import Scheduler
-from .step import StepItem, Stepper
+from .step import FEW_ROWS_PAD, StepItem, Stepper
 
 
 def _require_gpu(device: str):
@@ -64,12 +64,14 @@ class Engine:
         self.cache = CacheManager(needs, page_tokens=options.page_tokens, max_tokens=max_tokens,
                                   max_requests=options.max_requests, n_ctx=n_ctx, dtype=cache_dtype,
                                   device=self.device)
-        max_rows = max(options.n_batch, options.n_ubatch) + options.max_requests
+        # (a decode step of few rows may be filled up to FEW_ROWS_PAD)
+        max_items = max(options.max_requests, FEW_ROWS_PAD)
+        max_rows = max(options.n_batch, options.n_ubatch) + max_items
         for part in self.model.all_parts():
-            part.reserve(self.device, options.max_requests, n_ctx)
+            part.reserve(self.device, max_items, n_ctx)
         from .. import ops
         ops.register_weight_chain(self.model.weight_chain())
-        self.stepper = Stepper(self.model, self.cache, max_rows=max_rows, max_items=options.max_requests,
+        self.stepper = Stepper(self.model, self.cache, max_rows=max_rows, max_items=max_items,
                                device=self.device, cuda_graphs=options.cuda_graphs)
         self._sampler: Optional[Sampler] = None
         # sampled tokens (and the status word behind them) come back through a few pinned buffers in

@@ -162,8 +162,30 @@ StepBuffers.fill_decode = _fill_decode
 
 _NOT_TAKEN = object()       # _step_decode's answer when the general path has to run the step (None is a result: tokens without logits)
 MAX_ROW_GRAPHS = 8          # captured graphs of steps that are not pure decode (each keeps its activations)
+FEW_ROWS_PAD = 24           # rows that a decode step of fewer than 17 is filled up to where the few-rows tcgen05 products are the faster ones
 DECODE_ROWS_STEP = 8        # decode steps of more than 16 rows run with a multiple of this many rows (the last ones padding)
 MAX_DECODE_GRAPHS = 48      # captured decode steps (each keeps its logits [wanted, vocab]); the least recently used goes
+
+
+def few_rows_pad_from(model) -> int:
+    """From how many rows a decode step runs on the few-rows tcgen05 products, filled up to FEW_ROWS_PAD rows (17: as any other).
+    Up to 16 rows the products stream their weights through mma.sync slabs, K in slices of 8..10 chunks of 32 and a power of two
+    of slices a block: a width that is no power of two of such slices (1536: six) leaves that kernel with clusters of three that
+    are not resident together, and from nine rows on it runs every instruction twice.  Decode steps of 16 LFM2 layers on B200,
+    there and filled up to 24 rows: PAD_FIGURES
+    Only models of attention, short convolutions and dense feed-forwards: rows that belong to nobody would send experts' matrices
+    and recurrent states through memory."""
+    plain = all(b.mixer.kind in ("attention", "shortconv") and b.ffn is not None and b.ffn.kind == "swiglu" for b in model.blocks)
+    width = model.spec.hidden_size
+    if not plain or width <= 1024 or width % 32 or model.act_dtype != torch.bfloat16:
+        return 17
+    chunks = width // 32
+    if not any(chunks % (1 << i) == 0 and 8 <= chunks >> i <= 10 for i in range(8)):
+        return FEW_ROWS_ODD
+    return FEW_ROWS_WIDE if width >= 2048 else 17
+
+
+FEW_ROWS_ODD, FEW_ROWS_WIDE = 2, 9
 
 
 class Stepper:
@@ -193,6 +215,7 @@ class Stepper:
         self.launches = 0                      # kernels of ours launched, replays included
         self._decode_plans = {}
         self._plan_serial = 0
+        self.pad_from = few_rows_pad_from(model)
 
     def step(self, items: List[StepItem], device_tokens: Optional[torch.Tensor] = None,
              greedy_tokens: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -290,8 +313,9 @@ class Stepper:
         # own, a state row of its own), so that a batch that grows or drains by one request at a time meets a
         # new graph every eighth count, not at every one.  Up to 16 rows each count has kernels of its own cost.
         n_pad = n
-        if self.cuda_graphs and n > 16 and all(wants):
-            n_pad = -(-n // DECODE_ROWS_STEP) * DECODE_ROWS_STEP
+        # Models whose products of few rows are faster on tcgen05 are filled up to FEW_ROWS_PAD from fewer rows on.
+        if self.cuda_graphs and n >= min(17, self.pad_from) and all(wants):
+            n_pad = -(-max(n, FEW_ROWS_PAD if n < 17 else n) // DECODE_ROWS_STEP) * DECODE_ROWS_STEP
             if n_pad > self.buffers.max_items:
                 n_pad = n
         key = key + (n_pad,)
