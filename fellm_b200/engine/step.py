@@ -172,7 +172,9 @@ def few_rows_pad_from(model) -> int:
     Up to 16 rows the products stream their weights through mma.sync slabs, K in slices of 8..10 chunks of 32 and a power of two
     of slices a block: a width that is no power of two of such slices (1536: six) leaves that kernel with clusters of three that
     are not resident together, and from nine rows on it runs every instruction twice.  Decode steps of 16 LFM2 layers on B200,
-    there and filled up to 24 rows: PAD_FIGURES
+    there and filled up to 24 rows: width 1536 1 row 0.628 ms there, 2 rows 0.668 and 0.618, 8 rows 0.705 and 0.619, 16 rows 0.885
+    and 0.625; width 2048 8 rows 0.824 there, 9 rows 0.894 and 0.833, 16 rows 0.883 and 0.835; width 1024 stays (16 rows 0.415, 17
+    rows as 24 0.454).
     Only models of attention, short convolutions and dense feed-forwards: rows that belong to nobody would send experts' matrices
     and recurrent states through memory."""
     plain = all(b.mixer.kind in ("attention", "shortconv") and b.ffn is not None and b.ffn.kind == "swiglu" for b in model.blocks)

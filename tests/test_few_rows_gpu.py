@@ -1,0 +1,50 @@
+"""Decode steps of few rows that are filled up to a count the tcgen05 products take (engine/step.py): the logits of the rows
+asked for, whatever was filled in, and no trace of the filling in the requests' caches."""
+from __future__ import annotations
+
+import types
+
+import pytest
+import torch
+
+
+def test_which_models_are_filled_up():
+    from fellm_b200.engine.step import few_rows_pad_from
+
+    def model(width, mixer="shortconv", ffn="swiglu", dtype=torch.bfloat16):
+        block = types.SimpleNamespace(mixer=types.SimpleNamespace(kind=mixer), ffn=types.SimpleNamespace(kind=ffn))
+        return types.SimpleNamespace(blocks=[block], spec=types.SimpleNamespace(hidden_size=width), act_dtype=dtype)
+    assert [few_rows_pad_from(model(w)) for w in (512, 768, 1024, 1152, 1280, 1536, 1792, 2048, 2304, 3072)] == [17, 17, 17, 17, 17, 2, 2, 9, 9, 2]
+    assert few_rows_pad_from(model(1536, ffn="moe")) == few_rows_pad_from(model(1536, mixer="gated_delta")) == 17
+    assert few_rows_pad_from(model(1536, dtype=torch.float32)) == 17
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 7, 16])
+def test_filled_up_steps_give_the_rows_own_logits(n):
+    from fellm_b200.config import EngineOptions
+    from fellm_b200.engine import Engine, StepItem
+    cfg = dict(architectures=["Lfm2ForCausalLM"], vocab_size=640, hidden_size=1536, num_hidden_layers=3, num_attention_heads=24,
+               num_key_value_heads=8, head_dim=64, full_attn_idxs=[1], block_ff_dim=512, block_auto_adjust_ff_dim=False,
+               rope_theta=10000.0, rope_pairing="split_half", conv_L_cache=3, conv_bias=False, norm_eps=1e-5, tie_word_embeddings=True,
+               max_position_embeddings=512)
+    engines = [Engine.random(cfg, 7, EngineOptions(n_ctx=256, max_requests=16, max_tokens=16 * 64, cuda_graphs=g)) for g in (True, False)]
+    g = torch.Generator().manual_seed(n)
+    prompts = [torch.randint(0, 640, (3 + 5 * r,), generator=g).tolist() for r in range(n)]
+    follow = torch.randint(0, 640, (n, 5), generator=g).tolist()
+    got = []
+    for e in engines:
+        for r in range(n):
+            e.add_request(r)
+            e.step([StepItem(r, prompts[r], [])])
+        out = [e.step([StepItem(r, [follow[r][t]], [0]) for r in range(n)]).double().cpu() for t in range(4)]
+        # behind the filled-up steps, some rows alone and without logits: what the filling left must not show
+        e.step([StepItem(r, [follow[r][4]], []) for r in range(n)])
+        out.append(e.step([StepItem(0, [1], [0])]).double().cpu())
+        e.check_status()
+        e.cache.audit()
+        got.append(out)
+    for a, b in zip(*got):
+        assert a.shape == b.shape and torch.isfinite(a).all()
+        # two kernels of the same bfloat16 operands: other orders of float32 sums, then roundings of activations
+        assert float((a - b).norm() / b.norm()) < 2e-2
