@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import weakref
 from typing import Optional
 
 import torch
@@ -1572,7 +1573,10 @@ def register_weight_chain(weights):
     is followed by the first: the next step).  Replaces what was registered before for these matrices."""
     ws = [w for w in weights if w is not None and w.dtype == torch.bfloat16 and w.is_cuda and w.is_contiguous()]
     for w, nxt in zip(ws, ws[1:] + ws[:1]):
-        _next_weight[w.data_ptr()] = (nxt.data_ptr(), min(nxt.numel() * 2, PREFETCH_MAX_BYTES))
+        at = w.data_ptr()
+        _next_weight[at] = (nxt.data_ptr(), min(nxt.numel() * 2, PREFETCH_MAX_BYTES))
+        # (a matrix that goes takes its entry along: another tensor may come to lie there, and what was next is gone as well)
+        weakref.finalize(w, _next_weight.pop, at, None)
 
 
 PREFETCH_MAX_ROWS = 16     # measured on B200: 2% off a step of 1 or 8 rows, 1-6% ON a step of 64 (its products are short of bandwidth, not of latency)

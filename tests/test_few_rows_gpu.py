@@ -28,7 +28,7 @@ def test_filled_up_steps_give_the_rows_own_logits(n):
                num_key_value_heads=8, head_dim=64, full_attn_idxs=[1], block_ff_dim=512, block_auto_adjust_ff_dim=False,
                rope_theta=10000.0, rope_pairing="split_half", conv_L_cache=3, conv_bias=False, norm_eps=1e-5, tie_word_embeddings=True,
                max_position_embeddings=512)
-    engines = [Engine.random(cfg, 7, EngineOptions(n_ctx=256, max_requests=16, max_tokens=16 * 64, cuda_graphs=g)) for g in (True, False)]
+    engines = [Engine.random(cfg, 7, EngineOptions(n_ctx=256, max_requests=16, max_tokens=16 * 128, cuda_graphs=g)) for g in (True, False)]
     g = torch.Generator().manual_seed(n)
     prompts = [torch.randint(0, 640, (3 + 5 * r,), generator=g).tolist() for r in range(n)]
     follow = torch.randint(0, 640, (n, 5), generator=g).tolist()
