@@ -594,76 +594,102 @@ moe_gemm_mma_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__
   }
 }
 
-// Few rows (a decode step): the product is bound by reading each chosen expert's matrix once.  A warp owns one
-// output column of a row tile (and, GATED, the column's up partner): it streams the column's weight row(s) 16 bytes a
-// lane at a time against up to VR rows of A at once (more rows: again, the weights then come from L1 / L2), the lanes'
-// sums are added by a butterfly.  bfloat16 only; K a multiple of 8.
+// Few rows (a decode step): the product is bound by reading each chosen expert's matrix once.  A warp takes a slab of 16 weight
+// rows (GATED: eight gate rows and their eight up rows) as the rows of mma.m16n8k16 and a slice of K; its columns are up to
+// eight rows of A (more rows: again, the weights then come from L2).  A lane loads 8 consecutive k of rows g and g + 8 and
+// feeds them, and the same k of A's row g, as the k slots {2c, 2c + 1, 2c + 8, 2c + 9} of two MMAs: 16-byte loads of both
+// operands without shared memory, and VU chunks of 32 k (VU KB of weights a warp) on their way at once.  The slices of K of a slab
+// are warps of one block, added in their order.  bfloat16 only; K a multiple of 8.
+// A warp a column and float32 FMA, four rows at once, spent its time on the conversions and multiply-adds of the weights it
+// streamed: 8 tokens, two of twelve choices each, width 1,024, experts of 3,328: 27.3 us (up) and 20.6 us (down) there, 15.4
+// and 9.7 here (82 and 41 MB of matrices met); 30 tokens 67 and 64 us there, 26 and 16 here.
 #define VW 8            // warps a block
-#define VR 4            // rows at once
-// A warp's columns: n and, GATED, its up partner; not gated: n and n + 1 (two weight rows against the same rows of A).
-template <typename TO, bool GATED>
+#define VU 8            // chunks of 32 k on their way
+template <typename TO, bool GATED, int KS>
 __global__ void __launch_bounds__(VW * 32)
 moe_gemv_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__ gather, int top,
                 const bf16* __restrict__ W, TO* __restrict__ C, int ldc, int N, int K,
                 const int* __restrict__ table, const int* __restrict__ n_tiles, int inter, float act_limit, float act_alpha) {
+  __shared__ float4 part[VW][32];
   if ((int)blockIdx.x >= *n_tiles) return;
   const int e = table[3 * blockIdx.x], row0 = table[3 * blockIdx.x + 1], rows = table[3 * blockIdx.x + 2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = GATED ? blockIdx.y * VW + warp : 2 * (blockIdx.y * VW + warp);
-  if (n >= N) return;
-  const bool two = !GATED && n + 1 < N;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  const int slab = blockIdx.y * (VW / KS) + warp / KS, ks = warp % KS;
+  const int n0 = slab * (GATED ? 8 : 16), na = n0 + g, nb = GATED ? na : na + 8;         // this lane's columns of the result
   const bf16* We = W + (size_t)e * (GATED ? 2 : 1) * N * K;
-  const bf16* w0 = We + (size_t)(GATED ? gate_row(n, inter) : n) * K;
-  const bf16* w1 = GATED ? We + (size_t)up_row(n, N, inter) * K : (two ? w0 + K : w0);
-  for (int r0 = 0; r0 < rows; r0 += VR) {
-    const bf16* ar[VR];
+  const bf16* wa = We + (size_t)(GATED ? gate_row(min(na, N - 1), inter) : min(na, N - 1)) * K;
+  const bf16* wb = We + (size_t)(GATED ? up_row(min(nb, N - 1), N, inter) : min(nb, N - 1)) * K;
+  const int chunks = (K + 31) / 32, per = (chunks + KS - 1) / KS, first = ks * per, last = n0 < N ? min(chunks, first + per) : 0;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int r0 = 0; r0 < rows; r0 += 8) {
+    const int r = row0 + r0 + g;
+    const bool live = r0 + g < rows;
+    const bf16* ar = nullptr;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c0 = first; c0 < last; c0 += VU) {
+      uint4 a[VU], b[VU], x[VU];
 #pragma unroll
-    for (int i = 0; i < VR; ++i) {
-      const int r = min(r0 + i, rows - 1);
-      ar[i] = A + (size_t)(gather ? gather[row0 + r] / top : row0 + r) * lda;
-    }
-    const int nr = min(VR, rows - r0);
-    float s0[VR], s1[VR];
-#pragma unroll
-    for (int i = 0; i < VR; ++i) s0[i] = s1[i] = 0.f;
-    // two steps of K at once: four 16-byte loads of weights in flight a lane before the first is used
-    for (int k = lane * 8; k < K; k += 512) {
-      const bool second = k + 256 < K;
-      const uint4 zero = make_uint4(0, 0, 0, 0);
-      const uint4 ra0 = *(const uint4*)(w0 + k), rb0 = *(const uint4*)(w1 + k);
-      const uint4 ra1 = second ? *(const uint4*)(w0 + k + 256) : zero, rb1 = second ? *(const uint4*)(w1 + k + 256) : zero;
-      uint4 xa[VR], xb[VR];
-#pragma unroll
-      for (int i = 0; i < VR; ++i) {
-        xa[i] = i < nr ? *(const uint4*)(ar[i] + k) : zero;
-        xb[i] = (i < nr && second) ? *(const uint4*)(ar[i] + k + 256) : zero;
+      for (int u = 0; u < VU; ++u) {
+        const int k = (c0 + u) * 32 + 8 * c;
+        const bool in = c0 + u < last && k < K;
+        a[u] = in ? *(const uint4*)(wa + k) : zero;
+        b[u] = in ? *(const uint4*)(wb + k) : zero;
       }
-      float f0[8], f1[8], g0[8], g1[8];
-      unpack8(ra0, f0); unpack8(rb0, f1); unpack8(ra1, g0); unpack8(rb1, g1);
+      if (!ar && live) ar = A + (size_t)(gather ? gather[r] / top : r) * lda;           // (behind the first weights)
 #pragma unroll
-      for (int i = 0; i < VR; ++i) {
-        float fa[8], fb[8];
-        unpack8(xa[i], fa); unpack8(xb[i], fb);
+      for (int u = 0; u < VU; ++u) {
+        const int k = (c0 + u) * 32 + 8 * c;
+        x[u] = (live && c0 + u < last && k < K) ? *(const uint4*)(ar + k) : zero;
+      }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { s0[i] = fmaf(fa[j], f0[j], s0[i]); s1[i] = fmaf(fa[j], f1[j], s1[i]); }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { s0[i] = fmaf(fb[j], g0[j], s0[i]); s1[i] = fmaf(fb[j], g1[j], s1[i]); }
+      for (int u = 0; u < VU; ++u) {
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                     : "+f"(s[0]), "+f"(s[1]), "+f"(s[2]), "+f"(s[3])
+                     : "r"(a[u].x), "r"(b[u].x), "r"(a[u].y), "r"(b[u].y), "r"(x[u].x), "r"(x[u].y));
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                     : "+f"(s[0]), "+f"(s[1]), "+f"(s[2]), "+f"(s[3])
+                     : "r"(a[u].z), "r"(b[u].z), "r"(a[u].w), "r"(b[u].w), "r"(x[u].z), "r"(x[u].w));
       }
     }
+    if (KS > 1) {
+      __syncthreads();                             // (the parts before these have been added)
+      part[warp][lane] = make_float4(s[0], s[1], s[2], s[3]);
+      __syncthreads();
+      if (ks == 0) {
 #pragma unroll
-    for (int i = 0; i < VR; ++i) {
-      float a = warp_sum(s0[i]), b = warp_sum(s1[i]);
-      if (lane == 0 && r0 + i < rows) {
+        for (int w = 1; w < KS; ++w) {
+          const float4 p = part[warp + w][lane];
+          s[0] += p.x; s[1] += p.y; s[2] += p.z; s[3] += p.w;
+        }
+      }
+    }
+    if (ks == 0) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {                // result rows 2 c and 2 c + 1
+        const int rr = r0 + 2 * c + j;
+        if (rr >= rows) continue;
+        TO* to = C + (size_t)(row0 + rr) * ldc;
         if (GATED) {
-          a = to_f(from_f<bf16>(a)); b = to_f(from_f<bf16>(b));
-          C[(size_t)(row0 + r0 + i) * ldc + n] = from_f<TO>(glu_act(a, b, act_limit, act_alpha));
+          if (na < N) to[na] = from_f<TO>(glu_act(to_f(from_f<bf16>(s[j])), to_f(from_f<bf16>(s[2 + j])), act_limit, act_alpha));
         } else {
-          C[(size_t)(row0 + r0 + i) * ldc + n] = from_f<TO>(a);
-          if (two) C[(size_t)(row0 + r0 + i) * ldc + n + 1] = from_f<TO>(b);
+          if (na < N) to[na] = from_f<TO>(s[j]);
+          if (nb < N) to[nb] = from_f<TO>(s[2 + j]);
         }
       }
     }
   }
+}
+
+template <typename TO, bool GATED>
+static int moe_gemv_launch(const void* A, int lda, const int* gather, int top, const void* W, void* C, int ldc, int N, int K, const int* table,
+                           const int* n_tiles, int max_tiles, int inter, float act_limit, float act_alpha, cudaStream_t stream) {
+  // slices of K of a slab: VU chunks each where there are eight of them or fewer
+  const int chunks = (K + 31) / 32, slabs = ceil_div(N, GATED ? 8 : 16);
+#define MOE_GEMV(KS_) moe_gemv_kernel<TO, GATED, KS_><<<dim3(max_tiles, ceil_div(slabs, VW / KS_)), VW * 32, 0, stream>>>((const bf16*)A, lda, gather, \
+        top, (const bf16*)W, (TO*)C, ldc, N, K, table, n_tiles, inter, act_limit, act_alpha)
+  if (chunks > 4 * VU) MOE_GEMV(8); else if (chunks > 2 * VU) MOE_GEMV(4); else if (chunks > VU) MOE_GEMV(2); else MOE_GEMV(1);
+#undef MOE_GEMV
+  return launch_status();
 }
 
 // A [*, lda] (bfloat16 or float32), W [E][(gated ? 2 : 1) * N][K] of the same kind; C [P, ldc]: bfloat16 or float32
@@ -677,12 +703,8 @@ FELLM_API int fellm_moe_gemm(const void* A, int a_bf16, int lda, const int* gath
   if (a_bf16 != w_bf16 || (!gated && c_bf16) || (gated && c_bf16 != a_bf16)) return FELLM_ERR_ARG;
   const bool mma = use_mma && a_bf16 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0;
   if (mma && few_rows) {
-    dim3 grid(max_tiles, gated ? (N + VW - 1) / VW : (N + 2 * VW - 1) / (2 * VW));
-    if (gated)
-      moe_gemv_kernel<bf16, true><<<grid, VW * 32, 0, stream>>>((const bf16*)A, lda, gather, top, (const bf16*)W, (bf16*)C, ldc, N, K, table, n_tiles, inter, act_limit, act_alpha);
-    else
-      moe_gemv_kernel<float, false><<<grid, VW * 32, 0, stream>>>((const bf16*)A, lda, gather, top, (const bf16*)W, (float*)C, ldc, N, K, table, n_tiles, inter, act_limit, act_alpha);
-    return launch_status();
+    return gated ? moe_gemv_launch<bf16, true>(A, lda, gather, top, W, C, ldc, N, K, table, n_tiles, max_tiles, inter, act_limit, act_alpha, stream)
+                 : moe_gemv_launch<float, false>(A, lda, gather, top, W, C, ldc, N, K, table, n_tiles, max_tiles, inter, act_limit, act_alpha, stream);
   }
   if (mma) {
     dim3 grid(max_tiles, (N + TB - 1) / TB);
