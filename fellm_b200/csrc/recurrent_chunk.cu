@@ -352,11 +352,16 @@ __device__ __forceinline__ void rk_mma1(float (&c)[4], const unsigned (&a)[4], u
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// c += a b: the small products in one sum, the large ones in another that starts at zero, joined by float32 additions, since
+// an MMA cuts its sum off where an addition rounds it
 __device__ __forceinline__ void rk_mma(float (&c)[4], const RkSplit (&a)[4], const RkSplit (&b)[2]) {
   const unsigned hi[4] = {a[0].hi, a[1].hi, a[2].hi, a[3].hi}, lo[4] = {a[0].lo, a[1].lo, a[2].lo, a[3].lo};
-  rk_mma1(c, lo, b[0].hi, b[1].hi);
-  rk_mma1(c, hi, b[0].lo, b[1].lo);
-  rk_mma1(c, hi, b[0].hi, b[1].hi);
+  float s[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f};
+  rk_mma1(s, lo, b[0].hi, b[1].hi);
+  rk_mma1(s, hi, b[0].lo, b[1].lo);
+  rk_mma1(l, hi, b[0].hi, b[1].hi);
+#pragma unroll
+  for (int x = 0; x < 4; ++x) c[x] += l[x] + s[x];
 }
 
 template <bool DELTA, int DK, int THREADS>
