@@ -169,14 +169,91 @@ static int launch(const bf16* A, const bf16* W, const float* bias, void* out, in
   return launch_status();
 }
 
+// ---------------------------------------------------------------- a product per head for a handful of rows
+// The same product for up to 32 rows.  The weights are all there is to read (16 heads of 256 x 64: 0.5 MB), so what a tile of
+// 128 rows costs is its ring and its idle rows: HG_T us at 8 rows, HG_N here.  A warp takes 16 weight rows of a head as the
+// MMA's first operand, straight from memory, and the rows of the input, eight at a time, as the second: lane c's four
+// consecutive k are its slots {2c, 2c+1, 2c+8, 2c+9} in both, so that an MMA covers the same 16 k as the tile's and follows
+// it in K: the sums are the tile's, bit for bit, and a row's result stays free of the batch.
+#define HW_WARPS 2
+#define HW_STEPS 8        // MMAs whose operands are in flight
+
+__device__ __forceinline__ uint2 weights8(const bf16* at) {
+  uint2 v;
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(at));
+  return v;
+}
+
+template <int RG>
+__global__ void __launch_bounds__(HW_WARPS * 32)
+gemm_heads_few_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, bf16* __restrict__ out, int M, int N, int K, int lda, int ldw,
+                      int ldo, long long sa, long long sw, long long so) {
+  FELLM_TRACE_SCOPE(TRACE_GEMM_TILED);
+  const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  const int n0 = (blockIdx.x * HW_WARPS + (threadIdx.x >> 5)) * 16, na = n0 + g, nb = na + 8;
+  if (n0 >= N) return;
+  const bf16* wa = W + blockIdx.y * sw + (size_t)min(na, N - 1) * ldw;
+  const bf16* wb = W + blockIdx.y * sw + (size_t)min(nb, N - 1) * ldw;
+  const bf16* a = A + blockIdx.y * sa;
+  float s[RG][4];
+#pragma unroll
+  for (int r = 0; r < RG; ++r)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) s[r][x] = 0.f;
+  const uint2 zero = make_uint2(0, 0);
+  for (int k0 = 4 * c; k0 < K + 4 * c; k0 += 16 * HW_STEPS) {
+    uint2 p[HW_STEPS], q[HW_STEPS], x[RG][HW_STEPS];
+#pragma unroll
+    for (int u = 0; u < HW_STEPS; ++u) {
+      const int k = k0 + 16 * u;
+      p[u] = k < K ? weights8(wa + k) : zero;
+      q[u] = k < K ? weights8(wb + k) : zero;
+    }
+    if (k0 == 4 * c) { pdl_launch_dependents(); pdl_wait(); FELLM_TRACE_WAITED(); }      // the first weights are asked for in front of it
+#pragma unroll
+    for (int u = 0; u < HW_STEPS; ++u) {
+      const int k = k0 + 16 * u;
+#pragma unroll
+      for (int r = 0; r < RG; ++r) x[r][u] = (k < K && 8 * r + g < M) ? *(const uint2*)(a + (size_t)(8 * r + g) * lda + k) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < HW_STEPS; ++u)
+#pragma unroll
+      for (int r = 0; r < RG; ++r)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                     : "+f"(s[r][0]), "+f"(s[r][1]), "+f"(s[r][2]), "+f"(s[r][3])
+                     : "r"(p[u].x), "r"(q[u].x), "r"(p[u].y), "r"(q[u].y), "r"(x[r][u].x), "r"(x[r][u].y));
+  }
+#pragma unroll
+  for (int r = 0; r < RG; ++r)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int t = 8 * r + 2 * c + j;
+      if (t >= M) continue;
+      bf16* to = out + (size_t)t * ldo + blockIdx.y * so;
+      if (na < N) to[na] = from_f<bf16>(s[r][j]);
+      if (nb < N) to[nb] = from_f<bf16>(s[r][2 + j]);
+    }
+}
+
 // A batch of such products in one launch (the heads of a layer, each with a matrix of its own, on column blocks of
 // the same rows): member b computes C_b[M, N] = A_b[M, K] W_b[N, K]^T with A_b = A + b sa, W_b = W + b sw,
 // C_b = C + b sc (strides in elements; bfloat16 in and out).
 FELLM_API int fellm_gemm_tiled_batched(const void* A, const void* W, void* out, int batch, int M, int N, int K, int lda,
-                                       int ldw, int ldo, long long sa, long long sw, long long so, cudaStream_t stream) {
+                                       int ldw, int ldo, long long sa, long long sw, long long so, int few_rows, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (!A || !W || !out || K <= 0) return FELLM_ERR_ARG;
   if ((K % 8) || (lda % 8) || (ldw % 8) || (sa % 8) || (sw % 8) || batch > 65535) return FELLM_ERR_SIZE;
+  if (M <= few_rows) {
+    const dim3 slabs(ceil_div(N, 16 * HW_WARPS), batch);
+#define HEADS_FEW(RG_) return launch_k_class(1, gemm_heads_few_kernel<RG_>, slabs, dim3(HW_WARPS * 32), 0, stream, 1, (const bf16*)A, (const bf16*)W, \
+        (bf16*)out, M, N, K, lda, ldw, ldo, sa, sw, so)
+    if (M <= 8) HEADS_FEW(1);
+    if (M <= 16) HEADS_FEW(2);
+    if (M <= 32) HEADS_FEW(4);
+    return FELLM_ERR_SIZE;
+#undef HEADS_FEW
+  }
   size_t smem = (size_t)TSTAGES * (TBM + TBN) * 4 * sizeof(uint4);
   auto kern = gemm_tiled_kernel<EPI_STORE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -428,9 +428,9 @@ def head_gemm(a, w, out, *, a_head: int, out_head: int):
     if (_is_bf16(a) and _is_bf16(w) and _is_bf16(out) and K % 8 == 0 and a_head % 8 == 0 and a.stride(0) % 8 == 0
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and HEAD_GEMM_MMA):
         f = _fn("gemm_tiled", "fellm_gemm_tiled_batched", [_c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
-                                                           _c_ll, _c_ll, _c_ll, _c_p])
-        _check(f(_p(a), _p(w), _p(out), H, T, N, K, a.stride(0), K, out.stride(0), int(a_head), N * K, int(out_head), _stream()),
-               "head_gemm (tensor cores)")
+                                                           _c_ll, _c_ll, _c_ll, _c_int, _c_p])
+        _check(f(_p(a), _p(w), _p(out), H, T, N, K, a.stride(0), K, out.stride(0), int(a_head), N * K, int(out_head), HEAD_GEMM_FEW_ROWS,
+                 _stream()), "head_gemm (tensor cores)")
         return out
     f = _fn("gemm_simt", "fellm_gemm_simt_batched", [_c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                      _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_p])
@@ -440,6 +440,7 @@ def head_gemm(a, w, out, *, a_head: int, out_head: int):
 
 
 TOKEN_SIDE_MMA = os.environ.get("FELLM_B200_TOKEN_SIDE_MMA", "1") != "0"
+HEAD_GEMM_FEW_ROWS = 32
 HEAD_GEMM_MMA = os.environ.get("FELLM_B200_HEAD_GEMM_MMA", "1") != "0"
 
 
