@@ -180,12 +180,6 @@ static int launch(const bf16* A, const bf16* W, const float* bias, void* out, in
 #define HW_WARPS 2
 #define HW_STEPS 8        // MMAs whose operands are in flight
 
-__device__ __forceinline__ uint2 weights8(const bf16* at) {
-  uint2 v;
-  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(at));
-  return v;
-}
-
 template <int RG>
 __global__ void __launch_bounds__(HW_WARPS * 32)
 gemm_heads_few_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, bf16* __restrict__ out, int M, int N, int K, int lda, int ldw,
@@ -208,13 +202,8 @@ gemm_heads_few_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, bf
 #pragma unroll
     for (int u = 0; u < HW_STEPS; ++u) {
       const int k = k0 + 16 * u;
-      p[u] = k < K ? weights8(wa + k) : zero;
-      q[u] = k < K ? weights8(wb + k) : zero;
-    }
-    if (k0 == 4 * c) { pdl_launch_dependents(); pdl_wait(); FELLM_TRACE_WAITED(); }      // the first weights are asked for in front of it
-#pragma unroll
-    for (int u = 0; u < HW_STEPS; ++u) {
-      const int k = k0 + 16 * u;
+      p[u] = k < K ? *(const uint2*)(wa + k) : zero;
+      q[u] = k < K ? *(const uint2*)(wb + k) : zero;
 #pragma unroll
       for (int r = 0; r < RG; ++r) x[r][u] = (k < K && 8 * r + g < M) ? *(const uint2*)(a + (size_t)(8 * r + g) * lda + k) : zero;
     }
@@ -248,8 +237,8 @@ FELLM_API int fellm_gemm_tiled_batched(const void* A, const void* W, void* out, 
   if ((K % 8) || (lda % 8) || (ldw % 8) || (sa % 8) || (sw % 8) || batch > 65535) return FELLM_ERR_SIZE;
   if (M <= few_rows) {
     const dim3 slabs(ceil_div(N, 16 * HW_WARPS), batch);
-#define HEADS_FEW(RG_) return launch_k_class(1, gemm_heads_few_kernel<RG_>, slabs, dim3(HW_WARPS * 32), 0, stream, 1, (const bf16*)A, (const bf16*)W, \
-        (bf16*)out, M, N, K, lda, ldw, ldo, sa, sw, so)
+#define HEADS_FEW(RG_) return launch_k(gemm_heads_few_kernel<RG_>, slabs, dim3(HW_WARPS * 32), 0, stream, 1, (const bf16*)A, (const bf16*)W, (bf16*)out, \
+        M, N, K, lda, ldw, ldo, sa, sw, so)
     if (M <= 8) HEADS_FEW(1);
     if (M <= 16) HEADS_FEW(2);
     if (M <= 32) HEADS_FEW(4);
