@@ -76,8 +76,7 @@ template <bool DELTA, int DK>
 struct RkImage {
   static constexpr int NR = DELTA ? 2 * RK_C : RK_C;          // rows of the product with the state: W above Q, or Q alone
   static constexpr int AP = DK + 4;                           // their stride: eight rows' 16 bytes in different banks
-  static constexpr int KP = DK + 8;                           // stride of the rows of K: four rows' eight elements in different banks
-  static constexpr int A = 0, K = A + NR * AP, M = K + RK_C * KP, P = M + RK_C * RK_LP, FLOATS = P + DK;
+  static constexpr int A = 0, K = A + NR * AP, M = K + RK_C * DK, P = M + RK_C * RK_LP, FLOATS = P + DK;
 };
 
 // ---------------------------------------------------------------- prep
@@ -280,7 +279,7 @@ rk_prep_kernel(const RkArgs a) {
   for (int x = tid * 4; x < RK_C * DK; x += RK_THREADS * 4) {
     const int t = x / DK, i = x - t * DK;
     *(float4*)(img + I::A + (t + I::NR - RK_C) * I::AP + i) = *(const float4*)(B + x);
-    *(float4*)(img + I::K + t * I::KP + i) = *(const float4*)(KK + x);
+    *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
   }
   for (int x = tid * 4; x < RK_C * RK_LP; x += RK_THREADS * 4) *(float4*)(img + I::M + x) = *(const float4*)(Mm + x);
 
@@ -324,212 +323,177 @@ __device__ __forceinline__ void rk_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-// Two groups of DK / 16 warps.  The first walks the state: W S, U = U0 - W S, S = P S + K^T U; the second makes the
+// Two groups of eight warps.  The first walks the state: W S, U = U0 - W S, S = P S + K^T U; the second makes the
 // outputs, Q S + M U, from the state in front of the chunk as it lies in shared memory and the first group's U: what the
-// outputs cost runs beside the chain and not in it.
-//
-// The products with the state and the state's update run on mma.m16n8k8.tf32, every operand in two parts (x = hi + lo, each
-// rounded to the nearest tf32, 22 of 24 bits; lo lo, 2^-24 of a product, is left out) and float32 sums: three MMAs for one.
-// What that buys is the reads: a fragment's element is read by one lane, where a lane's own tile of 4 x 4 results read a
-// register from shared memory for every two multiply-adds (188 us a walk there, WALK_US here).  Against float64 the results
-// are as near as with float32 multiply-adds: RK_ERR.
-// M U stays in float32 multiply-adds: its masked pairs are skipped, not multiplied by zero.
-#define RK_PP (RK_NV + 8)  // row stride of the partial sums
-#define RK_UP (RK_NV + 8)  // row stride of U
-#define RK_SP 20           // column stride of a warp's part of the state
+// outputs cost runs beside the chain and not in it, and sixteen warps hide each other's waits.
+#define RK_WALK_THREADS 512
+#define RK_PP (RK_NV + 4)  // row stride of the partial sums
 
 __device__ __forceinline__ void rk_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void rk_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-struct RkSplit { unsigned hi, lo; };
-__device__ __forceinline__ RkSplit rk_split(float x) {
-  RkSplit r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r.hi) : "f"(x));
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r.lo) : "f"(x - __uint_as_float(r.hi)));
-  return r;
-}
-__device__ __forceinline__ void rk_mma1(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// c += a b: the small products in one sum, the large ones in another that starts at zero, joined by float32 additions, since
-// an MMA cuts its sum off where an addition rounds it
-__device__ __forceinline__ void rk_mma(float (&c)[4], const RkSplit (&a)[4], const RkSplit (&b)[2]) {
-  const unsigned hi[4] = {a[0].hi, a[1].hi, a[2].hi, a[3].hi}, lo[4] = {a[0].lo, a[1].lo, a[2].lo, a[3].lo};
-  float s[4] = {0.f, 0.f, 0.f, 0.f}, l[4] = {0.f, 0.f, 0.f, 0.f};
-  rk_mma1(s, lo, b[0].hi, b[1].hi);
-  rk_mma1(s, hi, b[0].lo, b[1].lo);
-  rk_mma1(l, hi, b[0].hi, b[1].hi);
-#pragma unroll
-  for (int x = 0; x < 4; ++x) c[x] += l[x] + s[x];
-}
-
-template <bool DELTA, int DK, int THREADS>
+template <bool DELTA, int DK>
 __device__ __forceinline__ void rk_fetch(const RkArgs& a, float* buf, size_t cell, int tile, int tid) {
   using I = RkImage<DELTA, DK>;
   const float* img = a.image + cell * I::FLOATS;
 #pragma unroll
-  for (int x = 4 * tid; x < I::FLOATS; x += 4 * THREADS) rk_copy16(buf + x, img + x);
+  for (int x = 4 * tid; x < I::FLOATS; x += 4 * RK_WALK_THREADS) rk_copy16(buf + x, img + x);
   const float* Ug = a.U + cell * ((size_t)RK_C * a.dv) + (size_t)tile * (RK_C * RK_NV);
-  if (tid < RK_C * RK_NV / 4) rk_copy16(buf + I::FLOATS + (tid >> 2) * RK_UP + (tid & 3) * 4, Ug + 4 * tid);
+  if (tid < RK_C * RK_NV / 4) rk_copy16(buf + I::FLOATS + 4 * tid, Ug + 4 * tid);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-// 32 rows (at A, stride AP, this warp's 16 key rows) times the state's 16 key rows (at Sw [16 columns][RK_SP]); the sums go to
-// part [32][RK_PP].
-template <int AP>
-__device__ __forceinline__ void rk_rows_by_state(const float* A, const float* Sw, float* part, int g, int c) {
-  float acc[2][2][4];
+// 32 rows (at A, stride AP) times the state, over a warp's KW key rows: a lane rows rg + 8 m, columns 4 cg + x; pairs of
+// key rows an operation.  The sums go to part [32][RK_PP].
+template <int KW, int AP>
+__device__ __forceinline__ void rk_rows_by_state(const float* A, const float* Sw, float* part, int rg, int cg) {
+  constexpr int GM = KW / 4 - 1;
+  unsigned long long acc[4][4];
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int m = 0; m < 4; ++m)
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+    for (int x = 0; x < 4; ++x) acc[m][x] = 0ull;
+  A += rg * AP;
 #pragma unroll
-      for (int x = 0; x < 4; ++x) acc[m][n][x] = 0.f;
+  for (int kk = 0; kk < KW / 4; ++kk) {
+    ulonglong2 sv[4];
 #pragma unroll
-  for (int k = 0; k < 16; k += 8) {
-    RkSplit b[2][2];
+    for (int x = 0; x < 4; ++x) sv[x] = *(const ulonglong2*)(Sw + (4 * cg + x) * KW + 4 * (kk ^ (cg & GM)));
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      b[n][0] = rk_split(Sw[(8 * n + g) * RK_SP + k + c]);
-      b[n][1] = rk_split(Sw[(8 * n + g) * RK_SP + k + c + 4]);
-    }
+    for (int m = 0; m < 4; ++m) {
+      const ulonglong2 av = *(const ulonglong2*)(A + 8 * m * AP + 4 * kk);
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const float* r = A + (16 * m + g) * AP + k + c;
-      const RkSplit av[4] = {rk_split(r[0]), rk_split(r[8 * AP]), rk_split(r[4]), rk_split(r[8 * AP + 4])};
-#pragma unroll
-      for (int n = 0; n < 2; ++n) rk_mma(acc[m][n], av, b[n]);
+      for (int x = 0; x < 4; ++x) { acc[m][x] = fma_f2(av.x, sv[x].x, acc[m][x]); acc[m][x] = fma_f2(av.y, sv[x].y, acc[m][x]); }
     }
   }
+  part += rg * RK_PP + 4 * cg;
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int m = 0; m < 4; ++m) {
+    float o[4];
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      *(float2*)(part + (16 * m + g) * RK_PP + 8 * n + 2 * c) = make_float2(acc[m][n][0], acc[m][n][1]);
-      *(float2*)(part + (16 * m + g + 8) * RK_PP + 8 * n + 2 * c) = make_float2(acc[m][n][2], acc[m][n][3]);
-    }
+    for (int x = 0; x < 4; ++x) { float lo, hi; unpack_f2(acc[m][x], lo, hi); o[x] = lo + hi; }
+    *(float4*)(part + 8 * m * RK_PP) = make_float4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+// the eight warps' sums of a row and two columns, in warp order
+__device__ __forceinline__ float2 rk_gather(const float* part, int row, int col) {
+  float2 r = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const float2 p = *(const float2*)(part + (w * RK_C + row) * RK_PP + col);
+    r.x += p.x; r.y += p.y;
+  }
+  return r;
 }
 
 template <bool DELTA, int DK>
-__global__ void __launch_bounds__(4 * DK)
+__global__ void __launch_bounds__(RK_WALK_THREADS)
 rk_walk_kernel(const RkArgs a) {
   extern __shared__ __align__(16) float sm[];
   using I = RkImage<DELTA, DK>;
-  constexpr int NW = DK / 16, GT = 32 * NW;        // warps (threads) of a group; a warp keeps 16 key rows of the state
-  constexpr int STAGE = I::FLOATS + RK_C * RK_UP;
-  constexpr int CPT = RK_NV / NW;                  // columns a thread gathers (2 or 4)
-  float* partQ = sm + 2 * STAGE;                   // [NW][32][RK_PP]
-  float* St = partQ + NW * RK_C * RK_PP;           // two of [NW][16 columns][RK_SP]
-  float* partW = St + 2 * NW * RK_NV * RK_SP;      // (delta) as partQ
-  float* Us = partW + NW * RK_C * RK_PP;           // (delta) [32][RK_UP]
+  constexpr int STAGE = I::FLOATS + RK_C * RK_NV;
+  constexpr int KW = DK / 8;                       // key rows of the state a warp keeps
+  constexpr int RPL = KW / 8;                      // of them a lane
+  constexpr int GM = KW / 4 - 1;                   // 16-byte groups of a column, less one
+  float* partQ = sm + 2 * STAGE;                   // [8 warps][32][RK_PP]
+  float* St = partQ + 8 * RK_C * RK_PP;            // two of [8 warps][16 columns][KW], 16-byte groups swizzled by column / 4
+  float* partW = St + 2 * RK_NV * DK;              // (delta) as partQ
+  float* Us = partW + 8 * RK_C * RK_PP;            // (delta) [32][16]
   const int item = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * RK_NV;
   const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0;
   if (n < a.min_rows || n <= 0) return;
   const int chunks = (n + RK_C - 1) / RK_C;
-  const int tid = threadIdx.x, gtid = tid % GT, warp = gtid >> 5, lane = tid & 31;
-  const bool walker = tid < GT;
-  const int g = lane >> 2, c4 = lane & 3;
+  const int tid = threadIdx.x, gtid = tid & 255, warp = (tid >> 5) & 7, lane = tid & 31;
+  const bool walker = tid < 256;
+  const int rg = lane >> 2, cg = lane & 3;
   const size_t cell0 = (size_t)rk_first_chunk(r0, item) * a.H + h;
-  rk_fetch<DELTA, DK, 2 * GT>(a, sm, cell0, blockIdx.x, tid);
+  rk_fetch<DELTA, DK>(a, sm, cell0, blockIdx.x, tid);
 
-  // a walker's part of the state, as the MMA's result lies: rows i0 and i0 + 8, columns j0 + 8 t + 2 c4 + {0, 1}
+  // a walker's part of the state: rows warp * KW + RPL * rg + r, columns j0 + 4 cg + x
   float* slot = a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv;
-  const int i0 = 16 * warp + g;
-  float s[2][4];
+  const int i0 = warp * KW + RPL * rg;
+  float s[RPL][4];
   auto put_state = [&](int c) {
-    float* Sw = St + ((c & 1) * NW + warp) * (RK_NV * RK_SP);
+    float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) Sw[(8 * t + 2 * c4 + (x & 1)) * RK_SP + g + 8 * (x >> 1)] = s[t][x];
+      for (int r = 0; r < RPL; ++r) {
+        const int i = RPL * rg + r, col = 4 * cg + x;
+        Sw[col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3)] = s[r][x];
+      }
   };
   if (walker) {
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) s[t][x] = slot[(size_t)(j0 + 8 * t + 2 * c4 + (x & 1)) * DK + i0 + 8 * (x >> 1)];
+      for (int r = 0; r < RPL; ++r) s[r][x] = slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r];
     put_state(0);
   }
-  const int row = gtid / NW, jc = CPT * (gtid % NW);             // gathering: a thread a row and CPT columns
+  const int row = gtid >> 3, jc = 2 * (gtid & 7);                // gathering: a thread a row and two columns
 
   for (int c = 0; c < chunks; ++c) {
     const float* buf = sm + (c & 1) * STAGE;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();          // this chunk's operands and state are here; the other buffers, the sums and U are free
-    if (c + 1 < chunks) rk_fetch<DELTA, DK, 2 * GT>(a, sm + ((c + 1) & 1) * STAGE, cell0 + (size_t)(c + 1) * a.H, blockIdx.x, tid);
+    if (c + 1 < chunks) rk_fetch<DELTA, DK>(a, sm + ((c + 1) & 1) * STAGE, cell0 + (size_t)(c + 1) * a.H, blockIdx.x, tid);
     const float* U = DELTA ? Us : buf + I::FLOATS;
-    const float* Sw = St + ((c & 1) * NW + warp) * (RK_NV * RK_SP);
-    auto gather = [&](const float* part, float (&r)[CPT]) {      // the warps' sums in warp order
-#pragma unroll
-      for (int x = 0; x < CPT; ++x) r[x] = 0.f;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-#pragma unroll
-        for (int x = 0; x < CPT; x += 2) {
-          const float2 p = *(const float2*)(part + (w * RK_C + row) * RK_PP + jc + x);
-          r[x] += p.x; r[x + 1] += p.y;
-        }
-      }
-    };
+    const float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
     if (walker) {
       if (DELTA) {
-        rk_rows_by_state<I::AP>(buf + I::A + 16 * warp, Sw, partW + warp * (RK_C * RK_PP), g, c4);
-        rk_bar_sync(1, GT);
-        float r[CPT];
-        gather(partW, r);
-        const float* u0 = buf + I::FLOATS + row * RK_UP + jc;
-#pragma unroll
-        for (int x = 0; x < CPT; ++x) Us[row * RK_UP + jc + x] = u0[x] - r[x];
-        rk_bar_sync(1, GT);
-        rk_bar_arrive(2, 2 * GT);                  // U is there for the other group
+        rk_rows_by_state<KW, I::AP>(buf + I::A + warp * KW, Sw, partW + warp * (RK_C * RK_PP), rg, cg);
+        rk_bar_sync(1, 256);
+        const float2 r = rk_gather(partW, row, jc), u0 = *(const float2*)(buf + I::FLOATS + row * RK_NV + jc);
+        *(float2*)(Us + row * RK_NV + jc) = make_float2(u0.x - r.x, u0.y - r.y);
+        rk_bar_sync(1, 256);
+        rk_bar_arrive(2, 512);                     // U is there for the other group
       }
-      const float p0 = buf[I::P + i0], p1 = buf[I::P + i0 + 8];
-#pragma unroll
-      for (int t = 0; t < 2; ++t) { s[t][0] *= p0; s[t][1] *= p0; s[t][2] *= p1; s[t][3] *= p1; }
       const float* Kb = buf + I::K + i0;
+      const float* Pb = buf + I::P + i0;
+      float k1[RPL];
 #pragma unroll
-      for (int k = 0; k < RK_C; k += 8) {
-        const float* r = Kb + (k + c4) * I::KP;
-        const RkSplit av[4] = {rk_split(r[0]), rk_split(r[8]), rk_split(r[4 * I::KP]), rk_split(r[4 * I::KP + 8])};
+      for (int q = 0; q < RPL; ++q) {
+        const float p = Pb[q];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const RkSplit b[2] = {rk_split(U[(k + c4) * RK_UP + 8 * t + g]), rk_split(U[(k + c4 + 4) * RK_UP + 8 * t + g])};
-          rk_mma(s[t], av, b);
+        for (int x = 0; x < 4; ++x) s[q][x] *= p;
+      }
+#pragma unroll 16
+      for (int t2 = 0; t2 < RK_C; ++t2) {
+        if (RPL == 2) { const float2 f = *(const float2*)(Kb + t2 * DK); k1[0] = f.x; k1[RPL - 1] = f.y; }
+        else k1[0] = Kb[t2 * DK];
+        const float4 u = *(const float4*)(U + t2 * RK_NV + 4 * cg);
+#pragma unroll
+        for (int q = 0; q < RPL; ++q) {
+          s[q][0] = fmaf(k1[q], u.x, s[q][0]); s[q][1] = fmaf(k1[q], u.y, s[q][1]);
+          s[q][2] = fmaf(k1[q], u.z, s[q][2]); s[q][3] = fmaf(k1[q], u.w, s[q][3]);
         }
       }
       put_state(c + 1);
     } else {
-      rk_rows_by_state<I::AP>(buf + I::A + (I::NR - RK_C) * I::AP + 16 * warp, Sw, partQ + warp * (RK_C * RK_PP), g, c4);
-      rk_bar_sync(3, GT);
-      float r[CPT];
-      gather(partQ, r);
-      if (DELTA) rk_bar_sync(2, 2 * GT);
+      rk_rows_by_state<KW, I::AP>(buf + I::A + (I::NR - RK_C) * I::AP + warp * KW, Sw, partQ + warp * (RK_C * RK_PP), rg, cg);
+      rk_bar_sync(3, 256);
+      float2 r = rk_gather(partQ, row, jc);
+      if (DELTA) rk_bar_sync(2, 512);
       const float* Mt = buf + I::M + row * RK_LP;
 #pragma unroll 2
-      for (int x = 0; x <= (row | (32 / NW - 1)); x += 4) {      // (a warp's 32 / NW rows end together)
+      for (int x = 0; x <= (row | 3); x += 4) {    // (a warp's four rows end together)
         const float4 m = *(const float4*)(Mt + x);
         const float mm[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          if (x + e <= row) {
-#pragma unroll
-            for (int y = 0; y < CPT; ++y) r[y] = fmaf(mm[e], U[(x + e) * RK_UP + jc + y], r[y]);
-          }
+          const float2 u = *(const float2*)(U + (x + e) * RK_NV + jc);
+          if (x + e <= row) { r.x = fmaf(mm[e], u.x, r.x); r.y = fmaf(mm[e], u.y, r.y); }
         }
       }
-      if (c * RK_C + row < n) {
-        float* to = a.out + (size_t)(r0 + c * RK_C + row) * ((size_t)a.H * a.dv) + (size_t)h * a.dv + j0 + jc;
-#pragma unroll
-        for (int x = 0; x < CPT; x += 2) *(float2*)(to + x) = make_float2(r[x], r[x + 1]);
-      }
+      if (c * RK_C + row < n) *(float2*)(a.out + (size_t)(r0 + c * RK_C + row) * ((size_t)a.H * a.dv) + (size_t)h * a.dv + j0 + jc) = r;
     }
   }
   if (walker) {
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) slot[(size_t)(j0 + 8 * t + 2 * c4 + (x & 1)) * DK + i0 + 8 * (x >> 1)] = s[t][x];
+      for (int r = 0; r < RPL; ++r) slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r] = s[r][x];
   }
 }
 
@@ -538,14 +502,13 @@ template <int MODE, int DK, typename TA>
 static int rk_launch(const RkArgs& a, int n_items, int max_rows, cudaStream_t stream) {
   constexpr bool DELTA = MODE <= RK_DELTA_CHANNEL;
   const size_t sm_prep = (size_t)(4 * RK_C * DK + 2 * RK_C * RK_LP + 2 * RK_C) * sizeof(float);
-  constexpr int NW = DK / 16;
-  const size_t sm_walk = (size_t)(2 * (RkImage<DELTA, DK>::FLOATS + RK_C * RK_UP) + NW * RK_C * RK_PP + 2 * NW * RK_NV * RK_SP +
-                                  (DELTA ? NW * RK_C * RK_PP + RK_C * RK_UP : 0)) * sizeof(float);
+  const size_t sm_walk = (size_t)(2 * (RkImage<DELTA, DK>::FLOATS + RK_C * RK_NV) + 8 * RK_C * RK_PP + 2 * RK_NV * DK +
+                                  (DELTA ? 8 * RK_C * RK_PP + RK_C * RK_NV : 0)) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(rk_prep_kernel<MODE, DK, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_prep);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(rk_walk_kernel<DELTA, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
   if (e != cudaSuccess) return (int)e;
   rk_prep_kernel<MODE, DK, TA><<<dim3((max_rows + RK_C - 1) / RK_C, a.H, n_items), RK_THREADS, sm_prep, stream>>>(a);
-  rk_walk_kernel<DELTA, DK><<<dim3(a.dv / RK_NV, a.H, n_items), 4 * DK, sm_walk, stream>>>(a);
+  rk_walk_kernel<DELTA, DK><<<dim3(a.dv / RK_NV, a.H, n_items), RK_WALK_THREADS, sm_walk, stream>>>(a);
   return launch_status();
 }
 
