@@ -918,15 +918,8 @@ MOE_PLAN_TILE = 1024
 MOE_MAX_TOP = 16
 MOE_MMA = os.environ.get("FELLM_B200_MOE_MMA", "1") != "0"
 MOE_UMMA = os.environ.get("FELLM_B200_MOE_UMMA", "1") != "0"
-# Which kernel a bfloat16 step's experts take goes by its (token, choice) pairs.  Slabs of 16 weight rows read a matrix once for
-# eight rows of an expert, the tcgen05 tiles once for 128, behind a start of their own and a gather.  Both products, slabs and
-# tcgen05 in us: 8 experts of [3328, 1024] 50 / 58 at 64 pairs, 62 / 58 at 96, 115 / 60 at 256; 16 of [1024, 1024] 30 / 37 at 64, 36 / 37
-# at 128, 40 / 38 at 192; 32 of [768, 1024] 33 / 45 at 64, 43 / 46 at 192, 49 / 48 at 256; 4 of [3328, 1024] 40 / 46 at 64, 52 / 47 at
-# 96.  So the line is eight rows an expert, between 96 and 256 pairs.  The mma.sync tiles of 64 rows (217, 102, 99, 214 us) are
-# the yardstick and stand in above 255 pairs where the tcgen05 product is switched off.
-MOE_UMMA_MIN_PAIRS = int(os.environ.get("FELLM_B200_MOE_UMMA_MIN_PAIRS", 96))
-MOE_UMMA_PER_EXPERT, MOE_UMMA_ALL_PAIRS = 8, 256
-MOE_FEW_PAIRS = int(os.environ.get("FELLM_B200_MOE_FEW_PAIRS", 255))               # up to this many off tcgen05: slabs
+MOE_UMMA_MIN_PAIRS = int(os.environ.get("FELLM_B200_MOE_UMMA_MIN_PAIRS", 256))     # fewer (token, choice) pairs: mma.sync tiles of 64 rows
+MOE_FEW_PAIRS = int(os.environ.get("FELLM_B200_MOE_FEW_PAIRS", 64))                # up to this many: a warp a column (weight streaming)
 
 
 def moe_route(logits, E: int, top: int, renormalize: bool = False):
@@ -984,10 +977,9 @@ class MoePlan:
     __slots__ = ("sorted", "place_of", "table", "n_tiles", "n_rows", "max_tiles", "pairs", "top", "row_tile")
 
 
-def moe_row_tile(pairs: int, bf16: bool, K_ok: bool, E: int = 0) -> int:
-    """Rows of a tile for a step of this many pairs over E experts: 128 where the tcgen05 grouped product takes the step."""
-    least = max(MOE_UMMA_MIN_PAIRS, min(MOE_UMMA_PER_EXPERT * E, MOE_UMMA_ALL_PAIRS))
-    return MOE_UMMA_ROW_TILE if (bf16 and K_ok and MOE_UMMA and USE_UMMA and pairs >= least) else MOE_ROW_TILE
+def moe_row_tile(pairs: int, bf16: bool, K_ok: bool) -> int:
+    """Rows of a tile for a step of this many pairs: 128 where the tcgen05 grouped product takes the step."""
+    return MOE_UMMA_ROW_TILE if (bf16 and K_ok and MOE_UMMA and USE_UMMA and pairs >= MOE_UMMA_MIN_PAIRS) else MOE_ROW_TILE
 
 
 def moe_plan(idx, E: int, row_tile: int = MOE_ROW_TILE) -> MoePlan:
@@ -1018,8 +1010,8 @@ def moe_gemm(a, w, plan: MoePlan, *, gated: bool, gather: bool, interleaved: boo
     a's dtype (w's rows: gate rows then up rows, or, interleaved, blocks of 8 gate and 8 up rows by turns); else
     float32.  act = (limit, alpha): the gated activation is the clamped form min(g, limit) sigmoid(alpha min(g, limit))
     (clamp(u, -limit, limit) + 1) instead.  Returns [P, N] in sorted order.
-    bfloat16: tcgen05 (tiles of 128 rows, the plan made for them), slabs of 16 weight rows for fewer pairs, mma.sync tiles
-    of 64 rows where neither is taken; float32, or sizes those do not take: float32 FMA."""
+    bfloat16: tcgen05 (tiles of 128 rows, the plan made for them), a warp a column for a handful of pairs, mma.sync
+    tiles of 64 rows between; float32, or sizes those do not take: float32 FMA."""
     _dev(a, w)
     assert a.stride(1) == 1 and w.is_contiguous() and a.dtype == w.dtype
     E, n_rows, K = w.shape

@@ -113,7 +113,7 @@ class RoutedExperts(FeedForward):
             hn = hn.to(first.dtype)
         bf = hn.dtype == torch.bfloat16
         k_ok = self.ff % 8 == 0 and self.size % 8 == 0 and hn.stride(0) % 8 == 0
-        tile = ops.moe_row_tile(idx.numel(), bf, k_ok and (self.interleaved or bool(self.plain)), self.E)
+        tile = ops.moe_row_tile(idx.numel(), bf, k_ok and (self.interleaved or bool(self.plain)))
         plan = ops.moe_plan(idx, self.E, tile)
         if self.plain:
             a = ops.relu2(ops.moe_gemm(hn, first, plan, gated=False, gather=True), hn.dtype)

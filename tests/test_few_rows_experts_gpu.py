@@ -37,21 +37,3 @@ def test_few_pairs(N, K, gated, interleaved, tokens):
         y = torch.nn.functional.silu(gate) * up
     # float32 sums of K exact products; gated: gate and up round to bfloat16 (2^-9 each), their product once more
     assert float((got - y).norm() / y.norm()) < (6e-3 if gated else 2e-6)
-
-
-@pytest.mark.parametrize("E,pairs,tile", [(4, 94, 64), (4, 96, 128), (16, 126, 64), (16, 128, 128), (40, 254, 64), (40, 256, 128)])
-@pytest.mark.parametrize("one", [False, True])
-def test_both_sides_of_the_line(E, pairs, tile, one):
-    """The last step that runs on slabs and the first on tcgen05 tiles, rows spread over the experts and all with one."""
-    from fellm_b200 import ops
-    g = torch.Generator().manual_seed(E + pairs)
-    N, K = 72, 136
-    idx = torch.full((pairs, 1), E - 1, dtype=torch.int32) if one else torch.randint(0, E, (pairs, 1), generator=g, dtype=torch.int32)
-    assert ops.moe_row_tile(pairs, True, True, E) == tile
-    plan = ops.moe_plan(idx.cuda(), E, tile)
-    a = torch.randn(pairs, K, generator=g).bfloat16().cuda()
-    w = (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16().cuda()
-    got = ops.moe_gemm(a, w, plan, gated=False, gather=True).double()
-    order = plan.sorted.long()
-    y = torch.einsum("pk,pnk->pn", a.double()[order], w.double()[idx.cuda().reshape(-1).long()[order]])
-    assert float((got - y).norm() / y.norm()) < 2e-6                    # (as above)
