@@ -171,9 +171,9 @@ static int launch(const bf16* A, const bf16* W, const float* bias, void* out, in
 
 // ---------------------------------------------------------------- a product per head for a handful of rows
 // The same product for up to 32 rows.  The weights are all there is to read (16 heads of 256 x 64: 0.5 MB), so what a tile of
-// 128 rows costs is its ring and its idle rows.  8 rows of 16 heads, device time in a graph, tile -> here: [256, 64] 2.84 ->
-// 1.36 us, [64, 256] 6.27 -> 1.78, [512, 128] 4.20 -> 1.65, [128, 512] 10.5 -> 2.8; at 32 rows 3.74 -> 1.78, 6.82 -> 2.58, 5.06 ->
-// 2.37, 11.5 -> 4.3.  Bound by the latency of one trip to memory and of the launch.  A warp takes 16 weight rows of a head as the
+// 128 rows costs is its ring and its idle rows.  8 rows of 16 heads, device time in a graph, tile -> here: [256, 64] 2.83 ->
+// 1.85 us, [64, 256] 6.37 -> 2.49, [512, 128] 4.15 -> 2.34, [128, 512] 10.5 -> 3.6; at 32 rows 3.79 -> 2.54, 6.83 -> 3.43, 4.87 ->
+// 3.16, 11.6 -> 4.9.  Bound by the latency of one trip to memory and of the launch.  A warp takes 16 weight rows of a head as the
 // MMA's first operand, straight from memory, and the rows of the input, eight at a time, as the second: lane c's four
 // consecutive k are its slots {2c, 2c+1, 2c+8, 2c+9} in both, so that an MMA covers the same 16 k as the tile's and follows
 // it in K: the sums are the tile's, bit for bit, and a row's result stays free of the batch.

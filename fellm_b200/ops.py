@@ -441,8 +441,8 @@ def head_gemm(a, w, out, *, a_head: int, out_head: int):
 
 TOKEN_SIDE_MMA = os.environ.get("FELLM_B200_TOKEN_SIDE_MMA", "1") != "0"
 # rows up to which a product per head takes slabs of 16 weight rows instead of tiles of 128 rows (the kernel's most: four groups of
-# eight rows in registers).  It is the faster one there at every size measured: 64 heads of [512, 128] 6.30 -> 3.12 us at 8 rows,
-# 8.01 -> 5.49 at 32, its smallest gain.
+# eight rows in registers).  It is the faster one there at every size measured: 64 heads of [512, 128] 6.30 -> 4.01 us at 8 rows,
+# 8.01 -> 6.65 at 32, its smallest gain.
 HEAD_GEMM_FEW_ROWS = 32
 HEAD_GEMM_MMA = os.environ.get("FELLM_B200_HEAD_GEMM_MMA", "1") != "0"
 
