@@ -359,13 +359,14 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
     const unsigned t_acc = t_row + AU_COL_O + grp * AU_VC * 32;
     const unsigned s_full = s_full0 + 16 * grp, p_full = p_full0 + 16 * grp, o_full = o_full0 + 16 * grp;
     const bool capped = AU_EXTENDED && a.cap_log2 > 0.f;
-    float scale = capped ? a.cap_log2 : a.scale_log2;            // (capped: of tanh's values)
-    if (AU_GENERAL && a.qt_every > 0) scale *= 1.0f + a.qt_coef * logf((float)((pos + 1) / a.qt_every + 1));
+    // (capped: of tanh's values; a temperature is the query's, so it goes into the tanh and not over it)
+    const float temp = (AU_GENERAL && a.qt_every > 0) ? 1.0f + a.qt_coef * logf((float)((pos + 1) / a.qt_every + 1)) : 1.0f;
+    float scale = capped ? a.cap_log2 : a.scale_log2 * temp;
     const bool sloped = AU_GENERAL && a.slopes != nullptr;
     const float slope = sloped ? a.slopes[g * R + head] * 1.4426950408889634f : 0.f;
     const float raw_scale = scale;
     if (sloped) scale = 1.f;                                     // (the scores are then scaled where their bias is added)
-    const float cap_in = capped ? a.scale_log2 / a.cap_log2 : 0.f;
+    const float cap_in = capped ? a.scale_log2 / a.cap_log2 * temp : 0.f;
     int lo = (AU_EXTENDED && a.window > 0) ? pos - a.window + 1 : 0;               // the first key the row sees
     if (AU_GENERAL && a.chunk > 0) lo = max(lo, pos / a.chunk * a.chunk);
     // The accumulator of P V stays in tensor memory, scaled by 2^-m where m is the row's REFERENCE

@@ -77,7 +77,9 @@ def close(got, want):
 
 
 FORMS = [dict(window=70), dict(chunk=48), dict(window=100, slopes=True, temp=(0.25, 16)), dict(cap=4.0, chunk=100, gate=True), dict(slopes=True),
-         dict(window=1, temp=(0.5, 128)), dict(window=64, out_gate=True), dict()]
+         dict(window=1, temp=(0.5, 128)), dict(window=64, out_gate=True), dict(),
+         # a cap and a temperature that is 1.6 to 2.5 at most of these positions: of the scores inside the cap
+         dict(cap=2.0, temp=(0.5, 16)), dict(cap=4.0, temp=(0.5, 16), slopes=True, window=100)]
 
 
 def form(spec, T, H, g):
