@@ -237,13 +237,15 @@ FELLM_API int fellm_gemm_tiled_batched(const void* A, const void* W, void* out, 
   if ((K % 8) || (lda % 8) || (ldw % 8) || (sa % 8) || (sw % 8) || batch > 65535) return FELLM_ERR_SIZE;
   if (M <= few_rows) {
     const dim3 slabs(ceil_div(N, 16 * HW_WARPS), batch);
-#define HEADS_FEW(RG_) return launch_k(gemm_heads_few_kernel<RG_>, slabs, dim3(HW_WARPS * 32), 0, stream, 1, (const bf16*)A, (const bf16*)W, (bf16*)out, \
-        M, N, K, lda, ldw, ldo, sa, sw, so)
+    if (M > 32) return FELLM_ERR_SIZE;
+    // (an ordinary launch: the kernel does not wait for the one in front, so it must never be a programmatic dependent)
+#define HEADS_FEW(RG_) gemm_heads_few_kernel<RG_><<<slabs, HW_WARPS * 32, 0, stream>>>((const bf16*)A, (const bf16*)W, (bf16*)out, M, N, K, lda, ldw, \
+        ldo, sa, sw, so)
     if (M <= 8) HEADS_FEW(1);
-    if (M <= 16) HEADS_FEW(2);
-    if (M <= 32) HEADS_FEW(4);
-    return FELLM_ERR_SIZE;
+    else if (M <= 16) HEADS_FEW(2);
+    else HEADS_FEW(4);
 #undef HEADS_FEW
+    return launch_status();
   }
   size_t smem = (size_t)TSTAGES * (TBM + TBN) * 4 * sizeof(uint4);
   auto kern = gemm_tiled_kernel<EPI_STORE>;

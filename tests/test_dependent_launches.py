@@ -1,0 +1,86 @@
+"""Launches that may be programmatic dependents of the kernel in front (launch_k, launch_k_class of csrc/common.cuh: by their class
+or, with FELLM_B200_PDL=1, all of them): the kernel has to wait for that kernel before it touches what it wrote.  Read from the
+sources; no GPU."""
+from __future__ import annotations
+
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "fellm_b200" / "csrc"
+SOURCES = sorted(CSRC.glob("*.cu"))
+
+
+def closing(text: str, at: int, pair: str) -> int:
+    """The index behind the bracket that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += (text[i] == pair[0]) - (text[i] == pair[1])
+        if depth == 0:
+            return i + 1
+    raise AssertionError("brackets do not close")
+
+
+def source(path: Path) -> str:
+    """The file with the sources it includes, without comments."""
+    text = path.read_text()
+    for inc in re.findall(r'#include\s+"([^"]+\.cu)"', text):
+        text += source(CSRC / inc)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def kernels(text: str):
+    """{name: (parameters, body)} of the file's kernels."""
+    got = {}
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\s*\([^;{]*?\)\s*)?(\w+)\s*\(", text):
+        end = closing(text, m.end() - 1, "()")
+        body = text.index("{", end)
+        got[m.group(1)] = (text[m.end():end - 1], text[body:closing(text, body, "{}")])
+    return got
+
+
+def dependents(text: str, names):
+    """The kernels that launch_k and launch_k_class are handed: by name, or by the function pointer declared last in front of the call."""
+    found = set()
+    for m in re.finditer(r"\blaunch_k(?:_class)?\s*\(", text):
+        call = text[m.end():closing(text, m.end() - 1, "()")]
+        direct = [n for n in names if re.search(rf"\b{n}\b", call)]
+        if not direct and re.search(r"\bkern\b", call):
+            start = max(text.rfind(decl, 0, m.start()) for decl in ("auto kern", "(*kern)"))
+            direct = [n for n in names if re.search(rf"\b{n}\b", text[start:m.start()])]
+            assert direct, f"which kernel is launched here? {call[:120]}"
+        found.update(direct)
+    return found
+
+
+def waits(name, all_kernels, text, seen=()):
+    """Whether the kernel's body, or a device function it calls, waits for the kernel in front."""
+    body = all_kernels[name][1]
+    if "pdl_wait()" in body:
+        return True
+    for callee in set(re.findall(r"\b(\w+)\s*(?:<[^;{}()]*>)?\(", body)):
+        m = re.search(rf"__device__[^;{{}}]*\b{callee}\s*\(", text)
+        if m:
+            end = closing(text, m.end() - 1, "()")
+            at = text.find("{", end)
+            if at >= 0 and "pdl_wait()" in text[at:closing(text, at, "{}")]:
+                return True
+    return False
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.stem)
+def test_dependent_kernels_wait(path):
+    text = source(path)
+    ks = kernels(text)
+    launched = dependents(text, ks)
+    without = sorted(n for n in launched if not waits(n, ks, text))
+    assert not without, f"{path.name}: launched as dependents, but without pdl_wait(): {without}"
+
+
+def test_the_reading_finds_the_launches():
+    """(the checks above would pass on files they cannot read)"""
+    found = {p.stem: dependents(source(p), kernels(source(p))) for p in SOURCES}
+    assert sum(len(v) for v in found.values()) > 40
+    assert "rmsnorm_vec_kernel" in found["elementwise"] and "attention_prefill_umma_kernel" in found["attention_umma"]
+    assert "latent_gather_kernel" in found["latent"] and "gemm_tiled_kernel" not in found["gemm_tiled"]
