@@ -9,9 +9,12 @@
 // lane, the 32 keys' K and V all in flight at once; the partial dot products of 32 keys go through the lanes by a
 // transposing butterfly that leaves lane j with the whole scores of key j; the softmax runs on a key a lane; then every lane
 // adds its 8 elements of its keys' values, the probabilities by shuffles.  A row and kv head's keys are dealt out in tiles of
-// 32 over the warps of a cluster of up to eight blocks (as many as fill the device: ~1 tile a warp for a window of 1,024 at
-// 48 rows x kv heads), merged through shared memory and then through the cluster's.  Bound by: latency, one round trip to
-// memory for the page numbers, one for keys and values, the two merges.
+// 32 over the warps of up to eight parts of four warps (a.parts, by the window or chunk alone: ~1 tile a warp for a window of
+// 1,024), whose sums lie in shared memory until all are there and are then added in one fixed order.  A cluster has as many
+// blocks as fill the device; a block of a smaller one takes several neighbouring parts one after another.  So a row's bits
+// do not depend on how many rows decode beside it (the same 12 rows: 9.5 us; 48 rows 20.9, 128 rows 63; with the shares by the
+// batch, in whose order rows were added before, 8.9, 19.3 and 62.5).  Bound by: latency, one round trip to memory for the page
+// numbers, one for keys and values, one to the other blocks' sums.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -19,12 +22,13 @@
 namespace cg = cooperative_groups;
 
 #define AR_WARPS 4
+#define AR_PARTS 8            // most parts of a row's keys
 
 struct ArArgs {
   const bf16* q; const bf16* pool; const int* block_table; const int* positions; const int* row_slot;
   bf16* out; int* status;
   const float* gate; const float* slopes; const bf16* og;
-  int ldq, max_pages, H, G, page_shift, layer, layers_in_group, window, chunk, ldg, ldog, qt_every, new_k_off, new_v_off;
+  int parts, ldq, max_pages, H, G, page_shift, layer, layers_in_group, window, chunk, ldg, ldog, qt_every, new_k_off, new_v_off;
   float scale, softcap, qt_coef;
 };
 
@@ -34,16 +38,14 @@ __device__ __forceinline__ void ar_unpack(const uint4& raw, float* f) {
   for (int e = 0; e < 4; ++e) { const float2 v = __bfloat1622float2(h[e]); f[2 * e] = v.x; f[2 * e + 1] = v.y; }
 }
 
-// What a part's sums are multiplied by on the way to the maximum M; a part without keys (m = -inf, l = 0) counts nothing,
-// one whose scores were no numbers keeps them.
-__device__ __forceinline__ float ar_factor(float m, float l, float M) { return (m == -INFINITY && l == 0.f) ? 0.f : expf(m - M); }
-
 template <int HD, int R, bool VK>
 __global__ void __launch_bounds__(AR_WARPS * 32)
 attention_rows_kernel(const ArArgs a) {
   constexpr int LPK = HD / 8, KPI = 32 / LPK, NI = 32 / KPI;        // lanes a key, keys a load, loads a tile (= LPK)
-  __shared__ __align__(16) float part[AR_WARPS][R][HD + 4];          // a warp's sums, then m, l
-  __shared__ __align__(16) float rec[R][HD + 4];                     // the block's
+  typedef float Sums[AR_WARPS][R][HD + 4];                           // a part's: per warp and head the elements, then m, l
+  extern __shared__ __align__(16) float ar_smem[];
+  Sums* sums = (Sums*)ar_smem;                                       // the block's parts'
+  __shared__ float factor[R][AR_PARTS * AR_WARPS], total[R];
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = gridDim.x, rank = blockIdx.x, g = blockIdx.y, row = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPK, sub = lane % LPK;
@@ -66,87 +68,112 @@ attention_rows_kernel(const ArArgs a) {
     for (int e = 0; e < 8; ++e) q[r][e] *= qt;
     slope[r] = a.slopes ? a.slopes[g * R + r] : 0.f;
   }
-  float acc[R][8], m[R], l[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    m[r] = -INFINITY; l[r] = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
-  }
 
-  for (int k0 = k_begin + 32 * (rank * AR_WARPS + warp); k0 <= pos; k0 += 32 * AR_WARPS * cs) {
-    const int mine = min(k0 + lane, pos);
-    const int page = max(bt[mine >> a.page_shift], 0);               // an unmapped entry (-1) must never become an address
-    uint4 kr[NI], vr[VK ? 1 : NI];
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const int j = i * KPI + grp, kj = min(k0 + j, pos);            // (beyond the row: the row's own key once more, masked below)
-      const int pg = __shfl_sync(0xffffffffu, page, j);
-      const bf16* krow = a.pool + ((size_t)pg * a.layers_in_group + a.layer) * record + ((size_t)g * pt + (kj & (pt - 1))) * HD;
-      const bf16* vrow = krow + (size_t)a.G * pt * HD;
-      if (fused && kj == pos) {
-        krow = qrow + a.new_k_off + (size_t)g * HD;
-        vrow = qrow + a.new_v_off + (size_t)g * HD;
-      }
-      kr[i] = *(const uint4*)(krow + 8 * sub);
-      if (!VK) vr[i] = *(const uint4*)(vrow + 8 * sub);
-    }
-    float s[R][NI];
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      float kf[8];
-      ar_unpack(kr[i], kf);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float d = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) d = fmaf(q[r][e], kf[e], d);
-        s[r][i] = d;
-      }
-    }
-    // a key's LPK partial sums, for NI = LPK keys of this lane group: lane `sub` ends with the whole of key sub * KPI + grp
-    float p[R];
+  const int n_parts = a.parts / cs, e0 = 8 * sub + (HD == 64 ? 4 * (grp & 1) + 2 * (grp >> 1) : 4 * grp);
+  for (int i = 0; i < n_parts; ++i) {
+    const int p = rank * n_parts + i;
+    float m[R], l[R];
+    float acc[R][8];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+      m[r] = -INFINITY; l[r] = 0.f;
 #pragma unroll
-      for (int w = LPK / 2; w > 0; w >>= 1) {
-        const bool up = sub & w;
+      for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
+    }
+
+    for (int k0 = k_begin + 32 * (p * AR_WARPS + warp); k0 <= pos; k0 += 32 * AR_WARPS * a.parts) {
+      const int mine = min(k0 + lane, pos);
+      const int page = max(bt[mine >> a.page_shift], 0);               // an unmapped entry (-1) must never become an address
+      uint4 kr[NI], vr[VK ? 1 : NI];
 #pragma unroll
-        for (int i = 0; i < w; ++i) {
-          const float give = up ? s[r][i] : s[r][i + w], keep = up ? s[r][i + w] : s[r][i];
-          s[r][i] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+      for (int i = 0; i < NI; ++i) {
+        const int j = i * KPI + grp, kj = min(k0 + j, pos);            // (beyond the row: the row's own key once more, masked below)
+        const int pg = __shfl_sync(0xffffffffu, page, j);
+        const bf16* krow = a.pool + ((size_t)pg * a.layers_in_group + a.layer) * record + ((size_t)g * pt + (kj & (pt - 1))) * HD;
+        const bf16* vrow = krow + (size_t)a.G * pt * HD;
+        if (fused && kj == pos) {
+          krow = qrow + a.new_k_off + (size_t)g * HD;
+          vrow = qrow + a.new_v_off + (size_t)g * HD;
+        }
+        kr[i] = *(const uint4*)(krow + 8 * sub);
+        if (!VK) vr[i] = *(const uint4*)(vrow + 8 * sub);
+      }
+      float s[R][NI];
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        float kf[8];
+        ar_unpack(kr[i], kf);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float d = 0.f;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) d = fmaf(q[r][e], kf[e], d);
+          s[r][i] = d;
+        }
+      }
+      // a key's LPK partial sums, for NI = LPK keys of this lane group: lane `sub` ends with the whole of key sub * KPI + grp
+      float pr[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int w = LPK / 2; w > 0; w >>= 1) {
+          const bool up = sub & w;
+#pragma unroll
+          for (int i = 0; i < w; ++i) {
+            const float give = up ? s[r][i] : s[r][i + w], keep = up ? s[r][i + w] : s[r][i];
+            s[r][i] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+          }
+        }
+      }
+      const int kj = k0 + sub * KPI + grp;
+      const bool seen = kj <= pos;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float x = s[r][0] * a.scale;
+        if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+        x -= slope[r] * (float)(pos - kj);
+        x = seen ? x : -INFINITY;
+        const float mn = fmaxf(m[r], warp_max(x));                     // (a tile holds a key that the row sees)
+        pr[r] = seen ? expf(x - mn) : 0.f;
+        const float corr = expf(m[r] - mn);
+        m[r] = mn;
+        l[r] = fmaf(l[r], corr, pr[r]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[r][e] *= corr;
+      }
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        const bool live = k0 + i * KPI + grp <= pos;                   // (a masked key's value is not touched: 0 * NaN)
+        float vf[8];
+        ar_unpack(VK ? kr[i] : vr[VK ? 0 : i], vf);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float pi = __shfl_sync(0xffffffffu, pr[r], i, LPK);
+          if (live) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(pi, vf[e], acc[r][e]);
+          }
         }
       }
     }
-    const int kj = k0 + sub * KPI + grp;
-    const bool seen = kj <= pos;
+
+    // the lane groups' sums: a lane ends with HD / 32 of the elements, from e0 on
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      float x = s[r][0] * a.scale;
-      if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
-      x -= slope[r] * (float)(pos - kj);
-      x = seen ? x : -INFINITY;
-      const float mn = fmaxf(m[r], warp_max(x));                     // (a tile holds a key that the row sees)
-      p[r] = seen ? expf(x - mn) : 0.f;
-      const float corr = expf(m[r] - mn);
-      m[r] = mn;
-      l[r] = fmaf(l[r], corr, p[r]);
+      l[r] = warp_sum(l[r]);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[r][e] *= corr;
-    }
+      for (int w = LPK, n = 4; w < 32; w <<= 1, n >>= 1) {
+        const bool up = lane & w;
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const bool live = k0 + i * KPI + grp <= pos;                   // (a masked key's value is not touched: 0 * NaN)
-      float vf[8];
-      ar_unpack(VK ? kr[i] : vr[VK ? 0 : i], vf);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const float pr = __shfl_sync(0xffffffffu, p[r], i, LPK);
-        if (live) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(pr, vf[e], acc[r][e]);
+        for (int e = 0; e < n; ++e) {
+          const float give = up ? acc[r][e] : acc[r][e + n], keep = up ? acc[r][e + n] : acc[r][e];
+          acc[r][e] = keep + __shfl_xor_sync(0xffffffffu, give, w);
         }
       }
+      float* to = sums[i][warp][r];
+      if (HD == 64) *(float2*)(to + e0) = make_float2(acc[r][0], acc[r][1]);
+      else *(float4*)(to + e0) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      if (lane == 0) *(float2*)(to + HD) = make_float2(m[r], l[r]);
     }
   }
 
@@ -162,49 +189,50 @@ attention_rows_kernel(const ArArgs a) {
     }
   }
 
-  // lane groups, then warps, then blocks
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    l[r] = warp_sum(l[r]);
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-#pragma unroll
-      for (int w = LPK; w < 32; w <<= 1) acc[r][e] += __shfl_xor_sync(0xffffffffu, acc[r][e], w);
-    if (grp == 0) {
-      *(float4*)&part[warp][r][8 * sub] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-      *(float4*)&part[warp][r][8 * sub + 4] = make_float4(acc[r][4], acc[r][5], acc[r][6], acc[r][7]);
-    }
-    if (lane == 0) { part[warp][r][HD] = m[r]; part[warp][r][HD + 1] = l[r]; }
+  if (cs > 1) cluster.sync(); else __syncthreads();
+  const int shift = __ffs(n_parts) - 1;                              // (a power of two)
+  auto sums_of = [&](int p, int w, int r) {
+    float* to = sums[p & (n_parts - 1)][w][r];
+    return cs > 1 ? cluster.map_shared_rank(to, p >> shift) : to;
+  };
+  // what a warp's sums count, a lane a (part, warp): -1 for one without keys
+  if (warp < R) {
+    const int p = lane / AR_WARPS;
+    const float2 ml = p < a.parts ? *(const float2*)(sums_of(p, lane % AR_WARPS, warp) + HD) : make_float2(-INFINITY, 0.f);
+    const bool none = ml.x == -INFINITY && ml.y == 0.f;
+    const float M = warp_max(ml.x), f = none ? 0.f : expf(ml.x - M), L = warp_sum(ml.y * f);
+    factor[warp][lane] = none ? -1.f : f;
+    if (lane == 0) total[warp] = L;
   }
   __syncthreads();
-  for (int x = threadIdx.x; x < R * HD; x += AR_WARPS * 32) {
-    const int r = x / HD, e = x - r * HD;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < AR_WARPS; ++w) M = fmaxf(M, part[w][r][HD]);
-    float o = 0.f, L = 0.f;
-#pragma unroll
-    for (int w = 0; w < AR_WARPS; ++w) {
-      const float f = ar_factor(part[w][r][HD], part[w][r][HD + 1], M);
-      o = fmaf(part[w][r][e], f, o); L = fmaf(part[w][r][HD + 1], f, L);
-    }
-    rec[r][e] = o;
-    if (e == 0) { rec[r][HD] = M; rec[r][HD + 1] = L; }
-  }
-  if (cs > 1) cluster.sync(); else __syncthreads();
-  // every block finishes its share of the elements
-  const int share = R * HD / cs;
-  for (int x = rank * share + threadIdx.x; x < (rank + 1) * share; x += AR_WARPS * 32) {
+  // every block finishes its share of the elements: four lanes an aligned four of them, a warp's sums each, then an element each
+  const int share = R * HD / cs, w = lane & 3;
+  for (int x0 = 0; x0 < share; x0 += AR_WARPS * 32) {
+    const bool live = x0 + (int)threadIdx.x < share;
+    const int x = rank * share + (live ? x0 + (int)threadIdx.x : w);
     const int r = x / HD, e = x - r * HD, h = g * R + r;
-    float M = -INFINITY;
-    for (int c = 0; c < cs; ++c) M = fmaxf(M, cs > 1 ? cluster.map_shared_rank(&rec[0][0], c)[r * (HD + 4) + HD] : rec[r][HD]);
-    float o = 0.f, L = 0.f;
-    for (int c = 0; c < cs; ++c) {
-      const float* rc = (cs > 1 ? cluster.map_shared_rank(&rec[0][0], c) : &rec[0][0]) + r * (HD + 4);
-      const float f = ar_factor(rc[HD], rc[HD + 1], M);
-      o = fmaf(rc[e], f, o); L = fmaf(rc[HD + 1], f, L);
+    float4 from[AR_PARTS];
+    float f[AR_PARTS], o4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int p = 0; p < AR_PARTS; ++p) {
+      f[p] = factor[r][p * AR_WARPS + w];
+      from[p] = !(f[p] < 0.f) ? *(const float4*)(sums_of(p, w, r) + (e & ~3)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float inv = 1.0f / L;
+#pragma unroll
+    for (int p = 0; p < AR_PARTS; ++p) {
+      if (f[p] < 0.f) continue;
+      o4[0] = fmaf(from[p].x, f[p], o4[0]); o4[1] = fmaf(from[p].y, f[p], o4[1]);
+      o4[2] = fmaf(from[p].z, f[p], o4[2]); o4[3] = fmaf(from[p].w, f[p], o4[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float give = (w & 2) ? o4[i] : o4[i + 2], keep = (w & 2) ? o4[i + 2] : o4[i];
+      o4[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+    const float give = (w & 1) ? o4[0] : o4[1], keep = (w & 1) ? o4[1] : o4[0];
+    float o = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+    if (!live) continue;
+    float inv = 1.0f / total[r];
     if (a.gate) inv *= 1.0f / (1.0f + expf(-a.gate[(size_t)row * a.ldg + h]));
     o *= inv;
     if (a.og) o *= 1.0f / (1.0f + expf(-__bfloat162float(a.og[(size_t)row * a.ldog + (size_t)h * HD + e])));
@@ -217,6 +245,11 @@ template <int HD, int R, bool VK>
 static int ar_launch(const ArArgs& a, int T, int cs, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs, a.G, T); cfg.blockDim = dim3(AR_WARPS * 32); cfg.stream = stream;
+  cfg.dynamicSmemBytes = (size_t)(a.parts / cs) * AR_WARPS * R * (HD + 4) * sizeof(float);
+  if (cfg.dynamicSmemBytes > 40 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<HD, R, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+    if (e != cudaSuccess) return (int)e;
+  }
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -228,23 +261,24 @@ static int ar_launch(const ArArgs& a, int T, int cs, cudaStream_t stream) {
 
 // Rows of q [T, ldq] (heads at column 0, H x hd bfloat16), each at its own position of its own slot; the other arguments as
 // fellm_paged_attention_general's, vd 0 (values that are the keys) or hd; og [T, ldog] bfloat16 (null: none): the result times
-// its sigmoid, element by element; cluster: 1, 2, 4 or 8 blocks a (row, kv head).
+// its sigmoid, element by element; parts: 1, 2, 4 or 8 shares of a row's keys (the order of its sums), cluster: as many blocks a
+// (row, kv head) or fewer.
 FELLM_API int fellm_attention_rows(const void* q, const void* pool, const int* block_table, int max_pages, const int* positions,
                                    const int* row_slot, void* out, int T, int H, int G, int hd, int vd, int page_tokens, int layer,
                                    int layers_in_group, float scale, int window, int ldq, float softcap, int chunk, const float* gate,
                                    int ldg, const float* slopes, float qt_coef, int qt_every, int new_k_off, int new_v_off, int* status,
-                                   const void* og, int ldog, int cluster, cudaStream_t stream) {
+                                   const void* og, int ldog, int parts, int cluster, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (!q || !pool || !block_table || !positions || !row_slot || !out) return FELLM_ERR_ARG;
   if (G < 1 || H % G || (hd != 64 && hd != 128) || (vd && vd != hd) || T > 65535 || G > 65535) return FELLM_ERR_SIZE;
   const int R = H / G;
   if ((R != 1 && R != 2 && R != 4) || page_tokens < 1 || (page_tokens & (page_tokens - 1))) return FELLM_ERR_SIZE;
-  if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return FELLM_ERR_ARG;
+  if ((parts != 1 && parts != 2 && parts != 4 && parts != AR_PARTS) || cluster < 1 || cluster > parts || parts % cluster) return FELLM_ERR_ARG;
   if ((((uintptr_t)q | (uintptr_t)pool) & 15) || (ldq & 7) || (new_k_off >= 0 && ((new_k_off & 7) || (vd && (new_v_off & 7))))) return FELLM_ERR_SIZE;
   ArArgs a;
   a.q = (const bf16*)q; a.pool = (const bf16*)pool; a.block_table = block_table; a.positions = positions; a.row_slot = row_slot;
   a.out = (bf16*)out; a.status = status; a.gate = gate; a.slopes = slopes; a.og = (const bf16*)og;
-  a.ldq = ldq; a.max_pages = max_pages; a.H = H; a.G = G; a.layer = layer; a.layers_in_group = layers_in_group;
+  a.parts = parts; a.ldq = ldq; a.max_pages = max_pages; a.H = H; a.G = G; a.layer = layer; a.layers_in_group = layers_in_group;
   a.window = window; a.chunk = chunk; a.ldg = ldg; a.ldog = ldog; a.qt_every = qt_every; a.new_k_off = new_k_off; a.new_v_off = new_v_off;
   a.scale = scale; a.softcap = softcap; a.qt_coef = qt_coef;
   a.page_shift = 0;

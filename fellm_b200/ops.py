@@ -1251,7 +1251,7 @@ def paged_attention_general(q, H, hd, vd, pool, block_table, positions, row_slot
     times its sigmoid, element by element.
     A bfloat16 decode step (write_new given, or out_gate) of the sizes `attention_rows_takes` names runs on a kernel that shares a
     key's reading among its heads and a row's keys among blocks (csrc/attention_rows.cu; the same float32 arithmetic in another
-    order).
+    order, which does not depend on the other rows of the step).
     Returns [T, H*vd] (H*hd, or H*out_dim, when the values are the keys) in q's dtype."""
     _dev(q, pool, block_table, positions, row_slot, gate, slopes, sinks)
     if sinks is not None:
@@ -1279,11 +1279,13 @@ def paged_attention_general(q, H, hd, vd, pool, block_table, positions, row_slot
             assert out_gate.dtype == q.dtype and out_gate.stride(1) == 1 and out_gate.shape == out.shape
         f = _fn("attention_rows", "fellm_attention_rows",
                 [_c_p, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p] + [_c_int] * 8 + [_c_f, _c_int, _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_f,
-                 _c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_p])
+                 _c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p])
+        cluster = attention_rows_cluster(T * G, window, chunk)
         _check(f(_p(q), _p(pool), _p(block_table), block_table.shape[1], _p(positions), _p(row_slot), _p(out), T, H, G, hd, vd, page_tokens,
                  layer, pool.shape[1], float(scale), int(window or 0), q.stride(0), float(softcap or 0.0), int(chunk or 0), _p(gate),
                  gate.stride(0) if gate is not None else 0, _p(slopes), float(qt_coef), int(qt_every), int(nk), int(nv), _p(status),
-                 _p(out_gate), out_gate.stride(0) if out_gate is not None else 0, attention_rows_cluster(T * G, window, chunk), _stream()),
+                 _p(out_gate), out_gate.stride(0) if out_gate is not None else 0, max(cluster, attention_rows_parts(window, chunk)), cluster,
+                 _stream()),
                "attention_rows")
         return out
     f = _fn("attention_simt", "fellm_paged_attention_general",
@@ -1307,12 +1309,20 @@ def attention_rows_takes(q, pool, H: int, G: int, hd: int, vd: int, page_tokens:
             and q.shape[0] <= 65535 and (not write_new or not (write_new[0] % 8 or (vd and write_new[1] % 8))))
 
 
-def attention_rows_cluster(items: int, window=None, chunk=None) -> int:
-    """Blocks (of four warps, a tile of 32 keys at a time) that share a row and kv head's keys: enough for two blocks an SM, no
-    more than have a tile each."""
+def attention_rows_parts(window=None, chunk=None) -> int:
+    """Parts (of four warps, a tile of 32 keys at a time) into which a row and kv head's keys are dealt out: by the window or chunk
+    alone, so that the order of a row's sums is the same in every step."""
     tiles = -(-min(window or 4096, chunk or 4096, 4096) // 32)
     n = 1
-    while n < 8 and items * n < 2 * sm_count() and 8 * n <= tiles:
+    while n < 8 and 8 * n <= tiles:
+        n *= 2
+    return n
+
+
+def attention_rows_cluster(items: int, window=None, chunk=None) -> int:
+    """Blocks that share those parts: enough for two blocks an SM."""
+    n = 1
+    while n < attention_rows_parts(window, chunk) and items * n < 2 * sm_count():
         n *= 2
     return n
 

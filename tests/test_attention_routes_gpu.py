@@ -173,6 +173,36 @@ def test_rows_over_a_cluster(spec, H, G, hd, page, keys_alone, cluster, monkeypa
     assert int(status) == 2 and torch.equal(before.view(torch.int16), pool.view(torch.int16))
 
 
+@pytest.mark.parametrize("window,chunk,G", [(None, None, 4), (1024, None, 4), (300, None, 2), (1024, 512, 8)])
+def test_a_row_keeps_its_bits_in_every_batch(window, chunk, G):
+    """However many rows decode together: the blocks that share a row's keys follow the batch, the order of its sums does not."""
+    from fellm_b200 import ops
+    g = torch.Generator().manual_seed(G)
+    lens = [1, 33, 700, 1500, 2100]
+    H, hd, page = 2 * G, 64, 64
+    pages = Pages(lens, G, hd, hd, page, 7)
+    T = 330
+    slots = torch.arange(T) % len(lens)
+    pos = torch.tensor(lens)[slots] - 1
+    q, gate = torch.randn(T, H * hd, generator=g).bfloat16().cuda(), torch.randn(T, H * hd, generator=g).bfloat16().cuda()
+    i32 = lambda x: x.to(torch.int32).cuda()  # noqa: E731
+
+    def call(n):
+        assert ops.attention_rows_takes(q[:n], pages.five(G, hd), H, G, hd, hd, page)
+        return ops.paged_attention_general(q[:n], H, hd, hd, pages.five(G, hd), pages.table.cuda(), i32(pos[:n]), i32(slots[:n]), 1, page, G, 0.125,
+                                           window=window, chunk=chunk, out_gate=gate[:n])
+    whole = call(T)
+    sizes = (1, 5, 12, 40, 80, 200)
+    clusters = {ops.attention_rows_cluster(n * G, window, chunk) for n in sizes + (T,)}
+    assert len(clusters) > 1
+    for n in sizes:
+        assert torch.equal(call(n), whole[:n])
+    for r in range(len(lens)):
+        want = attend(q[r:r + 1].double().cpu().view(1, H, hd), pages.k[r].double(), pages.v[r].double(), pos[r:r + 1], 0.125, window=window, chunk=chunk)
+        want = want.reshape(1, -1) * torch.sigmoid(gate[r:r + 1].double().cpu())
+        assert float((whole[r:r + 1].double().cpu() - want).norm() / want.norm()) < 2.5e-3
+
+
 @pytest.mark.parametrize("window,sink", [(64, True), (100, False), (1, True)])
 def test_latents_taken_out_per_head(window, sink):
     from fellm_b200 import ops
