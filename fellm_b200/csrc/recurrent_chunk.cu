@@ -1,5 +1,5 @@
 // Recurrences whose decay depends on the token (recurrent.cu's delta rule, decay with a bonus, gated write) over prompt
-// portions, in chunks of 32 tokens, float32 arithmetic on CUDA cores.
+// portions, in chunks of 32 tokens, on CUDA cores: float32, the sums that every later one hangs on in 64 bits.
 //
 // All of them are, per head with a state S [dk, dv] and per token vectors A, B, G, K [dk], v [dv] and scalars beta, c,
 //     u_t = beta_t (v_t - S_(t-1)^T A_t)   (delta rule)      or   u_t = v_t
@@ -20,20 +20,29 @@
 // every two multiply-adds, and a block's chunk of 32 tokens at dk = 128 is 0.2 M of those: ~5,000 of the 5,800 cycles a
 // chunk takes.  The scan walks one token after another, a reduction over dk and ~750 cycles each.  16 columns a block: a
 // prompt of 16 heads of 128 is 128 blocks for 148 SMs.  2,048 tokens of 16 heads of 128 x 128, delta rule: scan 791 us, here
-// prep 75 + walk 188; three prompts of 1,537 tokens, 8 heads, gated write: 274 us, here 28 + 77.
+// prep 81 + walk 188 (decay per channel: 96 + 188); three prompts of 1,537 tokens, 8 heads, gated write: 274 us, here 23 + 77.
 // 32 tokens a chunk: L and M cost 32 / 2 multiply-adds a token, channel and matrix, an eighth of the walk's.
 //
 // A later token's infinity or NaN stays out of an earlier token's sums, as in the walk token by token: masked pairs are
 // skipped or selected away, never multiplied by zero.
 //
-// Sums run in another order than the scan's (equal up to float32 rounding), so the engine uses this form for portions of
-// the bfloat16 engine; the 32-bit engine keeps the scan and with it the same bits for a prompt under every cut.
+// Rounding: with float32 throughout, the substitution's 31 steps and the sums of 128 products behind L, M and c made the delta
+// rule's results less exact than the walk token by token.  So in prep the lanes' partial sums of those products are joined
+// in 64 bits, the substitution runs in them (a finished row is rounded once, to what walk works with), and the running
+// products of the decays are sums of two floats.  Relative error against float64, scan / here, mean over five sizes and
+// three seeds: delta rule outputs 1.34e-7 / 1.22e-7, states 9.0e-8 / 8.6e-8, with keys nearly alike and beta 0.99 1.45e-7 /
+// 1.35e-7, 8.7e-8 / 8.4e-8; decay per channel 1.22e-7 / 1.08e-7, 7.8e-8 / 7.3e-8; decay and bonus 8.3e-8 / 6.8e-8, 3.15e-8 /
+// 3.09e-8; gated write 6.2e-8 / 5.9e-8, 1.09e-7 / 1.07e-7.  It costs 6 us of the 263 of the first size above (21 of 264 with a
+// decay per channel, 4 of 68 with a bonus; the gated write gains 5 of 106 through its smaller blocks).
+// Sums run in another order than the scan's, so the engine uses this form for portions of the bfloat16 engine; the 32-bit
+// engine keeps the scan and with it the same bits for a prompt under every cut.
 // A head's state lies column by column in its slot (element (i, j) at j * dk + i), as the scan keeps it.
 #include "common.cuh"
 
 #define RK_C 32            // tokens of a chunk
 #define RK_NV 16           // value columns of a walk's block
-#define RK_LP 36           // row stride of a chunk's 32 x 32 matrices
+#define RK_LP 36           // row stride of a chunk's 32 x 32 matrices in the image
+#define RK_LM 34           // and, in 64 bits, in prep's shared memory
 #define RK_THREADS 256
 
 enum RkMode { RK_DELTA_HEAD = 0, RK_DELTA_CHANNEL = 1, RK_DECAY_BONUS = 2, RK_GATED_WRITE = 3 };
@@ -71,6 +80,28 @@ template <int E> __device__ __forceinline__ void rk_store(float* p, const float*
 __device__ __forceinline__ float rk_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float rk_sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
 
+// warp_sum with one rounding at the end.
+__device__ __forceinline__ float rk_sum(float v) {
+  double d = v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  return (float)d;
+}
+
+// A running product of decays as an unrounded sum of two floats: its error stays below a rounding of the product, where a
+// single float's grows with every factor.
+struct RkProduct {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void by(float g) {
+    const float p = hi * g, rest = fmaf(hi, g, -p);
+    lo = fmaf(lo, g, rest); hi = p;
+  }
+  __device__ __forceinline__ float times(float v) const {
+    const float r = v * hi;
+    return fabsf(r) < INFINITY ? fmaf(v, hi, v * lo) : r;          // (an infinity times a rest of zero is not a number)
+  }
+};
+
 // What prep leaves for walk of a chunk and head, as it lies in walk's shared memory (its copies are then linear).
 template <bool DELTA, int DK>
 struct RkImage {
@@ -81,17 +112,16 @@ struct RkImage {
 
 // ---------------------------------------------------------------- prep
 template <int MODE, int DK, typename TA>
-__global__ void __launch_bounds__(RK_THREADS, 2)
+__global__ void __launch_bounds__(RK_THREADS, 3)
 rk_prep_kernel(const RkArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* A = sm;                                   // [32][DK]
   float* B = A + RK_C * DK;
   float* Gd = B + RK_C * DK;
   float* KK = Gd + RK_C * DK;
-  float* Lt = KK + RK_C * DK;                      // [s][t]: beta_t L_ts
-  float* Mm = Lt + RK_C * RK_LP;                   // [t][s]
-  float* beta = Mm + RK_C * RK_LP;
-  float* cc = beta + RK_C;
+  float* cc = KK + RK_C * DK;
+  double* beta = (double*)(cc + RK_C);             // (delta)
+  double* LM = beta + RK_C;                        // [32][RK_LM]: [s][t], t > s: beta_t L_ts; [t][s], s <= t: M_ts
   constexpr bool DELTA = MODE <= RK_DELTA_CHANNEL;
   constexpr int E = DK / 32;
   const int item = blockIdx.z, h = blockIdx.y, c = blockIdx.x;
@@ -101,7 +131,7 @@ rk_prep_kernel(const RkArgs a) {
   const size_t cell = (size_t)(rk_first_chunk(r0, item) + c) * a.H + h;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = h / (a.H / a.G);
-  for (int x = tid; x < 2 * RK_C * RK_LP; x += RK_THREADS) Lt[x] = 0.f;          // (and Mm behind it)
+  for (int x = tid; x < RK_C * RK_LM; x += RK_THREADS) LM[x] = 0.0;
 
   // ---- the token vectors: a warp takes tokens warp, warp + 8, ..; a lane E consecutive elements
   {
@@ -138,7 +168,7 @@ rk_prep_kernel(const RkArgs a) {
           float sq = 0.f, sk = 0.f, kq = 0.f;
 #pragma unroll
           for (int e = 0; e < E; ++e) { sq = fmaf(q[u][e], q[u][e], sq); sk = fmaf(k[u][e], k[u][e], sk); kq = fmaf(k[u][e], q[u][e], kq); }
-          sq = warp_sum(sq); sk = warp_sum(sk); kq = warp_sum(kq);
+          sq = rk_sum(sq); sk = rk_sum(sk); kq = rk_sum(kq);
           const float kn = 1.0f / sqrtf(sk + 1e-6f);
           const float qn = 1.0f / (sqrtf(sq + 1e-6f) * sqrtf((float)DK));
           const float gs = MODE == RK_DELTA_HEAD ? expf(-rate * rk_softplus(la[u] + bias)) : 0.f;
@@ -153,7 +183,7 @@ rk_prep_kernel(const RkArgs a) {
         } else if (MODE == RK_DECAY_BONUS) {
 #pragma unroll
           for (int e = 0; e < E; ++e) { bv[e] = q[u][e]; kv[e] = k[u][e]; gv[e] = w[u][e]; cv = fmaf(q[u][e] * x0[e], k[u][e], cv); }
-          cv = warp_sum(cv); be = 1.f;
+          cv = rk_sum(cv);
         } else {
 #pragma unroll
           for (int e = 0; e < E; ++e) {
@@ -162,13 +192,13 @@ rk_prep_kernel(const RkArgs a) {
             gv[e] = f; kv[e] = 1.0f - f; bv[e] = f * qq;
             cv = fmaf(kv[e], qq, cv);
           }
-          cv = warp_sum(cv); be = 1.f;
+          cv = rk_sum(cv);
         }
       }
       const int o = t * DK + lane * E;
       if (DELTA) rk_store<E>(A + o, av);
       rk_store<E>(B + o, bv); rk_store<E>(Gd + o, gv); rk_store<E>(KK + o, kv);
-      if (lane == 0) { beta[t] = be; cc[t] = cv; }
+      if (lane == 0) { cc[t] = cv; if (DELTA) beta[t] = be; }
     }
   }
   __syncthreads();
@@ -223,31 +253,26 @@ rk_prep_kernel(const RkArgs a) {
       }
       // lane ig ends with the whole of sum[4 (ig & 1) + 2 ((ig >> 1) & 1) + (ig >> 2)]
       const bool b0 = ig & 1, b1 = ig & 2, b2 = ig & 4;
-      float q4[4], q2[2], v;
-      if (DELTA) {
+      double q4[4], q2[2], v;                      // (the lanes' sums are joined in 64 bits, for half of the products' error)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float give = b0 ? sum[j] : sum[4 + j], keep = b0 ? sum[4 + j] : sum[j];
-          q4[j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) q4[j] = sum[j] + __shfl_xor_sync(0xffffffffu, sum[j], 1);
+      for (int j = 0; j < 4; ++j) {
+        const float give = DELTA && !b0 ? sum[4 + j] : sum[j], keep = DELTA && b0 ? sum[4 + j] : sum[j];
+        q4[j] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, give, 1);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const float give = b1 ? q4[j] : q4[2 + j], keep = b1 ? q4[2 + j] : q4[j];
+        const double give = b1 ? q4[j] : q4[2 + j], keep = b1 ? q4[2 + j] : q4[j];
         q2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
       }
       {
-        const float give = b2 ? q2[0] : q2[1], keep = b2 ? q2[1] : q2[0];
+        const double give = b2 ? q2[0] : q2[1], keep = b2 ? q2[1] : q2[0];
         v = keep + __shfl_xor_sync(0xffffffffu, give, 4);
       }
       const int t = t0 + (b1 ? 2 : 0) + (b2 ? 1 : 0);
       if (t > s) {
-        if (DELTA && b0) Lt[s * RK_LP + t] = beta[t] * v;
-        else if (!b0) Mm[t * RK_LP + s] = v;
-      } else if (t == s && !b0) Mm[t * RK_LP + t] = cc[t];
+        if (DELTA && b0) LM[s * RK_LM + t] = beta[t] * v;
+        else if (!b0) LM[t * RK_LM + s] = v;
+      } else if (t == s && !b0) LM[t * RK_LM + t] = (double)cc[t];
     }
   }
   __syncthreads();
@@ -256,23 +281,23 @@ rk_prep_kernel(const RkArgs a) {
   float* img = a.image + cell * I::FLOATS;
   // ---- running products of the decays: forward into A and B (up to the token before), backward into K (behind the token)
   if (tid < DK) {
-    float p = 1.f;
+    RkProduct p;
 #pragma unroll 8
     for (int t = 0; t < RK_C; ++t) {
       const int o = t * DK + tid;
       const float gd = Gd[o];
-      if (DELTA) A[o] *= p;
-      B[o] *= p;
-      p *= gd;
+      if (DELTA) A[o] = p.times(A[o]);
+      B[o] = p.times(B[o]);
+      p.by(gd);
     }
-    img[I::P + tid] = p;
+    img[I::P + tid] = p.hi + p.lo;
   } else if (tid < 2 * DK) {
-    float p = 1.f;
+    RkProduct p;
 #pragma unroll 8
     for (int t = RK_C - 1; t >= 0; --t) {
       const int o = t * DK + tid - DK;
-      KK[o] *= p;
-      p *= Gd[o];
+      KK[o] = p.times(KK[o]);
+      p.by(Gd[o]);
     }
   }
   __syncthreads();
@@ -281,7 +306,10 @@ rk_prep_kernel(const RkArgs a) {
     *(float4*)(img + I::A + (t + I::NR - RK_C) * I::AP + i) = *(const float4*)(B + x);
     *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
   }
-  for (int x = tid * 4; x < RK_C * RK_LP; x += RK_THREADS * 4) *(float4*)(img + I::M + x) = *(const float4*)(Mm + x);
+  for (int x = tid; x < RK_C * RK_C; x += RK_THREADS) {
+    const int t = x / RK_C, s = x % RK_C;
+    img[I::M + t * RK_LP + s] = s <= t ? (float)LM[t * RK_LM + s] : 0.f;
+  }
 
   // ---- (I + beta L) [W | U0] = beta [P A | V], a column a thread; without the delta rule U0 = V
   float* Ug = a.U + cell * ((size_t)RK_C * a.dv);
@@ -289,31 +317,60 @@ rk_prep_kernel(const RkArgs a) {
   for (int col = tid; col < (DELTA ? DK : 0) + a.dv; col += RK_THREADS) {
     const bool is_w = DELTA && col < DK;
     const int j = DELTA ? col - DK : col;
-    float x[RK_C];
-#pragma unroll
-    for (int t = 0; t < RK_C; ++t) {
-      x[t] = 0.f;
-      if (is_w) x[t] = A[t * DK + col];
-      else if (t < len) x[t] = to_f(vp[(size_t)(row0 + t) * a.ld + j]);
-    }
+    auto put = [&](int t, float x) {
+      if (is_w) img[I::A + t * I::AP + col] = x;
+      else Ug[((size_t)(j / RK_NV) * RK_C + t) * RK_NV + j % RK_NV] = x;
+    };
     if (DELTA) {
+      // products and sums in 64 bits, half of the tokens at a time (their registers); a finished value is the float that the
+      // walk over the chunks works with
+      constexpr int HC = RK_C / 2;
+      float done[HC];
 #pragma unroll
-      for (int t = 0; t < RK_C; ++t) x[t] *= beta[t];
+      for (int half = 0; half < 2; ++half) {
+        float in[HC];
+        double x[HC];
 #pragma unroll
-      for (int s = 0; s < RK_C - 1; ++s)
-#pragma unroll
-        for (int t0 = (s + 1) & ~3; t0 < RK_C; t0 += 4) {
-          const float4 l = *(const float4*)(Lt + s * RK_LP + t0);
-          if (t0 > s) x[t0] = fmaf(-l.x, x[s], x[t0]);
-          if (t0 + 1 > s) x[t0 + 1] = fmaf(-l.y, x[s], x[t0 + 1]);
-          if (t0 + 2 > s) x[t0 + 2] = fmaf(-l.z, x[s], x[t0 + 2]);
-          x[t0 + 3] = fmaf(-l.w, x[s], x[t0 + 3]);
+        for (int i = 0; i < HC; ++i) {
+          const int t = half * HC + i;
+          in[i] = 0.f;
+          if (is_w) in[i] = A[t * DK + col];
+          else if (t < len) in[i] = to_f(vp[(size_t)(row0 + t) * a.ld + j]);
         }
-    }
+        asm volatile("" ::: "memory");             // (all on their way before the first is waited for)
 #pragma unroll
-    for (int t = 0; t < RK_C; ++t) {
-      if (is_w) img[I::A + t * I::AP + col] = x[t];
-      else Ug[((size_t)(j / RK_NV) * RK_C + t) * RK_NV + j % RK_NV] = x[t];
+        for (int i = 0; i < HC; ++i) x[i] = (double)in[i] * beta[half * HC + i];
+        if (half) {
+#pragma unroll
+          for (int s = 0; s < HC; ++s) {
+            const double xs = (double)done[s];
+#pragma unroll
+            for (int i = 0; i < HC; i += 2) {
+              const double2 l = *(const double2*)(LM + s * RK_LM + HC + i);
+              x[i] = fma(-l.x, xs, x[i]); x[i + 1] = fma(-l.y, xs, x[i + 1]);
+            }
+          }
+        }
+#pragma unroll
+        for (int s = 0; s < HC; ++s) {
+          const float f = (float)x[s];
+          const double xs = (double)f;
+          done[s] = f;
+          put(half * HC + s, f);
+#pragma unroll
+          for (int i = (s + 1) & ~1; i < HC; i += 2) {
+            const double2 l = *(const double2*)(LM + (half * HC + s) * RK_LM + half * HC + i);
+            if (i > s) x[i] = fma(-l.x, xs, x[i]);
+            x[i + 1] = fma(-l.y, xs, x[i + 1]);
+          }
+        }
+      }
+    } else {
+      float x[RK_C];                               // (all on their way before the first is stored)
+#pragma unroll
+      for (int t = 0; t < RK_C; ++t) x[t] = t < len ? to_f(vp[(size_t)(row0 + t) * a.ld + j]) : 0.f;
+#pragma unroll
+      for (int t = 0; t < RK_C; ++t) put(t, x[t]);
     }
   }
 }
@@ -501,7 +558,7 @@ rk_walk_kernel(const RkArgs a) {
 template <int MODE, int DK, typename TA>
 static int rk_launch(const RkArgs& a, int n_items, int max_rows, cudaStream_t stream) {
   constexpr bool DELTA = MODE <= RK_DELTA_CHANNEL;
-  const size_t sm_prep = (size_t)(4 * RK_C * DK + 2 * RK_C * RK_LP + 2 * RK_C) * sizeof(float);
+  const size_t sm_prep = (size_t)(4 * RK_C * DK + RK_C) * sizeof(float) + (RK_C * RK_LM + RK_C) * sizeof(double);
   const size_t sm_walk = (size_t)(2 * (RkImage<DELTA, DK>::FLOATS + RK_C * RK_NV) + 8 * RK_C * RK_PP + 2 * RK_NV * DK +
                                   (DELTA ? 8 * RK_C * RK_PP + RK_C * RK_NV : 0)) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(rk_prep_kernel<MODE, DK, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_prep);
