@@ -210,11 +210,12 @@ FELLM_API int fellm_latent_rotate_q(const void* q, int bf16_, int ldq, int H, in
 // Blocks [0, T): a row's queries' rotated parts (dr elements behind the dn unrotated ones of every head), rotated where they
 // lie.  The others: a warp a key row of item i: the cached row of position first_i + k, first_i the position of the page of
 // the first key that the item's first row sees through the window; its rk latent elements into `lat`, its rotated part into
-// `rope`; zeros behind the item's last key (and where no page is mapped).
+// `rope`; zeros behind the item's last key (and where no page is mapped).  The kernel in front writes the step's rows into the
+// pool: `pool` is not __restrict__, as loads of what a kernel declares never to change need not stay behind its wait.
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(bf16* q, int ldq, int H, int dn, int dr, const float* __restrict__ freq, int n_rot, float mag,
                      const int* __restrict__ positions, const int* __restrict__ row_slot, const int* __restrict__ item_start,
-                     const int* __restrict__ block_table, int max_pages, const bf16* __restrict__ pool, int page_tokens, int layer,
+                     const int* __restrict__ block_table, int max_pages, const bf16* pool, int page_tokens, int layer,
                      int layers_in_group, int rk, int window, int key_rows, int T, bf16* __restrict__ lat, bf16* __restrict__ rope) {
   pdl_launch_dependents();
   pdl_wait();

@@ -78,6 +78,16 @@ def test_dependent_kernels_wait(path):
     assert not without, f"{path.name}: launched as dependents, but without pdl_wait(): {without}"
 
 
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.stem)
+def test_dependent_kernels_read_the_cache_behind_their_wait(path):
+    """A kernel in front may have written into the pool of pages: declared as never changing (const and __restrict__), its loads
+    may be moved in front of the wait."""
+    text = source(path)
+    ks = kernels(text)
+    frozen = sorted(n for n in dependents(text, ks) if re.search(r"\bconst\s+\w+\s*\*\s*__restrict__\s+pool\b", ks[n][0]))
+    assert not frozen, f"{path.name}: {frozen}"
+
+
 def test_the_reading_finds_the_launches():
     """(the checks above would pass on files they cannot read)"""
     found = {p.stem: dependents(source(p), kernels(source(p))) for p in SOURCES}
