@@ -654,7 +654,8 @@ def recurrent_chunk_rows(dtype) -> int:
 def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_items, max_item_rows, min_rows, H, G, dk, dv, out, *,
                      small=None, b_off=0, a_off=0, A_log=None, dt_bias=None, gch=None, bonus=None, lower=None, fbias=None) -> bool:
     """Runs the items of min_rows rows or more in chunks; False (nothing launched) for sizes and alignments the kernels do not
-    take: a lane reads dk / 32 neighbouring elements at once, a block keeps 16 value columns."""
+    take (a lane reads dk / 32 neighbouring elements at once, a block keeps 16 value columns) and for steps whose chunks would
+    take more than LAYER_SCRATCH_MAX_BYTES."""
     es = q.element_size()
     lane = dk // 32
     if dk not in (64, 128) or dv % 16 or n_items > 65535 or H > 65535 or (mode == 3 and es == 2):
@@ -666,7 +667,10 @@ def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_i
     T = out.shape[0]
     need = _fn("recurrent_chunk", "fellm_recurrent_chunk_scratch", [_c_int] * 6)
     need.restype = _c_ll
-    scratch = torch.empty(need(mode, T, n_items, H, dk, dv), dtype=torch.float32, device=out.device)
+    floats = need(mode, T, n_items, H, dk, dv)
+    if 4 * floats > LAYER_SCRATCH_MAX_BYTES:
+        return False
+    scratch = torch.empty(floats, dtype=torch.float32, device=out.device)
     sp, ss = _state_args(state)
     f = _fn("recurrent_chunk", "fellm_recurrent_chunk",
             [_c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int] + [_c_p] * 7 + [_c_ll] + [_c_p] * 4 + [_c_int] * 8 + [_c_p])
@@ -1371,6 +1375,11 @@ LATENT_SINGLE_ROWS = 32        # up to this many (token, head) rows an item: the
 LATENT_MAX_SPLITS = 16
 
 
+# Most bytes of scratch that a form of a layer may take which trades scratch for speed (keys and values per head out of latents,
+# chunks of a recurrence); a step that would take more runs in the form without.  An engine leaves 2 GB beside its cache for a
+# step's rows, and a prompt portion of the default 2,048 rows takes 29 MB (16 heads, a window of 1,024) and 75 MB (16 heads of
+# 128 x 128).
+LAYER_SCRATCH_MAX_BYTES = 512 << 20
 LATENT_EXPAND = os.environ.get("FELLM_B200_LATENT_EXPAND", "1") != "0"
 
 
@@ -1379,11 +1388,13 @@ def latent_expand_key_rows(H: int, dn: int, dr: int, dv: int, rk: int, window, p
     or 0 where the queries rather go into the latents' space (latent_attention).  Sizes: what the tcgen05 library is compiled for, a
     window (the rows an item can see are then known without its positions), pages of 64.  Worth it: a key row costs a product of
     rk x H (dn + dv) (~8 ns at 16 heads of 128, a latent of 512), a query row in the latents' space 0.2 us more over a window of
-    1,024 than per head, so up to 16 key rows a query row; below that a step is mostly single tokens or the last few of a prompt."""
+    1,024 than per head, so up to 16 key rows a query row; below that a step is mostly single tokens or the last few of a prompt.
+    Not where the rows of all items, their latents, rotated parts, keys and values per head, are beyond LAYER_SCRATCH_MAX_BYTES."""
     if not LATENT_EXPAND or not window or page_tokens != 64 or (dn, dr, dv) != (128, 64, 128) or rk % 64 or window > 4096:
         return 0
     rows = -(-(int(window) - 1 + 63 + max_item_rows) // 64) * 64
-    return rows if n_items * rows <= 16 * n_rows and n_rows >= 64 else 0
+    held = n_items * rows * (rk + dr + H * (dn + dv)) * 2
+    return rows if n_items * rows <= 16 * n_rows and n_rows >= 64 and held <= LAYER_SCRATCH_MAX_BYTES else 0
 
 
 def latent_expand_defines():

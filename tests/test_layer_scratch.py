@@ -1,0 +1,33 @@
+"""Forms of a layer that trade scratch for speed: how much they may take, and what is kept of their weights."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from fellm_b200 import ops
+
+
+def test_latents_per_head_have_a_limit():
+    """A step's latents, rotated parts, keys and values per head stay within the limit, whatever the heads and the requests."""
+    def rows(H, n_items, longest, T):
+        return ops.latent_expand_key_rows(H, 128, 64, 128, 512, 1024, 64, T, n_items, longest)
+    assert rows(16, 1, 2048, 2048) == 3136                           # a prompt's portion: 29 MB
+    for H in (16, 64, 128):
+        for n_items in range(1, 61):
+            for T in (512, 2048, 4096, 8192):
+                longest = -(-T // n_items)
+                n = rows(H, n_items, longest, T)
+                assert n_items * n * (512 + 64 + H * 256) * 2 <= ops.LAYER_SCRATCH_MAX_BYTES
+    assert rows(16, 53, 78, 4096) == 0 and rows(64, 4, 1024, 4096) > 0
+
+
+@pytest.mark.gpu
+def test_recurrences_beyond_the_limit_keep_the_scan(monkeypatch):
+    from test_recurrent_chunk_gpu import MODES, Step
+    for mode in MODES:
+        s = Step(mode, (70, 40), 2, 2, 64, 64, seed=3)
+        scan, _ = s.run(0)
+        assert not torch.equal(s.run(32)[0], scan)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "LAYER_SCRATCH_MAX_BYTES", 1 << 16)
+            assert torch.equal(s.run(32)[0], scan)
