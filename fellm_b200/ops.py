@@ -414,28 +414,29 @@ def gemm_simt(a, w, bias=None, out=None, out_dtype=None, accumulate=False, act=N
 
 def head_gemm(a, w, out, *, a_head: int, out_head: int):
     """One product per head in one launch: out[t, h * out_head + n] = sum_k a[t, h * a_head + k] w[h, n, k]
-    for h < H, n < N, k < K (w [H, N, K] contiguous; a and out are row-major with the heads side by side in a row,
+    for h < H, n < N, k < K (w [H, N, K], each w[h] contiguous; a and out are row-major with the heads side by side in a row,
     a head's block starting every a_head / out_head columns and possibly wider than K / N).  All bfloat16, with
     blocks that start on 16 bytes: tensor cores (mma.sync tiles, float32 sums); else float32 FMA, any mix of
     bfloat16 / float32.  A row's result does not depend on the batch."""
     _dev(a, w, out)
     H, N, K = w.shape
     T = a.shape[0]
-    assert w.is_contiguous() and a.stride(1) == 1 and out.stride(1) == 1 and out.shape[0] == T
+    assert w.stride(2) == 1 and (N == 1 or w.stride(1) == K) and a.stride(1) == 1 and out.stride(1) == 1 and out.shape[0] == T
+    wh = w.stride(0)
     assert a.shape[1] >= (H - 1) * a_head + K and out.shape[1] >= (H - 1) * out_head + N
     if _is_bf16(out) and not _is_bf16(a):
         raise KernelError("head_gemm: float32 activations do not round down to a bfloat16 result")
     if (_is_bf16(a) and _is_bf16(w) and _is_bf16(out) and K % 8 == 0 and a_head % 8 == 0 and a.stride(0) % 8 == 0
-            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and HEAD_GEMM_MMA):
+            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and wh % 8 == 0 and HEAD_GEMM_MMA):
         f = _fn("gemm_tiled", "fellm_gemm_tiled_batched", [_c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                            _c_ll, _c_ll, _c_ll, _c_int, _c_p])
-        _check(f(_p(a), _p(w), _p(out), H, T, N, K, a.stride(0), K, out.stride(0), int(a_head), N * K, int(out_head), HEAD_GEMM_FEW_ROWS,
+        _check(f(_p(a), _p(w), _p(out), H, T, N, K, a.stride(0), K, out.stride(0), int(a_head), wh, int(out_head), HEAD_GEMM_FEW_ROWS,
                  _stream()), "head_gemm (tensor cores)")
         return out
     f = _fn("gemm_simt", "fellm_gemm_simt_batched", [_c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                      _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_p])
     _check(f(_p(a), _is_bf16(a), _p(w), _is_bf16(w), _p(out), _is_bf16(out), H, T, N, K, a.stride(0), K, out.stride(0),
-             int(a_head), N * K, int(out_head), _stream()), "head_gemm")
+             int(a_head), wh, int(out_head), _stream()), "head_gemm")
     return out
 
 

@@ -99,7 +99,10 @@ class LatentAttention(Mixer):
             # portions of prompts: keys and values per head out of the latents, one product, rows [head: W_uk,h | W_uv,h]
             w["kv.weight"] = torch.cat([uk.view(H, dn, rk), w["uv.weight"].view(H, dv, rk).to(uk.dtype)], 1).reshape(H * (dn + dv), rk).contiguous()
         w["ukT.weight"] = uk.view(H, dn, rk).transpose(1, 2).contiguous()
-        w["uv.weight"] = w["uv.weight"].view(H, dv, rk).contiguous()
+        if "kv.weight" in w and w["uv.weight"].dtype == uk.dtype:
+            w["uv.weight"] = w["kv.weight"].view(H, dn + dv, rk)[:, dn:]          # (held once)
+        else:
+            w["uv.weight"] = w["uv.weight"].view(H, dv, rk).contiguous()
         w["o.weight"] = w["o.weight"].contiguous()
         self.position.to(uk.device)
 

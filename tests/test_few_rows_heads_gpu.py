@@ -25,3 +25,18 @@ def test_few_rows_are_the_tile_s(T, H, N, K, a_head, out_head):
         got = few[:, h * out_head:h * out_head + N].double().cpu()
         # K float32 sums and one rounding to 8 significant bits (half a unit in the last place: 2^-8 of the value at most)
         assert bool(((got - x @ m.T).abs() <= 2.0 ** -8 * (x @ m.T).abs() * 1.01 + K * 2.0 ** -23 * (x.abs() @ m.abs().T) + 1e-30).all())
+
+
+@pytest.mark.parametrize("T", [5, 40])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_matrices_in_a_wider_block(T, dtype):
+    """A head's matrix may be part of a larger block per head: the bits of the same matrices side by side."""
+    from fellm_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    H, N, K = 3, 40, 64
+    block = torch.randn(H, N + 24, K, generator=g).to(dtype).cuda()
+    a = torch.randn(T, H * K, generator=g).to(dtype).cuda()
+    out = [torch.empty(T, H * N, dtype=dtype, device="cuda") for _ in range(2)]
+    ops.head_gemm(a, block[:, 24:], out[0], a_head=K, out_head=N)
+    ops.head_gemm(a, block[:, 24:].contiguous(), out[1], a_head=K, out_head=N)
+    assert torch.equal(*out)

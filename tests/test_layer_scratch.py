@@ -5,6 +5,8 @@ import pytest
 import torch
 
 from fellm_b200 import ops
+from fellm_b200.parts.base import build_part
+from fellm_b200.parts.spec import PartSpec
 
 
 def test_latents_per_head_have_a_limit():
@@ -19,6 +21,19 @@ def test_latents_per_head_have_a_limit():
                 n = rows(H, n_items, longest, T)
                 assert n_items * n * (512 + 64 + H * 256) * 2 <= ops.LAYER_SCRATCH_MAX_BYTES
     assert rows(16, 53, 78, 4096) == 0 and rows(64, 4, 1024, 4096) > 0
+
+
+def test_value_projections_are_held_once():
+    spec = PartSpec.make("latent_attention", size=256, heads=2, dim=128, rot_dim=64, v_dim=128, q_rank=64, kv_rank=128, scale=0.1, norm_eps=1e-5,
+                         window=64, position=PartSpec.make("rope", rot_dim=64, theta=10000.0, pairing="adjacent"))
+    part = build_part("mixer", spec, "bfloat16")
+    g = torch.Generator().manual_seed(1)
+    w = {n: torch.randn(d.shape, generator=g).to(torch.bfloat16 if len(d.shape) > 1 else torch.float32) for n, d in part.param_decls().items()}
+    uv = w["uv.weight"].clone()
+    part.bind(dict(w))
+    kv, got = part.w["kv.weight"], part.w["uv.weight"]
+    assert got.untyped_storage().data_ptr() == kv.untyped_storage().data_ptr()
+    assert torch.equal(got.reshape(256, 128), uv)
 
 
 @pytest.mark.gpu
