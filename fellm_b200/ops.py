@@ -1596,13 +1596,19 @@ PREFETCH_MAX_BYTES = int(os.environ.get("FELLM_B200_WEIGHT_PREFETCH_MAX_MB", 48)
 
 def register_weight_chain(weights):
     """weights: the bfloat16 matrices of a decode step in the order its products read them (the last
-    is followed by the first: the next step).  Replaces what was registered before for these matrices."""
+    is followed by the first: the next step).  Replaces what was registered before for these matrices.  An entry lasts as long as
+    the memory of both its matrices, whichever tensors name it: another tensor may come to lie there afterwards."""
     ws = [w for w in weights if w is not None and w.dtype == torch.bfloat16 and w.is_cuda and w.is_contiguous()]
     for w, nxt in zip(ws, ws[1:] + ws[:1]):
-        at = w.data_ptr()
-        _next_weight[at] = (nxt.data_ptr(), min(nxt.numel() * 2, PREFETCH_MAX_BYTES))
-        # (a matrix that goes takes its entry along: another tensor may come to lie there, and what was next is gone as well)
-        weakref.finalize(w, _next_weight.pop, at, None)
+        at, entry = w.data_ptr(), (nxt.data_ptr(), min(nxt.numel() * 2, PREFETCH_MAX_BYTES))
+        _next_weight[at] = entry
+        for t in (w, nxt):
+            weakref.finalize(t.untyped_storage(), _forget_next, at, entry)
+
+
+def _forget_next(at, entry):
+    if _next_weight.get(at) is entry:
+        _next_weight.pop(at, None)
 
 
 PREFETCH_MAX_ROWS = 16     # measured on B200: 2% off a step of 1 or 8 rows, 1-6% ON a step of 64 (its products are short of bandwidth, not of latency)

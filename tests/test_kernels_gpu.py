@@ -934,3 +934,19 @@ def test_decode_conv_product_of_17_to_128_rows_equals_product_then_convolution(M
     untouched = [s for s in range(140) if s not in slots]
     assert torch.equal(st_a[untouched], state[untouched]) and torch.equal(st_a[:, 0], state[:, 0])
     ops.forget_norm_handoff()
+
+
+def test_weight_chain_lasts_as_long_as_the_memory():
+    """An entry of the prefetch chain stays while any tensor names its matrix's memory, and goes with it or with the next one's."""
+    before = dict(ops._next_weight)
+    a, b, c = (torch.zeros(16, 64, dtype=torch.bfloat16, device=DEV) for _ in range(3))
+    ops.register_weight_chain([a, b, c])
+    at = [t.data_ptr() for t in (a, b, c)]
+    view = a.view(64, 16)
+    del a
+    assert at[0] in ops._next_weight and ops._next_weight[at[0]][0] == at[1]
+    del c                                          # the last: what led to it goes too
+    assert at[2] not in ops._next_weight and at[1] not in ops._next_weight and at[0] in ops._next_weight
+    del view
+    assert at[0] not in ops._next_weight and {k: v for k, v in ops._next_weight.items() if k not in at} == {k: v for k, v in before.items() if k not in at}
+    del b
