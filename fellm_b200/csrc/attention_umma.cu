@@ -578,6 +578,21 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
 typedef CUresult (*AuEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static int au_encode(const void* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], CUtensorMap* out) {
+  static const AuEncodeTiledFn fn = []() -> AuEncodeTiledFn {         // (looked up once, whichever thread comes first)
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+               ? (AuEncodeTiledFn)p : nullptr;
+  }();
+  if (!fn) return FELLM_ERR_ARG;
+  const cuuint32_t box[3] = {64, AU_PT, 1}, estr[3] = {1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
+}
+
 static int au_pool_map(const bf16* base, int size, int per_key, long long records, int G, CUtensorMap* out) {
   static std::mutex mu;
   static struct { const void* base; long long records; int G, size, per_key; CUtensorMap map; } cache[16];
@@ -585,23 +600,11 @@ static int au_pool_map(const bf16* base, int size, int per_key, long long record
   std::lock_guard<std::mutex> lock(mu);
   for (int i = 0; i < n_cached; ++i)
     if (cache[i].base == base && cache[i].records == records && cache[i].G == G && cache[i].size == size && cache[i].per_key == per_key) { *out = cache[i].map; return 0; }
-  static AuEncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
-      return FELLM_ERR_ARG;
-    fn = (AuEncodeTiledFn)p;
-  }
-  cuuint64_t dims[3] = {(cuuint64_t)size, (cuuint64_t)G * AU_PT, (cuuint64_t)records};
-  cuuint64_t strides[2] = {(cuuint64_t)size * 2, (cuuint64_t)G * AU_PT * per_key * 2};
-  cuuint32_t box[3] = {64, AU_PT, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
+  const cuuint64_t dims[3] = {(cuuint64_t)size, (cuuint64_t)G * AU_PT, (cuuint64_t)records};
+  const cuuint64_t strides[2] = {(cuuint64_t)size * 2, (cuuint64_t)G * AU_PT * per_key * 2};
   CUtensorMap m;
-  CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return 1000 + (int)r;
+  const int e = au_encode(base, dims, strides, &m);
+  if (e) return e;
   cache[next].base = base; cache[next].records = records; cache[next].G = G; cache[next].size = size; cache[next].per_key = per_key; cache[next].map = m;
   next = (next + 1) % 16;
   if (n_cached < 16) ++n_cached;
@@ -685,26 +688,13 @@ FELLM_API int fellm_attn_latent_umma(const void* q, int ldq, const void* kv, con
   a.block_table = positions; a.row_slot = positions;            // (there are no pages: addresses that are valid, times max_pages = 0)
   a.max_pages = 0; a.sinks = sinks; a.H = H; a.G = H; a.layers_in_group = 1; a.scale_log2 = scale * 1.4426950408889634f;
   a.window = window; a.key_rows = key_rows;
-  static AuEncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess)
-      return FELLM_ERR_ARG;
-    fn = (AuEncodeTiledFn)p;
-  }
   CUtensorMap maps[2];
   const cuuint64_t cols[2] = {(cuuint64_t)H * (AU_KD - AU_LAT_ROPE + AU_VD), AU_LAT_ROPE};
   const void* base[2] = {kv, rope};
   for (int i = 0; i < 2; ++i) {
-    cuuint64_t dims[3] = {cols[i], (cuuint64_t)rows, 1};
-    cuuint64_t strides[2] = {cols[i] * 2, cols[i] * 2 * (cuuint64_t)rows};
-    cuuint32_t box[3] = {64, AU_PT, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base[i]), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return 1000 + (int)r;
+    const cuuint64_t dims[3] = {cols[i], (cuuint64_t)rows, 1}, strides[2] = {cols[i] * 2, cols[i] * 2 * (cuuint64_t)rows};
+    const int e = au_encode(base[i], dims, strides, &maps[i]);
+    if (e) return e;
   }
   const size_t smem = (size_t)AU_FIXED_B + (size_t)AU_STAGES * AU_STAGE_B + 1024;
   auto kern = attention_prefill_umma_kernel;
