@@ -546,7 +546,11 @@ attention_prefill_umma_kernel(const __grid_constant__ CUtensorMap k_map, const _
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float2 z = __bfloat1622float2(h2[e]);
-            o[8 * ch + 2 * e] *= __fdividef(1.0f, 1.0f + __expf(-z.x)); o[8 * ch + 2 * e + 1] *= __fdividef(1.0f, 1.0f + __expf(-z.y));
+            if constexpr (AU_GENERAL) {            // (the full functions, as the kernel has them that gated these layers' rows before)
+              o[8 * ch + 2 * e] *= 1.0f / (1.0f + expf(-z.x)); o[8 * ch + 2 * e + 1] *= 1.0f / (1.0f + expf(-z.y));
+            } else {
+              o[8 * ch + 2 * e] *= __fdividef(1.0f, 1.0f + __expf(-z.x)); o[8 * ch + 2 * e + 1] *= __fdividef(1.0f, 1.0f + __expf(-z.y));
+            }
           }
         }
       }
