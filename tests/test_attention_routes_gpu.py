@@ -82,11 +82,11 @@ FORMS = [dict(window=70), dict(chunk=48), dict(window=100, slopes=True, temp=(0.
          dict(cap=2.0, temp=(0.5, 16)), dict(cap=4.0, temp=(0.5, 16), slopes=True, window=100)]
 
 
-def form(spec, T, H, g):
+def form(spec, T, H, g, hd=64):
     kw = dict(spec)
     slopes = torch.rand(H, generator=g) * 0.2 if kw.pop("slopes", False) else None
     gate = torch.randn(T, H + 3, generator=g) if kw.pop("gate", False) else None
-    out_gate = torch.randn(T, H * 64 + 8, generator=g).bfloat16() if kw.pop("out_gate", False) else None
+    out_gate = torch.randn(T, H * hd + 8, generator=g).bfloat16() if kw.pop("out_gate", False) else None
     return kw, slopes, gate, out_gate
 
 
@@ -128,8 +128,6 @@ def test_portions_on_tcgen05(spec, H, G, keys_alone):
                                                            (8, 2, 64, 256, False, 1), (8, 2, 128, 32, True, 8)])
 def test_rows_over_a_cluster(spec, H, G, hd, page, keys_alone, cluster, monkeypatch):
     from fellm_b200 import ops
-    if hd != 64 and "out_gate" in spec:
-        return
     monkeypatch.setattr(ops, "attention_rows_cluster", lambda *a: cluster)
     g = torch.Generator().manual_seed(H + G)
     lens = [1, 31, 33, 130, 700]
@@ -142,7 +140,7 @@ def test_rows_over_a_cluster(spec, H, G, hd, page, keys_alone, cluster, monkeypa
         if vd:
             pages.v[r][-1] = q[r, (H + G) * hd:(H + 2 * G) * hd].view(G, hd)
     pos = torch.tensor([n - 1 for n in lens])
-    kw, slopes, gate, out_gate = form(spec, T, H, g)
+    kw, slopes, gate, out_gate = form(spec, T, H, g, hd)
     pool = pages.pool if keys_alone else pages.five(G, hd)
     i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()  # noqa: E731
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
@@ -158,6 +156,8 @@ def test_rows_over_a_cluster(spec, H, G, hd, page, keys_alone, cluster, monkeypa
     got = call(write)
     assert int(status) == 0
     again = call(None, with_gate=False)          # the CUDA-core kernel, which reads the rows' keys and values from their pages now
+    if out_gate is not None:
+        assert torch.equal(call(None), got)      # and this kernel, reading them from there
     for r in range(T):
         want = attend(q[r:r + 1, :H * hd].double().view(1, H, hd), pages.k[r].double(), pages.v[r].double(), pos[r:r + 1], hd ** -0.5,
                       slopes=None if slopes is None else slopes.double(), **kw)
