@@ -37,12 +37,14 @@ class StepContext:
     tokens[T], positions[T] (absolute), row_item[T] (index of the row's item), row_slot[T] (its
     request's slot: the row of block tables and state arrays), item_start[n_items+1] (row offsets),
     item_slot[n_items], item_len[n_items] (request length after this step), logit_rows[W].
+    own_rows: how many of the rows, the first ones, belong to a request (fewer than n_rows in a decode step that is filled up for
+    its products' sake: attention and the greedy head then run on these rows alone).
     carried: what a part leaves for a later part of the same step (rows of this step's tokens, by name); a model's
     forward() starts and ends with it empty.
     """
     __slots__ = ("tokens", "positions", "row_item", "row_slot", "item_start", "item_slot", "item_len",
                  "logit_rows", "n_rows", "n_items", "n_logit_rows", "all_single", "max_item_rows",
-                 "max_len", "status", "host", "logits_all", "fixed_addresses", "carried")
+                 "max_len", "status", "host", "logits_all", "fixed_addresses", "carried", "own_rows")
 
 
 class StepBuffers:
@@ -97,7 +99,7 @@ class StepBuffers:
         if self.on_gpu:
             self.ring_events[k].record()
             self.ring_used[k] = True
-        ctx.n_rows, ctx.n_items, ctx.n_logit_rows = T, n, W
+        ctx.n_rows, ctx.n_items, ctx.n_logit_rows, ctx.own_rows = T, n, W, T
         ctx.all_single = (T == n)
         ctx.logits_all = (W == T and list(logit_rows) == list(range(T)))
         ctx.max_item_rows, ctx.max_len = max_item_rows, max_len
@@ -107,8 +109,8 @@ class StepBuffers:
         return ctx
 
 
-def _fill_decode(self, plan, wants, toks, lens) -> StepContext:
-    """The decode form of fill(): n items of one row each.  The layout of the buffer is the one
+def _fill_decode(self, plan, wants, toks, lens, own_rows) -> StepContext:
+    """The decode form of fill(): n items of one row each, the first own_rows of them a request's.  The layout of the buffer is the one
     fill() makes for T = n; the parts that only depend on the composition are written once per
     staging buffer."""
     n = len(lens)
@@ -152,7 +154,7 @@ def _fill_decode(self, plan, wants, toks, lens) -> StepContext:
         ctx.status, ctx.host = self.status, None
         ctx.fixed_addresses = True
         self._decode_ctx[(n, W)] = ctx
-    ctx.logits_all = (W == n)
+    ctx.logits_all, ctx.own_rows = (W == n), own_rows
     ctx.max_len = int(lens.max()) + 1
     return ctx
 
@@ -175,9 +177,11 @@ def few_rows_pad_from(model) -> int:
     there and filled up to 24 rows: width 1536 1 row 0.628 ms there, 2 rows 0.668 and 0.618, 8 rows 0.705 and 0.619, 16 rows 0.885
     and 0.625; width 2048 8 rows 0.824 there, 9 rows 0.894 and 0.833, 16 rows 0.883 and 0.835; width 1024 stays (16 rows 0.415, 17
     rows as 24 0.454).
-    Only models of attention, short convolutions and dense feed-forwards: rows that belong to nobody would send experts' matrices
-    and recurrent states through memory."""
-    plain = all(b.mixer.kind in ("attention", "shortconv") and b.ffn is not None and b.ffn.kind == "swiglu" for b in model.blocks)
+    Only models of LFM2's parts (attention without further forms, short convolutions, dense feed-forwards): rows that belong to
+    nobody would send experts' matrices and recurrent states through memory, and the other attention kernels take them for
+    rows like any other."""
+    plain = all(b.mixer.kind in ("attention", "shortconv") and not getattr(b.mixer, "general", False) and b.ffn is not None
+                and b.ffn.kind == "swiglu" for b in model.blocks)
     width = model.spec.hidden_size
     if not plain or width <= 1024 or width % 32 or model.act_dtype != torch.bfloat16:
         return 17
@@ -313,9 +317,10 @@ class Stepper:
         # A graph is captured for every count of rows a decode step has; from 17 rows on the count is filled up
         # to a multiple of 8 with rows that belong to nobody (the cache's pad slot: position 0 of a page of its
         # own, a state row of its own), so that a batch that grows or drains by one request at a time meets a
-        # new graph every eighth count, not at every one.  Up to 16 rows each count has kernels of its own cost.
+        # new graph every eighth count, not at every one.  Up to 16 rows each count has kernels of its own cost and a
+        # graph of its own, also where the rows are filled up to FEW_ROWS_PAD because the products are then faster on
+        # tcgen05 (few_rows_pad_from): attention's key ranges are planned for the requests' rows.
         n_pad = n
-        # Models whose products of few rows are faster on tcgen05 are filled up to FEW_ROWS_PAD from fewer rows on.
         if self.cuda_graphs and n >= min(17, self.pad_from) and all(wants):
             n_pad = -(-max(n, FEW_ROWS_PAD if n < 17 else n) // DECODE_ROWS_STEP) * DECODE_ROWS_STEP
             if n_pad > self.buffers.max_items:
@@ -355,7 +360,7 @@ class Stepper:
             lens = np.concatenate([lens, fill])
             # (token 0 for the padding rows, also where the real rows' tokens come from the device)
             toks = np.zeros(n_pad, dtype=np.int64) if toks is None else np.concatenate([toks, fill])
-        ctx = self.buffers.fill_decode(plan, wants, toks, lens)
+        ctx = self.buffers.fill_decode(plan, wants, toks, lens, n if n < 17 else n_pad)
         if device_tokens is not None:
             ctx.tokens[:n].copy_(device_tokens[:n])
         cache.flush()
@@ -379,7 +384,7 @@ class Stepper:
         # key-range split of decode attention).  Other steps (portions of prompts, mixed batches)
         # repeat their shape when prompts are cut into equal portions: a few of their graphs are kept.
         if ctx.all_single:
-            key = (ctx.n_items, ctx.n_logit_rows, -(-ctx.max_len // 1024), greedy_key)
+            key = (ctx.n_items, ctx.n_logit_rows, -(-ctx.max_len // 1024), greedy_key, ctx.own_rows)
         else:
             key = ("rows", ctx.n_rows, ctx.n_items, ctx.n_logit_rows, ctx.max_item_rows, ctx.logits_all, greedy_key)
         entry = self.graphs.get(key)

@@ -357,8 +357,12 @@ class Model:
         else:
             xf = self.final_norm.forward(x, self.act_dtype, rows=ctx.logit_rows)
         ctx.carried = {}
-        if greedy_tokens is not None and self.head.forward_greedy(xf, greedy_tokens):
-            return None
+        if greedy_tokens is not None:
+            own, xg = getattr(ctx, "own_rows", xf.shape[0]), xf
+            if ctx.logits_all and own < xf.shape[0]:         # a step filled up with rows that are nobody's
+                xg = LazyNorm(xf.x[:own], xf.norm, xf.act_dtype) if isinstance(xf, LazyNorm) else xf[:own]
+            if self.head.forward_greedy(xg, greedy_tokens):
+                return None
         return self.head.forward(xf)
 
 

@@ -2424,8 +2424,11 @@ def paged_attention(q, cache, ctx, scale, window=None):
     brings one token."""
     if q.dtype == torch.bfloat16:
         if ctx.all_single:
-            return attention_decode(q, cache.pool, cache.block_table, ctx.positions, ctx.row_slot, cache.layer,
-                                    scale, window, ctx.max_len)
+            n = getattr(ctx, "own_rows", q.shape[0])
+            out = torch.empty((q.shape[0], q.shape[1] * q.shape[2]), dtype=q.dtype, device=q.device)
+            attention_decode(q[:n], cache.pool, cache.block_table, ctx.positions[:n], ctx.row_slot[:n], cache.layer, scale, window,
+                             ctx.max_len, out=out[:n])
+            return out
         return attention_prefill(q, cache.pool, cache.block_table, ctx.positions, ctx.row_slot, ctx.item_start,
                                  ctx.n_items, ctx.max_item_rows, cache.layer, scale, window)
     return paged_attention_simt(q, cache.pool, cache.block_table, ctx.positions, ctx.row_slot, cache.layer,

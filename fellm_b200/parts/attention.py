@@ -224,10 +224,13 @@ class Attention(Mixer):
         qkv = linear(xn, self.w["qkv.weight"])
         if (ctx.all_single and not self.shares_cache and qkv.dtype == torch.bfloat16 and self.rot_dim == self.hd
                 and ops.decode_fuses_rope(self.H, self.G, self.hd, cache.page_tokens, cache.pool)):
-            # a decode step: norm, rotation and the cache write happen inside the attention kernel
-            a = ops.attention_decode(None, cache.pool, cache.block_table, ctx.positions, ctx.row_slot, cache.layer,
-                                     self.scale, self.window, ctx.max_len,
-                                     fuse=(qkv, self.w.get("q_norm.weight"), self.w.get("k_norm.weight"), self.eps,
+            # a decode step: norm, rotation and the cache write happen inside the attention kernel (of the requests' rows:
+            # what the others read out is anything, and nobody reads their rows)
+            n = getattr(ctx, "own_rows", qkv.shape[0])
+            a = torch.empty((qkv.shape[0], self.H * self.hd), dtype=qkv.dtype, device=qkv.device)
+            ops.attention_decode(None, cache.pool, cache.block_table, ctx.positions[:n], ctx.row_slot[:n], cache.layer,
+                                     self.scale, self.window, ctx.max_len, out=a[:n],
+                                     fuse=(qkv[:n], self.w.get("q_norm.weight"), self.w.get("k_norm.weight"), self.eps,
                                            self.position.inv_freq, self.position.pairing))
             linear(a, self.w["out_proj.weight"], out=out, accumulate=True)
             return out

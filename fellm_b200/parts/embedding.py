@@ -62,6 +62,8 @@ class LinearHead(Head):
                 return True
         fused = isinstance(xf, LazyNorm) and xf.fusable_with(w)
         need = ops.head_argmax_scratch(rows, w.shape[0], w.shape[1], fused)
+        if fused and not need:           # (no plan with the norm inside the product: in front of it)
+            fused, need = False, ops.head_argmax_scratch(rows, w.shape[0], w.shape[1], False)
         if not need or need > keys.numel():
             return False
         if fused:
