@@ -173,10 +173,19 @@ def few_rows_pad_from(model) -> int:
     """From how many rows a decode step runs on the few-rows tcgen05 products, filled up to FEW_ROWS_PAD rows (17: as any other).
     Up to 16 rows the products stream their weights through mma.sync slabs, K in slices of 8..10 chunks of 32 and a power of two
     of slices a block: a width that is no power of two of such slices (1536: six) leaves that kernel with clusters of three that
-    are not resident together, and from nine rows on it runs every instruction twice.  Decode steps of 16 LFM2 layers on B200,
-    there and filled up to 24 rows: width 1536 1 row 0.628 ms there, 2 rows 0.668 and 0.618, 8 rows 0.705 and 0.619, 16 rows 0.885
-    and 0.625; width 2048 8 rows 0.824 there, 9 rows 0.894 and 0.833, 16 rows 0.883 and 0.835; width 1024 stays (16 rows 0.415, 17
-    rows as 24 0.454).
+    are not resident together, and from nine rows on it runs every instruction twice.  Decode steps of 16 LFM2 layers on B200 (ms,
+    as they are / filled up to 24 rows; width and feed-forward):
+        1536, 7168: 2 rows 0.683 / 0.650, 8 rows 0.715 / 0.640, 16 rows 0.903 / 0.635; contexts of 16,000: 2 rows 0.815 / 0.806,
+        16 rows 1.433 / 1.163
+        1536, 4608: 2 rows 0.518 / 0.571, 8 rows 0.552 / 0.548, 9 rows 0.674 / 0.576
+        1792, 8192: 2 rows 0.955 / 0.712, 16 rows 1.309 / 0.736
+        2048, 8192: 8 rows 0.835 / 0.859, 9 rows 0.906 / 0.879, 16 rows 0.899 / 0.848
+        2304, 10752: 4 rows 1.426 / 1.397, 9 rows 2.318 / 1.351;  2560, 12288: 8 rows 1.413 / 1.457, 9 rows 2.166 / 1.481
+        3072, 14336: 2 rows 2.974 / 1.685, 16 rows 3.088 / 1.642
+    and where gate and up together have more columns than the few-rows product takes:
+        1536, 9216: 8 rows 0.885 / 1.185, 16 rows 1.087 / 1.178;  2048, 10240: 9 rows 1.024 / 1.274, 16 rows 1.025 / 1.249
+    so such models keep their rows up to width 2048, above which the products of few rows are the slow ones anyway.  Width 1024
+    stays (16 rows 0.415, 17 rows as 24 0.454).
     Only models of LFM2's parts (attention without further forms, short convolutions, dense feed-forwards): rows that belong to
     nobody would send experts' matrices and recurrent states through memory, and the other attention kernels take them for
     rows like any other."""
@@ -185,9 +194,13 @@ def few_rows_pad_from(model) -> int:
     width = model.spec.hidden_size
     if not plain or width <= 1024 or width % 32 or model.act_dtype != torch.bfloat16:
         return 17
+    from .. import ops
+    ff = max(getattr(b.ffn, "ff", 4 * width) for b in model.blocks)
+    if width <= 2048 and 2 * ff > ops.SWAP_MAX_N:
+        return 17
     chunks = width // 32
     if not any(chunks % (1 << i) == 0 and 8 <= chunks >> i <= 10 for i in range(8)):
-        return FEW_ROWS_ODD
+        return FEW_ROWS_ODD if ff >= 4 * width else FEW_ROWS_WIDE          # (a small feed-forward is streamed in time)
     return FEW_ROWS_WIDE if width >= 2048 else 17
 
 

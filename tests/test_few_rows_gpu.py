@@ -19,6 +19,19 @@ def test_which_models_are_filled_up():
     assert few_rows_pad_from(model(1536, dtype=torch.float32)) == 17
 
 
+def test_which_feed_forwards_are_filled_up():
+    """Gate and up within the few-rows product's columns (up to width 2048), and large enough for two rows to gain; LFM2's own parts only."""
+    from fellm_b200.engine.step import few_rows_pad_from
+
+    def pad(width, ff, general=False):
+        block = types.SimpleNamespace(mixer=types.SimpleNamespace(kind="attention", general=general), ffn=types.SimpleNamespace(kind="swiglu", ff=ff))
+        return few_rows_pad_from(types.SimpleNamespace(blocks=[block], spec=types.SimpleNamespace(hidden_size=width), act_dtype=torch.bfloat16))
+    assert [pad(1536, ff) for ff in (4608, 6144, 7168, 8192, 9216)] == [9, 2, 2, 2, 17]
+    assert [pad(2048, ff) for ff in (8192, 9728, 10240)] == [9, 17, 17]
+    assert pad(1792, 8192) == 2 and pad(2304, 10752) == pad(2560, 12288) == 9 and pad(3072, 14336) == 2
+    assert pad(1536, 7168, general=True) == 17
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 2, 7, 16])
 def test_filled_up_steps_give_the_rows_own_logits(n):
@@ -59,7 +72,7 @@ def test_filled_up_steps_plan_for_the_requests_rows(width, n, monkeypatch):
     from fellm_b200.config import EngineOptions
     from fellm_b200.engine import Engine, StepItem
     cfg = dict(architectures=["Lfm2ForCausalLM"], vocab_size=640, hidden_size=width, num_hidden_layers=3, num_attention_heads=width // 64,
-               num_key_value_heads=8, head_dim=64, full_attn_idxs=[1], block_ff_dim=512, block_auto_adjust_ff_dim=False,
+               num_key_value_heads=8, head_dim=64, full_attn_idxs=[1], block_ff_dim=6144 if width == 1536 else 512, block_auto_adjust_ff_dim=False,
                rope_theta=10000.0, rope_pairing="split_half", conv_L_cache=3, conv_bias=False, norm_eps=1e-5, tie_word_embeddings=True,
                max_position_embeddings=4096)
     options = dict(n_ctx=2048, max_requests=16, max_tokens=16 * 1280, n_batch=2048)
@@ -67,6 +80,7 @@ def test_filled_up_steps_plan_for_the_requests_rows(width, n, monkeypatch):
     g = torch.Generator().manual_seed(n)
     prompts = [torch.randint(0, 640, (1025 + 7 * r,), generator=g).tolist() for r in range(n)]
     follow = torch.randint(0, 640, (n, 4), generator=g).tolist()
+    assert n >= engines[0].stepper.pad_from
     planned, picked = [], []
     split, argmax = ops.decode_split, ops.gemm_bf16_argmax
     monkeypatch.setattr(ops, "decode_split", lambda max_len, rows, *a, **k: planned.append(rows) or split(max_len, rows, *a, **k))
@@ -106,10 +120,11 @@ def test_greedy_generation_of_a_filled_up_batch(monkeypatch):
     from fellm_b200.config import EngineOptions
     from fellm_b200.engine import Engine, GenParams, StepItem
     cfg = dict(architectures=["Lfm2ForCausalLM"], vocab_size=640, hidden_size=1536, num_hidden_layers=3, num_attention_heads=24,
-               num_key_value_heads=8, head_dim=64, full_attn_idxs=[1], block_ff_dim=512, block_auto_adjust_ff_dim=False,
+               num_key_value_heads=8, head_dim=64, full_attn_idxs=[1], block_ff_dim=6144, block_auto_adjust_ff_dim=False,
                rope_theta=10000.0, rope_pairing="split_half", conv_L_cache=3, conv_bias=False, norm_eps=1e-5, tie_word_embeddings=True,
                max_position_embeddings=512)
     e = Engine.random(cfg, 7, EngineOptions(n_ctx=256, max_requests=16, max_tokens=16 * 128, cuda_graphs=True))
+    assert e.stepper.pad_from <= 5
     prompts = [torch.randint(0, 640, (3 + 5 * r,), generator=torch.Generator().manual_seed(r)).tolist() for r in range(5)]
     picked, argmax = [], ops.gemm_bf16_argmax
     monkeypatch.setattr(ops, "gemm_bf16_argmax", lambda x, *a, **k: picked.append(x.shape[0]) or argmax(x, *a, **k))
