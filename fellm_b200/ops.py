@@ -642,14 +642,27 @@ GATED_WRITE_PREP_MIN_ROWS = int(os.environ.get("FELLM_B200_GATED_WRITE_PREP_MIN_
 
 
 # Portions of prompts in chunks of 32 tokens (csrc/recurrent_chunk.cu) in the place of the token-by-token scan: from this many
-# rows of a request's portion on, a whole chunk (the scan costs ~0.3 us a token; a chunk 3 us behind two launches of ~10).
+# rows of a request's portion on, a whole chunk, in steps that have work enough for the two launches.
 RECURRENT_CHUNK_MIN_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_CHUNK_MIN_ROWS", 32))
+# ... by the step's rows beyond one an item, for keys of up to 64 elements and for longer ones.  A scan's time follows the rows of the
+# whole step (its blocks fill the device from one request on), the chunks' barely does: one portion of 32 / 64 / 96 rows, us scan and
+# chunks: delta rule of 16 heads 18.7 and 23.4 / 30.6 and 27.2 / 42.4 and 29.8, of 8 heads 15.3 and 23.7 / 23.1 and 26.7 / 31.5 and
+# 29.5, gated write 13.5 and 17.5 / 18.8 and 19.9 / 24.4 and 22.3, decay and bonus (keys of 64) 8.1 and 14.2 / 12.6 and 16.1 / 16.5 and
+# 18.2; two portions of 48: 47.9 and 35.7, 36.3 and 28.4, 27.1 and 21.6, 18.8 and 17.6.  One portion among single tokens, which keep a
+# scan of their own behind the chunks' launches (15 of them; a portion of 100 rows): 84.2 and 82.5, 71.8 and 77.4, 56.2 and 74.9, 48.3
+# and 54.5, 0.12..0.3 us a row there and half of it here.
+RECURRENT_CHUNK_STEP_ROWS = {64: 120, 128: 90}
+RECURRENT_CHUNK_MIXED_ROWS = 256
 
 
-def recurrent_chunk_rows(dtype) -> int:
-    """What a mixer passes as chunk_rows: the bfloat16 engine's portions run in chunks; the 32-bit engine keeps the scan, and with
-    it the same bits for a prompt under every cut (0: no chunks)."""
-    return RECURRENT_CHUNK_MIN_ROWS if dtype == torch.bfloat16 else 0
+def recurrent_chunk_rows(dtype, n_rows: int, n_items: int, max_item_rows: int, key_dim: int) -> int:
+    """What a mixer passes as chunk_rows for a step of n_rows rows of n_items requests, the longest max_item_rows: the bfloat16 engine's portions run in chunks
+    where the step has rows enough; the 32-bit engine keeps the scan, and with it the same bits for a prompt under every cut
+    (0: no chunks)."""
+    enough = n_rows - n_items >= RECURRENT_CHUNK_STEP_ROWS[64 if key_dim <= 64 else 128]
+    if n_items > 1 and n_rows - max_item_rows == n_items - 1:             # a portion among single tokens
+        enough = max_item_rows >= RECURRENT_CHUNK_MIXED_ROWS
+    return RECURRENT_CHUNK_MIN_ROWS if dtype == torch.bfloat16 and enough else 0
 
 
 def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_items, max_item_rows, min_rows, H, G, dk, dv, out, *,

@@ -139,7 +139,7 @@ class GatedDelta(Mixer):
         o = ops.delta_scan(qkv, off["k"], off["v"], p, off["b"], off["a"], w["A_log"],
                            None if gch is not None else w["dt_bias"], gch, mat_state.states, ctx.item_start,
                            mat_state.item_slot, ctx.n_items, H, G, dk, dv, max_item_rows=ctx.max_item_rows,
-                           chunk_rows=ops.recurrent_chunk_rows(xn.dtype))
+                           chunk_rows=ops.recurrent_chunk_rows(xn.dtype, xn.shape[0], ctx.n_items, ctx.max_item_rows, dk))
         if self.gate == "silu":
             gate, act = p[:, off["g"]:off["g"] + H * dv], "silu"
         else:

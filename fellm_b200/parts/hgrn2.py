@@ -57,7 +57,7 @@ class Hgrn2(Mixer):
         z = linear(h, w["qfv.weight"], out_dtype=torch.float32)
         o = ops.gated_write_scan(z, n, 2 * n, w["lower"], w["f.bias"], cache.states, ctx.item_start, cache.item_slot,
                                  ctx.n_items, self.H, self.dk, self.dv, max_item_rows=ctx.max_item_rows,
-                                 chunk_rows=ops.recurrent_chunk_rows(h.dtype))
+                                 chunk_rows=ops.recurrent_chunk_rows(h.dtype, h.shape[0], ctx.n_items, ctx.max_item_rows, self.dk))
         y = ops.head_norm_gate(o, w["norm.weight"], False, None, None, self.eps, self.H, self.dv, h.dtype)
         linear(y, w["o.weight"], out=out, accumulate=not store)
         return out

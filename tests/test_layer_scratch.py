@@ -36,6 +36,16 @@ def test_value_projections_are_held_once():
     assert torch.equal(got.reshape(256, 128), uv)
 
 
+def test_short_steps_keep_the_scan():
+    bf, rule = torch.bfloat16, ops.recurrent_chunk_rows
+    assert rule(torch.float32, 2048, 1, 2048, 128) == 0
+    for key_dim, rows in ((64, 121), (128, 91)):
+        assert rule(bf, rows, 1, rows, key_dim) == rule(bf, 4 * 32, 4, 32, key_dim) == ops.RECURRENT_CHUNK_MIN_ROWS
+        assert rule(bf, rows - 1, 1, rows - 1, key_dim) == rule(bf, 64, 1, 64, key_dim) == 0
+        assert rule(bf, 200 + 15, 16, 200, key_dim) == 0             # one portion among single tokens
+        assert rule(bf, 256 + 15, 16, 256, key_dim) > 0
+
+
 @pytest.mark.gpu
 def test_recurrences_beyond_the_limit_keep_the_scan(monkeypatch):
     from test_recurrent_chunk_gpu import MODES, Step
