@@ -599,15 +599,22 @@ moe_gemm_mma_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__
 // eight rows of A (more rows: again, the weights then come from L2).  A lane loads 8 consecutive k of rows g and g + 8 and
 // feeds them, and the same k of A's row g, as the k slots {2c, 2c + 1, 2c + 8, 2c + 9} of two MMAs: 16-byte loads of both
 // operands without shared memory, and VU chunks of 32 k (VU KB of weights a warp) on their way at once.  The slices of K of a slab
-// are warps of one block, added in their order.  bfloat16 only; K a multiple of 8.
+// are warps of one block, added in their order.  bfloat16 only; K a multiple of 8.  Every MMA starts from zero and the chunks' are
+// added in pairs, in float32: an MMA that adds into its accumulator truncates.  Relative error of float32 results of 3,328 (6,144)
+// products against float64: one chain of MMAs 3.8e-7 (7.4e-7), here 0.84e-7 (0.88e-7), float32 multiply-adds 0.90e-7 (1.09e-7); both
+// products of 8 tokens 28.8 us either way.
 // A warp a column and float32 FMA, four rows at once, spent its time on the conversions and multiply-adds of the weights it
 // streamed: 8 tokens, two of twelve choices each, width 1,024, experts of 3,328: 27.3 us (up) and 20.6 us (down) there, 15.4
 // and 9.7 here (82 and 41 MB of matrices met); 30 tokens 67 and 64 us there, 26 and 16 here.
 #define VW 8            // warps a block
 #define VU 8            // chunks of 32 k on their way
+__device__ __forceinline__ void slab_mma(float (&s)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(s[0]), "+f"(s[1]), "+f"(s[2]), "+f"(s[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 template <typename TO, bool GATED, int KS>
 __global__ void __launch_bounds__(VW * 32)
-moe_gemv_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__ gather, int top,
+moe_slabs_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__ gather, int top,
                 const bf16* __restrict__ W, TO* __restrict__ C, int ldc, int N, int K,
                 const int* __restrict__ table, const int* __restrict__ n_tiles, int inter, float act_limit, float act_alpha) {
   __shared__ float4 part[VW][32];
@@ -641,15 +648,23 @@ moe_gemv_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__ gat
         const int k = (c0 + u) * 32 + 8 * c;
         x[u] = (live && c0 + u < last && k < K) ? *(const uint4*)(ar + k) : zero;
       }
+      float t[VU][4];                              // a chunk's two MMAs, then sums of neighbours
 #pragma unroll
       for (int u = 0; u < VU; ++u) {
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                     : "+f"(s[0]), "+f"(s[1]), "+f"(s[2]), "+f"(s[3])
-                     : "r"(a[u].x), "r"(b[u].x), "r"(a[u].y), "r"(b[u].y), "r"(x[u].x), "r"(x[u].y));
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                     : "+f"(s[0]), "+f"(s[1]), "+f"(s[2]), "+f"(s[3])
-                     : "r"(a[u].z), "r"(b[u].z), "r"(a[u].w), "r"(b[u].w), "r"(x[u].z), "r"(x[u].w));
+        float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+        slab_mma(lo, a[u].x, b[u].x, a[u].y, b[u].y, x[u].x, x[u].y);
+        slab_mma(hi, a[u].z, b[u].z, a[u].w, b[u].w, x[u].z, x[u].w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[u][i] = lo[i] + hi[i];
       }
+#pragma unroll
+      for (int d = 1; d < VU; d *= 2)
+#pragma unroll
+        for (int u = 0; u < VU; u += 2 * d)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) t[u][i] += t[u + d][i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] += t[0][i];
     }
     if (KS > 1) {
       __syncthreads();                             // (the parts before these have been added)
@@ -681,14 +696,14 @@ moe_gemv_kernel(const bf16* __restrict__ A, int lda, const int* __restrict__ gat
 }
 
 template <typename TO, bool GATED>
-static int moe_gemv_launch(const void* A, int lda, const int* gather, int top, const void* W, void* C, int ldc, int N, int K, const int* table,
-                           const int* n_tiles, int max_tiles, int inter, float act_limit, float act_alpha, cudaStream_t stream) {
+static int moe_slabs_launch(const void* A, int lda, const int* gather, int top, const void* W, void* C, int ldc, int N, int K, const int* table,
+                            const int* n_tiles, int max_tiles, int inter, float act_limit, float act_alpha, cudaStream_t stream) {
   // slices of K of a slab: VU chunks each where there are eight of them or fewer
   const int chunks = (K + 31) / 32, slabs = ceil_div(N, GATED ? 8 : 16);
-#define MOE_GEMV(KS_) moe_gemv_kernel<TO, GATED, KS_><<<dim3(max_tiles, ceil_div(slabs, VW / KS_)), VW * 32, 0, stream>>>((const bf16*)A, lda, gather, \
+#define MOE_SLABS(KS_) moe_slabs_kernel<TO, GATED, KS_><<<dim3(max_tiles, ceil_div(slabs, VW / KS_)), VW * 32, 0, stream>>>((const bf16*)A, lda, gather, \
         top, (const bf16*)W, (TO*)C, ldc, N, K, table, n_tiles, inter, act_limit, act_alpha)
-  if (chunks > 4 * VU) MOE_GEMV(8); else if (chunks > 2 * VU) MOE_GEMV(4); else if (chunks > VU) MOE_GEMV(2); else MOE_GEMV(1);
-#undef MOE_GEMV
+  if (chunks > 4 * VU) MOE_SLABS(8); else if (chunks > 2 * VU) MOE_SLABS(4); else if (chunks > VU) MOE_SLABS(2); else MOE_SLABS(1);
+#undef MOE_SLABS
   return launch_status();
 }
 
@@ -703,8 +718,8 @@ FELLM_API int fellm_moe_gemm(const void* A, int a_bf16, int lda, const int* gath
   if (a_bf16 != w_bf16 || (!gated && c_bf16) || (gated && c_bf16 != a_bf16)) return FELLM_ERR_ARG;
   const bool mma = use_mma && a_bf16 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0;
   if (mma && few_rows) {
-    return gated ? moe_gemv_launch<bf16, true>(A, lda, gather, top, W, C, ldc, N, K, table, n_tiles, max_tiles, inter, act_limit, act_alpha, stream)
-                 : moe_gemv_launch<float, false>(A, lda, gather, top, W, C, ldc, N, K, table, n_tiles, max_tiles, inter, act_limit, act_alpha, stream);
+    return gated ? moe_slabs_launch<bf16, true>(A, lda, gather, top, W, C, ldc, N, K, table, n_tiles, max_tiles, inter, act_limit, act_alpha, stream)
+                 : moe_slabs_launch<float, false>(A, lda, gather, top, W, C, ldc, N, K, table, n_tiles, max_tiles, inter, act_limit, act_alpha, stream);
   }
   if (mma) {
     dim3 grid(max_tiles, (N + TB - 1) / TB);

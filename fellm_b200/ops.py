@@ -937,7 +937,7 @@ MOE_MAX_TOP = 16
 MOE_MMA = os.environ.get("FELLM_B200_MOE_MMA", "1") != "0"
 MOE_UMMA = os.environ.get("FELLM_B200_MOE_UMMA", "1") != "0"
 MOE_UMMA_MIN_PAIRS = int(os.environ.get("FELLM_B200_MOE_UMMA_MIN_PAIRS", 256))     # fewer (token, choice) pairs: mma.sync tiles of 64 rows
-MOE_FEW_PAIRS = int(os.environ.get("FELLM_B200_MOE_FEW_PAIRS", 64))                # up to this many: a warp a column (weight streaming)
+MOE_FEW_PAIRS = int(os.environ.get("FELLM_B200_MOE_FEW_PAIRS", 64))                # up to this many: slabs of 16 weight rows (weight streaming)
 
 
 def moe_route(logits, E: int, top: int, renormalize: bool = False):
@@ -1028,7 +1028,7 @@ def moe_gemm(a, w, plan: MoePlan, *, gated: bool, gather: bool, interleaved: boo
     a's dtype (w's rows: gate rows then up rows, or, interleaved, blocks of 8 gate and 8 up rows by turns); else
     float32.  act = (limit, alpha): the gated activation is the clamped form min(g, limit) sigmoid(alpha min(g, limit))
     (clamp(u, -limit, limit) + 1) instead.  Returns [P, N] in sorted order.
-    bfloat16: tcgen05 (tiles of 128 rows, the plan made for them), a warp a column for a handful of pairs, mma.sync
+    bfloat16: tcgen05 (tiles of 128 rows, the plan made for them), slabs of 16 weight rows for a handful of pairs, mma.sync
     tiles of 64 rows between; float32, or sizes those do not take: float32 FMA."""
     _dev(a, w)
     assert a.stride(1) == 1 and w.is_contiguous() and a.dtype == w.dtype

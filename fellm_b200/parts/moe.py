@@ -21,7 +21,7 @@ grouped products, the weighted sum reads h for them.
 
 Experts have no biases.  Nothing goes through the host: the router's choices are sorted by expert on the device
 (ops.moe_plan; the router's product and the routing are one launch, ops.moe_router) and two grouped products walk
-the sorted rows (tcgen05 for steps of many rows, mma.sync tiles between, a warp a column for a handful of tokens), the first gathering its input rows by token and
+the sorted rows (tcgen05 for steps of many rows, mma.sync tiles between, slabs of 16 weight rows for a handful of tokens), the first gathering its input rows by token and
 applying SiLU(gate) * up in its epilogue, the second leaving float32 rows that ops.moe_combine adds, weighted, into
 the residual stream.  A token's result does not depend on what else is in the step.
 """

@@ -37,3 +37,20 @@ def test_few_pairs(N, K, gated, interleaved, tokens):
         y = torch.nn.functional.silu(gate) * up
     # float32 sums of K exact products; gated: gate and up round to bfloat16 (2^-9 each), their product once more
     assert float((got - y).norm() / y.norm()) < (6e-3 if gated else 2e-6)
+
+
+@pytest.mark.parametrize("N,K,tokens", [(1024, 1024, 8), (1024, 3328, 8), (1024, 3328, 30), (2048, 6144, 8)])
+def test_sums_are_rounded_not_truncated(N, K, tokens):
+    """Float32 results: as near float64 as float32 multiply-adds are (0.7 to 1.1e-7 at these sizes; one chain of accumulating MMAs, which
+    truncate, is 2.4 to 7.4e-7 away)."""
+    from fellm_b200 import ops
+    g = torch.Generator().manual_seed(N + K + tokens)
+    E, top = 8, 2
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(tokens)]).to(torch.int32).cuda()
+    plan = ops.moe_plan(idx, E)
+    a = torch.randn(tokens, K, generator=g).bfloat16().cuda()
+    w = (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16().cuda()
+    got = ops.moe_gemm(a, w, plan, gated=False, gather=True).double()
+    order = plan.sorted.long()
+    want = torch.einsum("pk,pnk->pn", a.double()[order // top], w.double()[idx.reshape(-1).long()[order]])
+    assert float((got - want).norm() / want.norm()) < 1.3e-7
