@@ -108,29 +108,30 @@ struct UmmaArgs {
   float glu_limit = 0.f, glu_alpha = 1.f;     // the gated epilogue's activation (glu_act): 0 = SiLU(gate) * up
 };
 
-// One 32-column chunk of an output row: v[j] is C[m][n + j].
-// `res`: for EPI_ACC, the 32 values out already holds there, loaded while the MMAs ran (or null).
+// A warp's 32 rows x 32 columns of the result: lane r holds row m_w + r, v[j] is its column n + j.  Tensor memory gives a
+// lane a ROW, and a store of 16 bytes by 32 lanes a row apart is 32 half-filled sectors: the epilogue of a 128 x 256 tile of
+// float32 sums cost some 9 us of load/store slots so (out += of 2,048 x 2,048, K = 2,048: 38.1 us so, 20.2 with whole
+// rows; 2,048 x 2,048, K = 8,192 67.4 -> 51.5; float32 store of 1,537 x 3,072, K = 1,024 26.5 -> 19.2).  So the 4 KB go
+// through shared memory (`stage`, the warp's own; 16-byte pieces at their place XOR row, so that neither side meets a bank
+// twice) and leave as whole rows: 8 lanes x 16 bytes a row of float32, 4 lanes a row of bfloat16.
+// rows: how many of the 32 rows count.  `res`: for EPI_ACC, what load_residual() brought while the MMAs ran.
 template <int EPI>
-__device__ __forceinline__ void store_chunk(const UmmaArgs& a, float* v, int m, int n, const float4* res = nullptr) {
-  if (EPI == EPI_SWIGLU) {
-    // columns: 8 gate, 8 up, 8 gate, 8 up -> 16 features
-    bf16* dst = (bf16*)a.out + (size_t)m * a.ldo + (n >> 1);
+__device__ __forceinline__ bool chunk_rows_whole(const UmmaArgs& a, int n) {       // 16-byte pieces of a row are in or out as a whole
+  constexpr int PIECE = epi_bf16<EPI>() ? 8 : 4;
+  return (a.ldo % PIECE) == 0 && ((uintptr_t)a.out & 15) == 0 && (n + 32 <= a.N || (a.N % PIECE) == 0);
+}
+__device__ __forceinline__ void load_residual(const UmmaArgs& a, float4* res, int m_w, int rows, int n) {
+  const int lane = threadIdx.x & 31, c = n + 4 * (lane & 7);
+  if (!chunk_rows_whole<EPI_ACC>(a, n)) return;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (n + 16 * h >= a.N) break;
-      unsigned packed[4];
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        float g0 = v[16 * h + j], g1 = v[16 * h + j + 1], u0 = v[16 * h + 8 + j], u1 = v[16 * h + 9 + j];
-        if (a.bias) { g0 += a.bias[n + 16 * h + j]; g1 += a.bias[n + 16 * h + j + 1]; u0 += a.bias[n + 16 * h + 8 + j]; u1 += a.bias[n + 16 * h + 9 + j]; }
-        __nv_bfloat162 p = __floats2bfloat162_rn(glu_act(g0, u0, a.glu_limit, a.glu_alpha), glu_act(g1, u1, a.glu_limit, a.glu_alpha));
-        packed[j >> 1] = *(unsigned*)&p;
-      }
-      *(uint4*)(dst + 8 * h) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    }
-    return;
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3);
+    if (r < rows && c < a.N) res[i] = *(const float4*)((const float*)a.out + (size_t)(m_w + r) * a.ldo + c);
   }
-  const bool whole = n + 32 <= a.N;
+}
+template <int EPI>
+__device__ __forceinline__ void store_chunk(const UmmaArgs& a, float* v, int m_w, int rows, int n, const float4* res, uint4* stage) {
+  const int lane = threadIdx.x & 31;
   if (a.bias) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) if (n + j < a.N) v[j] += a.bias[n + j];
@@ -139,33 +140,92 @@ __device__ __forceinline__ void store_chunk(const UmmaArgs& a, float* v, int m, 
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = relu2_f(v[j]);
   }
-  if (epi_bf16<EPI>() && whole && (a.ldo % 8) == 0) {
-    uint4* dst = (uint4*)((bf16*)a.out + (size_t)m * a.ldo + n);         // 64 contiguous bytes of this row
+  if (!chunk_rows_whole<EPI>(a, n)) {
+    if (lane < rows) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (n + j >= a.N) break;
+        size_t o = (size_t)(m_w + lane) * a.ldo + n + j;
+        if (epi_bf16<EPI>()) ((bf16*)a.out)[o] = __float2bfloat16_rn(v[j]);
+        else if (EPI == EPI_ACC) ((float*)a.out)[o] += v[j];
+        else ((float*)a.out)[o] = v[j];
+      }
+    }
+    return;
+  }
+  if (epi_bf16<EPI>()) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      __nv_bfloat162 p0 = __floats2bfloat162_rn(v[8 * j], v[8 * j + 1]), p1 = __floats2bfloat162_rn(v[8 * j + 2], v[8 * j + 3]);
-      __nv_bfloat162 p2 = __floats2bfloat162_rn(v[8 * j + 4], v[8 * j + 5]), p3 = __floats2bfloat162_rn(v[8 * j + 6], v[8 * j + 7]);
-      dst[j] = make_uint4(*(unsigned*)&p0, *(unsigned*)&p1, *(unsigned*)&p2, *(unsigned*)&p3);
-    }
-  } else if (!epi_bf16<EPI>() && whole && (a.ldo % 4) == 0) {
-    float4* dst = (float4*)((float*)a.out + (size_t)m * a.ldo + n);       // 128 contiguous bytes of this row
+      __nv_bfloat162 p[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float4 r = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-      if (EPI == EPI_ACC) { float4 o = res ? res[j] : dst[j]; r.x += o.x; r.y += o.y; r.z += o.z; r.w += o.w; }
-      dst[j] = r;
+      for (int k = 0; k < 4; ++k) p[k] = __floats2bfloat162_rn(v[8 * j + 2 * k], v[8 * j + 2 * k + 1]);
+      stage[4 * lane + (j ^ ((lane >> 1) & 3))] = make_uint4(*(unsigned*)&p[0], *(unsigned*)&p[1], *(unsigned*)&p[2], *(unsigned*)&p[3]);
+    }
+    __syncwarp();
+    const int c = lane & 3;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = 8 * i + (lane >> 2);
+      const uint4 x = stage[4 * r + (c ^ ((r >> 1) & 3))];
+      if (r < rows && n + 8 * c < a.N) *(uint4*)((bf16*)a.out + (size_t)(m_w + r) * a.ldo + n + 8 * c) = x;
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if (n + j >= a.N) break;
-      size_t o = (size_t)m * a.ldo + n + j;
-      if (epi_bf16<EPI>()) ((bf16*)a.out)[o] = __float2bfloat16_rn(v[j]);
-      else if (EPI == EPI_ACC) ((float*)a.out)[o] += v[j];
-      else ((float*)a.out)[o] = v[j];
+    for (int j = 0; j < 8; ++j) ((float4*)stage)[8 * lane + (j ^ (lane & 7))] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    __syncwarp();
+    const int c = lane & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = 4 * i + (lane >> 3);
+      float4 x = ((const float4*)stage)[8 * r + (c ^ (r & 7))];
+      if (r < rows && n + 4 * c < a.N) {
+        if (EPI == EPI_ACC) { x.x += res[i].x; x.y += res[i].y; x.z += res[i].z; x.w += res[i].w; }
+        *(float4*)((float*)a.out + (size_t)(m_w + r) * a.ldo + n + 4 * c) = x;
+      }
     }
   }
+  __syncwarp();                                                // the next chunk writes the same 4 KB
 }
+// The gated form: columns are 8 gate, 8 up, 8 gate, 8 up, so a chunk is 16 features: 32 bytes of a row, a whole sector, which a lane
+// stores itself (transposed like the others: 1,800 x 14,336, K = 1,536 70.8 us for 66.3, the operands' own traffic through
+// shared memory being what binds there).
+__device__ __forceinline__ void store_gated(const UmmaArgs& a, const float* v, int m, int n) {
+  bf16* dst = (bf16*)a.out + (size_t)m * a.ldo + (n >> 1);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (n + 16 * h >= a.N) break;
+    unsigned packed[4];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float g0 = v[16 * h + j], g1 = v[16 * h + j + 1], u0 = v[16 * h + 8 + j], u1 = v[16 * h + 9 + j];
+      if (a.bias) { g0 += a.bias[n + 16 * h + j]; g1 += a.bias[n + 16 * h + j + 1]; u0 += a.bias[n + 16 * h + 8 + j]; u1 += a.bias[n + 16 * h + 9 + j]; }
+      __nv_bfloat162 p = __floats2bfloat162_rn(glu_act(g0, u0, a.glu_limit, a.glu_alpha), glu_act(g1, u1, a.glu_limit, a.glu_alpha));
+      packed[j >> 1] = *(unsigned*)&p;
+    }
+    *(uint4*)(dst + 8 * h) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  }
+}
+// What an epilogue warp does with its CHUNKS * 32 columns of a finished accumulator: `take(c0, v)` fetches 32 columns from column c0 of
+// the tile on.  res: the first two chunks' residual values, loaded by the caller under the MMAs; each later chunk's are asked
+// for as soon as their registers are free.
+template <int EPI, int CHUNKS, class Take>
+__device__ __forceinline__ void store_tile(const UmmaArgs& a, Take take, int m_w, int rows, int n0, int c_lo, float4 (*res)[8], uint4* stage) {
+#pragma unroll
+  for (int ch = 0; ch < CHUNKS; ++ch) {
+    const int c0 = c_lo + ch * 32;
+    float v[32];
+    take(c0, v);                                               // (whole warp, also for rows past the end)
+    if (n0 + c0 >= a.N) continue;
+    if (EPI == EPI_SWIGLU) {
+      const int lane = threadIdx.x & 31;
+      if (lane < rows) store_gated(a, v, m_w + lane, n0 + c0);
+      continue;
+    }
+    store_chunk<EPI>(a, v, m_w, rows, n0 + c0, res[EPI == EPI_ACC ? ch & 1 : 0], stage);
+    if (EPI == EPI_ACC && ch + 2 < CHUNKS) load_residual(a, res[ch & 1], m_w, rows, n0 + c0 + 64);
+  }
+}
+#define UM_EPI_STAGE 4096               // bytes of shared memory an epilogue warp transposes a chunk in
 
 // Persistent: a CTA walks over output tiles t = blockIdx.x, + gridDim.x, ... (tiles that follow one another share
 // their weight tile).  Two accumulators in tensor memory: while the epilogue warps read tile i out of one, the MMA
@@ -260,38 +320,25 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   } else {
     // epilogue warps: TMEM lanes 32*(warp%4) .. +32 = output rows; two warps share a quarter, a column half each
     const int q = warp & 3, half = (warp - 2) >> 2;
+    uint4* stage = reinterpret_cast<uint4*>(smem_raw + (tiles - smem_u32(smem_raw)) + STAGES * STAGE_BYTES + (warp - 2) * UM_EPI_STAGE);
     unsigned use = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++use) {
       const unsigned acc = use & 1;
       int m0, w0, n0, rows;
       coords(t, m0, w0, n0, rows);
-      const int m = m0 + q * 32 + lane;
-      const bool row_ok = q * 32 + lane < rows;
-      // += residual: what out holds in this thread's two chunks is fetched while the MMAs of the
+      // += residual: what out holds in this warp's first two chunks is fetched while the MMAs of the
       // tile still run (nothing else writes these elements during the launch)
       constexpr int CHUNKS = BN / 2 / 32;
-      constexpr int PRE = CHUNKS < 2 ? CHUNKS : 2;               // chunks fetched ahead (64 registers)
-      float4 res[EPI == EPI_ACC ? PRE : 1][8];
-      bool res_ok[CHUNKS];
-#pragma unroll
-      for (int ch = 0; ch < CHUNKS; ++ch) {
-        const int n = n0 + half * (BN / 2) + ch * 32;
-        res_ok[ch] = EPI == EPI_ACC && ch < PRE && row_ok && n + 32 <= a.N && (a.ldo % 4) == 0;
-        if (EPI == EPI_ACC && res_ok[ch]) {
-          const float4* src = (const float4*)((const float*)a.out + (size_t)m * a.ldo + n);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) res[ch][j] = src[j];
-        }
+      const int m_w = m0 + q * 32, rows_w = rows - q * 32, c_lo = half * (BN / 2);
+      float4 res[EPI == EPI_ACC ? 2 : 1][8];
+      if (EPI == EPI_ACC) {
+        load_residual(a, res[0], m_w, rows_w, n0 + c_lo);
+        load_residual(a, res[EPI == EPI_ACC ? 1 : 0], m_w, rows_w, n0 + c_lo + 32);
       }
       if (!mbar_wait(accfull0 + 8 * acc, (use >> 1) & 1, a.status, 103)) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll
-      for (int ch = 0; ch < CHUNKS; ++ch) {
-        const int c0 = half * (BN / 2) + ch * 32;
-        float v[32];
-        tmem_ld32(tmem_base + ((unsigned)(q * 32) << 16) + acc * BN + (unsigned)c0, v);      // whole warp, also for rows past M
-        if (row_ok && n0 + c0 < a.N) store_chunk<EPI>(a, v, m, n0 + c0, (EPI == EPI_ACC && res_ok[ch]) ? res[ch < PRE ? ch : 0] : nullptr);
-      }
+      store_tile<EPI, CHUNKS>(a, [&](int c0, float* v) { tmem_ld32(tmem_base + ((unsigned)(q * 32) << 16) + acc * BN + (unsigned)c0, v); },
+                              m_w, rows_w, n0, c_lo, res, stage);
       // this warp has read its part of the accumulator: one of the eight arrivals that free it
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
@@ -406,19 +453,12 @@ gemm_umma_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   } else {
     // epilogue warps: TMEM lanes 32*(warp%4) .. +32 = output rows; two warps share a quarter, a column half each
     const int q = warp & 3, half = (warp - 2) >> 2, row = q * 32 + lane;
-    const int m = m0 + row;
+    const int m_w = m0 + q * 32, rows_w = a.M - m_w, c_lo = half * (BN / 2);
     constexpr int CHUNKS = BN / 2 / 32;                       // 2
-    float4 res[EPI == EPI_ACC ? CHUNKS : 1][8];
-    bool res_ok[CHUNKS];
-#pragma unroll
-    for (int ch = 0; ch < CHUNKS; ++ch) {
-      const int n = n0 + half * (BN / 2) + ch * 32;
-      res_ok[ch] = EPI == EPI_ACC && rank == 0 && m < a.M && n + 32 <= a.N && (a.ldo % 4) == 0;
-      if (EPI == EPI_ACC && res_ok[ch]) {
-        const float4* src = (const float4*)((const float*)a.out + (size_t)m * a.ldo + n);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) res[ch][j] = src[j];
-      }
+    float4 res[EPI == EPI_ACC ? 2 : 1][8];
+    if (EPI == EPI_ACC && rank == 0) {
+      load_residual(a, res[0], m_w, rows_w, n0 + c_lo);
+      load_residual(a, res[EPI == EPI_ACC ? 1 : 0], m_w, rows_w, n0 + c_lo + 32);
     }
     const bool done = mbar_wait(accfull, 0, a.status, 133);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -440,11 +480,10 @@ gemm_umma_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       if (lane == 0) mbar_arrive_cluster(mapa_u32(recvfull, 0));       // (release at cluster scope: the stores above come first)
     } else {
       const bool got = mbar_wait_cluster(recvfull, 0, a.status, 134);
-      if (done && got) {
-#pragma unroll
-        for (int ch = 0; ch < CHUNKS; ++ch) {
-          const int c0 = half * (BN / 2) + ch * 32;
-          float v[32];
+      // (every MMA of this CTA is done and no copy is on its way: the operands' stages are free for the transposition)
+      uint4* stage = reinterpret_cast<uint4*>(smem_raw + (tiles - smem_u32(smem_raw)) + (warp - 2) * UM_EPI_STAGE);
+      if (done && got)
+        store_tile<EPI, CHUNKS>(a, [&](int c0, float* v) {
           tmem_ld32(tmem_base + ((unsigned)(q * 32) << 16) + (unsigned)c0, v);
           const float4* other = reinterpret_cast<const float4*>(recv + row * UK_RECV_LD + c0);
 #pragma unroll
@@ -452,9 +491,7 @@ gemm_umma_ksplit_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
             const float4 o = other[j];
             v[4 * j] += o.x; v[4 * j + 1] += o.y; v[4 * j + 2] += o.z; v[4 * j + 3] += o.w;
           }
-          if (m < a.M && n0 + c0 < a.N) store_chunk<EPI>(a, v, m, n0 + c0, (EPI == EPI_ACC && res_ok[ch]) ? res[ch] : nullptr);
-        }
-      }
+        }, m_w, rows_w, n0, c_lo, res, stage);
     }
   }
   // common exit: every role comes here, also after a wait that gave up.  The second CTA may leave before the first
@@ -596,34 +633,22 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
+    uint4* stage = reinterpret_cast<uint4*>(smem_raw + (tiles - smem_u32(smem_raw)) + STAGES * STAGE_BYTES + (warp - 2) * UM_EPI_STAGE);
     unsigned use = 0;
     for (int t = pair; t < total; t += n_pairs, ++use) {
       const unsigned acc = use & 1;
       const int m0 = (t % m_pairs) * 2 * UM_BM + (int)rank * UM_BM, n0 = (t / m_pairs) * BN;
-      const int m = m0 + q * 32 + lane;
       constexpr int CHUNKS = BN / 2 / 32;
-      constexpr int PRE = CHUNKS < 2 ? CHUNKS : 2;
-      float4 res[EPI == EPI_ACC ? PRE : 1][8];
-      bool res_ok[CHUNKS];
-#pragma unroll
-      for (int ch = 0; ch < CHUNKS; ++ch) {
-        const int n = n0 + half * (BN / 2) + ch * 32;
-        res_ok[ch] = EPI == EPI_ACC && ch < PRE && m < a.M && n + 32 <= a.N && (a.ldo % 4) == 0;
-        if (EPI == EPI_ACC && res_ok[ch]) {
-          const float4* src = (const float4*)((const float*)a.out + (size_t)m * a.ldo + n);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) res[ch][j] = src[j];
-        }
+      const int m_w = m0 + q * 32, rows_w = a.M - m_w, c_lo = half * (BN / 2);
+      float4 res[EPI == EPI_ACC ? 2 : 1][8];
+      if (EPI == EPI_ACC) {
+        load_residual(a, res[0], m_w, rows_w, n0 + c_lo);
+        load_residual(a, res[EPI == EPI_ACC ? 1 : 0], m_w, rows_w, n0 + c_lo + 32);
       }
       if (!mbar_wait(accfull0 + 8 * acc, (use >> 1) & 1, a.status, 123)) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll
-      for (int ch = 0; ch < CHUNKS; ++ch) {
-        const int c0 = half * (BN / 2) + ch * 32;
-        float v[32];
-        tmem_ld32(tmem_base + ((unsigned)(q * 32) << 16) + acc * BN + (unsigned)c0, v);
-        if (m < a.M && n0 + c0 < a.N) store_chunk<EPI>(a, v, m, n0 + c0, (EPI == EPI_ACC && res_ok[ch]) ? res[ch < PRE ? ch : 0] : nullptr);
-      }
+      store_tile<EPI, CHUNKS>(a, [&](int c0, float* v) { tmem_ld32(tmem_base + ((unsigned)(q * 32) << 16) + acc * BN + (unsigned)c0, v); },
+                              m_w, rows_w, n0, c_lo, res, stage);
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(accempty0_rank0 + 8 * acc);      // one of the sixteen arrivals that free the accumulator
@@ -668,7 +693,7 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int K, int ld,
 
 template <int EPI, int BN>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mw, const UmmaArgs& a, cudaStream_t stream) {
-  size_t smem = (size_t)(BN == 256 ? 4 : UM_STAGES) * (UM_BM + BN) * UM_BK * 2 + 1024;
+  size_t smem = (size_t)(BN == 256 ? 4 : UM_STAGES) * (UM_BM + BN) * UM_BK * 2 + 8 * UM_EPI_STAGE + 1024;
   auto kern = gemm_umma_kernel<EPI, BN>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -679,7 +704,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mw, const UmmaArgs& 
 
 template <int EPI, int BN>
 static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mw, const UmmaArgs& a, int max_tiles, cudaStream_t stream) {
-  size_t smem = (size_t)(BN == 256 ? 4 : UM_STAGES) * (UM_BM + BN) * UM_BK * 2 + 1024;
+  size_t smem = (size_t)(BN == 256 ? 4 : UM_STAGES) * (UM_BM + BN) * UM_BK * 2 + 8 * UM_EPI_STAGE + 1024;
   auto kern = gemm_umma_kernel<EPI, BN, true>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -690,7 +715,7 @@ static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mw, const Um
 
 template <int EPI, int BN>
 static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, const UmmaArgs& a, cudaStream_t stream) {
-  size_t smem = (size_t)(BN == 256 ? 6 : 8) * (UM_BM + BN / 2) * UM_BK * 2 + 1024;
+  size_t smem = (size_t)(BN == 256 ? 6 : 8) * (UM_BM + BN / 2) * UM_BK * 2 + 8 * UM_EPI_STAGE + 1024;
   auto kern = gemm_umma_pair_kernel<EPI, BN>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -719,28 +744,30 @@ FELLM_API int fellm_gemm_umma(const void* A, const void* W, const float* bias, v
   if ((K % 8) || (lda % 8) || (ldw % 8) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return FELLM_ERR_SIZE;
   if (epi == EPI_SWIGLU && ((N % 16) || (ldo % 8))) return FELLM_ERR_SIZE;
   // The tile: 128 x 128 or 128 x 256 by one CTA, or 256 x 256 / 256 x 128 by a CTA pair.  Chosen by an
-  // estimate: waves x k-blocks x the time a CTA takes for a k-block of its tile (measured on B200 at
-  // 2,048 rows: 0.37 us for 128 x 128, 0.47 us for 128 x 256, 0.44 us and 0.39 us for a pair's CTA on
-  // 256 x 256 and 256 x 128) + 4.5 us of filling and draining; within 5% one CTA a tile stays.
+  // estimate: waves x k-blocks x the time a CTA takes for a k-block of its tile + filling and draining.  Measured on B200 over
+  // 21 products of 130..2,048 rows: 0.28 us for 128 x 128 (32 KB written to and 32 KB read from shared memory a k-block: 512
+  // cycles at 128 bytes, twice the MMA's own), 0.40 us for 128 x 256, 0.345 us and 0.29 us for a pair's CTA on 256 x 256 and
+  // 256 x 128; 4.5 us of filling and draining, 5.2 us for a pair's; within 5% one CTA a tile stays.  (us; 128 x 256 / pair 256 x 256: 2,048 x 2,048 K 2,048 20.2 /
+  // 19.4, 1,537 x 3,072 K 1,024 19.1 / 17.6, 2,048 x 2,112 K 2,048 18.2 / 17.2; 2,048 x 1,280 K 1,024 9.5 / 10.3, 1,800 x 14,336 K 1,536 67 / 85.)
   // FELLM_B200_UMMA_PAIR=0: never pairs; =128 / =256: always that pair tile; FELLM_B200_UMMA_WIDE=0: no 128 x 256.
   const int m_tiles = ceil_div(M, UM_BM), m_pairs = ceil_div(M, 2 * UM_BM), kb = ceil_div(K, UM_BK);
   const int n_sm = fellm_sm_count(), pairs_dev = n_sm / 2;
   static int wide_ok = -1, pair_mode = -1;
   if (wide_ok < 0) { const char* ev = getenv("FELLM_B200_UMMA_WIDE"); wide_ok = (ev && ev[0] == '0') ? 0 : 1; }
   if (pair_mode < 0) { const char* ev = getenv("FELLM_B200_UMMA_PAIR"); pair_mode = ev ? atoi(ev) : 1; }
-  auto estimate = [&](int tiles, int units, float t_kb) { return 4.5f + (float)ceil_div(tiles, units) * kb * t_kb; };
-  float best = estimate(ceil_div(N, 128) * m_tiles, n_sm, 0.37f);
+  auto estimate = [&](int tiles, int units, float t_kb, float fixed) { return fixed + (float)ceil_div(tiles, units) * kb * t_kb; };
+  float best = estimate(ceil_div(N, 128) * m_tiles, n_sm, 0.28f, 4.5f);
   int choice = 0;                                           // 0: 128 x 128, 1: 128 x 256, 2: pair 256 x 256, 3: pair 256 x 128
   if (wide_ok && N >= 512) {
-    const float t = estimate(ceil_div(N, 256) * m_tiles, n_sm, 0.47f);
+    const float t = estimate(ceil_div(N, 256) * m_tiles, n_sm, 0.40f, 4.5f);
     if (t < best) { best = t; choice = 1; }
   }
   if (pair_mode && M >= 512 && pairs_dev >= 1) {
     if (N >= 256) {
-      const float t = estimate(ceil_div(N, 256) * m_pairs, pairs_dev, 0.44f);
+      const float t = estimate(ceil_div(N, 256) * m_pairs, pairs_dev, 0.345f, 5.2f);
       if (t < 0.95f * best) { best = t; choice = 2; }
     }
-    const float t = estimate(ceil_div(N, 128) * m_pairs, pairs_dev, 0.39f);
+    const float t = estimate(ceil_div(N, 128) * m_pairs, pairs_dev, 0.29f, 5.2f);
     if (t < 0.95f * best) { best = t; choice = 3; }
     if (pair_mode == 256 && N >= 256) choice = 2;
     if (pair_mode == 128) choice = 3;
@@ -750,10 +777,12 @@ FELLM_API int fellm_gemm_umma(const void* A, const void* W, const float* bias, v
   if (e) return e;
   UmmaArgs a; a.bias = bias; a.out = out; a.status = status; a.M = M; a.N = N; a.K = K; a.ldo = ldo;
   a.g_table = nullptr; a.g_tiles = nullptr; a.g_wrows = 0;
-  // few tiles and a long K (a few hundred rows, a narrow N): two CTAs a 128 x 128 tile, half of K each
+  // few tiles and a long K (a few hundred rows, a narrow N): two CTAs a 128 x 128 tile, half of K each.  Handing a part over
+  // costs some 4 us, a k-block of it saves 0.13 (us, whole / split: 600 x 1,024 K 1,024 7.8 / 9.7, K 2,048 12.1 / 12.0, K 3,072 16.4 / 14.2,
+  // K 8,192 38.2 / 27.3; 1,100 x 1,024 K 1,024 8.0 / 10.1, K 2,048 12.5 / 12.3)
   static int ksplit = -1;
   if (ksplit < 0) { const char* ev = getenv("FELLM_B200_UMMA_KSPLIT"); ksplit = (ev && ev[0] == '0') ? 0 : 1; }
-  if (ksplit && 2 * ceil_div(N, 128) * m_tiles <= n_sm && kb >= 8) {
+  if (ksplit && 2 * ceil_div(N, 128) * m_tiles <= n_sm && kb >= 32) {
     e = make_map(&mw, W, N, K, ldw, 128);
     if (e) return e;
     switch (epi) {
