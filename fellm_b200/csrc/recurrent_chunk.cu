@@ -13,14 +13,18 @@
 // Every factor is a product of decays, formed by multiplication alone: no logarithm, no division, so a decay of zero or
 // one that underflows is what it is in the token-by-token walk.
 //
-// Two kernels.  `prep` (a block a chunk and head, all side by side): the token vectors, L and M with one running product a
-// column, the substitution for (P A) and V, the scaled B and K.  `walk` (a block a head and 16 value columns): chunk
-// after chunk, the state in registers, three small products a chunk; the next chunk's operands arrive by cp.async meanwhile.
-// Bound by: the reads of shared memory.  A lane's tile of 4 x 4 (or 2 x 4) results takes a register from shared memory for
-// every two multiply-adds, and a block's chunk of 32 tokens at dk = 128 is 0.2 M of those: ~5,000 of the 5,800 cycles a
-// chunk takes.  The scan walks one token after another, a reduction over dk and ~750 cycles each.  16 columns a block: a
-// prompt of 16 heads of 128 is 128 blocks for 148 SMs.  2,048 tokens of 16 heads of 128 x 128, delta rule: scan 791 us, here
-// prep 81 + walk 188 (decay per channel: 96 + 188); three prompts of 1,537 tokens, 8 heads, gated write: 274 us, here 23 + 77.
+// `prep` (a block a chunk and head, all side by side): the token vectors, L and M with one running product a column, the
+// substitution for (P A) and V, the scaled B and K.  Then, in one `walk` (a block a head and 16 value columns), states and outputs
+// chunk after chunk; or, for long portions, what hangs together in a chain first and the outputs of all chunks side by
+// side behind it (`out`): with the delta rule the `chain` W S, K^T U (the state in front of every chunk goes to memory), without
+// it prep sums a chunk's K^T V and `states` is S' = P S + that, element by element.
+// Bound by: the reads of shared memory.  A load of 16 bytes a lane takes four wavefronts, or two where lanes one or two apart ask for the
+// same (of 8 bytes: two or one), whatever else they share; so a tile's row and column groups lie in alternate bits of the
+// lane's number (walk 188 -> 158 us, prep 85 -> 74 of the first size below, with the same bits).  A lane's tile of 4 x 4 (or 2 x 4) results then takes a wavefront for
+// about every FMA instruction of a warp.  16 columns a block: a prompt of 16 heads of 128 is 128 blocks for 148 SMs.
+// 2,048 tokens of 16 heads of 128 x 128, delta rule: scan 791 us, prep 85 + walk 188 as it was, here prep 74 + chain 105 + out 44 (one walk:
+// 158), graph of the three 269 -> 215; decay per channel 284 -> 226; three prompts of 1,537 tokens, 8 heads, gated write: scan 274, 100 -> 61;
+// 1,100 tokens in two prompts, 16 heads of 64, decay and bonus 71 -> 45.
 // 32 tokens a chunk: L and M cost 32 / 2 multiply-adds a token, channel and matrix, an eighth of the walk's.
 //
 // A later token's infinity or NaN stays out of an earlier token's sums, as in the walk token by token: masked pairs are
@@ -32,7 +36,7 @@
 // products of the decays are sums of two floats.  Relative error against float64, scan / here, mean over five sizes and
 // three seeds: delta rule outputs 1.34e-7 / 1.22e-7, states 9.0e-8 / 8.6e-8, with keys nearly alike and beta 0.99 1.45e-7 /
 // 1.35e-7, 8.7e-8 / 8.4e-8; decay per channel 1.22e-7 / 1.08e-7, 7.8e-8 / 7.3e-8; decay and bonus 8.3e-8 / 6.8e-8, 3.15e-8 /
-// 3.09e-8; gated write 6.2e-8 / 5.9e-8, 1.09e-7 / 1.07e-7.  It costs 6 us of the 263 of the first size above (21 of 264 with a
+// 3.10e-8; gated write 6.2e-8 / 5.9e-8, 1.09e-7 / 1.07e-7.  It costs 6 us of the 263 of the first size above (21 of 264 with a
 // decay per channel, 4 of 68 with a bonus; the gated write gains 5 of 106 through its smaller blocks).
 // Sums run in another order than the scan's, so the engine uses this form for portions of the bfloat16 engine; the 32-bit
 // engine keeps the scan and with it the same bits for a prompt under every cut.
@@ -44,6 +48,7 @@
 #define RK_LP 36           // row stride of a chunk's 32 x 32 matrices in the image
 #define RK_LM 34           // and, in 64 bits, in prep's shared memory
 #define RK_THREADS 256
+#define RK_LAST 3          // tokens at a chunk's end whose terms are added to the state one by one
 
 enum RkMode { RK_DELTA_HEAD = 0, RK_DELTA_CHANNEL = 1, RK_DECAY_BONUS = 2, RK_GATED_WRITE = 3 };
 
@@ -57,13 +62,26 @@ struct RkArgs {
   const int* item_start; const int* item_slot;
   float* state; long long slot_stride;
   float* out;                                                      // [T, H dv]
-  float* image; float* U;                                          // per (chunk, head): an RkImage; [dv / 16][32][16]
-  int H, G, dv, min_rows;
+  float* image; float* U; float* S;                                // per (chunk, head): an RkImage; [dv / 16][32][16]; the state in front of it [dv][dk] (or null: outputs in the walk)
+  int H, G, dv, min_rows, n_items, cells;                          // cells: places for the step's chunks
 };
 
 // Chunks of an item lie behind one another from here on: rows before it / 32 + its number is free of overlaps, and the
 // chunks of a step are at most T / 32 + items.
 __device__ __forceinline__ int rk_first_chunk(int row0, int item) { return row0 / RK_C + item; }
+
+// Which item the step's chunk x belongs to: the last one whose chunks start at or before x (a place between two items' chunks belongs to
+// nobody: its item's rows end before it).  The lanes of a warp look at 32 items at once.
+__device__ __forceinline__ int rk_item_of(const int* item_start, int n_items, int x) {
+  int item = 0;
+  for (int i0 = 0; i0 < n_items; i0 += 32) {
+    const int i = i0 + (threadIdx.x & 31);
+    const unsigned before = __ballot_sync(0xffffffffu, i < n_items && rk_first_chunk(item_start[i], i) <= x);
+    if (!before) break;
+    item = i0 + 31 - __clz(before);
+  }
+  return item;
+}
 
 template <int E> __device__ __forceinline__ void rk_load(const float* p, float* o) {
   if (E == 4) { const float4 f = *(const float4*)p; o[0] = f.x; o[1] = f.y; o[E - 2] = f.z; o[E - 1] = f.w; }
@@ -102,13 +120,59 @@ struct RkProduct {
   }
 };
 
-// What prep leaves for walk of a chunk and head, as it lies in walk's shared memory (its copies are then linear).
+// What prep leaves of a chunk and head, in the order its readers take it (their copies are then linear): walk reads W, K and
+// P, the outputs Q and M, the states of the recurrences without the delta rule P and, in K's
+// place, K of the last RK_LAST tokens.
 template <bool DELTA, int DK>
 struct RkImage {
-  static constexpr int NR = DELTA ? 2 * RK_C : RK_C;          // rows of the product with the state: W above Q, or Q alone
-  static constexpr int AP = DK + 4;                           // their stride: eight rows' 16 bytes in different banks
-  static constexpr int A = 0, K = A + NR * AP, M = K + RK_C * DK, P = M + RK_C * RK_LP, FLOATS = P + DK;
+  static constexpr int AP = DK + 4;                           // row stride of W and Q: eight rows' 16 bytes in different banks
+  static constexpr int W = 0, K = W + (DELTA ? RK_C * AP : 0), P = K + RK_C * DK, WALK = P + DK;
+  static constexpr int Q = WALK, M = Q + RK_C * AP, FLOATS = M + RK_C * RK_LP, OUT = FLOATS - Q;
 };
+
+// What a chunk's tokens but the last RK_LAST add to the state where u_t = v_t: K^T V, [dv][DK] at the cell's place in a.S, DK columns of V at a time (in V,
+// [32][DK]; the first of them are there).  A thread eight key rows and four value columns at a time, in the tokens' order.
+template <int DK, typename TA>
+__device__ __forceinline__ void rk_own_state(const RkArgs& a, size_t cell, float* V, const float* KK, const TA* vp, int row0, int len, int tid) {
+  float* S = a.S + cell * ((size_t)a.dv * DK);
+  for (int j0 = 0; j0 < a.dv; j0 += DK) {
+    if (j0) {
+      __syncthreads();
+      for (int x = tid; x < RK_C * DK; x += RK_THREADS) {
+        const int t = x / DK, j = j0 + x % DK;
+        V[x] = t < len && j < a.dv ? to_f(vp[(size_t)(row0 + t) * a.ld + j]) : 0.f;
+      }
+    }
+    __syncthreads();
+    for (int x = tid; x < (DK / 8) * (DK / 4); x += RK_THREADS) {
+      const int y = x >> 1, i = 8 * (y % (DK / 8)), j = 4 * ((x & 1) + 2 * (y / (DK / 8)));      // (neighbouring lanes read the same of K)
+      if (j0 + j >= a.dv) continue;
+      unsigned long long acc[4][4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[c][r] = 0ull;
+#pragma unroll 4
+      for (int t = 0; t < len - RK_LAST; ++t) {
+        const ulonglong2 k0 = *(const ulonglong2*)(KK + t * DK + i), k1 = *(const ulonglong2*)(KK + t * DK + i + 4);
+        const float4 v = *(const float4*)(V + t * DK + j);
+        const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const unsigned long long d = pack_f2(vv[c], vv[c]);
+          acc[c][0] = fma_f2(k0.x, d, acc[c][0]); acc[c][1] = fma_f2(k0.y, d, acc[c][1]);
+          acc[c][2] = fma_f2(k1.x, d, acc[c][2]); acc[c][3] = fma_f2(k1.y, d, acc[c][3]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        float* o = S + (size_t)(j0 + j + c) * DK + i;
+        *(ulonglong2*)o = make_ulonglong2(acc[c][0], acc[c][1]);
+        *(ulonglong2*)(o + 4) = make_ulonglong2(acc[c][2], acc[c][3]);
+      }
+    }
+  }
+}
 
 // ---------------------------------------------------------------- prep
 template <int MODE, int DK, typename TA>
@@ -124,11 +188,11 @@ rk_prep_kernel(const RkArgs a) {
   double* LM = beta + RK_C;                        // [32][RK_LM]: [s][t], t > s: beta_t L_ts; [t][s], s <= t: M_ts
   constexpr bool DELTA = MODE <= RK_DELTA_CHANNEL;
   constexpr int E = DK / 32;
-  const int item = blockIdx.z, h = blockIdx.y, c = blockIdx.x;
-  const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0;
+  const int item = rk_item_of(a.item_start, a.n_items, blockIdx.x), h = blockIdx.y;
+  const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0, c = blockIdx.x - rk_first_chunk(r0, item);
   if (n < a.min_rows || c * RK_C >= n) return;
   const int len = min(RK_C, n - c * RK_C), row0 = r0 + c * RK_C;
-  const size_t cell = (size_t)(rk_first_chunk(r0, item) + c) * a.H + h;
+  const size_t cell = (size_t)blockIdx.x * a.H + h;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = h / (a.H / a.G);
   for (int x = tid; x < RK_C * RK_LM; x += RK_THREADS) LM[x] = 0.0;
@@ -207,7 +271,7 @@ rk_prep_kernel(const RkArgs a) {
   // Four tokens a round: their (up to) eight sums go through the eight lanes together, seven shuffles for all of them.
   {
     constexpr int MB = DK / 32;
-    const int ig = lane & 7, s = 4 * warp + (lane >> 3);
+    const int ig = (lane >> 1) & 7, s = 4 * warp + (lane & 1) + 2 * (lane >> 4);        // (neighbouring lanes read the same)
     unsigned long long X[2 * MB];
 #pragma unroll
     for (int m = 0; m < 2 * MB; ++m) X[m] = 0ull;
@@ -257,16 +321,16 @@ rk_prep_kernel(const RkArgs a) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float give = DELTA && !b0 ? sum[4 + j] : sum[j], keep = DELTA && b0 ? sum[4 + j] : sum[j];
-        q4[j] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, give, 1);
+        q4[j] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, give, 2);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const double give = b1 ? q4[j] : q4[2 + j], keep = b1 ? q4[2 + j] : q4[j];
-        q2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+        q2[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
       }
       {
         const double give = b2 ? q2[0] : q2[1], keep = b2 ? q2[1] : q2[0];
-        v = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+        v = keep + __shfl_xor_sync(0xffffffffu, give, 8);
       }
       const int t = t0 + (b1 ? 2 : 0) + (b2 ? 1 : 0);
       if (t > s) {
@@ -303,8 +367,9 @@ rk_prep_kernel(const RkArgs a) {
   __syncthreads();
   for (int x = tid * 4; x < RK_C * DK; x += RK_THREADS * 4) {
     const int t = x / DK, i = x - t * DK;
-    *(float4*)(img + I::A + (t + I::NR - RK_C) * I::AP + i) = *(const float4*)(B + x);
-    *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
+    *(float4*)(img + I::Q + t * I::AP + i) = *(const float4*)(B + x);
+    if (DELTA || !a.S) *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
+    else if (t < len && t >= len - RK_LAST) *(float4*)(img + I::K + (t - len + RK_LAST) * DK + i) = *(const float4*)(KK + x);
   }
   for (int x = tid; x < RK_C * RK_C; x += RK_THREADS) {
     const int t = x / RK_C, s = x % RK_C;
@@ -318,7 +383,7 @@ rk_prep_kernel(const RkArgs a) {
     const bool is_w = DELTA && col < DK;
     const int j = DELTA ? col - DK : col;
     auto put = [&](int t, float x) {
-      if (is_w) img[I::A + t * I::AP + col] = x;
+      if (is_w) img[I::W + t * I::AP + col] = x;
       else Ug[((size_t)(j / RK_NV) * RK_C + t) * RK_NV + j % RK_NV] = x;
     };
     if (DELTA) {
@@ -371,8 +436,13 @@ rk_prep_kernel(const RkArgs a) {
       for (int t = 0; t < RK_C; ++t) x[t] = t < len ? to_f(vp[(size_t)(row0 + t) * a.ld + j]) : 0.f;
 #pragma unroll
       for (int t = 0; t < RK_C; ++t) put(t, x[t]);
+      if (a.S && j < DK) {                         // (A is free without the delta rule: it holds the values' first DK columns)
+#pragma unroll
+        for (int t = 0; t < RK_C; ++t) A[t * DK + j] = x[t];
+      }
     }
   }
+  if (!DELTA && a.S) rk_own_state<DK, TA>(a, cell, A, KK, vp, row0, len, tid);
 }
 
 // ---------------------------------------------------------------- walk
@@ -380,23 +450,18 @@ __device__ __forceinline__ void rk_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-// Two groups of eight warps.  The first walks the state: W S, U = U0 - W S, S = P S + K^T U; the second makes the
-// outputs, Q S + M U, from the state in front of the chunk as it lies in shared memory and the first group's U: what the
-// outputs cost runs beside the chain and not in it, and sixteen warps hide each other's waits.
-#define RK_WALK_THREADS 512
-#define RK_PP (RK_NV + 4)  // row stride of the partial sums
+// The delta rule's chain: W S, U = U0 - W S, S = P S + K^T U.  What the outputs need of it, the state in front of every chunk
+// and U, goes to memory.
+#define RK_PP RK_NV         // row stride of the partial sums (a warp writes eight whole rows, reads four)
 
-__device__ __forceinline__ void rk_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-__device__ __forceinline__ void rk_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-
-template <bool DELTA, int DK>
+template <int DK>
 __device__ __forceinline__ void rk_fetch(const RkArgs& a, float* buf, size_t cell, int tile, int tid) {
-  using I = RkImage<DELTA, DK>;
+  using I = RkImage<true, DK>;
   const float* img = a.image + cell * I::FLOATS;
 #pragma unroll
-  for (int x = 4 * tid; x < I::FLOATS; x += 4 * RK_WALK_THREADS) rk_copy16(buf + x, img + x);
+  for (int x = 4 * tid; x < I::WALK; x += 4 * RK_THREADS) rk_copy16(buf + x, img + x);
   const float* Ug = a.U + cell * ((size_t)RK_C * a.dv) + (size_t)tile * (RK_C * RK_NV);
-  if (tid < RK_C * RK_NV / 4) rk_copy16(buf + I::FLOATS + 4 * tid, Ug + 4 * tid);
+  if (tid < RK_C * RK_NV / 4) rk_copy16(buf + I::WALK + 4 * tid, Ug + 4 * tid);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
@@ -444,6 +509,110 @@ __device__ __forceinline__ float2 rk_gather(const float* part, int row, int col)
   return r;
 }
 
+template <int DK>
+__global__ void __launch_bounds__(RK_THREADS)
+rk_chain_kernel(const RkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  using I = RkImage<true, DK>;
+  constexpr int STAGE = I::WALK + RK_C * RK_NV;
+  constexpr int KW = DK / 8;                       // key rows of the state a warp keeps
+  constexpr int RPL = KW / 8;                      // of them a lane
+  constexpr int GM = KW / 4 - 1;                   // 16-byte groups of a column, less one
+  float* partW = sm + 2 * STAGE;                   // [8 warps][32][RK_PP]
+  float* St = partW + 8 * RK_C * RK_PP;            // [8 warps][16 columns][KW], 16-byte groups swizzled by column / 4
+  float* Us = St + RK_NV * DK;                     // [32][16]
+  const int item = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * RK_NV;
+  const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0;
+  if (n < a.min_rows || n <= 0) return;
+  const int chunks = (n + RK_C - 1) / RK_C;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rg = (lane & 1) + 2 * (lane >> 3), cg = (lane >> 1) & 3;       // (each shared by lanes one or two apart: see above)
+  const size_t cell0 = (size_t)rk_first_chunk(r0, item) * a.H + h;
+  rk_fetch<DK>(a, sm, cell0, blockIdx.x, tid);
+
+  // a lane's part of the state: rows warp * KW + RPL * rg + r, columns j0 + 4 cg + x
+  float* slot = a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv;
+  const int i0 = warp * KW + RPL * rg;
+  float s[RPL][4];
+  float* Sw = St + warp * (RK_NV * KW);            // (a warp's key rows: written and read by the warp alone)
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) s[r][x] = slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r];
+  const int row = tid >> 3, jc = 2 * (tid & 7);                // gathering: a thread a row and two columns
+
+  for (int c = 0; c < chunks; ++c) {
+    const float* buf = sm + (c & 1) * STAGE;
+    const size_t cell = cell0 + (size_t)c * a.H;
+    float* Sg = a.S + cell * ((size_t)a.dv * DK) + (size_t)j0 * DK + i0;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int i = RPL * rg, col = 4 * cg + x;
+      float* at = Sw + col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3);
+      if (RPL == 2) *(float2*)at = make_float2(s[0][x], s[RPL - 1][x]);
+      else *at = s[0][x];
+      if (RPL == 2) *(float2*)(Sg + (4 * cg + x) * DK) = make_float2(s[0][x], s[RPL - 1][x]);
+      else Sg[(4 * cg + x) * DK] = s[0][x];
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();          // this chunk's operands are here; the other buffer, the sums and U are free
+    if (c + 1 < chunks) rk_fetch<DK>(a, sm + ((c + 1) & 1) * STAGE, cell + a.H, blockIdx.x, tid);
+    rk_rows_by_state<KW, I::AP>(buf + I::W + warp * KW, Sw, partW + warp * (RK_C * RK_PP), rg, cg);
+    __syncthreads();
+    {
+      const float2 r = rk_gather(partW, row, jc), u0 = *(const float2*)(buf + I::WALK + row * RK_NV + jc);
+      const float2 u = make_float2(u0.x - r.x, u0.y - r.y);
+      *(float2*)(Us + row * RK_NV + jc) = u;
+      *(float2*)(a.U + cell * ((size_t)RK_C * a.dv) + (size_t)blockIdx.x * (RK_C * RK_NV) + row * RK_NV + jc) = u;
+    }
+    const float* Kb = buf + I::K + i0;
+    const float* Pb = buf + I::P + i0;
+    float k1[RPL];
+#pragma unroll
+    for (int q = 0; q < RPL; ++q) {
+      const float p = Pb[q];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) s[q][x] *= p;
+    }
+    __syncthreads();
+#pragma unroll 16
+    for (int t2 = 0; t2 < RK_C; ++t2) {
+      if (RPL == 2) { const float2 f = *(const float2*)(Kb + t2 * DK); k1[0] = f.x; k1[RPL - 1] = f.y; }
+      else k1[0] = Kb[t2 * DK];
+      const float4 u = *(const float4*)(Us + t2 * RK_NV + 4 * cg);
+#pragma unroll
+      for (int q = 0; q < RPL; ++q) {
+        s[q][0] = fmaf(k1[q], u.x, s[q][0]); s[q][1] = fmaf(k1[q], u.y, s[q][1]);
+        s[q][2] = fmaf(k1[q], u.z, s[q][2]); s[q][3] = fmaf(k1[q], u.w, s[q][3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) slot[(size_t)(j0 + 4 * cg + x) * DK + i0 + r] = s[r][x];
+}
+
+// ---------------------------------------------------------------- walk, outputs and all
+// Short portions wait for launches more than for work: states and outputs in one walk over the chunks, a launch less.
+// Two groups of eight warps.  The first walks the state: W S, U = U0 - W S, S = P S + K^T U; the second makes the
+// outputs, Q S + M U, from the state in front of the chunk as it lies in shared memory and the first group's U: what the
+// outputs cost runs beside the chain and not in it, and sixteen warps hide each other's waits.
+#define RK_WALK_THREADS 512
+__device__ __forceinline__ void rk_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void rk_bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+template <bool DELTA, int DK>
+__device__ __forceinline__ void rk_fetch_all(const RkArgs& a, float* buf, size_t cell, int tile, int tid) {
+  using I = RkImage<DELTA, DK>;
+  const float* img = a.image + cell * I::FLOATS;
+#pragma unroll
+  for (int x = 4 * tid; x < I::FLOATS; x += 4 * RK_WALK_THREADS) rk_copy16(buf + x, img + x);
+  const float* Ug = a.U + cell * ((size_t)RK_C * a.dv) + (size_t)tile * (RK_C * RK_NV);
+  if (tid < RK_C * RK_NV / 4) rk_copy16(buf + I::FLOATS + 4 * tid, Ug + 4 * tid);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
 template <bool DELTA, int DK>
 __global__ void __launch_bounds__(RK_WALK_THREADS)
 rk_walk_kernel(const RkArgs a) {
@@ -463,9 +632,9 @@ rk_walk_kernel(const RkArgs a) {
   const int chunks = (n + RK_C - 1) / RK_C;
   const int tid = threadIdx.x, gtid = tid & 255, warp = (tid >> 5) & 7, lane = tid & 31;
   const bool walker = tid < 256;
-  const int rg = lane >> 2, cg = lane & 3;
+  const int rg = (lane & 1) + 2 * (lane >> 3), cg = (lane >> 1) & 3;
   const size_t cell0 = (size_t)rk_first_chunk(r0, item) * a.H + h;
-  rk_fetch<DELTA, DK>(a, sm, cell0, blockIdx.x, tid);
+  rk_fetch_all<DELTA, DK>(a, sm, cell0, blockIdx.x, tid);
 
   // a walker's part of the state: rows warp * KW + RPL * rg + r, columns j0 + 4 cg + x
   float* slot = a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv;
@@ -475,10 +644,11 @@ rk_walk_kernel(const RkArgs a) {
     float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
 #pragma unroll
     for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = RPL * rg + r, col = 4 * cg + x;
-        Sw[col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3)] = s[r][x];
+{
+        const int i = RPL * rg, col = 4 * cg + x;
+        float* at = Sw + col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3);
+        if (RPL == 2) *(float2*)at = make_float2(s[0][x], s[RPL - 1][x]);
+        else *at = s[0][x];
       }
   };
   if (walker) {
@@ -494,12 +664,12 @@ rk_walk_kernel(const RkArgs a) {
     const float* buf = sm + (c & 1) * STAGE;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();          // this chunk's operands and state are here; the other buffers, the sums and U are free
-    if (c + 1 < chunks) rk_fetch<DELTA, DK>(a, sm + ((c + 1) & 1) * STAGE, cell0 + (size_t)(c + 1) * a.H, blockIdx.x, tid);
+    if (c + 1 < chunks) rk_fetch_all<DELTA, DK>(a, sm + ((c + 1) & 1) * STAGE, cell0 + (size_t)(c + 1) * a.H, blockIdx.x, tid);
     const float* U = DELTA ? Us : buf + I::FLOATS;
     const float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
     if (walker) {
       if (DELTA) {
-        rk_rows_by_state<KW, I::AP>(buf + I::A + warp * KW, Sw, partW + warp * (RK_C * RK_PP), rg, cg);
+        rk_rows_by_state<KW, I::AP>(buf + I::W + warp * KW, Sw, partW + warp * (RK_C * RK_PP), rg, cg);
         rk_bar_sync(1, 256);
         const float2 r = rk_gather(partW, row, jc), u0 = *(const float2*)(buf + I::FLOATS + row * RK_NV + jc);
         *(float2*)(Us + row * RK_NV + jc) = make_float2(u0.x - r.x, u0.y - r.y);
@@ -528,7 +698,7 @@ rk_walk_kernel(const RkArgs a) {
       }
       put_state(c + 1);
     } else {
-      rk_rows_by_state<KW, I::AP>(buf + I::A + (I::NR - RK_C) * I::AP + warp * KW, Sw, partQ + warp * (RK_C * RK_PP), rg, cg);
+      rk_rows_by_state<KW, I::AP>(buf + I::Q + warp * KW, Sw, partQ + warp * (RK_C * RK_PP), rg, cg);
       rk_bar_sync(3, 256);
       float2 r = rk_gather(partQ, row, jc);
       if (DELTA) rk_bar_sync(2, 512);
@@ -554,18 +724,192 @@ rk_walk_kernel(const RkArgs a) {
   }
 }
 
+// Without the delta rule the states are S' = P S + (what the chunk adds), element by element: a thread four key rows of a column,
+// what it reads of RK_AHEAD chunks on its way at once.  The state in front of a chunk takes the place of what prep summed.  The
+// terms of a chunk's last tokens, which later decays have left large, are added here and last, as in the walk token by token: summed
+// with the others in prep, a state's error rose from 3.1e-8 to 3.4e-8 (decay and bonus).
+#define RK_AHEAD 4
+template <int DK>
+__global__ void __launch_bounds__(RK_THREADS)
+rk_states_kernel(const RkArgs a) {
+  using I = RkImage<false, DK>;
+  const int item = blockIdx.z, h = blockIdx.y, x = 4 * (blockIdx.x * RK_THREADS + threadIdx.x), i = x % DK, j = x / DK;
+  const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0;
+  if (n < a.min_rows || n <= 0 || x >= a.dv * DK) return;
+  const int chunks = (n + RK_C - 1) / RK_C;
+  const size_t cell0 = (size_t)rk_first_chunk(r0, item) * a.H + h;
+  float4* slot = (float4*)(a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv + x);
+  float* S = a.S + cell0 * ((size_t)a.dv * DK) + x;
+  const float* img = a.image + cell0 * I::FLOATS + i;
+  const float* U = a.U + cell0 * ((size_t)RK_C * a.dv) + (size_t)(j / RK_NV) * (RK_C * RK_NV) + j % RK_NV;
+  const size_t s_step = (size_t)a.H * a.dv * DK, i_step = (size_t)a.H * I::FLOATS, u_step = (size_t)a.H * RK_C * a.dv;
+  float4 s = *slot;
+  for (int c = 0; c < chunks; c += RK_AHEAD) {
+    float4 add[RK_AHEAD], p[RK_AHEAD], k[RK_AHEAD][RK_LAST];
+    float u[RK_AHEAD][RK_LAST];
+#pragma unroll
+    for (int e = 0; e < RK_AHEAD; ++e)
+      if (c + e < chunks) {
+        add[e] = *(const float4*)(S + (c + e) * s_step);
+        p[e] = *(const float4*)(img + (c + e) * i_step + I::P);
+        const int len = min(RK_C, n - (c + e) * RK_C);
+#pragma unroll
+        for (int l = 0; l < RK_LAST; ++l) {
+          k[e][l] = make_float4(0.f, 0.f, 0.f, 0.f); u[e][l] = 0.f;
+          if (len - RK_LAST + l >= 0) {
+            k[e][l] = *(const float4*)(img + (c + e) * i_step + I::K + l * DK);
+            u[e][l] = U[(c + e) * u_step + (len - RK_LAST + l) * RK_NV];
+          }
+        }
+      }
+#pragma unroll
+    for (int e = 0; e < RK_AHEAD; ++e)
+      if (c + e < chunks) {
+        *(float4*)(S + (c + e) * s_step) = s;
+        s = make_float4(fmaf(p[e].x, s.x, add[e].x), fmaf(p[e].y, s.y, add[e].y), fmaf(p[e].z, s.z, add[e].z), fmaf(p[e].w, s.w, add[e].w));
+#pragma unroll
+        for (int l = 0; l < RK_LAST; ++l)
+          s = make_float4(fmaf(k[e][l].x, u[e][l], s.x), fmaf(k[e][l].y, u[e][l], s.y), fmaf(k[e][l].z, u[e][l], s.z), fmaf(k[e][l].w, u[e][l], s.w));
+      }
+  }
+  *slot = s;
+}
+
+// ---------------------------------------------------------------- outputs
+// O = Q S + M U of every chunk, side by side: a block a chunk, head and 64 columns; a warp 16 rows x 32 columns, a lane rows
+// rg + 4 m and four neighbouring columns.  The 32 floats of a key row pair a lane takes from shared memory feed 32 multiply-adds: bound by those.
+// Sums as the eight warps of one chain would make them: DK / 8 key rows at a time, pairs of rows an operation, then the parts in order.
+#define RK_OUT_THREADS 128
+#define RK_OUT_COLS 64
+template <bool DELTA, int DK>
+__global__ void __launch_bounds__(RK_OUT_THREADS)
+rk_out_kernel(const RkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  using I = RkImage<DELTA, DK>;
+  constexpr int KW = DK / 8, SP = DK + 4, UP = RK_OUT_COLS + 4;
+  float* Q = sm;                                   // [32][AP], and M [32][RK_LP] behind it
+  float* M = Q + RK_C * I::AP;
+  float* S = Q + I::OUT;                 // [64 columns][SP]: column j of 32 at row 8 (j % 4) + j / 4, so that a lane's four are 8 rows apart
+  float* U = S + RK_OUT_COLS * SP;                 // [32][UP]
+  const int item = rk_item_of(a.item_start, a.n_items, blockIdx.x), h = blockIdx.y, j0 = blockIdx.z * RK_OUT_COLS;
+  const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0, c = blockIdx.x - rk_first_chunk(r0, item);
+  if (n < a.min_rows || c * RK_C >= n) return;
+  const int cols = min(RK_OUT_COLS, a.dv - j0);    // (a multiple of 16)
+  const size_t cell = (size_t)blockIdx.x * a.H + h;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* img = a.image + cell * I::FLOATS + I::Q;
+  const float* Sg = a.S + cell * ((size_t)a.dv * DK) + (size_t)j0 * DK;
+  const float* Ug = a.U + cell * ((size_t)RK_C * a.dv) + (size_t)(j0 / RK_NV) * (RK_C * RK_NV);
+  // four groups of copies, a quarter of the key rows each: the products start behind the first
+  constexpr int KQ = DK / 4;
+#pragma unroll
+  for (int part = 0; part < 4; ++part) {
+    if (part == 0) for (int x = 4 * tid; x < I::OUT; x += 4 * RK_OUT_THREADS) rk_copy16(Q + x, img + x);
+    for (int x = 4 * tid; x < cols * KQ; x += 4 * RK_OUT_THREADS) {
+      const int j = x / KQ, k = part * KQ + x % KQ;
+      rk_copy16(S + ((j & ~31) + 8 * (j & 3) + ((j & 31) >> 2)) * SP + k, Sg + (size_t)j * DK + k);
+    }
+    if (part == 3)
+      for (int x = 4 * tid; x < cols * RK_C; x += 4 * RK_OUT_THREADS) {
+        const int tile = x / (RK_C * RK_NV), y = x % (RK_C * RK_NV);
+        rk_copy16(U + (y / RK_NV) * UP + tile * RK_NV + y % RK_NV, Ug + x);
+      }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  const int rg = (lane & 1) + 2 * (lane >> 4), cg = (lane >> 1) & 7, row0 = 16 * (warp & 1) + rg, col0 = 32 * (warp >> 1);
+  float r[4][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) r[m][x] = 0.f;
+  const float* Qr = Q + row0 * I::AP;
+  const float* Sc = S + (col0 + cg) * SP;
+#pragma unroll 1
+  for (int w = 0; w < 8; ++w) {
+    if (w == 0) asm volatile("cp.async.wait_group 3;\n" ::: "memory");
+    else if (w == 2) asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+    else if (w == 4) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    else if (w == 6) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (!(w & 1)) __syncthreads();
+    unsigned long long acc[4][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) acc[m][x] = 0ull;
+#pragma unroll
+    for (int kk = 0; kk < KW / 4; ++kk) {
+      const int k = w * KW + 4 * kk;
+      ulonglong2 sv[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) sv[x] = *(const ulonglong2*)(Sc + 8 * x * SP + k);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const ulonglong2 qv = *(const ulonglong2*)(Qr + 4 * m * I::AP + k);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) { acc[m][x] = fma_f2(qv.x, sv[x].x, acc[m][x]); acc[m][x] = fma_f2(qv.y, sv[x].y, acc[m][x]); }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) { float lo, hi; unpack_f2(acc[m][x], lo, hi); r[m][x] += lo + hi; }
+  }
+  const float* Uc = U + col0 + 4 * cg;
+#pragma unroll 1
+  for (int t = 0; t < 16 * (warp & 1) + 16; t += 4) {
+    float4 mv[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) mv[m] = *(const float4*)(M + (row0 + 4 * m) * RK_LP + t);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 u = *(const float4*)(Uc + (t + e) * UP);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const float f = e == 0 ? mv[m].x : e == 1 ? mv[m].y : e == 2 ? mv[m].z : mv[m].w;
+        if (t + e <= row0 + 4 * m) {               // (a later token's values stay out, whatever they are)
+          r[m][0] = fmaf(f, u.x, r[m][0]); r[m][1] = fmaf(f, u.y, r[m][1]);
+          r[m][2] = fmaf(f, u.z, r[m][2]); r[m][3] = fmaf(f, u.w, r[m][3]);
+        }
+      }
+    }
+  }
+  if (col0 + 4 * cg >= cols) return;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int t = c * RK_C + row0 + 4 * m;
+    if (t < n) *(float4*)(a.out + (size_t)(r0 + t) * ((size_t)a.H * a.dv) + (size_t)h * a.dv + j0 + col0 + 4 * cg) = make_float4(r[m][0], r[m][1], r[m][2], r[m][3]);
+  }
+}
+
 // ---------------------------------------------------------------- launches
 template <int MODE, int DK, typename TA>
-static int rk_launch(const RkArgs& a, int n_items, int max_rows, cudaStream_t stream) {
+static int rk_launch(const RkArgs& a, cudaStream_t stream) {
   constexpr bool DELTA = MODE <= RK_DELTA_CHANNEL;
+  using I = RkImage<DELTA, DK>;
   const size_t sm_prep = (size_t)(4 * RK_C * DK + RK_C) * sizeof(float) + (RK_C * RK_LM + RK_C) * sizeof(double);
-  const size_t sm_walk = (size_t)(2 * (RkImage<DELTA, DK>::FLOATS + RK_C * RK_NV) + 8 * RK_C * RK_PP + 2 * RK_NV * DK +
-                                  (DELTA ? 8 * RK_C * RK_PP + RK_C * RK_NV : 0)) * sizeof(float);
+  // (more than half of an SM's shared memory: two blocks on one SM and none on another made one portion among single tokens, whose blocks
+  // have nothing to do, a third longer)
+  size_t sm_chain = (size_t)(2 * (RkImage<true, DK>::WALK + RK_C * RK_NV) + 8 * RK_C * RK_PP + RK_NV * DK + RK_C * RK_NV) * sizeof(float);
+  if (sm_chain < 116 * 1024) sm_chain = 116 * 1024;
+  const size_t sm_out = (size_t)(I::OUT + RK_OUT_COLS * (DK + 4) + RK_C * (RK_OUT_COLS + 4)) * sizeof(float);
+  const size_t sm_walk = (size_t)(2 * (I::FLOATS + RK_C * RK_NV) + 8 * RK_C * RK_PP + 2 * RK_NV * DK + (DELTA ? 8 * RK_C * RK_PP + RK_C * RK_NV : 0)) * sizeof(float);
+  const int tiles = (a.dv + RK_OUT_COLS - 1) / RK_OUT_COLS;
+  if (tiles > 65535) return FELLM_ERR_SIZE;
   cudaError_t e = cudaFuncSetAttribute(rk_prep_kernel<MODE, DK, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_prep);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(rk_walk_kernel<DELTA, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
+  if (e == cudaSuccess && !a.S) e = cudaFuncSetAttribute(rk_walk_kernel<DELTA, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_walk);
+  if (e == cudaSuccess && a.S && DELTA) e = cudaFuncSetAttribute(rk_chain_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_chain);
+  if (e == cudaSuccess && a.S) e = cudaFuncSetAttribute(rk_out_kernel<DELTA, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_out);
   if (e != cudaSuccess) return (int)e;
-  rk_prep_kernel<MODE, DK, TA><<<dim3((max_rows + RK_C - 1) / RK_C, a.H, n_items), RK_THREADS, sm_prep, stream>>>(a);
-  rk_walk_kernel<DELTA, DK><<<dim3(a.dv / RK_NV, a.H, n_items), RK_WALK_THREADS, sm_walk, stream>>>(a);
+  // (ordinary launches: as programmatic dependents the next kernel's blocks take the SMs' shared memory while they wait; 2,048 tokens of
+  // the delta rule 214 -> 291 us)
+  rk_prep_kernel<MODE, DK, TA><<<dim3(a.cells, a.H), RK_THREADS, sm_prep, stream>>>(a);
+  if (!a.S) {
+    rk_walk_kernel<DELTA, DK><<<dim3(a.dv / RK_NV, a.H, a.n_items), RK_WALK_THREADS, sm_walk, stream>>>(a);
+    return launch_status();
+  }
+  if (DELTA) rk_chain_kernel<DK><<<dim3(a.dv / RK_NV, a.H, a.n_items), RK_THREADS, sm_chain, stream>>>(a);
+  else rk_states_kernel<DK><<<dim3((a.dv * DK / 4 + RK_THREADS - 1) / RK_THREADS, a.H, a.n_items), RK_THREADS, 0, stream>>>(a);
+  rk_out_kernel<DELTA, DK><<<dim3(a.cells, a.H, tiles), RK_OUT_THREADS, sm_out, stream>>>(a);
   return launch_status();
 }
 
@@ -575,20 +919,20 @@ static long long rk_image_floats(int mode, int dk) {
 }
 
 // Floats of scratch for a step of T rows.
-FELLM_API long long fellm_recurrent_chunk_scratch(int mode, int T, int n_items, int H, int dk, int dv) {
-  return (T / RK_C + (long long)n_items) * H * (rk_image_floats(mode, dk) + (long long)RK_C * dv);
+FELLM_API long long fellm_recurrent_chunk_scratch(int mode, int T, int n_items, int H, int dk, int dv, int apart) {
+  return (T / RK_C + (long long)n_items) * H * (rk_image_floats(mode, dk) + (long long)(RK_C + (apart ? dk : 0)) * dv);
 }
 
 // mode 0 / 1: the delta rule with a decay per head / channel (q, k [T, G dk] and v [T, H dv] in rows of ld elements, as
 // fellm_delta_scan takes them); 2: decay and bonus (r, k, v [T, H dk]); 3: gated write (q raw, f raw, v).  Items of fewer
-// than min_rows rows are left alone.  16-byte rows: see the checks.
+// than min_rows rows are left alone.  apart: the outputs beside one another behind the states (scratch for that), else in one walk with them.  16-byte rows: see the checks.
 FELLM_API int fellm_recurrent_chunk(int mode, const void* q, const void* k, const void* v, int is_bf16, int ld, int v_off,
                                     const float* small, int lds, int b_off, int a_off, const float* A_log, const float* dt_bias,
                                     const float* gch, const float* bonus, const float* lower, const float* fbias, float* state,
                                     long long slot_stride, const int* item_start, const int* item_slot, float* out, float* scratch,
-                                    int T, int n_items, int max_rows, int min_rows, int H, int G, int dk, int dv, cudaStream_t stream) {
+                                    int T, int n_items, int min_rows, int H, int G, int dk, int dv, int apart, cudaStream_t stream) {
   if (n_items <= 0 || T <= 0) return 0;
-  if ((dk != 64 && dk != 128) || dv < RK_NV || dv % RK_NV || H < 1 || G < 1 || H % G || max_rows < 1 || min_rows < 1 || mode < 0 || mode > 3 ||
+  if ((dk != 64 && dk != 128) || dv < RK_NV || dv % RK_NV || H < 1 || G < 1 || H % G || min_rows < 1 || mode < 0 || mode > 3 ||
       n_items > 65535 || H > 65535) return FELLM_ERR_SIZE;
   if (!q || !k || !v || !state || !item_start || !item_slot || !out || !scratch) return FELLM_ERR_ARG;
   if ((mode <= 1 && !small) || (mode == 0 && (!A_log || !dt_bias)) || ((mode == 1 || mode == 2) && !gch) || (mode == 2 && !bonus) ||
@@ -602,10 +946,10 @@ FELLM_API int fellm_recurrent_chunk(int mode, const void* q, const void* k, cons
   a.q = q; a.k = k; a.v = v; a.ld = ld; a.v_off = v_off; a.small = small; a.lds = lds; a.b_off = b_off; a.a_off = a_off;
   a.A_log = A_log; a.dt_bias = dt_bias; a.gch = gch; a.bonus = bonus; a.lower = lower; a.fbias = fbias;
   a.item_start = item_start; a.item_slot = item_slot; a.state = state; a.slot_stride = slot_stride; a.out = out;
-  a.H = H; a.G = G; a.dv = dv; a.min_rows = min_rows;
+  a.H = H; a.G = G; a.dv = dv; a.min_rows = min_rows; a.n_items = n_items; a.cells = T / RK_C + n_items;
   const size_t cells = (size_t)(T / RK_C + n_items) * H;
-  a.image = scratch; a.U = scratch + cells * (size_t)rk_image_floats(mode, dk);
-#define RK_GO(MODE_, TA_) (dk == 128 ? rk_launch<MODE_, 128, TA_>(a, n_items, max_rows, stream) : rk_launch<MODE_, 64, TA_>(a, n_items, max_rows, stream))
+  a.image = scratch; a.U = scratch + cells * (size_t)rk_image_floats(mode, dk); a.S = apart ? a.U + cells * ((size_t)RK_C * dv) : nullptr;
+#define RK_GO(MODE_, TA_) (dk == 128 ? rk_launch<MODE_, 128, TA_>(a, stream) : rk_launch<MODE_, 64, TA_>(a, stream))
   if (mode == 0) return is_bf16 ? RK_GO(0, bf16) : RK_GO(0, float);
   if (mode == 1) return is_bf16 ? RK_GO(1, bf16) : RK_GO(1, float);
   if (mode == 2) return is_bf16 ? RK_GO(2, bf16) : RK_GO(2, float);

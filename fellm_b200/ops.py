@@ -653,6 +653,14 @@ RECURRENT_CHUNK_MIN_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_CHUNK_MIN_RO
 # and 54.5, 0.12..0.3 us a row there and half of it here.
 RECURRENT_CHUNK_STEP_ROWS = {64: 120, 128: 90}
 RECURRENT_CHUNK_MIXED_ROWS = 256
+# Portions of this many rows or more: states first, then all outputs side by side; up to it one walk makes both, a launch less.  Without
+# the delta rule the states are then no chain of products any more.  With it (modes 0, 1) the chain keeps its products and only the
+# outputs' leave it, which pays later where the walk's blocks fill the device.  us, one walk / apart: decay and bonus, 16 heads of 64: 192
+# rows 22.5 / 22.6, 256 25.3 / 23.0, 400 among 15 single tokens 69.3 / 63.8; gated write, 8 heads of 128: 192 25.3 / 27.4, 384 36.0 / 30.2, 300
+# among single tokens 85.4 / 88.6, 400 90.9 / 89.9; delta rule of 8 heads 320 43.7 / 43.3, 768 80.8 / 72.1; of 16 heads 320 48.0 / 50.3,
+# 768 87.4 / 87.8, 2,048 225 / 215.
+RECURRENT_APART_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_APART_ROWS", 320))
+RECURRENT_APART_ROWS_FULL = max(RECURRENT_APART_ROWS, 1024)        # the delta rule with more than 96 blocks a portion (H dv / 16)
 
 
 def recurrent_chunk_rows(dtype, n_rows: int, n_items: int, max_item_rows: int, key_dim: int) -> int:
@@ -669,7 +677,8 @@ def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_i
                      small=None, b_off=0, a_off=0, A_log=None, dt_bias=None, gch=None, bonus=None, lower=None, fbias=None) -> bool:
     """Runs the items of min_rows rows or more in chunks; False (nothing launched) for sizes and alignments the kernels do not
     take (a lane reads dk / 32 neighbouring elements at once, a block keeps 16 value columns) and for steps whose chunks would
-    take more than LAYER_SCRATCH_MAX_BYTES."""
+    take more than LAYER_SCRATCH_MAX_BYTES.  The outputs are made apart from the states where a portion is long enough and the
+    states in front of all chunks fit that limit too."""
     es = q.element_size()
     lane = dk // 32
     if dk not in (64, 128) or dv % 16 or n_items > 65535 or H > 65535 or (mode == 3 and es == 2):
@@ -679,9 +688,11 @@ def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_i
     if out.data_ptr() % 16 or not out.is_contiguous():
         return False
     T = out.shape[0]
-    need = _fn("recurrent_chunk", "fellm_recurrent_chunk_scratch", [_c_int] * 6)
+    need = _fn("recurrent_chunk", "fellm_recurrent_chunk_scratch", [_c_int] * 7)
     need.restype = _c_ll
-    floats = need(mode, T, n_items, H, dk, dv)
+    apart_from = RECURRENT_APART_ROWS_FULL if mode <= 1 and H * dv > 96 * 16 else RECURRENT_APART_ROWS
+    apart = max_item_rows >= apart_from and 4 * need(mode, T, n_items, H, dk, dv, 1) <= LAYER_SCRATCH_MAX_BYTES
+    floats = need(mode, T, n_items, H, dk, dv, int(apart))
     if 4 * floats > LAYER_SCRATCH_MAX_BYTES:
         return False
     scratch = torch.empty(floats, dtype=torch.float32, device=out.device)
@@ -690,8 +701,14 @@ def _recurrent_chunk(mode, q, k, v, ld, v_off, state, item_start, item_slot, n_i
             [_c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_int, _c_int] + [_c_p] * 7 + [_c_ll] + [_c_p] * 4 + [_c_int] * 8 + [_c_p])
     _check(f(mode, _p(q), _p(k), _p(v), _is_bf16(q), ld, int(v_off), _p(small), small.stride(0) if small is not None else 0, int(b_off),
              int(a_off), _p(A_log), _p(dt_bias), _p(gch), _p(bonus), _p(lower), _p(fbias), sp, ss, _p(item_start), _p(item_slot), _p(out),
-             _p(scratch), T, n_items, int(max_item_rows), int(min_rows), H, G, dk, dv, _stream()), "recurrent_chunk")
+             _p(scratch), T, n_items, int(min_rows), H, G, dk, dv, int(apart), _stream()), "recurrent_chunk")
     return True
+
+
+def _no_item_below(rows: int, T: int, n_items: int, max_item_rows: int) -> bool:
+    """Whether T rows in n_items portions of up to max_item_rows leave none with fewer than `rows`: then nothing is left for the scan
+    behind the chunks, an empty launch of 2 us."""
+    return T - (n_items - 1) * max_item_rows >= rows
 
 
 def gated_write_scan(z, f_off, v_off, lower, bias, state, item_start, item_slot, n_items, H, dk, dv, out=None,
@@ -721,7 +738,7 @@ def gated_write_scan(z, f_off, v_off, lower, bias, state, item_start, item_slot,
     skip = 0
     if 0 < chunk_rows <= max_item_rows and _recurrent_chunk(3, z, z[:, f_off:], z, z.stride(0), v_off, state, item_start, item_slot, n_items,
                                                             max_item_rows, chunk_rows, H, H, dk, dv, out, lower=lower, fbias=bias):
-        if n_items == 1:
+        if _no_item_below(chunk_rows, T, n_items, max_item_rows):
             return out
         skip, max_item_rows, block, prepared = chunk_rows, chunk_rows - 1, 0, False
     sp, ss = _state_args(state)
@@ -790,7 +807,7 @@ def delta_scan(qkv, k_off, v_off, small, b_off, a_off, A_log, dt_bias, gch, stat
     if 0 < chunk_rows <= max_item_rows and _recurrent_chunk(
             0 if gch is None else 1, qkv, qkv[:, k_off:], qkv, qkv.stride(0), v_off, state, item_start, item_slot, n_items, max_item_rows,
             chunk_rows, H, G, dk, dv, out, small=small, b_off=b_off, a_off=a_off, A_log=A_log, dt_bias=dt_bias, gch=gch):
-        if n_items == 1:
+        if _no_item_below(chunk_rows, T, n_items, max_item_rows):
             return out
         skip, max_item_rows = chunk_rows, chunk_rows - 1
     sp, ss = _state_args(state)
@@ -821,7 +838,7 @@ def decay_bonus_scan(r, k, v, w, u, state, item_start, item_slot, n_items, H, dk
     skip = 0
     if 0 < chunk_rows <= max_item_rows and _recurrent_chunk(2, r, k, v, r.stride(0), 0, state, item_start, item_slot, n_items, max_item_rows,
                                                             chunk_rows, H, H, dk, dk, out, gch=w, bonus=u):
-        if n_items == 1:
+        if _no_item_below(chunk_rows, T, n_items, max_item_rows):
             return out
         skip, max_item_rows = chunk_rows, chunk_rows - 1
     sp, ss = _state_args(state)
