@@ -1,7 +1,7 @@
 // Causal GQA attention over the paged float32 cache, heads of 64, 1, 2 or 4 of them a kv head: the 32-bit engine's attention
 // of the LFM2 shapes, float32 arithmetic on CUDA cores.  What paged_attention_simt_kernel (attention_simt.cu) computes; there a
 // block is a (row, head), so every row and head reads its keys and values again, a lane a key (104 us for 201 rows of 16
-// heads behind 250 tokens each; 44 here).
+// heads behind 250 tokens each; 39 here).
 //
 // Here a block of four warps takes a kv head and RB neighbouring rows: a tile of 32 keys is read once for its RB x R queries,
 // 8 lanes a key and 32 bytes a lane.  The partial dot products of a lane's eight keys go through the eight lanes by a
@@ -171,13 +171,19 @@ FELLM_API int fellm_attention_f32(const float* q, int ldq, const float* pool, co
   if (!q || !pool || !block_table || !positions || !row_slot || !out) return FELLM_ERR_ARG;
   if (hd != AF_HD || G < 1 || G > 65535 || H % G || page_tokens < 1 || (ldq & 3) || (((uintptr_t)q | (uintptr_t)pool) & 15)) return FELLM_ERR_SIZE;
   const AfArgs a = {q, pool, block_table, positions, row_slot, out, max_pages, T, H, G, page_tokens, layer, layers_in_group, window, ldq, scale};
-  // neighbouring rows share a tile's reading where there are rows enough for every SM and no window
+  // Neighbouring rows share a tile's reading where there are rows enough and no window: eight queries a block where their blocks go three
+  // times (two heads a kv head) or one and a half times (one, four) into the SMs, else four: more blocks, each with half the registers.
+  // us, eight / four queries a block, 8 kv heads; two heads: 201 rows behind 300 40.7 / 36.0, 64 behind 500 29.5 / 18.1, 32 behind 100 12.9 /
+  // 7.6, 256 behind 500 64.6 / 71.6, 1,024 194 / 212; one head: 200 rows 35.1 / 17.3, 256 behind 500 34.7 / 38.2; four heads: 32 behind 100
+  // 13.5 / 8.9, 64 behind 500 29.9 / 36.5.
   const bool many = window <= 0 && T >= 32;
+  const int R = H / G;
+  const bool eight = R <= 4 && 2ll * ceil_div(T, 8 / (R < 1 ? 1 : R)) * G >= (R == 2 ? 6ll : 3ll) * fellm_sm_count();
 #define AF_GO(R_, RB_) attention_f32_kernel<R_, RB_><<<dim3(ceil_div(T, RB_), G), AF_WARPS * 32, 0, stream>>>(a)
-  switch (H / G) {
-    case 1: if (many) AF_GO(1, 8); else AF_GO(1, 1); break;
-    case 2: if (many) AF_GO(2, 4); else AF_GO(2, 1); break;
-    case 4: if (many) AF_GO(4, 2); else AF_GO(4, 1); break;
+  switch (R) {
+    case 1: if (many && eight) AF_GO(1, 8); else if (many) AF_GO(1, 4); else AF_GO(1, 1); break;
+    case 2: if (many && eight) AF_GO(2, 4); else if (many) AF_GO(2, 2); else AF_GO(2, 1); break;
+    case 4: if (many && eight) AF_GO(4, 2); else AF_GO(4, 1); break;
     default: return FELLM_ERR_SIZE;
   }
 #undef AF_GO

@@ -77,12 +77,14 @@ gemm_tn_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const fl
 
 // All three float32, rows that start on 16 bytes and K a multiple of 4: the same chains, fed by cp.async through a ring of
 // FP_STAGES stages of 32 k.  A thread keeps TM x TN outputs whose rows and columns are TBM / TM and TBN / TN apart, and reads
-// four k of a row at a time (row stride 36 floats: the 8 rows of a quarter warp in different banks).  Bound by those reads
-// where rows are many (4 x 4 outputs: 32 floats from shared memory for 64 multiply-adds) and by the warps' latency: 8 x 4
-// outputs a thread halve the warps and take 49 and 63 us where 4 x 4 take 48 ([201, 2048, 1024]) and 44 ([201, 1024, 1024]); the
-// kernel above, without loads in flight under its sums, takes 95 for either.  Tiles of 64 x 64 where they fill three
-// quarters of the SMs, of 32 x 64 where those fill half, else 16 x 32 and 8 x 32 with few outputs a thread: a product of a
-// decode step is a few chains of K dependent multiply-adds, and more warps walk them side by side.
+// four k of a row at a time (row stride 36 floats: the 8 rows of a quarter warp in different banks), the next four's on their
+// way under the sums.  A 16-byte load takes four wavefronts of shared memory, two where lanes one or two apart ask for the same: a
+// warp's 4 x 8 threads have rows and columns in alternate bits of the lane's number, 16 wavefronts for the 16 cycles of its 4 x 4 x 4
+// multiply-adds (24 before).  Bound by those and, with few warps, by their latency.  us at K = 1,024, loads numbered row after row and
+// used as they came / now: [201, 2048] 47 / 33, [201, 1024] 39 / 20, [256, 9216] 146 / 114, [48, 1024] 25 / 10, [8, 1024] 18 / 10.
+// The tile: 16 x 32 of 2 x 2 outputs a thread takes some 5.6 us a block and SM side by side, 64 x 64 of 4 x 4 29 and never less
+// than 33: the latter where that is less and its rows are filled ([256, 9216] 114 / 163, [33, 6176] 34 / 23, [201, 2048] 35 / 33, [256, 1024],
+// K = 4,608 151 / 94).  8 x 32 for up to 8 rows.
 #define FP_STAGES 4
 #define FP_BK 32
 #define FP_LD 36
@@ -98,18 +100,30 @@ gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, con
   FELLM_TRACE_SCOPE(TRACE_GEMM_SIMT);
   extern __shared__ __align__(16) float fp_smem[];
   constexpr int THREADS = TBM * TBN / (TN * TM), TX = TBN / TN, TY = TBM / TM, STAGE = (TBM + TBN) * FP_LD;
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  // a warp is 4 x 8 threads of the tile, rows in bits 0 and 4 of the lane's number, columns in bits 1 to 3
+  static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp is 4 x 8 threads");
+  const int tid = threadIdx.x, lane = tid & 31, wx = (tid >> 5) % (TX / 8), wy = (tid >> 5) / (TX / 8);
+  const int tx = 8 * wx + ((lane >> 1) & 7), ty = 4 * wy + (lane & 1) + 2 * (lane >> 4);
   const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
+  // a thread's copies: the same rows in every step, 16 bytes each
+  constexpr int COPIES = ((TBM + TBN) * (FP_BK / 4) + THREADS - 1) / THREADS, APART = THREADS / (FP_BK / 4);
+  constexpr bool WHOLE = COPIES * THREADS == (TBM + TBN) * (FP_BK / 4);           // every thread has as many
+  const float* src[COPIES];
+  bool in[COPIES];
+  const int r0 = tid / (FP_BK / 4), kq = (tid % (FP_BK / 4)) * 4;
+#pragma unroll
+  for (int c = 0; c < COPIES; ++c) {
+    const int r = r0 + c * APART, row = r < TBM ? m0 + r : n0 + r - TBM;
+    in[c] = row < (r < TBM ? M : N);
+    src[c] = !in[c] ? A : (r < TBM ? A + (size_t)row * lda : W + (size_t)row * ldw) + kq;
+  }
   auto fetch = [&](int step) {
-    float* st = fp_smem + (step % FP_STAGES) * STAGE;
+    float* st = fp_smem + (step % FP_STAGES) * STAGE + r0 * FP_LD + kq;
     const int k0 = step * FP_BK;
-    for (int x = tid; x < (TBM + TBN) * (FP_BK / 4); x += THREADS) {
-      const int r = x / (FP_BK / 4), k = k0 + (x % (FP_BK / 4)) * 4;
-      const bool is_a = r < TBM;
-      const int row = is_a ? m0 + r : n0 + r - TBM;
-      const bool live = k < K && row < (is_a ? M : N);
-      fp_copy16(st + r * FP_LD + k - k0, live ? (is_a ? A + (size_t)row * lda + k : W + (size_t)row * ldw + k) : A, live);
-    }
+    const bool k_in = k0 + kq < K;
+#pragma unroll
+    for (int c = 0; c < COPIES; ++c)
+      if (WHOLE || r0 + c * APART < TBM + TBN) fp_copy16(st + c * APART * FP_LD, in[c] && k_in ? src[c] + k0 : A, in[c] && k_in);
   };
   const int steps = (K + FP_BK - 1) / FP_BK;
 #pragma unroll
@@ -129,20 +143,36 @@ gemm_tn_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, con
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     const float* As = fp_smem + (s % FP_STAGES) * STAGE + ty * FP_LD;
     const float* Ws = fp_smem + (s % FP_STAGES) * STAGE + (TBM + tx) * FP_LD;
+    // four k at a time, the next four's on their way under the sums
+    float4 a[2][TM], w[2][TN];
+    auto read = [&](int k, int to) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[to][i] = *(const float4*)(As + TY * i * FP_LD + k);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[to][j] = *(const float4*)(Ws + TX * j * FP_LD + k);
+    };
+    read(0, 0);
 #pragma unroll
     for (int k = 0; k < FP_BK; k += 4) {
-      float4 a[TM], w[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *(const float4*)(As + TY * i * FP_LD + k);
-#pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = *(const float4*)(Ws + TX * j * FP_LD + k);
+      const int at = (k >> 2) & 1;
+      if (k + 4 < FP_BK) read(k + 4, at ^ 1);
+      // (each output's chain in the order of k)
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {              // (each output's chain in the order of k)
-          acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]); acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
-          acc[i][j] = fmaf(a[i].z, w[j].z, acc[i][j]); acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
-        }
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[at][i].x, w[at][j].x, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[at][i].y, w[at][j].y, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[at][i].z, w[at][j].z, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[at][i].w, w[at][j].w, acc[i][j]);
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -199,8 +229,8 @@ FELLM_API int fellm_gemm_simt(const void* A, int a_dt, const void* W, int w_dt, 
     const float *a = (const float*)A, *w = (const float*)W;
     int sms = 0, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    if (M > 32 && (long long)ceil_div(N, 64) * ceil_div(M, 64) >= sms * 3 / 4) return launch_f32<64, 64, 4, 4>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
-    if (M > 16 && (long long)ceil_div(N, 64) * ceil_div(M, 32) >= sms / 2) return launch_f32<32, 64, 4, 4>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
+    const long long large = (long long)ceil_div(N, 64) * ceil_div(M, 64), small = (long long)ceil_div(N, 32) * ceil_div(M, 16);
+    if (10 * small > 59ll * sms && 10 * small > 52 * large) return launch_f32<64, 64, 4, 4>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
     if (M > 8) return launch_f32<16, 32, 2, 2>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
     return launch_f32<8, 32, 2, 1>(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, epi, s);
   }
