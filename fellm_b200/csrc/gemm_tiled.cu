@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(HW_WARPS * 32)
 gemm_heads_few_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, bf16* __restrict__ out, int M, int N, int K, int lda, int ldw,
                       int ldo, long long sa, long long sw, long long so) {
   FELLM_TRACE_SCOPE(TRACE_GEMM_TILED);
+  pdl_launch_dependents();              // (launched the ordinary way itself; a dependent behind it may start, and waits for its end)
   const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
   const int n0 = (blockIdx.x * HW_WARPS + (threadIdx.x >> 5)) * 16, na = n0 + g, nb = na + 8;
   if (n0 >= N) return;

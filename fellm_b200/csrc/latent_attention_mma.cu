@@ -4,24 +4,35 @@
 //
 // A token's cache row is [c (RK) | rotated key part (DR)], one for all heads; a query row is [W_uk,h^T qn (RK) |
 // rotated qr (DR)] per (token, head).  score = scale (query . row); the value of a key is the first RK elements of
-// its row.  So all H heads of a token are rows of ONE product against the same keys: a CTA takes MQ = 16 NG
-// consecutive (token, head) rows of one item, walks the keys its rows can see in tiles of KT = 16 NC, and its NG x NC
-// warps split a tile two ways: warp (i, j) computes the scores of row group i against keys [16 j, 16 j + 16) of the
-// tile and leaves them in shared memory; after a barrier it reads its group's scores for the whole tile, does the
-// online softmax for them (the NC warps of a group do the same arithmetic and hold the same m and l), and adds
-// P V for the value elements [j RK / NC, (j + 1) RK / NC), which it alone accumulates: a row's read-out of RK
-// float32 sums lies across NC warps' registers.
+// its row.  So all H heads of a token are rows of ONE product against the same keys.  Two kernels:
 //
-//   NG = 4, NC = 2   portions of prompts: 64 rows, key tiles of 32 through a two-stage cp.async ring
-//   NG = 1, NC = 4   single tokens (16 rows = the heads of a token), key tiles of 64; NC = 2 where RK / 4 is not a
-//                    multiple of 16.  The key range can be split over gridDim.z CTAs, which leave (m, l, sums) in a
-//                    scratch buffer that latent_merge_kernel puts together (a block a row: 8 x the parallelism of
-//                    a merge by the CTA that finishes last, which was tried and cost 40 us a layer).
+// Portions of prompts (latent_attention_kernel): a CTA takes MQ = 16 NG consecutive (token, head) rows of one item, walks
+// the keys its rows can see in tiles of KT = 16 NC through a two-stage cp.async ring, and its NG x NC warps split a tile two
+// ways: warp (i, j) computes the scores of row group i against keys [16 j, 16 j + 16) of the tile and leaves them in shared
+// memory; after a barrier it reads its group's scores for the whole tile, does the online softmax for them (the NC warps of
+// a group do the same arithmetic and hold the same m and l), and adds P V for the value elements [j RK / NC,
+// (j + 1) RK / NC), which it alone accumulates: a row's read-out of RK float32 sums lies across NC warps' registers.  NG = 4,
+// NC = 2: 64 rows, key tiles of 32.
+//
+// Single tokens (latent_tokens_kernel): 16 rows (the heads of a token) and a share of their keys a CTA of eight warps, tiles of
+// 64 keys.  A warp makes the scores of eight keys, a thread the probabilities of four (16 threads a row), a warp the sums of
+// an eighth of the value elements.  A token's keys are shared out in portions of 16; up to eight shares are a cluster, whose
+// sums stay in shared memory and are put together through distributed shared memory, every CTA an eighth of the
+// elements.  More shares (long contexts of few requests) leave (m, l, sums) in a scratch buffer that latent_merge_kernel puts
+// together (a block a row: 8 x the parallelism of a merge by the CTA that finishes last, which was tried and cost 40 us a
+// layer).  Index arrays and cache rows are read ahead of the wait for the kernel in front: see the kernel.
+// Bound by: latency, of the index arrays, of the keys, of the chains of a tile (tiles by four warps that each did the softmax of all
+// rows took 6,700 instructions a warp, 17 us; eight warps, 3,300, 14.5 us; one page a warp and angles ahead of the wait 12.6 us by itself
+// and 9 behind the product in front; 8 tokens of 8 heads over 1,024 keys of 1,152 bytes, 11.7 + 5.7 us for the merge before).
 //
 // A key counts for the row of a token at position p iff p - window < key <= p (window 0: every key up to p).  A
 // sink per head joins the denominator once: exp(sink_h), not scaled, no value.  Rows of an item have consecutive
 // positions; key tiles start at multiples of KT, so a tile lies in one page (page_tokens % KT == 0).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 #ifndef LAT_RK
 #define LAT_RK 512
@@ -78,9 +89,9 @@ struct LatArgs {
   const int* block_table; int max_pages;
   const int* positions; const int* row_slot; const int* item_start;
   bf16* out;                // [rows][H][RK]
-  float* scratch;           // n_splits > 1: [rows * H][n_splits][RK + 2]
+  float* scratch;           // n_splits > 1 and no cluster: [rows * H][n_splits][RK + 2]
   const float* sinks;       // [H] or null
-  int H, page_tokens, layer, layers_in_group, window, n_splits;
+  int H, page_tokens, layer, layers_in_group, window, n_splits, cluster, single;       // single: every item is one token
   float scale_log2;
 };
 
@@ -105,8 +116,6 @@ __global__ void __launch_bounds__(NG * NC * 32, 1) latent_attention_kernel(LatAr
   int key_begin = a.window > 0 ? max(0, pos_lo - a.window + 1) : 0;
   key_begin &= ~(KT - 1);
   const int n_tiles = (pos_hi + 1 - key_begin + KT - 1) / KT;
-  const int per = (n_tiles + a.n_splits - 1) / a.n_splits;
-  const int t_begin = blockIdx.z * per, t_end = min(n_tiles, t_begin + per);
 
   const unsigned q_s = (unsigned)__cvta_generic_to_shared(smem), k_s = q_s + MQ * ROWB;
   float* S_s = (float*)(smem + (MQ + 2 * KT) * ROWB);
@@ -165,13 +174,13 @@ __global__ void __launch_bounds__(NG * NC * 32, 1) latent_attention_kernel(LatAr
   for (int n = 0; n < NT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
-  if (t_begin < t_end) load_tile(t_begin, 0);
+  load_tile(0, 0);
   cp_async_commit();
-  for (int t = t_begin; t < t_end; ++t) {
-    const int buf = (t - t_begin) & 1;
+  for (int t = 0; t < n_tiles; ++t) {
+    const int buf = t & 1;
     cp_async_wait_all();
     __syncthreads();                   // tile t has landed; everyone is done with the other buffer and with S_s
-    if (t + 1 < t_end) load_tile(t + 1, buf ^ 1);
+    if (t + 1 < n_tiles) load_tile(t + 1, buf ^ 1);
     cp_async_commit();
     const int k0 = key_begin + t * KT;
     const bool live = k0 <= grp_hi && k0 + KT - 1 >= grp_first;        // some row of the group sees some key of the tile
@@ -253,32 +262,271 @@ __global__ void __launch_bounds__(NG * NC * 32, 1) latent_attention_kernel(LatAr
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   const size_t row_g0 = (size_t)r_begin * H + Rg0;         // the (token, head) row among all rows of the step
-  if (a.n_splits == 1) {
-    if (a.sinks) {
-      l0 += exp2f(a.sinks[Rg0 % H] * LOG2E - m0);
-      l1 += exp2f(a.sinks[Rg1 % H] * LOG2E - m1);
-    }
-    const float inv0 = 1.0f / l0, inv1 = 1.0f / l1;
+  if (a.sinks) {
+    l0 += exp2f(a.sinks[Rg0 % H] * LOG2E - m0);
+    l1 += exp2f(a.sinks[Rg1 % H] * LOG2E - m1);
+  }
+  const float inv0 = 1.0f / l0, inv1 = 1.0f / l1;
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      const int col = wj * DVW + 8 * n + 2 * c;
-      if (Rg0 < n_rows) *(__nv_bfloat162*)(a.out + row_g0 * RK + col) = __floats2bfloat162_rn(o[n][0] * inv0, o[n][1] * inv0);
-      if (Rg1 < n_rows) *(__nv_bfloat162*)(a.out + (row_g0 + 8) * RK + col) = __floats2bfloat162_rn(o[n][2] * inv1, o[n][3] * inv1);
-    }
-  } else {
-    float* r0 = a.scratch + (row_g0 * a.n_splits + blockIdx.z) * (RK + 2);
-    float* r1 = a.scratch + ((row_g0 + 8) * a.n_splits + blockIdx.z) * (RK + 2);
+  for (int n = 0; n < NT; ++n) {
+    const int col = wj * DVW + 8 * n + 2 * c;
+    if (Rg0 < n_rows) *(__nv_bfloat162*)(a.out + row_g0 * RK + col) = __floats2bfloat162_rn(o[n][0] * inv0, o[n][1] * inv0);
+    if (Rg1 < n_rows) *(__nv_bfloat162*)(a.out + (row_g0 + 8) * RK + col) = __floats2bfloat162_rn(o[n][2] * inv1, o[n][3] * inv1);
+  }
+}
+
+// ---------------------------------------------------------------- single tokens
+constexpr int LT_WARPS = 8, LT_KT = 64, LT_ROWS = 16;
+constexpr int LT_SLD = LT_KT + 4, LT_PLD = LT_KT + 8;        // row strides of the scores (float32) and the probabilities (bfloat16)
+constexpr int LT_OLD = RK + 4;                               // and of the sums that a cluster puts together
+constexpr int LT_GROUPS = (RK / 16 + LT_WARPS - 1) / LT_WARPS;                // 16 value elements each, a warp's: warp, warp + 8, ..
+constexpr size_t LT_KEYS = (size_t)2 * LT_KT * ROWB;
+constexpr size_t LT_SUMS = (size_t)LT_ROWS * LT_OLD * sizeof(float);
+constexpr size_t LT_SMEM = LT_ROWS * ROWB + (LT_KEYS > LT_SUMS ? LT_KEYS : LT_SUMS);
+
+__global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs a) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(16) float S_s[LT_ROWS * LT_SLD];
+  __shared__ __align__(16) bf16 P_s[LT_ROWS * LT_PLD];
+  __shared__ float corr_s[LT_ROWS];
+  __shared__ float2 ml_s[LT_ROWS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3, H = a.H;
+  const int rank = blockIdx.x, item = blockIdx.y, R0 = blockIdx.z * LT_ROWS;
+  pdl_launch_dependents();
+  // Launched as a programmatic dependent of the product that makes q, which is launched the ordinary way: all that was written in front
+  // of that one is there, the index arrays and the cache with this step's own rows.  Only q is waited for.
+  const int r_begin = a.single ? item : a.item_start[item], n_rows = a.single ? H : (a.item_start[item + 1] - r_begin) * H;
+  if (R0 >= n_rows) { pdl_wait(); return; }        // (the same for a whole cluster)
+  const int rows_here = min(LT_ROWS, n_rows - R0), pos0 = a.positions[r_begin];
+  const int* bt = a.block_table + (size_t)a.row_slot[r_begin] * a.max_pages;
+  auto token_of = [&](int R) { return a.single ? 0 : R / H; };                  // which of the item's tokens a row belongs to
+  const int pos_lo = pos0 + token_of(R0), pos_hi = pos0 + token_of(R0 + rows_here - 1);
+  // this CTA's share of the keys, in portions of 16
+  int key_begin = (a.window > 0 ? max(0, pos_lo - a.window + 1) : 0) & ~15;
+  const int portions = (pos_hi + 1 - key_begin + 15) / 16, per = (portions + a.n_splits - 1) / a.n_splits;
+  const int mine = max(0, min(per, portions - rank * per));
+  key_begin += 16 * rank * per;
+  const int key_end = min(pos_hi + 1, key_begin + 16 * mine), n_tiles = (16 * mine + LT_KT - 1) / LT_KT;
+
+  const unsigned q_s = (unsigned)__cvta_generic_to_shared(smem), k_s = q_s + LT_ROWS * ROWB;
+  // A tile's portions with a key, two warps each, eight rows a warp: 16 keys lie in one page, so a warp looks one page up and its
+  // rows lie behind one another.  Keys beyond the last visible one are zeros: they are masked, but a value of a freed page's
+  // bits must not reach a product (0 * NaN).
+  auto rows_of = [&](int t) {                      // this warp's eight rows of a tile (an address without keys is not read)
+    const int k0 = min(key_begin + t * LT_KT + 16 * (warp >> 1), max(key_end - 1, 0)) & ~15;
+    const int page = max(bt[k0 / a.page_tokens], 0);             // an unmapped entry (-1) must never become an address
+    return a.pool + (((size_t)page * a.layers_in_group + a.layer) * a.page_tokens + (k0 % a.page_tokens + 8 * (warp & 1))) * D;
+  };
+  auto load_tile = [&](int t, const bf16* src) {
+    const int at = 16 * (warp >> 1) + 8 * (warp & 1), n_keys = key_end - (key_begin + t * LT_KT) - at;
+    if (n_keys + 8 * (warp & 1) > 0) {             // (the portion has a key)
+      const unsigned dst = k_s + (t & 1) * LT_KT * ROWB;
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      const int col = wj * DVW + 8 * n + 2 * c;
-      if (Rg0 < n_rows) *(float2*)(r0 + col) = make_float2(o[n][0], o[n][1]);
-      if (Rg1 < n_rows) *(float2*)(r1 + col) = make_float2(o[n][2], o[n][3]);
+      for (int i = 0; i < (8 * CPR + 31) / 32; ++i) {
+        const int ch = lane + 32 * i, r = ch / CPR;
+        if (8 * CPR % 32 && r >= 8) break;
+        if (r < n_keys) cp_async16(dst + tile_off(at + r, ch - r * CPR), src + ch * 8);
+        else st_shared_zero16(dst + tile_off(at + r, ch - r * CPR));
+      }
     }
-    if (wj == 0 && c == 0) {
-      if (Rg0 < n_rows) { r0[RK] = m0; r0[RK + 1] = l0; }
-      if (Rg1 < n_rows) { r1[RK] = m1; r1[RK + 1] = l1; }
+    cp_async_commit();
+  };
+  if (n_tiles > 0) {
+    const bf16 *first = rows_of(0), *second = rows_of(1);
+    load_tile(0, first);
+    if (n_tiles > 1) load_tile(1, second);
+  }
+  // the rotated part's pairs (a thread's PAIRS): their angles do not wait either
+  constexpr int PAIRS = (LT_ROWS * DR / 2 + LT_WARPS * 32 - 1) / (LT_WARPS * 32), HALF = DR / 2 > 0 ? DR / 2 : 1;
+  float sn[PAIRS > 0 ? PAIRS : 1], cs[PAIRS > 0 ? PAIRS : 1];
+  if (a.qsrc) {
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      const int x = tid + LT_WARPS * 32 * i, r = x / HALF, p = x % HALF;
+      sn[i] = 0.f; cs[i] = 1.f;
+      if (r < rows_here && 2 * p < a.n_rot) {
+        sincosf((float)(pos0 + token_of(R0 + r)) * a.freq[p], &sn[i], &cs[i]);
+        sn[i] *= a.mag; cs[i] *= a.mag;
+      }
     }
   }
+  pdl_wait();
+  // the query rows (rows beyond the item's end are zeros)
+  {
+    const int q_ld = a.qsrc ? RK : D, chunks = q_ld / 8;
+    const bf16* qg = a.q + ((size_t)r_begin * H + R0) * q_ld;
+    for (int r = warp; r < LT_ROWS; r += LT_WARPS)
+      for (int cc = lane; cc < chunks; cc += 32) {
+        if (r < rows_here) cp_async16(q_s + tile_off(r, cc), qg + (size_t)r * q_ld + cc * 8);
+        else st_shared_zero16(q_s + tile_off(r, cc));
+      }
+    if (a.qsrc) {
+#pragma unroll
+      for (int i = 0; i < PAIRS; ++i) {
+        const int x = tid + LT_WARPS * 32 * i, r = x / HALF, p = x % HALF;
+        if (r >= LT_ROWS) break;
+        __nv_bfloat162 v = __floats2bfloat162_rn(0.f, 0.f);
+        if (r < rows_here) {
+          const int t = token_of(R0 + r), h = R0 + r - t * H;
+          v = *(const __nv_bfloat162*)(a.qsrc + (size_t)(r_begin + t) * a.ldq + (size_t)h * a.q_head + a.q_rot_off + 2 * p);
+          if (2 * p < a.n_rot) {
+            const float2 uv = __bfloat1622float2(v);
+            v = __floats2bfloat162_rn(uv.x * cs[i] - uv.y * sn[i], uv.y * cs[i] + uv.x * sn[i]);
+          }
+        }
+        asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(q_s + tile_off(r, RK / 8 + p / 4) + 4 * (p % 4)), "r"(*(const unsigned*)&v));
+      }
+    }
+    cp_async_commit();
+  }
+  // a thread's row and four keys of the softmax
+  const int sr = tid >> 4, sk = 4 * (tid & 15);
+  const int hi = pos0 + token_of(min(R0 + sr, n_rows - 1)), lo = a.window > 0 ? hi - a.window + 1 : 0;
+  float m = -INFINITY, l = 0.f;
+  float o[LT_GROUPS][2][4];
+#pragma unroll
+  for (int i = 0; i < LT_GROUPS; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) o[i][j][0] = o[i][j][1] = o[i][j][2] = o[i][j][3] = 0.f;
+
+  for (int t = 0; t < n_tiles; ++t) {
+    if (t > 0 && t + 1 < n_tiles) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    else cp_async_wait_all();
+    __syncthreads();                   // the tile and q are here
+    const int k0 = key_begin + t * LT_KT, n16 = min(LT_KT / 16, (key_end - k0 + 15) / 16);
+    const unsigned kb = k_s + (t & 1) * LT_KT * ROWB;
+    if (warp < 2 * n16) {
+      // scores of keys 8 warp .. + 8: two steps of 16 elements a load of theirs, a chain of MMAs each
+      float s[2][4] = {};
+      const unsigned krow = 8 * warp + (lane & 7);
+#pragma unroll 6
+      for (int ks = 0; ks < KS / 2; ++ks) {
+        unsigned a0[4], a1[4], b[4];
+        ldsm_x4(a0, q_s + tile_off(lane & 15, 4 * ks + (lane >> 4)));
+        ldsm_x4(a1, q_s + tile_off(lane & 15, 4 * ks + 2 + (lane >> 4)));
+        ldsm_x4(b, kb + tile_off(krow, 4 * ks + (lane >> 3)));
+        mma16816(s[0], a0, b[0], b[1]);
+        mma16816(s[1], a1, b[2], b[3]);
+      }
+      if (KS & 1) {
+        unsigned a0[4], b[4];
+        ldsm_x4(a0, q_s + tile_off(lane & 15, 2 * (KS - 1) + (lane >> 4)));
+        ldsm_x4(b, kb + tile_off(krow, 2 * (KS - 1) + ((lane >> 3) & 1)));        // (the last two matrices: the first two once more)
+        mma16816(s[0], a0, b[0], b[1]);
+      }
+      float* to = S_s + g * LT_SLD + 8 * warp + 2 * c;
+      *(float2*)to = make_float2(s[0][0] + s[1][0], s[0][1] + s[1][1]);
+      *(float2*)(to + 8 * LT_SLD) = make_float2(s[0][2] + s[1][2], s[0][3] + s[1][3]);
+    }
+    __syncthreads();
+    {
+      const float4 raw = *(const float4*)(S_s + sr * LT_SLD + sk);
+      float x[4] = {raw.x, raw.y, raw.z, raw.w}, mx = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int kj = k0 + sk + e;
+        x[e] = kj <= hi && kj >= lo && kj < key_end ? x[e] * a.scale_log2 : -INFINITY;
+        mx = fmaxf(mx, x[e]);
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+      const float mn = fmaxf(m, mx), mu = mn == -INFINITY ? 0.f : mn;              // (a row that has seen nothing yet)
+      const float corr = exp2f(m - mu);
+      float sum = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { x[e] = exp2f(x[e] - mu); sum += x[e]; }
+      l = l * corr + sum;
+      m = mn;
+      *(uint2*)(P_s + sr * LT_PLD + sk) = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
+      if ((tid & 15) == 0) corr_s[sr] = corr;
+    }
+    __syncthreads();
+    const float corr0 = corr_s[g], corr1 = corr_s[g + 8];
+#pragma unroll
+    for (int i = 0; i < LT_GROUPS; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) { o[i][j][0] *= corr0; o[i][j][1] *= corr0; o[i][j][2] *= corr1; o[i][j][3] *= corr1; }
+#pragma unroll
+    for (int kk = 0; kk < LT_KT / 16; ++kk) {
+      if (kk >= n16) break;
+      unsigned pa[4];
+      ldsm_x4(pa, (unsigned)__cvta_generic_to_shared(P_s + (lane & 15) * LT_PLD + 16 * kk + 8 * (lane >> 4)));
+#pragma unroll
+      for (int i = 0; i < LT_GROUPS; ++i) {
+        const int grp = warp + LT_WARPS * i;
+        if ((RK / 16) % LT_WARPS && grp >= RK / 16) break;
+        unsigned vb[4];
+        ldsm_x4_trans(vb, kb + tile_off(16 * kk + (lane & 15), 2 * grp + (lane >> 4)));
+        mma16816(o[i][0], pa, vb[0], vb[1]);
+        mma16816(o[i][1], pa, vb[2], vb[3]);
+      }
+    }
+    if (t + 2 < n_tiles) {
+      const bf16* src = rows_of(t + 2);
+      __syncthreads();                 // everyone is done with the tile
+      load_tile(t + 2, src);
+    }
+  }
+#pragma unroll
+  for (int w = 8; w > 0; w >>= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
+  cp_async_wait_all();
+  __syncthreads();                     // (the keys' place is free; P_s and corr_s are read)
+  const size_t row_g = (size_t)r_begin * H + R0;
+  const bool apart = a.n_splits > 1 && !a.cluster;
+  // the rows' sums, in shared memory for the cluster (in the keys' place) or in the scratch buffer
+  float* const os = (float*)(smem + LT_ROWS * ROWB);
+#pragma unroll
+  for (int i = 0; i < LT_GROUPS; ++i) {
+    const int grp = warp + LT_WARPS * i;
+    if ((RK / 16) % LT_WARPS && grp >= RK / 16) break;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int col = 16 * grp + 8 * j + 2 * c;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = g + 8 * e;
+        const float2 v = make_float2(o[i][j][2 * e], o[i][j][2 * e + 1]);
+        if (!apart) *(float2*)(os + r * LT_OLD + col) = v;
+        else if (r < rows_here) *(float2*)(a.scratch + ((row_g + r) * a.n_splits + rank) * (RK + 2) + col) = v;
+      }
+    }
+  }
+  if ((tid & 15) == 0) {
+    if (!apart) ml_s[sr] = make_float2(m, l);
+    else if (sr < rows_here) *(float2*)(a.scratch + ((row_g + sr) * a.n_splits + rank) * (RK + 2) + RK) = make_float2(m, l);
+  }
+  if (apart) return;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int n = a.n_splits;
+  if (n > 1) cluster.sync(); else __syncthreads();
+  // every CTA a share of the elements, four a thread
+  const int total = rows_here * (RK / 4), share = (total + n - 1) / n, end = min(total, (rank + 1) * share);
+  for (int x = rank * share + tid; x < end; x += LT_WARPS * 32) {
+    const int r = x / (RK / 4), col = 4 * (x - r * (RK / 4));
+    float4 v[8];
+    float2 ml[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < n) {
+        v[q] = *(const float4*)(cluster.map_shared_rank(os, q) + r * LT_OLD + col);
+        ml[q] = *(const float2*)(cluster.map_shared_rank(ml_s, q) + r);
+      }
+    float M = -INFINITY, L = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) if (q < n) M = fmaxf(M, ml[q].x);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < n && ml[q].x > -INFINITY) {          // (a share without a visible key counts nothing)
+        const float w = exp2f(ml[q].x - M);
+        L = fmaf(ml[q].y, w, L);
+        acc.x = fmaf(v[q].x, w, acc.x); acc.y = fmaf(v[q].y, w, acc.y); acc.z = fmaf(v[q].z, w, acc.z); acc.w = fmaf(v[q].w, w, acc.w);
+      }
+    if (a.sinks) L += exp2f(a.sinks[(R0 + r) % H] * LOG2E - M);
+    const float inv = 1.0f / L;
+    *(uint2*)(a.out + (row_g + r) * RK + col) = make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+  }
+  if (n > 1) cluster.sync();                       // nobody leaves while its sums are being read
 }
 
 // The ranges of a split key walk put together, in the order of the ranges: out = sum_s O_s 2^(m_s - m) / (sum_s l_s
@@ -324,39 +572,66 @@ static int launch_latent(const LatArgs& a, int n_items, int max_item_rows, int r
   auto kern = latent_attention_kernel<NG, NC>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  dim3 grid(ceil_div(max_item_rows * a.H, MQ), n_items, a.n_splits);
-  const int cls = launch_class_for_rows(rows_total, 0);
-  int rc = launch_k_class(cls, kern, grid, dim3(NG * NC * 32), smem, stream, 1, a);
-  if (rc || a.n_splits == 1) return rc;
-  return launch_k_class(cls, latent_merge_kernel, dim3(rows_total * a.H), dim3(RK / 2 < 32 ? 32 : RK / 2), 0, stream, 1, (const float*)a.scratch, a.out,
-                        a.sinks, a.H, a.n_splits);
+  dim3 grid(ceil_div(max_item_rows * a.H, MQ), n_items, 1);
+  return launch_k_class(launch_class_for_rows(rows_total, 0), kern, grid, dim3(NG * NC * 32), smem, stream, 1, a);
+}
+
+static int launch_tokens(const LatArgs& a, int n_items, int max_item_rows, int rows_total, cudaStream_t stream) {
+  if (a.page_tokens % 16) return FELLM_ERR_SIZE;
+  cudaError_t e = cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT_SMEM);
+  if (e != cudaSuccess) return (int)e;
+  dim3 grid(a.n_splits, n_items, ceil_div(max_item_rows * a.H, LT_ROWS));
+  int rc = launch_k_class(1, latent_tokens_kernel, grid, dim3(LT_WARPS * 32), LT_SMEM, stream, a.cluster ? a.n_splits : 1, a);
+  if (rc || a.n_splits == 1 || a.cluster) return rc;
+  return launch_k_class(launch_class_for_rows(rows_total, 0), latent_merge_kernel, dim3(rows_total * a.H), dim3(RK / 2 < 32 ? 32 : RK / 2), 0, stream, 1,
+                        (const float*)a.scratch, a.out, a.sinks, a.H, a.n_splits);
+}
+
+// How many clusters of `size` CTAs of the single tokens' kernel the device holds at once (asked once per device and size; 0: none).
+FELLM_API int fellm_latent_token_clusters(int size) {
+  static int cached[64][9];
+  int dev = 0;
+  if (size < 1 || size > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (!cached[dev][size]) {
+    int n = 0;
+    if (cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT_SMEM) != cudaSuccess) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size); cfg.blockDim = dim3(LT_WARPS * 32); cfg.dynamicSmemBytes = LT_SMEM;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = size; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, latent_tokens_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    cached[dev][size] = n > 0 ? n + 1 : 1;
+  }
+  return cached[dev][size] - 1;
 }
 
 FELLM_API int fellm_latent_attention_rk() { return RK; }
 FELLM_API int fellm_latent_attention_dr() { return DR; }
 // the key tile of a variant (0: portions, 1: single tokens): pages hold a multiple of it
-FELLM_API int fellm_latent_attention_key_tile(int variant) { return variant != 1 ? 32 : (RK % 64 == 0 ? 64 : 32); }
+FELLM_API int fellm_latent_attention_key_tile(int variant) { return variant != 1 ? 32 : 16; }
 
 // variant 0: 64 rows a CTA (portions of prompts), n_splits must be 1; variant 1: 16 rows a CTA (single tokens),
 // qsrc (or null): the queries' rotated parts are read from there and rotated in the kernel, and q holds the RK
-// elements of a (token, head) row alone.  n_splits >= 1 (up to 32) with scratch of rows * H * n_splits * (RK + 2) floats when above 1.
+// elements of a (token, head) row alone.  n_splits >= 1 shares of the keys: as a cluster (up to 8), or (up to 32) with scratch of rows * H * n_splits * (RK + 2) floats when above 1.
 FELLM_API int fellm_latent_attention_mma(const void* q, const void* pool, const int* block_table, int max_pages,
                                          const int* positions, const int* row_slot, const int* item_start, int n_items,
                                          int max_item_rows, int rows_total, void* out, float* scratch, int n_splits, int H,
                                          int page_tokens, int layer, int layers_in_group, float scale, int window,
                                          const float* sinks, int variant, const void* qsrc, int ldq, int q_head, int q_rot_off,
-                                         const float* freq, int n_rot, float mag, cudaStream_t stream) {
+                                         const float* freq, int n_rot, float mag, int cluster, cudaStream_t stream) {
   if (n_items <= 0 || rows_total <= 0 || max_item_rows <= 0) return 0;
   if (!q || !pool || !block_table || !positions || !row_slot || !item_start || !out) return FELLM_ERR_ARG;
-  if (H < 1 || page_tokens < 1 || n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && (!scratch || variant != 1))) return FELLM_ERR_ARG;
+  if (H < 1 || page_tokens < 1 || n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && variant != 1) || (cluster && n_splits > 8) ||
+      (n_splits > 1 && !cluster && !scratch)) return FELLM_ERR_ARG;
   if (qsrc && ((ldq | q_head | q_rot_off) % 8 || ((size_t)qsrc & 15) || n_rot < 0 || n_rot > DR || (n_rot & 1) || (n_rot && !freq))) return FELLM_ERR_SIZE;
   LatArgs a;
   a.qsrc = DR ? (const bf16*)qsrc : nullptr; a.ldq = ldq; a.q_head = q_head; a.q_rot_off = q_rot_off; a.n_rot = n_rot; a.freq = freq; a.mag = mag;
   a.q = (const bf16*)q; a.pool = (const bf16*)pool; a.block_table = block_table; a.max_pages = max_pages;
   a.positions = positions; a.row_slot = row_slot; a.item_start = item_start; a.out = (bf16*)out; a.scratch = scratch;
   a.sinks = sinks; a.H = H; a.page_tokens = page_tokens; a.layer = layer; a.layers_in_group = layers_in_group;
-  a.window = window > 0 ? window : 0; a.n_splits = n_splits; a.scale_log2 = scale * LOG2E;
+  a.window = window > 0 ? window : 0; a.n_splits = n_splits; a.cluster = cluster && n_splits > 1; a.single = max_item_rows == 1 && n_items == rows_total; a.scale_log2 = scale * LOG2E;
   if (variant == 0) return launch_latent<4, 2>(a, n_items, max_item_rows, rows_total, stream);
-  if constexpr (RK % 64 == 0) return launch_latent<1, 4>(a, n_items, max_item_rows, rows_total, stream);
-  else return launch_latent<1, 2>(a, n_items, max_item_rows, rows_total, stream);
+  return launch_tokens(a, n_items, max_item_rows, rows_total, stream);
 }

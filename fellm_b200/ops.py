@@ -1404,6 +1404,10 @@ def latent_rotate_q(q, H, dn, dr, q_abs, rk, freq, n_rot, mag, positions):
 LATENT_ATTENTION_MMA = os.environ.get("FELLM_B200_LATENT_ATTENTION_MMA", "1") != "0"
 LATENT_SINGLE_ROWS = 32        # up to this many (token, head) rows an item: the kernel's form for single tokens
 LATENT_MAX_SPLITS = 16
+# So many shares of a token's keys or fewer are one cluster (of up to 8) and put together in it, more go through memory and a merge behind.
+# us a layer of 8 heads, merge / cluster: 8 tokens over 1,024 keys 38 / 32, 1 token over 100 30 / 22, 24 tokens 45 / 40, 48 (shares of three) 63 / 63;
+# clusters of 8 where only 15 are resident: 16 tokens 43 / 47.
+LATENT_CLUSTER_TO = int(os.environ.get("FELLM_B200_LATENT_CLUSTER_TO", 10))
 
 
 # Most bytes of scratch that a form of a layer may take which trades scratch for speed (keys and values per head out of latents,
@@ -1513,7 +1517,7 @@ def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, i
     if out is None:
         out = torch.empty((T, H * rk), dtype=torch.bfloat16, device=q_abs.device)
     variant = 1 if max_item_rows * H <= LATENT_SINGLE_ROWS else 0
-    n_splits, scratch = 1, None
+    n_splits, scratch, cluster = 1, None, 0
     if variant == 1:
         # few CTAs walk many keys: split the walk so that the SMs have work (a constant of the step's shape)
         kt = 64 if rk % 64 == 0 else 32
@@ -1522,15 +1526,20 @@ def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, i
         tiles = span // kt + 2
         ctas = n_items * (-(-max_item_rows * H // 16))
         n_splits = max(1, min(tiles // 2, 148 // max(ctas, 1), LATENT_MAX_SPLITS))
-        if n_splits > 1:
+        if 1 < n_splits <= LATENT_CLUSTER_TO:
+            # as one cluster, of a size that the device holds for all tokens at once (a second round costs more than fewer shares)
+            fits = _fn("latent_attention_mma", "fellm_latent_token_clusters", [_c_int], defines={"LAT_RK": rk, "LAT_DR": dr})
+            cluster = next((s for s in range(min(n_splits, 8), 1, -1) if fits(s) >= ctas), 0)
+        n_splits = cluster or n_splits
+        if n_splits > 1 and not cluster:
             scratch = torch.empty((T * H * n_splits * (rk + 2),), dtype=torch.float32, device=q_abs.device)
     f = _fn("latent_attention_mma", "fellm_latent_attention_mma",
             [_c_p, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
-             _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_f, _c_p], defines={"LAT_RK": rk, "LAT_DR": dr})
+             _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_f, _c_int, _c_p], defines={"LAT_RK": rk, "LAT_DR": dr})
     _check(f(_p(q_abs), _p(pool), _p(block_table), block_table.shape[1], _p(positions), _p(row_slot), _p(item_start),
              int(n_items), int(max_item_rows), T, _p(out), _p(scratch), n_splits, H, page_tokens, layer, pool.shape[1],
              float(scale), int(window or 0), _p(sinks), variant, _p(qsrc), ldq, int(q_head), int(q_off), _p(freq), int(n_rot), float(mag),
-             _stream()), "latent_attention")
+             int(cluster), _stream()), "latent_attention")
     return out
 
 

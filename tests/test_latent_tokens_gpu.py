@@ -1,0 +1,45 @@
+"""Latent attention of single tokens: a token's keys shared out in portions of 16 over the blocks of a cluster, or over blocks that leave
+their sums in memory, against float64, at the edges of portions, tiles, windows and shares."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rk,dr,H", [(512, 64, 8), (512, 64, 16), (64, 16, 4), (64, 16, 24)])
+@pytest.mark.parametrize("window,contexts", [(None, (1, 16, 17, 64, 65, 300)), (100, (1, 99, 101, 513)), (1024, (1500, 1039, 64)), (64, (63, 64, 128, 1000)),
+                                             (None, (3100,))])
+@pytest.mark.parametrize("share", [0, 10, 100])
+def test_a_token_over_its_keys(monkeypatch, rk, dr, H, window, contexts, share):
+    from fellm_b200 import ops
+    monkeypatch.setattr(ops, "LATENT_CLUSTER_TO", share)             # 0: always through memory, 100: always a cluster
+    D, PT, n = rk + dr, 64, len(contexts)
+    g = torch.Generator().manual_seed(rk + H + n)
+    pages = [-(-c // PT) for c in contexts]
+    pool = torch.randn(sum(pages) + 1, 1, PT, D, generator=g).bfloat16()
+    table = torch.full((n, max(pages) + 1), -1, dtype=torch.int32)
+    for i, (p, c) in enumerate(zip(pages, contexts)):
+        table[i, :p] = torch.randperm(p, generator=g) + 1 + sum(pages[:i])
+        pool[table[i, p - 1], 0, (c - 1) % PT + 1:] = float("nan")   # behind the last key: a freed page's bits
+        if window is not None:
+            table[i, :max(0, c - window) // PT] = -1                 # pages wholly behind the window are given back
+    q = (torch.randn(n, H, D, generator=g) * 0.5).bfloat16()
+    sinks = torch.randn(H, generator=g)
+    scale = D ** -0.5
+    pos = torch.tensor([c - 1 for c in contexts], dtype=torch.int32)
+    got = ops.latent_attention(q.reshape(n, H * D).cuda(), H, rk, dr, pool.cuda(), table.cuda(), pos.cuda(), torch.arange(n, dtype=torch.int32).cuda(),
+                               torch.arange(n + 1, dtype=torch.int32).cuda(), n, 1, max(contexts), 0, PT, scale, window=window, sinks=sinks.cuda())
+    got = got.double().cpu().view(n, H, rk)
+    for i, c in enumerate(contexts):
+        first = 0 if window is None else max(0, c - window)
+        at = torch.arange(first, c)
+        rows = pool[table[i, at // PT].long(), 0, at % PT].double()
+        s = q[i].double() @ rows.T * scale
+        m = torch.maximum(s.max(-1).values, sinks.double())
+        p = torch.exp(s - m[:, None])
+        want = p @ rows[:, :rk] / (p.sum(-1) + torch.exp(sinks.double() - m))[:, None]
+        # probabilities rounded to bfloat16 (2^-9 each) of values of size ~1, then the result
+        room = 2.0 ** -8 * (p @ rows[:, :rk].abs() / p.sum(-1, keepdim=True)) + 2.0 ** -8 * want.abs() + 1e-4
+        assert ((got[i] - want).abs() <= room).all(), (c, float(((got[i] - want).abs() / room).max()))
