@@ -39,7 +39,7 @@ __device__ __forceinline__ void ar_unpack(const uint4& raw, float* f) {
 }
 
 template <int HD, int R, bool VK>
-__global__ void __launch_bounds__(AR_WARPS * 32)
+__global__ void __launch_bounds__(AR_WARPS * 32, HD != 64 || VK ? 1 : R == 2 ? 4 : R == 4 ? 3 : 1)       // (blocks an SM: see ar_launch)
 attention_rows_kernel(const ArArgs a) {
   constexpr int LPK = HD / 8, KPI = 32 / LPK, NI = 32 / KPI;        // lanes a key, keys a load, loads a tile (= LPK)
   typedef float Sums[AR_WARPS][R][HD + 4];                           // a part's: per warp and head the elements, then m, l
@@ -49,6 +49,8 @@ attention_rows_kernel(const ArArgs a) {
   cg::cluster_group cluster = cg::this_cluster();
   const int cs = gridDim.x, rank = blockIdx.x, g = blockIdx.y, row = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LPK, sub = lane % LPK;
+  // Launched as a programmatic dependent of the kernel that makes q (and this token's key and value): who is where is read ahead of
+  // the wait, a warp's first page number with it (copies from the host write them, no kernel of a step).
   const int pos = a.positions[row];
   const int* bt = a.block_table + (size_t)a.row_slot[row] * a.max_pages;
   int k_begin = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
@@ -57,6 +59,11 @@ attention_rows_kernel(const ArArgs a) {
   const size_t record = (size_t)a.G * pt * (VK ? HD : 2 * HD);
   const bf16* qrow = a.q + (size_t)row * a.ldq;
   const bool fused = a.new_k_off >= 0;
+
+  const int n_parts = a.parts / cs, e0 = 8 * sub + (HD == 64 ? 4 * (grp & 1) + 2 * (grp >> 1) : 4 * grp);
+  const int first = k_begin + 32 * (rank * n_parts * AR_WARPS + warp);
+  int page = first <= pos ? bt[min(first + lane, pos) >> a.page_shift] : 0;
+  pdl_wait();
 
   float q[R][8];
   const float qt = a.qt_every > 0 ? 1.0f + a.qt_coef * logf((float)((pos + 1) / a.qt_every + 1)) : 1.0f;
@@ -69,7 +76,6 @@ attention_rows_kernel(const ArArgs a) {
     slope[r] = a.slopes ? a.slopes[g * R + r] : 0.f;
   }
 
-  const int n_parts = a.parts / cs, e0 = 8 * sub + (HD == 64 ? 4 * (grp & 1) + 2 * (grp >> 1) : 4 * grp);
   for (int i = 0; i < n_parts; ++i) {
     const int p = rank * n_parts + i;
     float m[R], l[R];
@@ -82,8 +88,8 @@ attention_rows_kernel(const ArArgs a) {
     }
 
     for (int k0 = k_begin + 32 * (p * AR_WARPS + warp); k0 <= pos; k0 += 32 * AR_WARPS * a.parts) {
-      const int mine = min(k0 + lane, pos);
-      const int page = max(bt[mine >> a.page_shift], 0);               // an unmapped entry (-1) must never become an address
+      if (k0 != first) page = bt[min(k0 + lane, pos) >> a.page_shift];
+      page = max(page, 0);                                          // an unmapped entry (-1) must never become an address
       uint4 kr[NI], vr[VK ? 1 : NI];
 #pragma unroll
       for (int i = 0; i < NI; ++i) {
@@ -177,6 +183,7 @@ attention_rows_kernel(const ArArgs a) {
     }
   }
 
+  pdl_launch_dependents();                         // (the next product's weights beside the merge, not beside the keys)
   // the step's own key and value into their page: nobody in this launch reads them from there
   if (fused && rank == 0 && warp == 0) {
     const int page = bt[pos >> a.page_shift];
@@ -241,6 +248,29 @@ attention_rows_kernel(const ArArgs a) {
   if (cs > 1) cluster.sync();                                        // nobody leaves while its sums are being read
 }
 
+// How many clusters of cs blocks the device holds at once (asked once per device and size of the cluster, the shared memory of a block
+// following it; 0: not known).
+template <int HD, int R, bool VK>
+static int ar_resident_clusters(int cs, size_t smem) {
+  static int cached[64][AR_PARTS + 1][AR_PARTS + 1];
+  const int per = (int)(smem / (AR_WARPS * R * (HD + 4) * sizeof(float)));          // parts a block, 1..8
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || per > AR_PARTS) return 0;
+  int& n = cached[dev][cs][per];
+  if (!n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs); cfg.blockDim = dim3(AR_WARPS * 32); cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int got = 0;
+    if (cudaOccupancyMaxActiveClusters(&got, attention_rows_kernel<HD, R, VK>, &cfg) != cudaSuccess) { cudaGetLastError(); got = 0; }
+    n = got + 1;
+  }
+  return n - 1;
+}
+
 template <int HD, int R, bool VK>
 static int ar_launch(const ArArgs& a, int T, int cs, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
@@ -250,13 +280,15 @@ static int ar_launch(const ArArgs& a, int T, int cs, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<HD, R, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
     if (e != cudaSuccess) return (int)e;
   }
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, attention_rows_kernel<HD, R, VK>, a);
-  if (e != cudaSuccess) return (int)e;
-  return launch_status();
+  // A programmatic dependent (four layers with their products, us before / so: two heads a kv head, 1 token 68.8 / 56.6, 24 tokens 148.6 /
+  // 128.0; four heads, 1 token 73.6 / 63.3, 12 tokens 94.1 / 91.0), except where its clusters just fill a device that holds two blocks an SM: beside the
+  // blocks of the kernel in front not all of them find room, and a second round costs more (values that are keys, 4 tokens, 32 heads, 8
+  // kv heads, clusters of 8: 70 / 81 us for four layers).  Blocks an SM matter as much: 12 tokens of four heads a kv head (384 blocks)
+  // 86 us with three, 108 with two and more registers; of two heads, 8 tokens, 275 with four and 290 with three.
+  const long long clusters = (long long)a.G * T;
+  const int fit = ar_resident_clusters<HD, R, VK>(cs, cfg.dynamicSmemBytes);
+  const bool full = fit * cs <= 2 * fellm_sm_count() && clusters <= fit && 10 * clusters > 9ll * fit;
+  return launch_k_class(full ? 0 : 1, attention_rows_kernel<HD, R, VK>, cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes, stream, cs, a);
 }
 
 // Rows of q [T, ldq] (heads at column 0, H x hd bfloat16), each at its own position of its own slot; the other arguments as
