@@ -234,7 +234,10 @@ __device__ __forceinline__ void store_tile(const UmmaArgs& a, Take take, int m_w
 // Persistent: a CTA walks over output tiles t = blockIdx.x, + gridDim.x, ... (tiles that follow one another share
 // their weight tile).  Two accumulators in tensor memory: while the epilogue warps read tile i out of one, the MMA
 // thread fills the other with tile i+1, and the TMA thread is already fetching operands further ahead.
-template <int EPI, int BN, bool GROUPED = false>
+// HALVES: a tile's two halves of K have an accumulator each, which the epilogue adds (the first half's plus the second's, rounded): an MMA
+// that adds into its accumulator truncates, so two chains of half the length are nearer to the sum, and they are the bits of the kernel
+// below, which gives each half a CTA.
+template <int EPI, int BN, bool GROUPED = false, bool HALVES = false>
 __global__ void __launch_bounds__(UM_THREADS)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, UmmaArgs a) {
   FELLM_TRACE_SCOPE(TRACE_GEMM_UMMA);
@@ -249,6 +252,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const unsigned full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[STAGES]);
   const unsigned accfull0 = smem_u32(&bars[2 * STAGES]), accempty0 = smem_u32(&bars[2 * STAGES + 2]);
   const int k_blocks = (a.K + UM_BK - 1) / UM_BK;
+  const int k_mid = HALVES ? k_blocks / 2 : k_blocks;       // the second accumulator's first k-block
   const int n_tiles = (a.N + BN - 1) / BN;
   int m_tiles = (a.M + UM_BM - 1) / UM_BM;
 
@@ -297,12 +301,12 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   } else if (warp == 1) {
     if (lane == 0) {
       const unsigned idesc = umma_idesc(UM_BM, BN);
-      unsigned it = 0, use = 0;      // use: tiles done so far; accumulator = use & 1
+      unsigned it = 0, use = 0;      // use: tiles done so far; accumulator = use & 1 (HALVES: both, one tile at a time)
       bool ok = true;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++use) {
-        const unsigned acc = use & 1, d_tmem = tmem_base + acc * BN;
-        if (use >= 2) {              // the epilogue must have drained this accumulator's previous tile
-          ok = mbar_wait(accempty0 + 8 * acc, ((use >> 1) - 1) & 1, a.status, 104);
+        const unsigned acc = HALVES ? 0 : use & 1, turn = HALVES ? use : use >> 1;
+        if (turn >= 1) {             // the epilogue must have drained this accumulator's previous tile
+          ok = mbar_wait(accempty0 + 8 * acc, (turn - 1) & 1, a.status, 104);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         }
@@ -313,9 +317,11 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           unsigned sa = tiles + s * STAGE_BYTES, sb = sa + UM_BM * UM_BK * 2;
           unsigned long long da = umma_desc(sa), db = umma_desc(sb);
+          const unsigned second = HALVES && kb >= k_mid, d_tmem = tmem_base + (HALVES ? second : acc) * BN;
+          const int k_first = second ? k_mid : 0;
 #pragma unroll
           for (int k = 0; k < UM_BK / 16; ++k)          // 32 bytes further along K inside the swizzle atom
-            umma_f16(d_tmem, da + (unsigned long long)(k * 2), db + (unsigned long long)(k * 2), idesc, (kb | k) ? 1u : 0u);
+            umma_f16(d_tmem, da + (unsigned long long)(k * 2), db + (unsigned long long)(k * 2), idesc, (kb > k_first || k) ? 1u : 0u);
           umma_commit(empty0 + 8 * s);                  // the stage is free once these MMAs have read it
         }
         if (ok) umma_commit(accfull0 + 8 * acc);        // arrives when every MMA of this tile is done
@@ -327,7 +333,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     uint4* stage = reinterpret_cast<uint4*>(smem_raw + (tiles - smem_u32(smem_raw)) + STAGES * STAGE_BYTES + (warp - 2) * UM_EPI_STAGE);
     unsigned use = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++use) {
-      const unsigned acc = use & 1;
+      const unsigned acc = HALVES ? 0 : use & 1, turn = HALVES ? use : use >> 1;
       int m0, w0, n0, rows;
       coords(t, m0, w0, n0, rows);
       // += residual: what out holds in this warp's first two chunks is fetched while the MMAs of the
@@ -339,10 +345,18 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         load_residual(a, res[0], m_w, rows_w, n0 + c_lo);
         load_residual(a, res[EPI == EPI_ACC ? 1 : 0], m_w, rows_w, n0 + c_lo + 32);
       }
-      if (!mbar_wait(accfull0 + 8 * acc, (use >> 1) & 1, a.status, 103)) break;
+      if (!mbar_wait(accfull0 + 8 * acc, turn & 1, a.status, 103)) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      store_tile<EPI, CHUNKS, GROUPED>(a, [&](int c0, float* v) { tmem_ld32(tmem_base + ((unsigned)(q * 32) << 16) + acc * BN + (unsigned)c0, v); },
-                              m_w, rows_w, n0, c_lo, res, stage);
+      const unsigned mine = tmem_base + ((unsigned)(q * 32) << 16) + acc * BN;
+      store_tile<EPI, CHUNKS, GROUPED>(a, [&](int c0, float* v) {
+        tmem_ld32(mine + (unsigned)c0, v);
+        if (HALVES) {
+          float o[32];
+          tmem_ld32(mine + BN + (unsigned)c0, o);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += o[j];
+        }
+      }, m_w, rows_w, n0, c_lo, res, stage);
       // this warp has read its part of the accumulator: one of the eight arrivals that free it
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       __syncwarp();
@@ -695,10 +709,10 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int K, int ld,
   return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
 }
 
-template <int EPI, int BN>
+template <int EPI, int BN, bool HALVES = false>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mw, const UmmaArgs& a, cudaStream_t stream) {
   size_t smem = (size_t)(BN == 256 ? 4 : UM_STAGES) * (UM_BM + BN) * UM_BK * 2 + 8 * UM_EPI_STAGE + 1024;
-  auto kern = gemm_umma_kernel<EPI, BN>;
+  auto kern = gemm_umma_kernel<EPI, BN, false, HALVES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int n_sm = fellm_sm_count();
@@ -781,20 +795,23 @@ FELLM_API int fellm_gemm_umma(const void* A, const void* W, const float* bias, v
   if (e) return e;
   UmmaArgs a; a.bias = bias; a.out = out; a.status = status; a.M = M; a.N = N; a.K = K; a.ldo = ldo;
   a.g_table = nullptr; a.g_tiles = nullptr; a.g_wrows = 0;
-  // few tiles and a long K (a few hundred rows, a narrow N): two CTAs a 128 x 128 tile, half of K each.  Handing a part over
-  // costs some 4 us, a k-block of it saves 0.13 (us, whole / split: 600 x 1,024 K 1,024 7.8 / 9.7, K 2,048 12.1 / 12.0, K 3,072 16.4 / 14.2,
-  // K 8,192 38.2 / 27.3; 1,100 x 1,024 K 1,024 8.0 / 10.1, K 2,048 12.5 / 12.3)
+  // few tiles (a few hundred rows, a narrow N): each half of K has a sum of its own.  Long ones, two CTAs a 128 x 128 tile; handing a part
+  // over costs some 4 us, a k-block of it saves 0.13, so up to 31 k-blocks one CTA makes both halves, with the same bits.  us, two CTAs / one
+  // CTA with two sums / one with a single sum over all of K, which is less exact: 600 x 1,024 K 512 8.1 / 5.4 / 5.3, K 1,024 9.3 / 7.5 / 7.5,
+  // K 1,536 10.5 / 9.5 / 9.5, K 1,984 11.5 / 11.6 / 11.4; 1,100 x 1,024 K 1,024 9.7 / 7.6 / 7.7; out += of it 10.2 / 8.3 / 8.1.  Two CTAs / one
+  // with a single sum beyond: K 3,072 14.2 / 16.4, K 8,192 27.3 / 38.2.
   static int ksplit = -1;
   if (ksplit < 0) { const char* ev = getenv("FELLM_B200_UMMA_KSPLIT"); ksplit = (ev && ev[0] == '0') ? 0 : 1; }
-  if (ksplit && 2 * ceil_div(N, 128) * m_tiles <= n_sm && kb >= 32) {
+  if (ksplit && 2 * ceil_div(N, 128) * m_tiles <= n_sm && kb >= 8) {
+    const bool apart = kb >= 32;
     e = make_map(&mw, W, N, K, ldw, 128);
     if (e) return e;
     switch (epi) {
-      case EPI_STORE: return launch_ksplit<EPI_STORE>(ma, mw, a, stream);
-      case EPI_ACC: return launch_ksplit<EPI_ACC>(ma, mw, a, stream);
-      case EPI_SWIGLU: return launch_ksplit<EPI_SWIGLU>(ma, mw, a, stream);
-      case EPI_F32: return launch_ksplit<EPI_F32>(ma, mw, a, stream);
-      case EPI_RELU2: return launch_ksplit<EPI_RELU2>(ma, mw, a, stream);
+      case EPI_STORE: return apart ? launch_ksplit<EPI_STORE>(ma, mw, a, stream) : launch<EPI_STORE, 128, true>(ma, mw, a, stream);
+      case EPI_ACC: return apart ? launch_ksplit<EPI_ACC>(ma, mw, a, stream) : launch<EPI_ACC, 128, true>(ma, mw, a, stream);
+      case EPI_SWIGLU: return apart ? launch_ksplit<EPI_SWIGLU>(ma, mw, a, stream) : launch<EPI_SWIGLU, 128, true>(ma, mw, a, stream);
+      case EPI_F32: return apart ? launch_ksplit<EPI_F32>(ma, mw, a, stream) : launch<EPI_F32, 128, true>(ma, mw, a, stream);
+      case EPI_RELU2: return apart ? launch_ksplit<EPI_RELU2>(ma, mw, a, stream) : launch<EPI_RELU2, 128, true>(ma, mw, a, stream);
       default: return FELLM_ERR_ARG;
     }
   }

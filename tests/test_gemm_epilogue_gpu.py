@@ -63,3 +63,34 @@ def test_gated_columns_that_end_anywhere(M, N, K):
     room = 1.1 * sums * (gate.abs() + up.abs() + 1) + 2.0 ** -7 * want.abs() + 1e-6          # (|silu'| <= 1.1; the exponential's own 2^-21)
     assert ((held[:M, :N // 2].double() - want).abs() <= room).all()
     assert (held[M:] == 3).all() and (held[:, N // 2:] == 3).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [512, 584, 1024, 1976, 2048])
+@pytest.mark.parametrize("M,N", [(129, 1000), (600, 1024), (1100, 1024), (300, 96)])
+@pytest.mark.parametrize("epi", ["f32", "acc", "store"])
+def test_few_tiles_add_two_halves_of_k(M, N, K, epi):
+    """Products of few tiles: two sums over half of K each, added with rounding, whether one CTA or two make them (an MMA that adds into
+    its accumulator truncates: one sum over all of K is less exact).  The halves' own sums: the same rows in a product of so many tiles that
+    none is halved."""
+    from fellm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    dt = torch.bfloat16 if epi == "store" else torch.float32
+    out = torch.randn(M, N, generator=g, device=DEV).to(dt)
+    held = out.clone()
+    ops.gemm_bf16(x, w, out=out, accumulate=epi == "acc")
+    cut = 64 * (-(-K // 64) // 2)
+    many = -(-148 * 128 // M) + 1
+    parts = [ops.gemm_bf16(x[:, at].repeat(many, 1), w[:, at].contiguous(), out_dtype=torch.float32)[:M] for at in (slice(0, cut), slice(cut, K))]
+    ops.check_umma_status(DEV)
+    want = parts[0] + parts[1]
+    if epi == "acc":
+        want = want + held
+    assert torch.equal(out, want.to(dt))
+    x, w = x.double(), w.double()
+    exact = x @ w.T + (held.double() if epi == "acc" else 0.0)
+    whole = ops.gemm_bf16(x.bfloat16().repeat(many, 1), w.bfloat16(), out_dtype=torch.float32)[:M].double()
+    if epi == "f32":
+        assert float((out.double() - exact).norm()) < float((whole - exact).norm())
