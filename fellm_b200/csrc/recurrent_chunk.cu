@@ -17,14 +17,14 @@
 // substitution for (P A) and V, the scaled B and K.  Then, in one `walk` (a block a head and 16 value columns), states and outputs
 // chunk after chunk; or, for long portions, what hangs together in a chain first and the outputs of all chunks side by
 // side behind it (`out`): with the delta rule the `chain` W S, K^T U (the state in front of every chunk goes to memory), without
-// it prep sums a chunk's K^T V and `states` is S' = P S + that, element by element.
+// it the `states` S' = P S + K^T V, element by element.  Each sum in the walk's order: a portion's bits do not depend on which of the two runs.
 // Bound by: the reads of shared memory.  A load of 16 bytes a lane takes four wavefronts, or two where lanes one or two apart ask for the
 // same (of 8 bytes: two or one), whatever else they share; so a tile's row and column groups lie in alternate bits of the
 // lane's number (walk 188 -> 158 us, prep 85 -> 74 of the first size below, with the same bits).  A lane's tile of 4 x 4 (or 2 x 4) results then takes a wavefront for
 // about every FMA instruction of a warp.  16 columns a block: a prompt of 16 heads of 128 is 128 blocks for 148 SMs.
 // 2,048 tokens of 16 heads of 128 x 128, delta rule: scan 791 us, prep 85 + walk 188 as it was, here prep 74 + chain 105 + out 44 (one walk:
-// 158), graph of the three 269 -> 215; decay per channel 284 -> 226; three prompts of 1,537 tokens, 8 heads, gated write: scan 274, 100 -> 61;
-// 1,100 tokens in two prompts, 16 heads of 64, decay and bonus 71 -> 45.
+// 158), graph of the three 269 -> 215; decay per channel 284 -> 226; three prompts of 1,537 tokens, 8 heads, gated write: scan 274, 100 -> 64;
+// 1,100 tokens in two prompts, 16 heads of 64, decay and bonus 69 -> 44.
 // 32 tokens a chunk: L and M cost 32 / 2 multiply-adds a token, channel and matrix, an eighth of the walk's.
 //
 // A later token's infinity or NaN stays out of an earlier token's sums, as in the walk token by token: masked pairs are
@@ -36,7 +36,7 @@
 // products of the decays are sums of two floats.  Relative error against float64, scan / here, mean over five sizes and
 // three seeds: delta rule outputs 1.34e-7 / 1.22e-7, states 9.0e-8 / 8.6e-8, with keys nearly alike and beta 0.99 1.45e-7 /
 // 1.35e-7, 8.7e-8 / 8.4e-8; decay per channel 1.22e-7 / 1.08e-7, 7.8e-8 / 7.3e-8; decay and bonus 8.3e-8 / 6.8e-8, 3.15e-8 /
-// 3.10e-8; gated write 6.2e-8 / 5.9e-8, 1.09e-7 / 1.07e-7.  It costs 6 us of the 263 of the first size above (21 of 264 with a
+// 3.09e-8; gated write 6.2e-8 / 5.9e-8, 1.09e-7 / 1.07e-7.  It costs 6 us of the 263 of the first size above (21 of 264 with a
 // decay per channel, 4 of 68 with a bonus; the gated write gains 5 of 106 through its smaller blocks).
 // Sums run in another order than the scan's, so the engine uses this form for portions of the bfloat16 engine; the 32-bit
 // engine keeps the scan and with it the same bits for a prompt under every cut.
@@ -48,7 +48,6 @@
 #define RK_LP 36           // row stride of a chunk's 32 x 32 matrices in the image
 #define RK_LM 34           // and, in 64 bits, in prep's shared memory
 #define RK_THREADS 256
-#define RK_LAST 3          // tokens at a chunk's end whose terms are added to the state one by one
 
 enum RkMode { RK_DELTA_HEAD = 0, RK_DELTA_CHANNEL = 1, RK_DECAY_BONUS = 2, RK_GATED_WRITE = 3 };
 
@@ -120,59 +119,14 @@ struct RkProduct {
   }
 };
 
-// What prep leaves of a chunk and head, in the order its readers take it (their copies are then linear): walk reads W, K and
-// P, the outputs Q and M, the states of the recurrences without the delta rule P and, in K's
-// place, K of the last RK_LAST tokens.
+// What prep leaves of a chunk and head, in the order its readers take it (their copies are then linear): the chain reads W, K and
+// P, the states of the recurrences without the delta rule K and P, the outputs Q and M.
 template <bool DELTA, int DK>
 struct RkImage {
   static constexpr int AP = DK + 4;                           // row stride of W and Q: eight rows' 16 bytes in different banks
   static constexpr int W = 0, K = W + (DELTA ? RK_C * AP : 0), P = K + RK_C * DK, WALK = P + DK;
   static constexpr int Q = WALK, M = Q + RK_C * AP, FLOATS = M + RK_C * RK_LP, OUT = FLOATS - Q;
 };
-
-// What a chunk's tokens but the last RK_LAST add to the state where u_t = v_t: K^T V, [dv][DK] at the cell's place in a.S, DK columns of V at a time (in V,
-// [32][DK]; the first of them are there).  A thread eight key rows and four value columns at a time, in the tokens' order.
-template <int DK, typename TA>
-__device__ __forceinline__ void rk_own_state(const RkArgs& a, size_t cell, float* V, const float* KK, const TA* vp, int row0, int len, int tid) {
-  float* S = a.S + cell * ((size_t)a.dv * DK);
-  for (int j0 = 0; j0 < a.dv; j0 += DK) {
-    if (j0) {
-      __syncthreads();
-      for (int x = tid; x < RK_C * DK; x += RK_THREADS) {
-        const int t = x / DK, j = j0 + x % DK;
-        V[x] = t < len && j < a.dv ? to_f(vp[(size_t)(row0 + t) * a.ld + j]) : 0.f;
-      }
-    }
-    __syncthreads();
-    for (int x = tid; x < (DK / 8) * (DK / 4); x += RK_THREADS) {
-      const int y = x >> 1, i = 8 * (y % (DK / 8)), j = 4 * ((x & 1) + 2 * (y / (DK / 8)));      // (neighbouring lanes read the same of K)
-      if (j0 + j >= a.dv) continue;
-      unsigned long long acc[4][4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[c][r] = 0ull;
-#pragma unroll 4
-      for (int t = 0; t < len - RK_LAST; ++t) {
-        const ulonglong2 k0 = *(const ulonglong2*)(KK + t * DK + i), k1 = *(const ulonglong2*)(KK + t * DK + i + 4);
-        const float4 v = *(const float4*)(V + t * DK + j);
-        const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const unsigned long long d = pack_f2(vv[c], vv[c]);
-          acc[c][0] = fma_f2(k0.x, d, acc[c][0]); acc[c][1] = fma_f2(k0.y, d, acc[c][1]);
-          acc[c][2] = fma_f2(k1.x, d, acc[c][2]); acc[c][3] = fma_f2(k1.y, d, acc[c][3]);
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float* o = S + (size_t)(j0 + j + c) * DK + i;
-        *(ulonglong2*)o = make_ulonglong2(acc[c][0], acc[c][1]);
-        *(ulonglong2*)(o + 4) = make_ulonglong2(acc[c][2], acc[c][3]);
-      }
-    }
-  }
-}
 
 // ---------------------------------------------------------------- prep
 template <int MODE, int DK, typename TA>
@@ -368,8 +322,7 @@ rk_prep_kernel(const RkArgs a) {
   for (int x = tid * 4; x < RK_C * DK; x += RK_THREADS * 4) {
     const int t = x / DK, i = x - t * DK;
     *(float4*)(img + I::Q + t * I::AP + i) = *(const float4*)(B + x);
-    if (DELTA || !a.S) *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
-    else if (t < len && t >= len - RK_LAST) *(float4*)(img + I::K + (t - len + RK_LAST) * DK + i) = *(const float4*)(KK + x);
+    *(float4*)(img + I::K + x) = *(const float4*)(KK + x);
   }
   for (int x = tid; x < RK_C * RK_C; x += RK_THREADS) {
     const int t = x / RK_C, s = x % RK_C;
@@ -436,13 +389,8 @@ rk_prep_kernel(const RkArgs a) {
       for (int t = 0; t < RK_C; ++t) x[t] = t < len ? to_f(vp[(size_t)(row0 + t) * a.ld + j]) : 0.f;
 #pragma unroll
       for (int t = 0; t < RK_C; ++t) put(t, x[t]);
-      if (a.S && j < DK) {                         // (A is free without the delta rule: it holds the values' first DK columns)
-#pragma unroll
-        for (int t = 0; t < RK_C; ++t) A[t * DK + j] = x[t];
-      }
     }
   }
-  if (!DELTA && a.S) rk_own_state<DK, TA>(a, cell, A, KK, vp, row0, len, tid);
 }
 
 // ---------------------------------------------------------------- walk
@@ -643,13 +591,12 @@ rk_walk_kernel(const RkArgs a) {
   auto put_state = [&](int c) {
     float* Sw = St + (c & 1) * (RK_NV * DK) + warp * (RK_NV * KW);
 #pragma unroll
-    for (int x = 0; x < 4; ++x)
-{
-        const int i = RPL * rg, col = 4 * cg + x;
-        float* at = Sw + col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3);
-        if (RPL == 2) *(float2*)at = make_float2(s[0][x], s[RPL - 1][x]);
-        else *at = s[0][x];
-      }
+    for (int x = 0; x < 4; ++x) {
+      const int i = RPL * rg, col = 4 * cg + x;
+      float* at = Sw + col * KW + 4 * ((i >> 2) ^ (cg & GM)) + (i & 3);
+      if (RPL == 2) *(float2*)at = make_float2(s[0][x], s[RPL - 1][x]);
+      else *at = s[0][x];
+    }
   };
   if (walker) {
 #pragma unroll
@@ -724,55 +671,79 @@ rk_walk_kernel(const RkArgs a) {
   }
 }
 
-// Without the delta rule the states are S' = P S + (what the chunk adds), element by element: a thread four key rows of a column,
-// what it reads of RK_AHEAD chunks on its way at once.  The state in front of a chunk takes the place of what prep summed.  The
-// terms of a chunk's last tokens, which later decays have left large, are added here and last, as in the walk token by token: summed
-// with the others in prep, a state's error rose from 3.1e-8 to 3.4e-8 (decay and bonus).
+// Without the delta rule the states are S' = P S + K^T V, element by element: the walk's multiply-adds in the walk's order and so with its
+// bits, without the outputs.  A block of two warps a head, RK_SR key rows and 16 value columns, a thread four key rows of two columns, so
+// that a portion of 8 heads of 128 gives every SM quarter a warp; RK_AHEAD chunks' operands on their way under the sums.  (Blocks of all
+// key rows, four columns a thread, reach 64 SMs there: prep, states and outputs of 2,048 tokens 134 us for 90.  K^T V summed in prep, chunks
+// side by side, takes 85, but rounds in another order and makes a state's error larger, 3.09e-8 -> 3.4e-8 with decay and bonus.)
 #define RK_AHEAD 4
+#define RK_SR 32           // key rows a block
+#define RK_STATES_THREADS 64
 template <int DK>
-__global__ void __launch_bounds__(RK_THREADS)
+__global__ void __launch_bounds__(RK_STATES_THREADS)
 rk_states_kernel(const RkArgs a) {
   using I = RkImage<false, DK>;
-  const int item = blockIdx.z, h = blockIdx.y, x = 4 * (blockIdx.x * RK_THREADS + threadIdx.x), i = x % DK, j = x / DK;
+  constexpr int P = RK_C * RK_SR, V = P + RK_SR, STAGE = V + RK_C * RK_NV;
+  __shared__ __align__(16) float sm[(RK_AHEAD + 1) * STAGE];           // [32][RK_SR] of K, P, [32][16] of V
+  const int item = blockIdx.z, h = blockIdx.y, tile = blockIdx.x / (DK / RK_SR), i0 = RK_SR * (blockIdx.x % (DK / RK_SR));
   const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0;
-  if (n < a.min_rows || n <= 0 || x >= a.dv * DK) return;
+  if (n < a.min_rows || n <= 0) return;
   const int chunks = (n + RK_C - 1) / RK_C;
+  const int tid = threadIdx.x, lane = tid & 31;
+  // a thread's key rows i .. i + 3, columns j and j + 1 (each shared by lanes one or two apart)
+  const int i = 4 * ((lane & 1) + 2 * (lane >> 3)), j = 8 * (tid >> 5) + 2 * ((lane >> 1) & 3);
   const size_t cell0 = (size_t)rk_first_chunk(r0, item) * a.H + h;
-  float4* slot = (float4*)(a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv + x);
-  float* S = a.S + cell0 * ((size_t)a.dv * DK) + x;
-  const float* img = a.image + cell0 * I::FLOATS + i;
-  const float* U = a.U + cell0 * ((size_t)RK_C * a.dv) + (size_t)(j / RK_NV) * (RK_C * RK_NV) + j % RK_NV;
-  const size_t s_step = (size_t)a.H * a.dv * DK, i_step = (size_t)a.H * I::FLOATS, u_step = (size_t)a.H * RK_C * a.dv;
-  float4 s = *slot;
-  for (int c = 0; c < chunks; c += RK_AHEAD) {
-    float4 add[RK_AHEAD], p[RK_AHEAD], k[RK_AHEAD][RK_LAST];
-    float u[RK_AHEAD][RK_LAST];
+  auto fetch = [&](int c, int at) {
+    if (c < chunks) {
+      const size_t cell = cell0 + (size_t)c * a.H;
+      float* to = sm + at * STAGE;
+      const float* img = a.image + cell * I::FLOATS + i0;
 #pragma unroll
-    for (int e = 0; e < RK_AHEAD; ++e)
-      if (c + e < chunks) {
-        add[e] = *(const float4*)(S + (c + e) * s_step);
-        p[e] = *(const float4*)(img + (c + e) * i_step + I::P);
-        const int len = min(RK_C, n - (c + e) * RK_C);
+      for (int x = tid; x < P / 4; x += RK_STATES_THREADS) rk_copy16(to + 4 * x, img + I::K + (x / (RK_SR / 4)) * DK + 4 * (x % (RK_SR / 4)));
+      if (tid < RK_SR / 4) rk_copy16(to + P + 4 * tid, img + I::P + 4 * tid);
+      const float* Vg = a.U + cell * ((size_t)RK_C * a.dv) + (size_t)tile * (RK_C * RK_NV);
 #pragma unroll
-        for (int l = 0; l < RK_LAST; ++l) {
-          k[e][l] = make_float4(0.f, 0.f, 0.f, 0.f); u[e][l] = 0.f;
-          if (len - RK_LAST + l >= 0) {
-            k[e][l] = *(const float4*)(img + (c + e) * i_step + I::K + l * DK);
-            u[e][l] = U[(c + e) * u_step + (len - RK_LAST + l) * RK_NV];
-          }
-        }
-      }
+      for (int x = tid; x < RK_C * RK_NV / 4; x += RK_STATES_THREADS) rk_copy16(to + V + 4 * x, Vg + 4 * x);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
 #pragma unroll
-    for (int e = 0; e < RK_AHEAD; ++e)
-      if (c + e < chunks) {
-        *(float4*)(S + (c + e) * s_step) = s;
-        s = make_float4(fmaf(p[e].x, s.x, add[e].x), fmaf(p[e].y, s.y, add[e].y), fmaf(p[e].z, s.z, add[e].z), fmaf(p[e].w, s.w, add[e].w));
+  for (int c = 0; c < RK_AHEAD; ++c) fetch(c, c);
+
+  const size_t at0 = (size_t)(tile * RK_NV + j) * DK + i0 + i;
+  float* slot = a.state + (size_t)a.item_slot[item] * a.slot_stride + (size_t)h * DK * a.dv + at0;
+  float* Sg = a.S + cell0 * ((size_t)a.dv * DK) + at0;
+  const size_t s_step = (size_t)a.H * a.dv * DK;
+  float s[2][4];
 #pragma unroll
-        for (int l = 0; l < RK_LAST; ++l)
-          s = make_float4(fmaf(k[e][l].x, u[e][l], s.x), fmaf(k[e][l].y, u[e][l], s.y), fmaf(k[e][l].z, u[e][l], s.z), fmaf(k[e][l].w, u[e][l], s.w));
-      }
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[x][r] = slot[x * DK + r];
+  int now = 0, free = RK_AHEAD;
+  for (int c = 0; c < chunks; ++c, Sg += s_step) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x) *(float4*)(Sg + x * DK) = make_float4(s[x][0], s[x][1], s[x][2], s[x][3]);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(RK_AHEAD - 1) : "memory");
+    __syncthreads();          // this chunk's operands are here, everyone is done with the chunk before
+    fetch(c + RK_AHEAD, free);
+    const float* K = sm + now * STAGE;
+    const float4 p = *(const float4*)(K + P + i);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) { s[x][0] *= p.x; s[x][1] *= p.y; s[x][2] *= p.z; s[x][3] *= p.w; }
+#pragma unroll 16
+    for (int t = 0; t < RK_C; ++t) {
+      const float4 k = *(const float4*)(K + t * RK_SR + i);
+      const float2 v = *(const float2*)(K + V + t * RK_NV + j);
+      s[0][0] = fmaf(k.x, v.x, s[0][0]); s[0][1] = fmaf(k.y, v.x, s[0][1]); s[0][2] = fmaf(k.z, v.x, s[0][2]); s[0][3] = fmaf(k.w, v.x, s[0][3]);
+      s[1][0] = fmaf(k.x, v.y, s[1][0]); s[1][1] = fmaf(k.y, v.y, s[1][1]); s[1][2] = fmaf(k.z, v.y, s[1][2]); s[1][3] = fmaf(k.w, v.y, s[1][3]);
+    }
+    free = now;
+    now = now == RK_AHEAD ? 0 : now + 1;
   }
-  *slot = s;
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) slot[x * DK + r] = s[x][r];
 }
 
 // ---------------------------------------------------------------- outputs
@@ -908,7 +879,7 @@ static int rk_launch(const RkArgs& a, cudaStream_t stream) {
     return launch_status();
   }
   if (DELTA) rk_chain_kernel<DK><<<dim3(a.dv / RK_NV, a.H, a.n_items), RK_THREADS, sm_chain, stream>>>(a);
-  else rk_states_kernel<DK><<<dim3((a.dv * DK / 4 + RK_THREADS - 1) / RK_THREADS, a.H, a.n_items), RK_THREADS, 0, stream>>>(a);
+  else rk_states_kernel<DK><<<dim3(a.dv / RK_NV * (DK / RK_SR), a.H, a.n_items), RK_STATES_THREADS, 0, stream>>>(a);
   rk_out_kernel<DELTA, DK><<<dim3(a.cells, a.H, tiles), RK_OUT_THREADS, sm_out, stream>>>(a);
   return launch_status();
 }

@@ -654,10 +654,11 @@ RECURRENT_CHUNK_MIN_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_CHUNK_MIN_RO
 RECURRENT_CHUNK_STEP_ROWS = {64: 120, 128: 90}
 RECURRENT_CHUNK_MIXED_ROWS = 256
 # Portions of this many rows or more: states first, then all outputs side by side; up to it one walk makes both, a launch less.  Without
-# the delta rule the states are then no chain of products any more.  With it (modes 0, 1) the chain keeps its products and only the
-# outputs' leave it, which pays later where the walk's blocks fill the device.  us, one walk / apart: decay and bonus, 16 heads of 64: 192
-# rows 22.5 / 22.6, 256 25.3 / 23.0, 400 among 15 single tokens 69.3 / 63.8; gated write, 8 heads of 128: 192 25.3 / 27.4, 384 36.0 / 30.2, 300
-# among single tokens 85.4 / 88.6, 400 90.9 / 89.9; delta rule of 8 heads 320 43.7 / 43.3, 768 80.8 / 72.1; of 16 heads 320 48.0 / 50.3,
+# the delta rule the states are then split among more blocks than the walk's (element by element).  With it (modes 0, 1) the chain keeps its
+# products and only the outputs' leave it, which pays later where the walk's blocks fill the device.  A portion's bits are the same
+# either way.  us, one walk / apart: decay and bonus, 16 heads of 64: 192 rows 20.8 / 20.3, 320 27.8 / 23.4, 400 among three single tokens
+# 41.4 / 34.1; gated write, 8 heads of 128: 192 26.3 / 24.9, 384 37.2 / 29.2, 16 heads 192 26.8 / 28.8, 320 36.7 / 37.4, 400 among three
+# single tokens 55.4 / 55.2; delta rule of 8 heads 320 43.7 / 43.3, 768 80.8 / 72.1; of 16 heads 320 48.0 / 50.3,
 # 768 87.4 / 87.8, 2,048 225 / 215.
 RECURRENT_APART_ROWS = int(os.environ.get("FELLM_B200_RECURRENT_APART_ROWS", 320))
 RECURRENT_APART_ROWS_FULL = max(RECURRENT_APART_ROWS, 1024)        # the delta rule with more than 96 blocks a portion (H dv / 16)
