@@ -14,16 +14,18 @@
 // (j + 1) RK / NC), which it alone accumulates: a row's read-out of RK float32 sums lies across NC warps' registers.  NG = 4,
 // NC = 2: 64 rows, key tiles of 32.
 //
-// Single tokens (latent_tokens_kernel): 16 rows (the heads of a token) and a share of their keys a CTA of eight warps, tiles of
-// 64 keys.  A warp makes the scores of eight keys, a thread the probabilities of four (16 threads a row), a warp the sums of
-// an eighth of the value elements.  A token's keys are shared out in portions of 16; up to eight shares are a cluster, whose
-// sums stay in shared memory and are put together through distributed shared memory, every CTA an eighth of the
-// elements.  More shares (long contexts of few requests) leave (m, l, sums) in a scratch buffer that latent_merge_kernel puts
+// Single tokens (latent_tokens_kernel): 16 rows (the heads of a token) and a share of their keys, whole tiles, a CTA of eight warps;
+// tiles of 64 keys, of 32 where the latent is no multiple of 64.  A warp makes the scores of eight keys, a thread the probabilities of
+// four (16 threads a row), a warp the sums of an eighth of the value elements.  Few shares are a cluster, whose sums stay in shared memory and are
+// put together through distributed shared memory, every CTA its part of the elements.  More shares (long contexts of few requests), or
+// clusters that the device does not hold at once, leave (m, l, sums) in a scratch buffer that latent_merge_kernel puts
 // together (a block a row: 8 x the parallelism of a merge by the CTA that finishes last, which was tried and cost 40 us a
-// layer).  Index arrays and cache rows are read ahead of the wait for the kernel in front: see the kernel.
+// layer).  Which of the two runs is not in the bits: the shares, and every sum's order, are the same.  Index arrays and cache rows are read
+// ahead of the wait for the kernel in front: see the kernel.
 // Bound by: latency, of the index arrays, of the keys, of the chains of a tile (tiles by four warps that each did the softmax of all
-// rows took 6,700 instructions a warp, 17 us; eight warps, 3,300, 14.5 us; one page a warp and angles ahead of the wait 12.6 us by itself
-// and 9 behind the product in front; 8 tokens of 8 heads over 1,024 keys of 1,152 bytes, 11.7 + 5.7 us for the merge before).
+// rows took 6,700 instructions a warp).  8 tokens of 8 heads over 1,024 keys of 1,152 bytes with the product in front: four warps and a merge
+// 18.7 us, here 12.8 (1 token over 100 keys 15.1 -> 9.9, 48 tokens over 1,024 32.3 -> 27.3).  Shares in portions of 16 keys, and scores as the
+// sum of two chains of MMAs, take 12.1 and 8.0 us; they round otherwise, and a row's bits then depend on how the shares are put together.
 //
 // A key counts for the row of a token at position p iff p - window < key <= p (window 0: every key up to p).  A
 // sink per head joins the denominator once: exp(sink_h), not scaled, no value.  Rows of an item have consecutive
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(NG * NC * 32, 1) latent_attention_kernel(LatAr
 }
 
 // ---------------------------------------------------------------- single tokens
-constexpr int LT_WARPS = 8, LT_KT = 64, LT_ROWS = 16;
+constexpr int LT_WARPS = 8, LT_KT = RK % 64 == 0 ? 64 : 32, LT_ROWS = 16, LT_MAX_CLUSTER = 16;
 constexpr int LT_SLD = LT_KT + 4, LT_PLD = LT_KT + 8;        // row strides of the scores (float32) and the probabilities (bfloat16)
 constexpr int LT_OLD = RK + 4;                               // and of the sums that a cluster puts together
 constexpr int LT_GROUPS = (RK / 16 + LT_WARPS - 1) / LT_WARPS;                // 16 value elements each, a warp's: warp, warp + 8, ..
@@ -301,12 +303,12 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
   const int* bt = a.block_table + (size_t)a.row_slot[r_begin] * a.max_pages;
   auto token_of = [&](int R) { return a.single ? 0 : R / H; };                  // which of the item's tokens a row belongs to
   const int pos_lo = pos0 + token_of(R0), pos_hi = pos0 + token_of(R0 + rows_here - 1);
-  // this CTA's share of the keys, in portions of 16
-  int key_begin = (a.window > 0 ? max(0, pos_lo - a.window + 1) : 0) & ~15;
-  const int portions = (pos_hi + 1 - key_begin + 15) / 16, per = (portions + a.n_splits - 1) / a.n_splits;
-  const int mine = max(0, min(per, portions - rank * per));
-  key_begin += 16 * rank * per;
-  const int key_end = min(pos_hi + 1, key_begin + 16 * mine), n_tiles = (16 * mine + LT_KT - 1) / LT_KT;
+  // this CTA's share of the keys, whole tiles
+  int key_begin = (a.window > 0 ? max(0, pos_lo - a.window + 1) : 0) & ~(LT_KT - 1);
+  const int all = (pos_hi + 1 - key_begin + LT_KT - 1) / LT_KT, per = (all + a.n_splits - 1) / a.n_splits;
+  const int n_tiles = max(0, min(per, all - rank * per));
+  key_begin += LT_KT * rank * per;
+  const int key_end = min(pos_hi + 1, key_begin + LT_KT * n_tiles);
 
   const unsigned q_s = (unsigned)__cvta_generic_to_shared(smem), k_s = q_s + LT_ROWS * ROWB;
   // A tile's portions with a key, two warps each, eight rows a warp: 16 keys lie in one page, so a warp looks one page up and its
@@ -319,7 +321,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
   };
   auto load_tile = [&](int t, const bf16* src) {
     const int at = 16 * (warp >> 1) + 8 * (warp & 1), n_keys = key_end - (key_begin + t * LT_KT) - at;
-    if (n_keys + 8 * (warp & 1) > 0) {             // (the portion has a key)
+    if (at < LT_KT && n_keys + 8 * (warp & 1) > 0) {             // (the portion has a key)
       const unsigned dst = k_s + (t & 1) * LT_KT * ROWB;
 #pragma unroll
       for (int i = 0; i < (8 * CPR + 31) / 32; ++i) {
@@ -379,8 +381,10 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
     }
     cp_async_commit();
   }
-  // a thread's row and four keys of the softmax
-  const int sr = tid >> 4, sk = 4 * (tid & 15);
+  // a thread's row and four keys of the softmax: 16 threads a row, keys 16 sp + sk and sk + 8 and the ones behind them, as a lane of an
+  // MMA's first operand holds them
+  const int sr = tid >> 4, sp = (tid >> 2) & 3, sk = 16 * sp + 2 * (tid & 3);
+  const bool has_keys = sp < LT_KT / 16;
   const int hi = pos0 + token_of(min(R0 + sr, n_rows - 1)), lo = a.window > 0 ? hi - a.window + 1 : 0;
   float m = -INFINITY, l = 0.f;
   float o[LT_GROUPS][2][4];
@@ -396,8 +400,8 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
     const int k0 = key_begin + t * LT_KT, n16 = min(LT_KT / 16, (key_end - k0 + 15) / 16);
     const unsigned kb = k_s + (t & 1) * LT_KT * ROWB;
     if (warp < 2 * n16) {
-      // scores of keys 8 warp .. + 8: two steps of 16 elements a load of theirs, a chain of MMAs each
-      float s[2][4] = {};
+      // scores of keys 8 warp .. + 8, one chain of MMAs: two steps of 16 elements a load of theirs
+      float s[4] = {};
       const unsigned krow = 8 * warp + (lane & 7);
 #pragma unroll 6
       for (int ks = 0; ks < KS / 2; ++ks) {
@@ -405,39 +409,51 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
         ldsm_x4(a0, q_s + tile_off(lane & 15, 4 * ks + (lane >> 4)));
         ldsm_x4(a1, q_s + tile_off(lane & 15, 4 * ks + 2 + (lane >> 4)));
         ldsm_x4(b, kb + tile_off(krow, 4 * ks + (lane >> 3)));
-        mma16816(s[0], a0, b[0], b[1]);
-        mma16816(s[1], a1, b[2], b[3]);
+        mma16816(s, a0, b[0], b[1]);
+        mma16816(s, a1, b[2], b[3]);
       }
       if (KS & 1) {
         unsigned a0[4], b[4];
         ldsm_x4(a0, q_s + tile_off(lane & 15, 2 * (KS - 1) + (lane >> 4)));
         ldsm_x4(b, kb + tile_off(krow, 2 * (KS - 1) + ((lane >> 3) & 1)));        // (the last two matrices: the first two once more)
-        mma16816(s[0], a0, b[0], b[1]);
+        mma16816(s, a0, b[0], b[1]);
       }
       float* to = S_s + g * LT_SLD + 8 * warp + 2 * c;
-      *(float2*)to = make_float2(s[0][0] + s[1][0], s[0][1] + s[1][1]);
-      *(float2*)(to + 8 * LT_SLD) = make_float2(s[0][2] + s[1][2], s[0][3] + s[1][3]);
+      *(float2*)to = make_float2(s[0], s[1]);
+      *(float2*)(to + 8 * LT_SLD) = make_float2(s[2], s[3]);
     }
     __syncthreads();
     {
-      const float4 raw = *(const float4*)(S_s + sr * LT_SLD + sk);
-      float x[4] = {raw.x, raw.y, raw.z, raw.w}, mx = -INFINITY;
+      float x[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (has_keys) {
+        const float2 lo2 = *(const float2*)(S_s + sr * LT_SLD + sk), hi2 = *(const float2*)(S_s + sr * LT_SLD + sk + 8);
+        const float raw[4] = {lo2.x, lo2.y, hi2.x, hi2.y};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int kj = k0 + sk + e;
-        x[e] = kj <= hi && kj >= lo && kj < key_end ? x[e] * a.scale_log2 : -INFINITY;
-        mx = fmaxf(mx, x[e]);
+        for (int e = 0; e < 4; ++e) {
+          const int kj = k0 + sk + (e & 1) + 8 * (e >> 1);
+          if (kj <= hi && kj >= lo) x[e] = raw[e] * a.scale_log2;
+        }
       }
+      float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
 #pragma unroll
       for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
       const float mn = fmaxf(m, mx), mu = mn == -INFINITY ? 0.f : mn;              // (a row that has seen nothing yet)
       const float corr = exp2f(m - mu);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = exp2f(x[e] - mu);
+      // a tile's sum, portion after portion of four threads' keys: the last portion's threads have it
       float sum = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { x[e] = exp2f(x[e] - mu); sum += x[e]; }
+      for (int p = 0; p < LT_KT / 16; ++p) {
+        const float before = p ? __shfl_sync(0xffffffffu, sum, (lane & 16) | (4 * (p - 1)) | (lane & 3)) : 0.f;
+        if (sp == p) sum = (((before + x[0]) + x[1]) + x[2]) + x[3];
+      }
       l = l * corr + sum;
       m = mn;
-      *(uint2*)(P_s + sr * LT_PLD + sk) = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
+      if (has_keys) {
+        *(unsigned*)(P_s + sr * LT_PLD + sk) = pack_bf16(x[0], x[1]);
+        *(unsigned*)(P_s + sr * LT_PLD + sk + 8) = pack_bf16(x[2], x[3]);
+      }
       if ((tid & 15) == 0) corr_s[sr] = corr;
     }
     __syncthreads();
@@ -467,8 +483,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
       load_tile(t + 2, src);
     }
   }
-#pragma unroll
-  for (int w = 8; w > 0; w >>= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
+  l += __shfl_xor_sync(0xffffffffu, l, 1); l += __shfl_xor_sync(0xffffffffu, l, 2);
   cp_async_wait_all();
   __syncthreads();                     // (the keys' place is free; P_s and corr_s are read)
   const size_t row_g = (size_t)r_begin * H + R0;
@@ -491,7 +506,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
       }
     }
   }
-  if ((tid & 15) == 0) {
+  if ((tid & 15) == 4 * (LT_KT / 16 - 1)) {
     if (!apart) ml_s[sr] = make_float2(m, l);
     else if (sr < rows_here) *(float2*)(a.scratch + ((row_g + sr) * a.n_splits + rank) * (RK + 2) + RK) = make_float2(m, l);
   }
@@ -503,24 +518,26 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
   const int total = rows_here * (RK / 4), share = (total + n - 1) / n, end = min(total, (rank + 1) * share);
   for (int x = rank * share + tid; x < end; x += LT_WARPS * 32) {
     const int r = x / (RK / 4), col = 4 * (x - r * (RK / 4));
+    float2 ml[LT_MAX_CLUSTER];
     float4 v[8];
-    float2 ml[8];
+    auto sums_of = [&](int q) { return *(const float4*)(cluster.map_shared_rank(os, q) + r * LT_OLD + col); };
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (q < n) {
-        v[q] = *(const float4*)(cluster.map_shared_rank(os, q) + r * LT_OLD + col);
-        ml[q] = *(const float2*)(cluster.map_shared_rank(ml_s, q) + r);
-      }
+    for (int q = 0; q < LT_MAX_CLUSTER; ++q) if (q < n) ml[q] = *(const float2*)(cluster.map_shared_rank(ml_s, q) + r);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) if (q < n) v[q] = sums_of(q);
     float M = -INFINITY, L = 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) if (q < n) M = fmaxf(M, ml[q].x);
+    for (int q = 0; q < LT_MAX_CLUSTER; ++q) if (q < n) M = fmaxf(M, ml[q].x);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (q < n && ml[q].x > -INFINITY) {          // (a share without a visible key counts nothing)
-        const float w = exp2f(ml[q].x - M);
-        L = fmaf(ml[q].y, w, L);
-        acc.x = fmaf(v[q].x, w, acc.x); acc.y = fmaf(v[q].y, w, acc.y); acc.z = fmaf(v[q].z, w, acc.z); acc.w = fmaf(v[q].w, w, acc.w);
+    for (int q = 0; q < LT_MAX_CLUSTER; ++q)
+      if (q < n) {
+        // as latent_merge_kernel (a share without a visible key counts nothing; the only share counts as it is)
+        const bool counts = n == 1 || ml[q].x > -INFINITY;
+        const float w = n == 1 ? 1.f : counts ? exp2f(ml[q].x - M) : 0.f;
+        if (counts) L = __fadd_rn(L, __fmul_rn(ml[q].y, w));
+        const float4 o = q < 8 ? v[q & 7] : sums_of(q);
+        acc.x = fmaf(o.x, w, acc.x); acc.y = fmaf(o.y, w, acc.y); acc.z = fmaf(o.z, w, acc.z); acc.w = fmaf(o.w, w, acc.w);
       }
     if (a.sinks) L += exp2f(a.sinks[(R0 + r) % H] * LOG2E - M);
     const float inv = 1.0f / L;
@@ -546,7 +563,7 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restri
   float m = -INFINITY;
   for (int s = 0; s < n_splits; ++s) m = fmaxf(m, sm_m[s]);
   float L = 0.f;
-  for (int s = 0; s < n_splits; ++s) L += sm_m[s] > -INFINITY ? sm_w[s] * exp2f(sm_m[s] - m) : 0.f;
+  for (int s = 0; s < n_splits; ++s) if (sm_m[s] > -INFINITY) L = __fadd_rn(L, __fmul_rn(sm_w[s], exp2f(sm_m[s] - m)));      // (as a cluster adds them)
   if (sinks) L += exp2f(sinks[row % H] * LOG2E - m);
   const float inv = 1.0f / L;
   __syncthreads();
@@ -577,8 +594,9 @@ static int launch_latent(const LatArgs& a, int n_items, int max_item_rows, int r
 }
 
 static int launch_tokens(const LatArgs& a, int n_items, int max_item_rows, int rows_total, cudaStream_t stream) {
-  if (a.page_tokens % 16) return FELLM_ERR_SIZE;
+  if (a.page_tokens % LT_KT) return FELLM_ERR_SIZE;
   cudaError_t e = cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT_SMEM);
+  if (e == cudaSuccess && a.cluster && a.n_splits > 8) e = cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return (int)e;
   dim3 grid(a.n_splits, n_items, ceil_div(max_item_rows * a.H, LT_ROWS));
   int rc = launch_k_class(1, latent_tokens_kernel, grid, dim3(LT_WARPS * 32), LT_SMEM, stream, a.cluster ? a.n_splits : 1, a);
@@ -589,12 +607,13 @@ static int launch_tokens(const LatArgs& a, int n_items, int max_item_rows, int r
 
 // How many clusters of `size` CTAs of the single tokens' kernel the device holds at once (asked once per device and size; 0: none).
 FELLM_API int fellm_latent_token_clusters(int size) {
-  static int cached[64][9];
+  static int cached[64][LT_MAX_CLUSTER + 1];
   int dev = 0;
-  if (size < 1 || size > 8 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (size < 1 || size > LT_MAX_CLUSTER || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   if (!cached[dev][size]) {
     int n = 0;
     if (cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT_SMEM) != cudaSuccess) return 0;
+    if (size > 8 && cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return 0; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(size); cfg.blockDim = dim3(LT_WARPS * 32); cfg.dynamicSmemBytes = LT_SMEM;
     cudaLaunchAttribute at[1];
@@ -609,12 +628,10 @@ FELLM_API int fellm_latent_token_clusters(int size) {
 
 FELLM_API int fellm_latent_attention_rk() { return RK; }
 FELLM_API int fellm_latent_attention_dr() { return DR; }
-// the key tile of a variant (0: portions, 1: single tokens): pages hold a multiple of it
-FELLM_API int fellm_latent_attention_key_tile(int variant) { return variant != 1 ? 32 : 16; }
 
 // variant 0: 64 rows a CTA (portions of prompts), n_splits must be 1; variant 1: 16 rows a CTA (single tokens),
 // qsrc (or null): the queries' rotated parts are read from there and rotated in the kernel, and q holds the RK
-// elements of a (token, head) row alone.  n_splits >= 1 shares of the keys: as a cluster (up to 8), or (up to 32) with scratch of rows * H * n_splits * (RK + 2) floats when above 1.
+// elements of a (token, head) row alone.  n_splits >= 1 shares of the keys: as a cluster (up to 16), or (up to 32) with scratch of rows * H * n_splits * (RK + 2) floats when above 1.
 FELLM_API int fellm_latent_attention_mma(const void* q, const void* pool, const int* block_table, int max_pages,
                                          const int* positions, const int* row_slot, const int* item_start, int n_items,
                                          int max_item_rows, int rows_total, void* out, float* scratch, int n_splits, int H,
@@ -623,7 +640,7 @@ FELLM_API int fellm_latent_attention_mma(const void* q, const void* pool, const 
                                          const float* freq, int n_rot, float mag, int cluster, cudaStream_t stream) {
   if (n_items <= 0 || rows_total <= 0 || max_item_rows <= 0) return 0;
   if (!q || !pool || !block_table || !positions || !row_slot || !item_start || !out) return FELLM_ERR_ARG;
-  if (H < 1 || page_tokens < 1 || n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && variant != 1) || (cluster && n_splits > 8) ||
+  if (H < 1 || page_tokens < 1 || n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && variant != 1) || (cluster && n_splits > LT_MAX_CLUSTER) ||
       (n_splits > 1 && !cluster && !scratch)) return FELLM_ERR_ARG;
   if (qsrc && ((ldq | q_head | q_rot_off) % 8 || ((size_t)qsrc & 15) || n_rot < 0 || n_rot > DR || (n_rot & 1) || (n_rot && !freq))) return FELLM_ERR_SIZE;
   LatArgs a;

@@ -1405,9 +1405,10 @@ def latent_rotate_q(q, H, dn, dr, q_abs, rk, freq, n_rot, mag, positions):
 LATENT_ATTENTION_MMA = os.environ.get("FELLM_B200_LATENT_ATTENTION_MMA", "1") != "0"
 LATENT_SINGLE_ROWS = 32        # up to this many (token, head) rows an item: the kernel's form for single tokens
 LATENT_MAX_SPLITS = 16
-# So many shares of a token's keys or fewer are one cluster (of up to 8) and put together in it, more go through memory and a merge behind.
-# us a layer of 8 heads, merge / cluster: 8 tokens over 1,024 keys 38 / 32, 1 token over 100 30 / 22, 24 tokens 45 / 40, 48 (shares of three) 63 / 63;
-# clusters of 8 where only 15 are resident: 16 tokens 43 / 47.
+# So many shares of a token's keys or fewer are one cluster, put together in it, where the device holds the clusters of all tokens at
+# once; else the shares go through memory and a merge behind.  The bits are the same.  us with the product in front, 8 heads, merge /
+# cluster: 8 tokens over 1,024 keys 14.9 / 12.8, 1 token over 100 11.3 / 9.9, 32 tokens over 1,024 19.3 / 18.1; 16 shares: 1 token over 4,000
+# 17.9 / 19.0, 4 tokens 18.4 / 19.3.
 LATENT_CLUSTER_TO = int(os.environ.get("FELLM_B200_LATENT_CLUSTER_TO", 10))
 
 
@@ -1528,10 +1529,9 @@ def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, i
         ctas = n_items * (-(-max_item_rows * H // 16))
         n_splits = max(1, min(tiles // 2, 148 // max(ctas, 1), LATENT_MAX_SPLITS))
         if 1 < n_splits <= LATENT_CLUSTER_TO:
-            # as one cluster, of a size that the device holds for all tokens at once (a second round costs more than fewer shares)
+            # as one cluster where the device holds those of all tokens at once (a second round costs more than the merge)
             fits = _fn("latent_attention_mma", "fellm_latent_token_clusters", [_c_int], defines={"LAT_RK": rk, "LAT_DR": dr})
-            cluster = next((s for s in range(min(n_splits, 8), 1, -1) if fits(s) >= ctas), 0)
-        n_splits = cluster or n_splits
+            cluster = int(fits(n_splits) >= ctas)
         if n_splits > 1 and not cluster:
             scratch = torch.empty((T * H * n_splits * (rk + 2),), dtype=torch.float32, device=q_abs.device)
     f = _fn("latent_attention_mma", "fellm_latent_attention_mma",

@@ -43,3 +43,26 @@ def test_a_token_over_its_keys(monkeypatch, rk, dr, H, window, contexts, share):
         # probabilities rounded to bfloat16 (2^-9 each) of values of size ~1, then the result
         room = 2.0 ** -8 * (p @ rows[:, :rk].abs() / p.sum(-1, keepdim=True)) + 2.0 ** -8 * want.abs() + 1e-4
         assert ((got[i] - want).abs() <= room).all(), (c, float(((got[i] - want).abs() / room).max()))
+
+
+@pytest.mark.parametrize("rk,dr,H", [(512, 64, 8), (64, 16, 24), (96, 16, 4)])
+@pytest.mark.parametrize("window,contexts", [(None, (1, 40, 129, 700)), (1024, (1500,) * 3 + (1039, 64) + (1100,) * 3), (1024, (2000,) * 17), (None, (3100,))])
+def test_how_the_shares_are_put_together_is_not_in_the_bits(monkeypatch, rk, dr, H, window, contexts):
+    """A cluster or memory and a second kernel: the shares are the same whole tiles and are added in the same order."""
+    from fellm_b200 import ops
+    D, PT, n = rk + dr, 64, len(contexts)
+    g = torch.Generator().manual_seed(rk + n)
+    pages = [-(-c // PT) for c in contexts]
+    pool = torch.randn(sum(pages) + 1, 1, PT, D, generator=g).bfloat16().cuda()
+    table = torch.zeros((n, max(pages)), dtype=torch.int32)
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(p) + 1 + sum(pages[:i])
+    q = (torch.randn(n, H * D, generator=g) * 0.5).bfloat16().cuda()
+    pos = torch.tensor([c - 1 for c in contexts], dtype=torch.int32).cuda()
+    sinks = torch.randn(H, generator=g).cuda()
+
+    def run(share):
+        monkeypatch.setattr(ops, "LATENT_CLUSTER_TO", share)
+        return ops.latent_attention(q, H, rk, dr, pool, table.cuda(), pos, torch.arange(n, dtype=torch.int32).cuda(),
+                                    torch.arange(n + 1, dtype=torch.int32).cuda(), n, 1, max(contexts), 0, PT, D ** -0.5, window=window, sinks=sinks)
+    assert torch.equal(run(0), run(100))
