@@ -94,6 +94,7 @@ struct LatArgs {
   float* scratch;           // n_splits > 1 and no cluster: [rows * H][n_splits][RK + 2]
   const float* sinks;       // [H] or null
   int H, page_tokens, layer, layers_in_group, window, n_splits, cluster, single;       // single: every item is one token
+  int ready;                // the index arrays and the cache are complete before the kernel in front ends: see latent_tokens_kernel
   float scale_log2;
 };
 
@@ -295,8 +296,10 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3, H = a.H;
   const int rank = blockIdx.x, item = blockIdx.y, R0 = blockIdx.z * LT_ROWS;
   pdl_launch_dependents();
-  // Launched as a programmatic dependent of the product that makes q, which is launched the ordinary way: all that was written in front
-  // of that one is there, the index arrays and the cache with this step's own rows.  Only q is waited for.
+  // With `ready` launched as a programmatic dependent, and what the caller vouches for is read ahead of the wait: a kernel launched the
+  // ordinary way (the product that makes q) lies between this one and whatever wrote the index arrays and the cache with this
+  // step's own rows, and it started when those had ended.  Only q is waited for.
+  if (!a.ready) pdl_wait();
   const int r_begin = a.single ? item : a.item_start[item], n_rows = a.single ? H : (a.item_start[item + 1] - r_begin) * H;
   if (R0 >= n_rows) { pdl_wait(); return; }        // (the same for a whole cluster)
   const int rows_here = min(LT_ROWS, n_rows - R0), pos0 = a.positions[r_begin];
@@ -599,7 +602,7 @@ static int launch_tokens(const LatArgs& a, int n_items, int max_item_rows, int r
   if (e == cudaSuccess && a.cluster && a.n_splits > 8) e = cudaFuncSetAttribute(latent_tokens_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return (int)e;
   dim3 grid(a.n_splits, n_items, ceil_div(max_item_rows * a.H, LT_ROWS));
-  int rc = launch_k_class(1, latent_tokens_kernel, grid, dim3(LT_WARPS * 32), LT_SMEM, stream, a.cluster ? a.n_splits : 1, a);
+  int rc = launch_k_class(a.ready ? 1 : launch_class_for_rows(rows_total, 0), latent_tokens_kernel, grid, dim3(LT_WARPS * 32), LT_SMEM, stream, a.cluster ? a.n_splits : 1, a);
   if (rc || a.n_splits == 1 || a.cluster) return rc;
   return launch_k_class(launch_class_for_rows(rows_total, 0), latent_merge_kernel, dim3(rows_total * a.H), dim3(RK / 2 < 32 ? 32 : RK / 2), 0, stream, 1,
                         (const float*)a.scratch, a.out, a.sinks, a.H, a.n_splits);
@@ -632,12 +635,13 @@ FELLM_API int fellm_latent_attention_dr() { return DR; }
 // variant 0: 64 rows a CTA (portions of prompts), n_splits must be 1; variant 1: 16 rows a CTA (single tokens),
 // qsrc (or null): the queries' rotated parts are read from there and rotated in the kernel, and q holds the RK
 // elements of a (token, head) row alone.  n_splits >= 1 shares of the keys: as a cluster (up to 16), or (up to 32) with scratch of rows * H * n_splits * (RK + 2) floats when above 1.
+// ready (variant 1): see latent_tokens_kernel.
 FELLM_API int fellm_latent_attention_mma(const void* q, const void* pool, const int* block_table, int max_pages,
                                          const int* positions, const int* row_slot, const int* item_start, int n_items,
                                          int max_item_rows, int rows_total, void* out, float* scratch, int n_splits, int H,
                                          int page_tokens, int layer, int layers_in_group, float scale, int window,
                                          const float* sinks, int variant, const void* qsrc, int ldq, int q_head, int q_rot_off,
-                                         const float* freq, int n_rot, float mag, int cluster, cudaStream_t stream) {
+                                         const float* freq, int n_rot, float mag, int cluster, int ready, cudaStream_t stream) {
   if (n_items <= 0 || rows_total <= 0 || max_item_rows <= 0) return 0;
   if (!q || !pool || !block_table || !positions || !row_slot || !item_start || !out) return FELLM_ERR_ARG;
   if (H < 1 || page_tokens < 1 || n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && variant != 1) || (cluster && n_splits > LT_MAX_CLUSTER) ||
@@ -648,7 +652,7 @@ FELLM_API int fellm_latent_attention_mma(const void* q, const void* pool, const 
   a.q = (const bf16*)q; a.pool = (const bf16*)pool; a.block_table = block_table; a.max_pages = max_pages;
   a.positions = positions; a.row_slot = row_slot; a.item_start = item_start; a.out = (bf16*)out; a.scratch = scratch;
   a.sinks = sinks; a.H = H; a.page_tokens = page_tokens; a.layer = layer; a.layers_in_group = layers_in_group;
-  a.window = window > 0 ? window : 0; a.n_splits = n_splits; a.cluster = cluster && n_splits > 1; a.single = max_item_rows == 1 && n_items == rows_total; a.scale_log2 = scale * LOG2E;
+  a.window = window > 0 ? window : 0; a.n_splits = n_splits; a.cluster = cluster && n_splits > 1; a.ready = ready; a.single = max_item_rows == 1 && n_items == rows_total; a.scale_log2 = scale * LOG2E;
   if (variant == 0) return launch_latent<4, 2>(a, n_items, max_item_rows, rows_total, stream);
   return launch_tokens(a, n_items, max_item_rows, rows_total, stream);
 }

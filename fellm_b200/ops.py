@@ -1492,7 +1492,7 @@ def latent_attention_modules(rk: int, dr: int):
 
 
 def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, item_start, n_items, max_item_rows, max_len,
-                     layer, page_tokens, scale, *, window=None, sinks=None, out=None, q_rot=None):
+                     layer, page_tokens, scale, *, window=None, sinks=None, out=None, q_rot=None, cache_ready=False):
     """Latent attention on tensor cores (bfloat16): q_abs [T, H * (rk + dr)] contiguous, the queries taken into the
     cache rows' space; pool's page-layer record is [page_tokens][rk + dr]; rows of item i are
     item_start[i]..item_start[i + 1] with consecutive positions.  A key's value is the first rk elements of its row.
@@ -1500,7 +1500,9 @@ def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, i
     sizes the split of a single token's key walk).  q_rot = (q, q_head, off, freq, n_rot, mag): q_abs is [T, H * rk], and
     head h's rotated part is read from columns [h q_head + off, + dr) of q [T, >= H q_head] and rotated by the row's
     position inside the kernel (pairs (2i, 2i + 1) of its first n_rot elements, angle = position * freq[i], cos and sin
-    times mag); see latent_rotate_fusable.  Returns [T, H * rk]."""
+    times mag); see latent_rotate_fusable.  cache_ready: a kernel launched the ordinary way, as head_gemm's are, lies between this call and
+    the last one that wrote the cache or the index arrays; single tokens then read those while the kernel in front still runs.  Returns
+    [T, H * rk]."""
     _dev(q_abs, pool, block_table, positions, row_slot, item_start, sinks)
     T = q_abs.shape[0]
     assert latent_attention_takes(q_abs, pool, rk, dr, page_tokens)
@@ -1536,11 +1538,11 @@ def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, i
             scratch = torch.empty((T * H * n_splits * (rk + 2),), dtype=torch.float32, device=q_abs.device)
     f = _fn("latent_attention_mma", "fellm_latent_attention_mma",
             [_c_p, _c_p, _c_p, _c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
-             _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_f, _c_int, _c_p], defines={"LAT_RK": rk, "LAT_DR": dr})
+             _c_int, _c_f, _c_int, _c_p, _c_int, _c_p, _c_int, _c_int, _c_int, _c_p, _c_int, _c_f, _c_int, _c_int, _c_p], defines={"LAT_RK": rk, "LAT_DR": dr})
     _check(f(_p(q_abs), _p(pool), _p(block_table), block_table.shape[1], _p(positions), _p(row_slot), _p(item_start),
              int(n_items), int(max_item_rows), T, _p(out), _p(scratch), n_splits, H, page_tokens, layer, pool.shape[1],
              float(scale), int(window or 0), _p(sinks), variant, _p(qsrc), ldq, int(q_head), int(q_off), _p(freq), int(n_rot), float(mag),
-             int(cluster), _stream()), "latent_attention")
+             int(cluster), int(bool(cache_ready)), _stream()), "latent_attention")
     return out
 
 

@@ -137,7 +137,7 @@ class LatentAttention(Mixer):
             ops.head_gemm(q, w["ukT.weight"], qa, a_head=dn + dr, out_head=rk)
             a = ops.latent_attention(qa, H, rk, dr, cache.pool, cache.block_table, ctx.positions, ctx.row_slot, ctx.item_start,
                                      ctx.n_items, ctx.max_item_rows, ctx.max_len, cache.layer, cache.page_tokens, self.scale,
-                                     window=self.window, sinks=w.get("sink"),
+                                     window=self.window, sinks=w.get("sink"), cache_ready=True,        # (head_gemm: an ordinary launch)
                                      q_rot=(q, dn + dr, dn, self.position.inv_freq, self.n_rot, self.magnitude))
             return self._read_out(a, T, out, store)
         qa = torch.empty((T, H * (rk + dr)), dtype=q.dtype, device=q.device)
@@ -146,7 +146,7 @@ class LatentAttention(Mixer):
         if on_mma:
             a = ops.latent_attention(qa, H, rk, dr, cache.pool, cache.block_table, ctx.positions, ctx.row_slot, ctx.item_start,
                                      ctx.n_items, ctx.max_item_rows, ctx.max_len, cache.layer, cache.page_tokens, self.scale,
-                                     window=self.window, sinks=w.get("sink"))
+                                     window=self.window, sinks=w.get("sink"), cache_ready=True)
         else:
             # the 32-bit engine, and sizes the tensor-core kernel does not take
             a = ops.paged_attention_general(qa, H, rk + dr, 0, cache.pool, cache.block_table, ctx.positions, ctx.row_slot,

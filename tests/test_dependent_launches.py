@@ -88,6 +88,33 @@ def test_dependent_kernels_read_the_cache_behind_their_wait(path):
     assert not frozen, f"{path.name}: {frozen}"
 
 
+def test_the_cache_is_read_ahead_of_a_wait_only_where_the_caller_says_so():
+    """latent_tokens_kernel reads index arrays and cache in front of its wait, or waits first: as the caller says.  Who says so has launched
+    a product per head in front, an ordinary launch on every route, and writes nothing behind it."""
+    text = source(CSRC / "latent_attention_mma.cu")
+    body = kernels(text)["latent_tokens_kernel"][1]
+    first = body.index("if (!a.ready) pdl_wait();")
+    assert all(first < body.index(read) for read in ("a.item_start", "a.positions", "a.block_table", "a.row_slot", "a.pool"))
+    assert "launch_k_class(a.ready ? 1 :" in text
+    entry = {"fellm_gemm_tiled_batched": ("gemm_tiled", {"gemm_heads_few_kernel", "gemm_tiled_kernel"}),
+             "fellm_gemm_simt_batched": ("gemm_simt", {"gemm_tn_simt_kernel"})}
+    ops = (CSRC.parent / "ops.py").read_text()
+    head_gemm = ops[ops.index("def head_gemm("):ops.index("\n\n\n", ops.index("def head_gemm("))]
+    assert set(re.findall(r'"(fellm_\w+)"', head_gemm)) == set(entry)
+    for name, (module, launched) in entry.items():
+        text = source(CSRC / f"{module}.cu")
+        at = text.index(f"{name}(")
+        body = text[text.index("{", at):closing(text, text.index("{", at), "{}")]
+        assert "launch_k" not in body and "<<<" in body
+        assert {k for k in kernels(text) if re.search(rf"\b{k}\b", body)} == launched
+    for path in CSRC.parent.rglob("*.py"):
+        text = path.read_text()
+        for m in re.finditer(r"cache_ready=True", text):
+            call = text.rindex("ops.latent_attention(", 0, m.start())
+            product = text.rindex("ops.head_gemm(", 0, call)
+            assert set(re.findall(r"\bops\.(\w+)\(", text[product:call])) <= {"head_gemm", "latent_rotate_q"}, path
+
+
 def test_the_reading_finds_the_launches():
     """(the checks above would pass on files they cannot read)"""
     found = {p.stem: dependents(source(p), kernels(source(p))) for p in SOURCES}

@@ -66,3 +66,34 @@ def test_how_the_shares_are_put_together_is_not_in_the_bits(monkeypatch, rk, dr,
         return ops.latent_attention(q, H, rk, dr, pool, table.cuda(), pos, torch.arange(n, dtype=torch.int32).cuda(),
                                     torch.arange(n + 1, dtype=torch.int32).cuda(), n, 1, max(contexts), 0, PT, D ** -0.5, window=window, sinks=sinks)
     assert torch.equal(run(0), run(100))
+
+
+@pytest.mark.parametrize("n", [1, 8, 140])
+def test_directly_behind_the_kernel_that_writes_the_cache(n):
+    """Without cache_ready nothing of a step is read before the kernel in front has ended: this one writes the step's own rows, and lets its
+    dependents start before it does.  New rows in every pass, a context of one key beside others: a row not yet written would show."""
+    from types import SimpleNamespace
+    from fellm_b200 import ops
+    rk, dr, H, PT, rq = 512, 64, 8, 64, 768
+    D = rk + dr
+    contexts = [1 + 37 * i % 200 for i in range(n)]
+    g = torch.Generator().manual_seed(n)
+    pool = torch.randn(4 * n + 1, 1, PT, D, generator=g).bfloat16().cuda()
+    table = (torch.arange(4 * n, dtype=torch.int32).view(n, 4) + 1).cuda()
+    pos = torch.tensor([c - 1 for c in contexts], dtype=torch.int32).cuda()
+    slot, starts = torch.arange(n, dtype=torch.int32).cuda(), torch.arange(n + 1, dtype=torch.int32).cuda()
+    cache = SimpleNamespace(pool=pool, block_table=table, page_tokens=PT, layer=0)
+    wq, wc = torch.ones(rq).cuda(), torch.ones(rk).cuda()
+    freq = (0.5 ** torch.arange(dr // 2)).cuda()
+    q = torch.randn(n, H * D, generator=g).bfloat16().cuda()
+    z = [torch.randn(n, rq + D, generator=g).cuda() for _ in range(8)]
+
+    def step(i, wait):
+        ops.latent_prep(z[i], 0, rq, rq, rk, rq + rk, dr, wq, wc, 1e-5, freq, dr, 1.0, pos, slot, cache, torch.bfloat16)
+        if wait:
+            torch.cuda.synchronize()
+        return ops.latent_attention(q, H, rk, dr, pool, table, pos, slot, starts, n, 1, max(contexts), 0, PT, D ** -0.5)
+    want = [step(i, True) for i in range(8)]
+    torch.cuda.synchronize()
+    got = [step(i, False) for i in range(8)]
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
