@@ -94,7 +94,9 @@ __device__ __forceinline__ float tanh_any(float x) {
 // predecessor in the stream is still running.  What does not depend on the predecessor (weight
 // prefetch, index set-up) goes before pdl_wait(); everything that reads or writes data another
 // kernel of the step touches goes after it.  pdl_wait() returns once the predecessor has completed
-// and its writes are visible; it is a no-op for a kernel launched the ordinary way.
+// and its writes are visible; it is a no-op for a kernel launched the ordinary way.  Loads through a pointer that the kernel
+// declares __restrict__ need not stay behind the wait (nobody else is taken to write there; const as well, never to change): so of
+// its parameters only weights, the step's index arrays and what it merely writes are declared so.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -150,11 +152,13 @@ struct TraceScope {
 #include <cstdlib>
 static inline bool pdl_enabled(int launch_class) {
   static int on = -1;
-  // FELLM_B200_PDL: 0 = never; 2 (the default) = only launches of class 1, the weight-streaming
-  // products, which request their weights before they wait for the kernel before them; 3 = also
-  // class 2 (short element-wise kernels); 1 = every launch.  Measured on B200, one decode step of
-  // 88 dependent launches replayed from a CUDA graph (batch 8, 16 layers of width 1024): 465 us
-  // with 0, 404 us with 2, 429 us with 3, 421 us with 1: kernels with nothing to do before their
+  // FELLM_B200_PDL: 0 = never; 2 (the default) = only launches of class 1; 3 = also class 2 (short
+  // element-wise kernels); 1 = every launch.  Class 1: the weight-streaming products, which request
+  // their weights before they wait for the kernel in front; decode attention that reads page numbers or
+  // keys ahead of its wait; the kernels around a handful of rows' experts and those of steps of many rows
+  // (launch_class_for_rows), whose launch hides under the kernel in front.  Measured on B200, one
+  // decode step of 88 dependent launches replayed from a CUDA graph (batch 8, 16 layers of width 1024): 465 us
+  // with 0, 404 us with 2, 429 us with 3, 421 us with 1: most kernels with nothing to do before their
   // wait only take SM room from the kernel they wait for.
   if (on < 0) { const char* e = getenv("FELLM_B200_PDL"); on = (e && e[0] >= '0' && e[0] <= '3') ? e[0] - '0' : 2; }
   return on == 1 || (on == 2 && launch_class == 1) || (on == 3 && (launch_class == 1 || launch_class == 2));

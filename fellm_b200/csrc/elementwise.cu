@@ -8,7 +8,7 @@
 
 // ---------------------------------------------------------------- embedding
 template <typename TW>
-__global__ void embed_rows_kernel(const int* __restrict__ tokens, const TW* __restrict__ table,
+__global__ void embed_rows_kernel(const int* tokens, const TW* __restrict__ table,
                                   float* __restrict__ out, int d, int vocab, int* __restrict__ status, float scale) {
   FELLM_TRACE_SCOPE(TRACE_EMBED_ROWS);
   pdl_launch_dependents();
@@ -40,7 +40,7 @@ FELLM_API int fellm_embed_rows(const int* tokens, const void* table, int table_i
 // One block per output row; the reduction order depends on d and the block size only, so a row's
 // result does not depend on which other rows are in the batch.
 template <typename TO, int THREADS>
-__global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w,
                                TO* __restrict__ out, const int* __restrict__ rows, int d, float eps) {
   FELLM_TRACE_SCOPE(TRACE_RMSNORM);
   __shared__ float partial[THREADS / 32];
@@ -78,7 +78,7 @@ __device__ __forceinline__ void store4(bf16* o, float a, float b, float c, float
 // the sum and the scaling (rows longer than 128*VPL are read a second time).  A row's sum has the
 // same order whatever else is in the batch.
 template <typename TO, int VPL>
-__global__ void rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_vec_kernel(const float* x, const float* __restrict__ w,
                                    TO* __restrict__ out, const int* __restrict__ rows, int n_rows, int d, float eps) {
   FELLM_TRACE_SCOPE(TRACE_RMSNORM_VEC);
   pdl_launch_dependents();
@@ -140,6 +140,12 @@ FELLM_API int fellm_rmsnorm(const float* x, const float* w, void* out, int out_i
       if (out_is_bf16) return launch_k_class(norm_class(n_out_rows), rmsnorm_vec_kernel<bf16, 8>, vgrid, dim3(warps * 32), 0, stream, 1, x, w, (bf16*)out, rows, n_out_rows, d, eps);
       return launch_k_class(norm_class(n_out_rows), rmsnorm_vec_kernel<float, 8>, vgrid, dim3(warps * 32), 0, stream, 1, x, w, (float*)out, rows, n_out_rows, d, eps);
     }
+    // Rows of more than 2,048 stay in registers too where their warps, three blocks an SM, are there at once; else they are read a second
+    // time (us at 4,096, read twice / kept: 1 row 5.9 / 4.3, 1,024 rows 7.7 / 6.1, 2,048 rows 8.5 / 10.2)
+    if (d > 2048 && n_out_rows <= 12 * fellm_sm_count()) {
+      if (out_is_bf16) return launch_k_class(norm_class(n_out_rows), rmsnorm_vec_kernel<bf16, 32>, vgrid, dim3(warps * 32), 0, stream, 1, x, w, (bf16*)out, rows, n_out_rows, d, eps);
+      return launch_k_class(norm_class(n_out_rows), rmsnorm_vec_kernel<float, 32>, vgrid, dim3(warps * 32), 0, stream, 1, x, w, (float*)out, rows, n_out_rows, d, eps);
+    }
     if (out_is_bf16) return launch_k_class(norm_class(n_out_rows), rmsnorm_vec_kernel<bf16, 16>, vgrid, dim3(warps * 32), 0, stream, 1, x, w, (bf16*)out, rows, n_out_rows, d, eps);
     return launch_k_class(norm_class(n_out_rows), rmsnorm_vec_kernel<float, 16>, vgrid, dim3(warps * 32), 0, stream, 1, x, w, (float*)out, rows, n_out_rows, d, eps);
   }
@@ -155,7 +161,7 @@ FELLM_API int fellm_rmsnorm(const float* x, const float* w, void* out, int out_i
 // ---------------------------------------------------------------- SiLU gate
 // in [T, 2F]: gate in columns [0,F), up in [F,2F); out [T,F] = gate/(1+exp(-gate)) * up.
 template <typename T>
-__global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, int rows, int F) {
+__global__ void silu_mul_kernel(const T* gu, T* __restrict__ out, int rows, int F) {
   FELLM_TRACE_SCOPE(TRACE_SILU_MUL);
   pdl_launch_dependents();
   pdl_wait(); FELLM_TRACE_WAITED();
@@ -179,7 +185,7 @@ FELLM_API int fellm_silu_mul(const void* gu, void* out, int is_bf16, int rows, i
 // ---------------------------------------------------------------- Dynamic Tanh norm
 // y = tanh(alpha * x) * w + b: no mean, no variance, nothing that couples the elements of a row.
 template <typename TO>
-__global__ void dyt_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
+__global__ void dyt_norm_kernel(const float* x, const float* __restrict__ w, const float* __restrict__ b,
                                 float alpha, TO* __restrict__ out, const int* __restrict__ rows, int n_rows, int d) {
   pdl_launch_dependents();
   pdl_wait();
@@ -204,14 +210,14 @@ FELLM_API int fellm_dyt_norm(const float* x, const float* w, const float* b, flo
 // ---------------------------------------------------------------- [a | b] rows in the activation dtype
 // out[t, 0:d] = a[t, :], out[t, d:2d] = b[t, :] (float32 in): the input of a product over two streams.
 template <typename TO>
-__global__ void concat_cast_kernel(const float* __restrict__ a, const float* __restrict__ b, TO* __restrict__ out,
+__global__ void concat_cast_kernel(const float* left, const float* right, TO* __restrict__ out,
                                    int rows, int d) {
   pdl_launch_dependents();
   pdl_wait();
   size_t n = (size_t)rows * 2 * d;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     size_t r = i / (2 * d); int c = (int)(i - r * 2 * d);
-    out[i] = from_f<TO>(c < d ? a[r * d + c] : b[r * d + c - d]);
+    out[i] = from_f<TO>(c < d ? left[r * d + c] : right[r * d + c - d]);
   }
 }
 
@@ -277,7 +283,7 @@ __device__ __forceinline__ float block_sum(float v, float* scratch /* [33] */) {
 // y[c] = x[c] / sqrt(mean over c's part of x^2 + eps) * w[c].  A block per (row, part); float32 in, activation dtype out.
 template <typename TO>
 __global__ void __launch_bounds__(256)
-rmsnorm_groups_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __restrict__ out,
+rmsnorm_groups_kernel(const float* x, const float* __restrict__ w, TO* __restrict__ out,
                       const int* __restrict__ rows, int d, int groups, float eps) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
@@ -297,7 +303,7 @@ rmsnorm_groups_kernel(const float* __restrict__ x, const float* __restrict__ w, 
 // kept in registers between the sum and the scaling (a lane's share in order, then a butterfly: the same order whatever
 // else the step holds).
 template <typename TO, int VPL>
-__global__ void rmsnorm_groups_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __restrict__ out,
+__global__ void rmsnorm_groups_vec_kernel(const float* x, const float* __restrict__ w, TO* __restrict__ out,
                                           const int* __restrict__ rows, int n_rows, int d, int groups, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -359,7 +365,7 @@ FELLM_API int fellm_rmsnorm_groups(const float* x, const float* w, void* out, in
 // coef = (a, b, c, e) on the device.  z float32 [T, F] (the product's sums as they are; rows ldz apart), out in the activation dtype.
 template <typename TO>
 __global__ void __launch_bounds__(256)
-poly_norm_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ coef, TO* __restrict__ out, int F, float eps) {
+poly_norm_kernel(const float* z, int ldz, const float* __restrict__ coef, TO* __restrict__ out, int F, float eps) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
   pdl_wait();
@@ -384,7 +390,7 @@ poly_norm_kernel(const float* __restrict__ z, int ldz, const float* __restrict__
 // between the three sums and the result (the sums: a thread's share in order, warps in order, as above).
 template <typename TO, int KEEP>
 __global__ void __launch_bounds__(256)
-poly_norm_vec_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ coef, TO* __restrict__ out, int F, float eps) {
+poly_norm_vec_kernel(const float* z, int ldz, const float* __restrict__ coef, TO* __restrict__ out, int F, float eps) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
   pdl_wait();
@@ -445,8 +451,8 @@ FELLM_API int fellm_poly_norm(const float* z, int ldz, const float* coef, void* 
 // ---------------------------------------------------------------- sublayers through sigmoid gates into the stream
 // x[t, c] += sum over the n sublayers s of y_s[t, c] * sigmoid(zg[t, s * d + c])   (zg: the gates' logits, bias
 // included, float32 [T, ldg]; y_s float32 [T, d]; n = 1 or 2; the sublayers are added up first, in order)
-__global__ void gated_add_kernel(float* __restrict__ x, const float* __restrict__ y0, const float* __restrict__ y1,
-                                 const float* __restrict__ zg, int ldg, long long n, int d) {
+__global__ void gated_add_kernel(float* x, const float* y0, const float* y1,
+                                 const float* zg, int ldg, long long n, int d) {
   pdl_launch_dependents();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -476,7 +482,7 @@ __device__ __forceinline__ float gelu_tanh_f(float z) {
 }
 template <typename TW>
 __global__ void __launch_bounds__(256)
-token_side_kernel(float* __restrict__ x, const int* __restrict__ tokens, const TW* __restrict__ table, int ldt, int off,
+token_side_kernel(float* x, const int* tokens, const TW* __restrict__ table, int ldt, int off,
                   int vocab, const TW* __restrict__ Wg, const TW* __restrict__ Wp, const float* __restrict__ w, int d, int m,
                   float eps, int* __restrict__ status) {
   extern __shared__ float sh[];            // [d] the row, then its y; [m] g
@@ -548,8 +554,8 @@ __device__ __forceinline__ void ts_mma16816(float* d, const unsigned* a, unsigne
 
 template <int NT, int W>
 __global__ void __launch_bounds__(32 * W)
-token_side_mma_kernel(float* __restrict__ x, const float* __restrict__ y0, const float* __restrict__ y1,
-                      const float* __restrict__ zg, int ldz, const int* __restrict__ tokens, const bf16* __restrict__ table,
+token_side_mma_kernel(float* x, const float* y0, const float* y1,
+                      const float* zg, int ldz, const int* tokens, const bf16* __restrict__ table,
                       int ldt, int off, int vocab, const bf16* __restrict__ Wg, const bf16* __restrict__ Wp,
                       const float* __restrict__ w, int T, int d, int m, float eps, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char ts_smem[];

@@ -1096,7 +1096,7 @@ FELLM_API int fellm_gemm_skinny(const void* x, const float* xf, const float* nor
 // rows (FeLLM: bf16_matmul_rows then argmax_token, plugins/cuda_kernels/src/oxide_kernels.rs:3165,116).
 // The single-shot product's CTAs each leave the best (value, index) of their part of a row as a key; a
 // second, tiny kernel takes the best key of each row.  Ties go to the lower index.
-__global__ void __launch_bounds__(32) argmax_keys_kernel(const unsigned long long* __restrict__ keys, int n_ctas, int* __restrict__ out_tokens) {
+__global__ void __launch_bounds__(32) argmax_keys_kernel(const unsigned long long* keys, int n_ctas, int* __restrict__ out_tokens) {
   FELLM_TRACE_SCOPE(TRACE_ARGMAX_FINAL);
   pdl_launch_dependents();
   pdl_wait(); FELLM_TRACE_WAITED();

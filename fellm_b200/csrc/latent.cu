@@ -26,7 +26,7 @@ __device__ __forceinline__ void rotate_pair(float& u, float& v, int pos, float f
 
 template <typename TO, typename TC>
 __global__ void __launch_bounds__(128)
-latent_prep_kernel(const float* __restrict__ z, int ldz, int q_off, int rq, int c_off, int rk, int r_off, int dr,
+latent_prep_kernel(const float* z, int ldz, int q_off, int rq, int c_off, int rk, int r_off, int dr,
                    const float* __restrict__ wq, const float* __restrict__ wc, float eps,
                    const float* __restrict__ freq, int n_rot, float mag,
                    const int* __restrict__ positions, const int* __restrict__ row_slot,
@@ -85,7 +85,7 @@ __device__ __forceinline__ void lp_put4(bf16* o, float4 v) {
 #define LP_VPT 4
 template <typename TO, typename TC>
 __global__ void __launch_bounds__(LP_THREADS)
-latent_prep_vec_kernel(const float* __restrict__ z, int ldz, int q_off, int rq, int c_off, int rk, int r_off, int dr,
+latent_prep_vec_kernel(const float* z, int ldz, int q_off, int rq, int c_off, int rk, int r_off, int dr,
                        const float* __restrict__ wq, const float* __restrict__ wc, float eps,
                        const float* __restrict__ freq, int n_rot, float mag,
                        const int* __restrict__ positions, const int* __restrict__ row_slot,
@@ -170,7 +170,7 @@ FELLM_API int fellm_latent_prep(const float* z, int ldz, int q_off, int rq, int 
 
 template <typename TA>
 __global__ void __launch_bounds__(128)
-latent_rotate_q_kernel(const TA* __restrict__ q, int ldq, int H, int dn, int dr, TA* __restrict__ q_abs, int rk,
+latent_rotate_q_kernel(const TA* q, int ldq, int H, int dn, int dr, TA* __restrict__ q_abs, int rk,
                        const float* __restrict__ freq, int n_rot, float mag, const int* __restrict__ positions) {
   pdl_launch_dependents();
   pdl_wait();

@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 1) latent_tokens_kernel(LatArgs
 
 // The ranges of a split key walk put together, in the order of the ranges: out = sum_s O_s 2^(m_s - m) / (sum_s l_s
 // 2^(m_s - m) + 2^(sink - m)), m = max_s m_s.  A block per (token, head) row.
-__global__ void __launch_bounds__(256) latent_merge_kernel(const float* __restrict__ scratch, bf16* __restrict__ out,
+__global__ void __launch_bounds__(256) latent_merge_kernel(const float* scratch, bf16* __restrict__ out,
                                                            const float* __restrict__ sinks, int H, int n_splits) {
   __shared__ float sm_m[MAX_SPLITS], sm_w[MAX_SPLITS];
   pdl_launch_dependents();

@@ -14,7 +14,7 @@
 #include "common.cuh"
 
 template <typename TA, typename TC>
-__global__ void qk_rope_write_kernel(const TA* __restrict__ qkv, const float* __restrict__ q_w,
+__global__ void qk_rope_write_kernel(const TA* qkv, const float* __restrict__ q_w,
                                      const float* __restrict__ k_w, float eps,
                                      const float* __restrict__ inv_freq, int pairing,
                                      const int* __restrict__ positions, const int* __restrict__ row_slot,
@@ -104,7 +104,7 @@ __device__ __forceinline__ uint4 rw_pack8(const float* f) {
 }
 
 template <int GL>
-__global__ void qk_rope_write_vec_kernel(const bf16* __restrict__ qkv, const float* __restrict__ q_w,
+__global__ void qk_rope_write_vec_kernel(const bf16* qkv, const float* __restrict__ q_w,
                                          const float* __restrict__ k_w, float eps,
                                          const float* __restrict__ inv_freq, int pairing,
                                          const int* __restrict__ positions, const int* __restrict__ row_slot,
@@ -247,7 +247,7 @@ FELLM_API int fellm_qk_rope_write(const void* qkv, int act_bf16, const float* q_
 #define RN_MAXT 16     // unrotated elements a lane
 template <typename TA>
 __global__ void __launch_bounds__(128)
-qk_rotate_norm_kernel(TA* __restrict__ qkv, int ld, int T, int n_q, int n_k, int k_off, int hd, int rot_dim,
+qk_rotate_norm_kernel(TA* qkv, int ld, int T, int n_q, int n_k, int k_off, int hd, int rot_dim,
                       const float* __restrict__ inv_freq, int pairing, const int* __restrict__ positions, float eps,
                       int unit_norm) {
   pdl_launch_dependents();
@@ -304,7 +304,7 @@ qk_rotate_norm_kernel(TA* __restrict__ qkv, int ld, int T, int n_q, int n_k, int
 // goes round its lanes by shuffles.  All loads of a warp lie in front of its stores.
 template <int LANES>
 __global__ void __launch_bounds__(128)
-qk_rotate_norm_vec_kernel(bf16* __restrict__ qkv, int ld, int T, int n_q, int n_k, int k_off, int rot_dim,
+qk_rotate_norm_vec_kernel(bf16* qkv, int ld, int T, int n_q, int n_k, int k_off, int rot_dim,
                           const float* __restrict__ inv_freq, const int* __restrict__ positions, float eps, int unit_norm) {
   pdl_launch_dependents();
   pdl_wait();
@@ -407,7 +407,7 @@ struct RotateWriteArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-qkv_rotate_write_kernel(T* __restrict__ qkv, const T* __restrict__ v0, T* __restrict__ pool, RotateWriteArgs a) {
+qkv_rotate_write_kernel(T* qkv, const T* v0, T* __restrict__ pool, RotateWriteArgs a) {
   __shared__ float sn_s[RWM_HALF], cs_s[RWM_HALF];
   pdl_launch_dependents();
   const int row = blockIdx.x, pos = a.positions[row], half = a.rot_dim >> 1;
@@ -461,7 +461,7 @@ qkv_rotate_write_kernel(T* __restrict__ qkv, const T* __restrict__ v0, T* __rest
 // bfloat16, pairs (i, i + rot_dim/2), hd and vd multiples of 8, rot_dim of 16, rows on 16-byte boundaries: a thread eight
 // elements (and the eight they are paired with) by 16-byte loads and stores.
 __global__ void __launch_bounds__(128)
-qkv_rotate_write_vec_kernel(bf16* __restrict__ qkv, const bf16* __restrict__ v0, bf16* __restrict__ pool, RotateWriteArgs a) {
+qkv_rotate_write_vec_kernel(bf16* qkv, const bf16* v0, bf16* __restrict__ pool, RotateWriteArgs a) {
   __shared__ float sn_s[RWM_HALF], cs_s[RWM_HALF];
   pdl_launch_dependents();
   const int row = blockIdx.x, pos = a.positions[row], half = a.rot_dim >> 1;
@@ -567,7 +567,7 @@ __device__ __forceinline__ void nrw_block_sums(float& x, float& y, float (*red)[
 
 template <typename T>
 __global__ void __launch_bounds__(NRW_THREADS)
-qkv_norm_rotate_write_kernel(T* __restrict__ qkv, T* __restrict__ pool, NormRotateWriteArgs a) {
+qkv_norm_rotate_write_kernel(T* qkv, T* __restrict__ pool, NormRotateWriteArgs a) {
   __shared__ float sn_s[RWM_HALF], cs_s[RWM_HALF], red[2][NRW_THREADS / 32];
   pdl_launch_dependents();
   const int row = blockIdx.x, pos = a.positions[row], half = a.rot_dim >> 1;
@@ -614,7 +614,7 @@ qkv_norm_rotate_write_kernel(T* __restrict__ qkv, T* __restrict__ pool, NormRota
 // a thread eight elements by 16-byte loads and stores (and, SPLIT, the eight they are paired with).
 template <bool SPLIT>
 __global__ void __launch_bounds__(NRW_THREADS)
-qkv_norm_rotate_write_vec_kernel(bf16* __restrict__ qkv, bf16* __restrict__ pool, NormRotateWriteArgs a) {
+qkv_norm_rotate_write_vec_kernel(bf16* qkv, bf16* __restrict__ pool, NormRotateWriteArgs a) {
   __shared__ float sn_s[RWM_HALF], cs_s[RWM_HALF], red[2][NRW_THREADS / 32];
   pdl_launch_dependents();
   const int row = blockIdx.x, pos = a.positions[row], half = a.rot_dim >> 1;

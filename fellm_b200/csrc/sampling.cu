@@ -204,8 +204,8 @@ __device__ __forceinline__ u64 splitmix64(u64 x) {
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, int V, const RowParams* __restrict__ params,
-              int* __restrict__ counts, const int* __restrict__ bias_tok, const float* __restrict__ bias_val,
+sample_kernel(const float* logits, int V, const RowParams* __restrict__ params,
+              int* counts, const int* __restrict__ bias_tok, const float* __restrict__ bias_val,
               int* __restrict__ out_tokens, float* __restrict__ out_probs, int update_counts) {
   FELLM_TRACE_SCOPE(TRACE_SAMPLE);
   __shared__ Shared s;
@@ -371,7 +371,7 @@ FELLM_API int fellm_count_tokens(int* counts, int V, const int* slots, const int
 // Ties go to the lower id at both stages (sampling.rs:588-604).
 #define ARGMAX_CHUNKS 64
 __global__ void __launch_bounds__(256)
-argmax_partial_kernel(const float* __restrict__ logits, int V, float* __restrict__ pval, int* __restrict__ pidx) {
+argmax_partial_kernel(const float* logits, int V, float* __restrict__ pval, int* __restrict__ pidx) {
   FELLM_TRACE_SCOPE(TRACE_ARGMAX_PARTIAL);
   pdl_launch_dependents();
   pdl_wait(); FELLM_TRACE_WAITED();
@@ -400,7 +400,7 @@ argmax_partial_kernel(const float* __restrict__ logits, int V, float* __restrict
   }
 }
 __global__ void __launch_bounds__(32)
-argmax_final_kernel(const float* __restrict__ pval, const int* __restrict__ pidx, int* __restrict__ out_tokens) {
+argmax_final_kernel(const float* pval, const int* pidx, int* __restrict__ out_tokens) {
   FELLM_TRACE_SCOPE(TRACE_ARGMAX_FINAL);
   pdl_launch_dependents();
   pdl_wait(); FELLM_TRACE_WAITED();

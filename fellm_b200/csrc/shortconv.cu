@@ -121,8 +121,8 @@ __device__ void shortconv_body_vec(const bf16* __restrict__ bcx, const float* __
 }
 
 template <typename TA, int VLC>
-__global__ void shortconv_kernel(const TA* __restrict__ bcx, const float* __restrict__ w,
-                                 const float* __restrict__ conv_bias, float* __restrict__ state,
+__global__ void shortconv_kernel(const TA* bcx, const float* __restrict__ w,
+                                 const float* __restrict__ conv_bias, float* state,
                                  long long slot_stride, const int* __restrict__ item_slot,
                                  const int* __restrict__ item_start, const int* __restrict__ row_item,
                                  TA* __restrict__ y, int T, int n_items, int d, int Lc, int n_body_tiles, int blocked) {

@@ -78,7 +78,7 @@ __device__ __forceinline__ float4 ln4(float4 v, float mean, float rstd, float4 w
 // x (may be null: the plain norm) += LN(y rows); out / cast (may be null) gets the result in TO.
 template <typename TO, int VPL>
 __global__ void __launch_bounds__(LN_WARPS * 32)
-layernorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, const float* __restrict__ b,
+layernorm_vec_kernel(float* x, const float* y, const float* __restrict__ w, const float* __restrict__ b,
                      TO* __restrict__ out, const int* __restrict__ rows, int n_rows, int d, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -123,7 +123,7 @@ static inline bool ln_vec_ok(const void* a, const void* b, const void* c, const 
 
 template <typename TO>
 __global__ void __launch_bounds__(LN_WARPS * 32)
-layernorm_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b, TO* __restrict__ out,
+layernorm_kernel(const float* x, const float* __restrict__ w, const float* __restrict__ b, TO* __restrict__ out,
                  const int* __restrict__ rows, int n_rows, int d, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -157,7 +157,7 @@ FELLM_API int fellm_layernorm(const float* x, const float* w, const float* b, vo
 // the stream itself next.
 template <typename TO>
 __global__ void __launch_bounds__(LN_WARPS * 32)
-add_layernorm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, const float* __restrict__ b,
+add_layernorm_kernel(float* x, const float* y, const float* __restrict__ w, const float* __restrict__ b,
                      TO* __restrict__ cast, int n_rows, int d, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -194,13 +194,25 @@ FELLM_API int fellm_add_layernorm(float* x, const float* y, const float* w, cons
 }
 
 // ---------------------------------------------------------------- float32 -> bfloat16 rows
-__global__ void cast_rows_kernel(const float* __restrict__ x, bf16* __restrict__ out, long long n) {
+// A thread U vectors, all their loads in front of their stores; a number each where an address or the end does not allow that.  One vector a
+// thread up to some two million numbers, four from there (us, number after number in a loop / one / four vectors: 1,024 x 1,024 3.4 / 1.5 / -,
+// 2,048 x 1,536 4.9 / 3.7 / 2.7, 2,048 x 4,096 8.0 / 9.0 / 4.4).
+template <int U>
+__global__ void cast_rows_kernel(const float* x, bf16* __restrict__ out, long long n) {
   pdl_launch_dependents();
   pdl_wait();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = __float2bfloat16_rn(x[i]);
+  const long long i = (long long)blockIdx.x * blockDim.x * (U ? U : 1) + threadIdx.x;
+  if (U == 0) { if (i < n) out[i] = __float2bfloat16_rn(x[i]); return; }
+  float4 v[U ? U : 1];
+#pragma unroll
+  for (int u = 0; u < U; ++u) if (i + u * blockDim.x < n / 4) v[u] = ((const float4*)x)[i + u * blockDim.x];
+#pragma unroll
+  for (int u = 0; u < U; ++u) if (i + u * blockDim.x < n / 4) put4(out + 4 * (i + u * blockDim.x), v[u]);
 }
 
+// vectors a thread (0: a number) and blocks of 256 threads for n numbers
+static inline int ew_vectors(const void* a, const void* b, long long n) { return n % 4 || (((uintptr_t)a | (uintptr_t)b) & 15) ? 0 : n <= 1 << 21 ? 1 : 4; }
+static inline unsigned ew_all(int vectors, long long n) { const long long per = vectors ? 1024ll * vectors : 256; return (unsigned)((n + per - 1) / per); }
 static inline int ew_blocks(long long n) {
   long long b = (n + 255) / 256, cap = (long long)fellm_sm_count() * 16;
   return (int)(b > cap ? cap : (b < 1 ? 1 : b));
@@ -209,13 +221,16 @@ static inline int ew_blocks(long long n) {
 FELLM_API int fellm_cast_rows(const float* x, void* out, long long n, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (!x || !out) return FELLM_ERR_ARG;
-  return launch_k_class(launch_class_for_rows(n / 256, 0), cast_rows_kernel, dim3(ew_blocks(n)), dim3(256), 0, stream, 1, x, (bf16*)out, n);
+  if (n >> 38) return FELLM_ERR_SIZE;              // (more blocks than a grid has)
+  const int v = ew_vectors(x, out, n);
+  return launch_k_class(launch_class_for_rows(n / 256, 0), v == 4 ? cast_rows_kernel<4> : v ? cast_rows_kernel<1> : cast_rows_kernel<0>, dim3(ew_all(v, n)),
+                        dim3(256), 0, stream, 1, x, (bf16*)out, n);
 }
 
 // ---------------------------------------------------------------- act(gate) * up
 // gu [T, ld]: gate in columns [0, F), up in [F, 2F); out [T, F].  act 0: SiLU; 1: GELU, tanh form.
 template <typename T>
-__global__ void act_mul_kernel(const T* __restrict__ gu, int ld, T* __restrict__ out, int rows, int F, int act) {
+__global__ void act_mul_kernel(const T* gu, int ld, T* __restrict__ out, int rows, int F, int act) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t n = (size_t)rows * F;
@@ -227,7 +242,7 @@ __global__ void act_mul_kernel(const T* __restrict__ gu, int ld, T* __restrict__
 }
 
 // bfloat16, F % 8 == 0, rows 16-byte aligned: eight elements a thread.
-__global__ void act_mul_vec_kernel(const bf16* __restrict__ gu, int ld, bf16* __restrict__ out, int rows, int F, int act) {
+__global__ void act_mul_vec_kernel(const bf16* gu, int ld, bf16* __restrict__ out, int rows, int F, int act) {
   pdl_launch_dependents();
   pdl_wait();
   const int per = F >> 3;
@@ -261,7 +276,7 @@ FELLM_API int fellm_act_mul(const void* gu, int ld, void* out, int is_bf16, int 
 // ---------------------------------------------------------------- a *= sigmoid(g)
 // a [T, N] contiguous, g [T, ldg] (the gate's logits); the sigmoid and the product in float32.
 template <typename T>
-__global__ void gate_mul_kernel(T* __restrict__ a, const T* __restrict__ g, int ldg, int rows, int N) {
+__global__ void gate_mul_kernel(T* a, const T* g, int ldg, int rows, int N) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t n = (size_t)rows * N;
@@ -272,7 +287,7 @@ __global__ void gate_mul_kernel(T* __restrict__ a, const T* __restrict__ g, int 
 }
 
 // bfloat16, N % 8 == 0, 16-byte aligned rows: eight elements a thread.
-__global__ void gate_mul_vec_kernel(bf16* __restrict__ a, const bf16* __restrict__ g, int ldg, int rows, int N) {
+__global__ void gate_mul_vec_kernel(bf16* a, const bf16* g, int ldg, int rows, int N) {
   pdl_launch_dependents();
   pdl_wait();
   const int per = N >> 3;
@@ -303,22 +318,30 @@ FELLM_API int fellm_gate_mul(void* a, const void* g, int ldg, int is_bf16, int r
 }
 
 // ---------------------------------------------------------------- max(z, 0)^2
-template <typename TO>
-__global__ void relu2_kernel(const float* __restrict__ z, TO* __restrict__ out, long long n) {
+template <int U, typename TO>
+__global__ void relu2_kernel(const float* z, TO* __restrict__ out, long long n) {       // (as cast_rows_kernel)
   pdl_launch_dependents();
   pdl_wait();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float v = fmaxf(z[i], 0.f);
-    out[i] = from_f<TO>(v * v);
-  }
+  const long long i = (long long)blockIdx.x * blockDim.x * (U ? U : 1) + threadIdx.x;
+  auto f = [](float a) { const float v = fmaxf(a, 0.f); return v * v; };
+  if (U == 0) { if (i < n) out[i] = from_f<TO>(f(z[i])); return; }
+  float4 v[U ? U : 1];
+#pragma unroll
+  for (int u = 0; u < U; ++u) if (i + u * blockDim.x < n / 4) v[u] = ((const float4*)z)[i + u * blockDim.x];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (i + u * blockDim.x < n / 4) put4(out + 4 * (i + u * blockDim.x), make_float4(f(v[u].x), f(v[u].y), f(v[u].z), f(v[u].w)));
 }
 
 FELLM_API int fellm_relu2(const float* z, void* out, int out_is_bf16, long long n, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (!z || !out) return FELLM_ERR_ARG;
-  const int cls = launch_class_for_rows(n / 256, 0);
-  if (out_is_bf16) return launch_k_class(cls, relu2_kernel<bf16>, dim3(ew_blocks(n)), dim3(256), 0, stream, 1, z, (bf16*)out, n);
-  return launch_k_class(cls, relu2_kernel<float>, dim3(ew_blocks(n)), dim3(256), 0, stream, 1, z, (float*)out, n);
+  if (n >> 38) return FELLM_ERR_SIZE;
+  const int cls = launch_class_for_rows(n / 256, 0), v = ew_vectors(z, out, n);
+#define RELU2(TO_) launch_k_class(cls, v == 4 ? relu2_kernel<4, TO_> : v ? relu2_kernel<1, TO_> : relu2_kernel<0, TO_>, dim3(ew_all(v, n)), dim3(256), 0, \
+                                  stream, 1, z, (TO_*)out, n)
+  return out_is_bf16 ? RELU2(bf16) : RELU2(float);
+#undef RELU2
 }
 
 // ---------------------------------------------------------------- x += RMSNorm(y), and the norm that reads x next
@@ -327,7 +350,7 @@ FELLM_API int fellm_relu2(const float* z, void* out, int out_is_bf16, long long 
 // (VPT 16-byte vectors a thread); the number of threads depends on the row's length alone, and so does every sum's order.
 template <int VPT, typename TO>
 __global__ void __launch_bounds__(1024)
-add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, float eps,
+add_rmsnorm_vec_kernel(float* x, const float* y, const float* __restrict__ w, float eps,
                        const float* __restrict__ wn, float eps_n, TO* __restrict__ h, int d) {
   __shared__ float part[2][32];
   pdl_launch_dependents();
@@ -385,7 +408,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const
 // Any width and alignment: the rows are read again instead of kept.
 template <typename TO>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, float eps,
+add_rmsnorm_kernel(float* x, const float* y, const float* __restrict__ w, float eps,
                    const float* __restrict__ wn, float eps_n, TO* __restrict__ h, int d) {
   __shared__ float part[2][8];
   pdl_launch_dependents();

@@ -88,6 +88,26 @@ def test_dependent_kernels_read_the_cache_behind_their_wait(path):
     assert not frozen, f"{path.name}: {frozen}"
 
 
+# What no kernel of a step writes: weights, and the step's index arrays and sampling parameters, which copies from the host bring.
+CONSTANT = {"w", "wq", "wc", "wn", "b", "q_w", "k_w", "coef", "table", "Wg", "Wp", "W", "Wr", "corr", "bias", "conv_bias", "freq", "inv_freq", "sinks",
+            "positions", "row_slot", "block_table", "item_start", "item_slot", "row_item", "rows", "params", "bias_tok", "bias_val"}
+# What kernels only write to.
+WRITTEN = {"out", "status", "cq", "lat", "rope", "pool", "q_out", "h", "cast", "y", "out_tokens", "out_probs", "pval", "pidx", "q_abs"}
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.stem)
+def test_dependent_kernels_read_their_inputs_behind_their_wait(path):
+    """Loads through a __restrict__ parameter need not stay behind the wait: nobody else is taken to write there, and where it is const it is
+    taken never to change.  So of what a dependent declares __restrict__, no kernel in front writes what it reads."""
+    text = source(path)
+    ks = kernels(text)
+    for name in dependents(text, ks):
+        for p in ks[name][0].split(","):
+            m = re.search(r"__restrict__\s+(\w+)", p)
+            assert not m or m.group(1) in (CONSTANT if re.search(r"\bconst\b[^*]*\*", p) else WRITTEN), \
+                f"{path.name}: {name} may read {m.group(1)} ahead of its wait"
+
+
 def test_the_cache_is_read_ahead_of_a_wait_only_where_the_caller_says_so():
     """latent_tokens_kernel reads index arrays and cache in front of its wait, or waits first: as the caller says.  Who says so has launched
     a product per head in front, an ordinary launch on every route, and writes nothing behind it."""

@@ -950,3 +950,31 @@ def test_weight_chain_lasts_as_long_as_the_memory():
     del view
     assert at[0] not in ops._next_weight and {k: v for k, v in ops._next_weight.items() if k not in at} == {k: v for k, v in before.items() if k not in at}
     del b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 3, 4, 255, 1023, 1024, 1028, (1 << 21) - 4, 1 << 21, (1 << 21) + 4, (1 << 21) + 4096 + 7])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_casts_and_squares_anywhere(n, shift):
+    """Numbers one by one, a vector a thread, four vectors a thread: at the edges of each, from any address, and nothing beside them."""
+    from fellm_b200 import ops
+    x = torch.randn(1, n + shift, device=DEV)[:, shift:]
+    for f, want in ((ops.cast_rows, x.bfloat16()), (ops.relu2, (x.clamp(min=0) ** 2).bfloat16())):
+        held = torch.full((1, n + shift + 9), 3.0, dtype=torch.bfloat16, device=DEV)
+        f(x, torch.bfloat16, out=held[:, shift:shift + n])
+        assert torch.equal(held[:, shift:shift + n], want) and (held[:, :shift] == 3).all() and (held[:, shift + n:] == 3).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [2048, 2052, 3072, 4096, 4100, 5000])
+@pytest.mark.parametrize("T", [1, 40, 1777])
+def test_rmsnorm_of_wide_rows(d, T):
+    """Rows kept in registers or read twice: the same bits, whatever the number of rows."""
+    from fellm_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(d + T)
+    x, w = torch.randn(T, d, generator=g, device=DEV), torch.rand(d, generator=g, device=DEV)
+    got = ops.rmsnorm(x, w, 1e-5, torch.float32)
+    many = ops.rmsnorm(x[:1].repeat(1800, 1), w, 1e-5, torch.float32)
+    assert torch.equal(many[-1], got[0])
+    want = x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert float((got - want).abs().max()) < 1e-5 * float(want.abs().max())
