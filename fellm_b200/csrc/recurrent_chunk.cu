@@ -144,7 +144,7 @@ rk_prep_kernel(const RkArgs a) {
   constexpr int E = DK / 32;
   const int item = rk_item_of(a.item_start, a.n_items, blockIdx.x), h = blockIdx.y;
   const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0, c = blockIdx.x - rk_first_chunk(r0, item);
-  if (n < a.min_rows || c * RK_C >= n) return;
+  if (n < a.min_rows || c < 0 || c * RK_C >= n) return;           // (c < 0: rows in front of the first item)
   const int len = min(RK_C, n - c * RK_C), row0 = r0 + c * RK_C;
   const size_t cell = (size_t)blockIdx.x * a.H + h;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -764,7 +764,7 @@ rk_out_kernel(const RkArgs a) {
   float* U = S + RK_OUT_COLS * SP;                 // [32][UP]
   const int item = rk_item_of(a.item_start, a.n_items, blockIdx.x), h = blockIdx.y, j0 = blockIdx.z * RK_OUT_COLS;
   const int r0 = a.item_start[item], n = a.item_start[item + 1] - r0, c = blockIdx.x - rk_first_chunk(r0, item);
-  if (n < a.min_rows || c * RK_C >= n) return;
+  if (n < a.min_rows || c < 0 || c * RK_C >= n) return;           // (c < 0: rows in front of the first item)
   const int cols = min(RK_OUT_COLS, a.dv - j0);    // (a multiple of 16)
   const size_t cell = (size_t)blockIdx.x * a.H + h;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

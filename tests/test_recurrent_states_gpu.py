@@ -115,3 +115,26 @@ def test_the_scan_behind_the_chunks_is_left_out_for_nobody(mode, lens):
     o, st = s.run(32)
     want, want_state = s.oracle()
     assert near(o, want) and near(st, want_state)
+
+
+@pytest.mark.parametrize("mode", ["decay_bonus", "gated_write"])
+def test_rows_in_front_of_the_first_item_are_nobodys(form, mode):
+    from fellm_b200 import ops
+    H, dk, front, n = 2, 64, 70, 75
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    z, decay, bonus = rnd(front + n, 3 * H * dk), torch.rand(front + n, H * dk, generator=g, device="cuda"), rnd(H, dk)
+    lower, bias = torch.rand(H * dk, generator=g, device="cuda"), rnd(H * dk)
+
+    def run(first):
+        m, w, state = z[front - first:].contiguous(), decay[front - first:].contiguous(), torch.zeros(1, H, dk, dk, device="cuda")
+        out = torch.full((first + n, H * dk), 3.0, device="cuda")
+        at = dict(item_start=torch.tensor([first, first + n], dtype=torch.int32, device="cuda"), item_slot=torch.zeros(1, dtype=torch.int32, device="cuda"))
+        if mode == "decay_bonus":
+            ops.decay_bonus_scan(m[:, :H * dk], m[:, H * dk:2 * H * dk], m[:, 2 * H * dk:], w, bonus, state, n_items=1, H=H, dk=dk, out=out,
+                                 max_item_rows=n, chunk_rows=32, **at)
+        else:
+            ops.gated_write_scan(m, H * dk, 2 * H * dk, lower, bias, state, n_items=1, H=H, dk=dk, dv=dk, out=out, max_item_rows=n, chunk_rows=32, **at)
+        return out, state
+    (out, state), (alone, alone_state) = run(front), run(0)
+    assert (out[:front] == 3).all() and torch.equal(out[front:], alone) and torch.equal(state, alone_state)
