@@ -48,3 +48,64 @@ def test_router(E, T, K, dtype):
         h.zero_()
         assert torch.allclose(scores.gather(1, idx.long()), w.double(), rtol=3e-5, atol=0)
         assert torch.allclose(scores.topk(2, 1).values, w.double(), rtol=3e-5, atol=0)      # (a close call may fall the other way)
+
+
+@pytest.mark.parametrize("T", [1, 8, 40])
+def test_a_layer_behind_a_kernel_that_lets_it_start(T):
+    """The kernels of a layer one behind the other, the first behind an RMSNorm that lets its dependents start before it has written a row:
+    new numbers in the same buffers in every pass, the rows poisoned in between, launched one by one and from a graph.  A read ahead of a
+    wait would show against passes in which every kernel is waited for; those are held against float64."""
+    from fellm_b200 import ops
+    E, top, d, ff, passes = 8, 2, 1024, 768, 6
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    wr = (rnd(E + 2, d) * 2 * d ** -0.5).bfloat16()                         # (two identity experts)
+    gate, up = ((rnd(E, ff, d) * d ** -0.5).bfloat16() for _ in range(2))
+    both = torch.stack([ops.interleave_gate_up(gate[e], up[e]) for e in range(E)]).contiguous()
+    down = (rnd(E, d, ff) * ff ** -0.5).bfloat16()
+    ones = torch.ones(d, device="cuda")
+    xs = [rnd(T, d) for _ in range(passes)]
+    x, h, out = torch.empty(T, d, device="cuda"), torch.empty(T, d, dtype=torch.bfloat16, device="cuda"), torch.empty(T, d, device="cuda")
+
+    def layer(wait=lambda: None):
+        h.fill_(float("nan"))
+        ops.rmsnorm(x, ones, 1e-5, torch.bfloat16, out=h)
+        wait()
+        idx, score = ops.moe_router(h, wr, top)
+        wait()
+        plan = ops.moe_plan(idx, E, ops.moe_row_tile(idx.numel(), True, True))
+        wait()
+        a = ops.moe_gemm(h, both, plan, gated=True, gather=True, interleaved=True)
+        wait()
+        y = ops.moe_gemm(a, down, plan, gated=False, gather=False)
+        wait()
+        ops.moe_combine(out, y, plan, score, store=True, identity=h)
+        return idx, score
+
+    want = []
+    for p in range(passes):
+        x.copy_(xs[p])
+        idx, score = layer(torch.cuda.synchronize)
+        torch.cuda.synchronize()
+        want.append(out.clone())
+        hd = h.double()
+        logits = torch.softmax(hd @ wr.double().T, 1)
+        assert torch.allclose(logits.gather(1, idx.long()), score.double(), rtol=3e-5, atol=0)
+        ref = torch.zeros(T, d, dtype=torch.float64, device="cuda")
+        for t in range(T):
+            for e, s in zip(idx[t].tolist(), score[t].double()):
+                act = torch.nn.functional.silu(gate[e].double() @ hd[t]) * (up[e].double() @ hd[t]) if e < E else None
+                ref[t] += s * (down[e].double() @ act if e < E else hd[t])
+        # (the activations are rounded to 8 bits of mantissa, their errors add up at random over ff of them)
+        assert float((out - ref).norm()) < 2.0 ** -8 * float(ref.norm())
+    for p in range(passes):
+        x.copy_(xs[p])
+        layer()
+        assert torch.equal(out, want[p])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer()
+    for p in range(passes):
+        x.copy_(xs[p])
+        graph.replay()
+        assert torch.equal(out, want[p])
