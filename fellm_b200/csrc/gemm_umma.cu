@@ -187,10 +187,9 @@ __device__ __forceinline__ void store_chunk(const UmmaArgs& a, float* v, int m_w
   __syncwarp();                                                // the next chunk writes the same 4 KB
 }
 // The gated form: columns are 8 gate, 8 up, 8 gate, 8 up, so a chunk is 16 features: 32 bytes of a row, a whole sector, which a lane
-// stores itself (transposed like the others: 1,800 x 14,336, K = 1,536 70.8 us for 66.3, the operands' own traffic through
-// shared memory being what binds there).
-// LIMITED: the clamped activation may be asked for (the grouped products); without its code a tile's 16,384 activations take some
-// 0.4 us less (2,048 x 16,384, K = 2,048 98.1 -> 95.0 us, 1,800 x 14,336, K = 1,536 on pairs 70.8 -> 66.3).
+// stores itself: nothing is gained by a way through shared memory, which the operands keep busy.
+// LIMITED: the clamped activation may be asked for (the grouped products).  us with its code everywhere / without it: 1,800 x 14,336,
+// K = 1,536 85.6 / 69.4, on pairs 87 / 75; 2,048 x 16,384, K = 2,048 118 / 108; 600 x 9,216, K = 1,024 24.4 / 21.5.
 template <bool LIMITED>
 __device__ __forceinline__ void store_gated(const UmmaArgs& a, const float* v, int m, int n) {
   const float limit = LIMITED ? a.glu_limit : 0.f, alpha = LIMITED ? a.glu_alpha : 1.f;
@@ -765,8 +764,9 @@ FELLM_API int fellm_gemm_umma(const void* A, const void* W, const float* bias, v
   // estimate: waves x k-blocks x the time a CTA takes for a k-block of its tile + filling and draining.  Measured on B200 over
   // 21 products of 130..2,048 rows: 0.28 us for 128 x 128 (32 KB written to and 32 KB read from shared memory a k-block: 512
   // cycles at 128 bytes, twice the MMA's own), 0.40 us for 128 x 256, 0.345 us and 0.29 us for a pair's CTA on 256 x 256 and
-  // 256 x 128; 4.5 us of filling and draining, 5.2 us for a pair's; within 5% one CTA a tile stays.  (us; 128 x 256 / pair 256 x 256: 2,048 x 2,048 K 2,048 20.2 /
-  // 19.4, 1,537 x 3,072 K 1,024 19.1 / 17.6, 2,048 x 2,112 K 2,048 18.2 / 17.2; 2,048 x 1,280 K 1,024 9.5 / 10.3, 1,800 x 14,336 K 1,536 67 / 85.)
+  // 256 x 128; 4.5 us of filling and draining, 5.2 us for a pair's; within 5% one CTA a tile stays.  (us with W from memory, one CTA a tile / pairs: out = of 2,048 x 2,048 K 2,048
+  // 15.8 / 15.9, K 4,608 30.4 / 28.6, 600 x 4,096 K 2,048 16.8 / 16.1, 1,537 x 3,072 K 1,024 15.6 / 15.0, out += of it 19.2 / 18.6; with W in the
+  // L2 one CTA a tile is 1 us ahead at K 2,048.  Gated, 1,800 x 14,336 K 1,536 69 / 75.)
   // FELLM_B200_UMMA_PAIR=0: never pairs; =128 / =256: always that pair tile; FELLM_B200_UMMA_WIDE=0: no 128 x 256.
   const int m_tiles = ceil_div(M, UM_BM), m_pairs = ceil_div(M, 2 * UM_BM), kb = ceil_div(K, UM_BK);
   const int n_sm = fellm_sm_count(), pairs_dev = n_sm / 2;

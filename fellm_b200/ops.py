@@ -1529,7 +1529,7 @@ def latent_attention(q_abs, H, rk, dr, pool, block_table, positions, row_slot, i
         span = min(int(window), longest) if window else longest
         tiles = span // kt + 2
         ctas = n_items * (-(-max_item_rows * H // 16))
-        n_splits = max(1, min(tiles // 2, 148 // max(ctas, 1), LATENT_MAX_SPLITS))
+        n_splits = max(1, min(tiles // 2, sm_count(q_abs.device) // max(ctas, 1), LATENT_MAX_SPLITS))
         if 1 < n_splits <= LATENT_CLUSTER_TO:
             # as one cluster where the device holds those of all tokens at once (a second round costs more than the merge)
             fits = _fn("latent_attention_mma", "fellm_latent_token_clusters", [_c_int], defines={"LAT_RK": rk, "LAT_DR": dr})
